@@ -221,11 +221,6 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
   ctx->bh_attr.release();
   ctx->bh_attr32.release();
   ctx->pinned.release();
-  for (int k = 0; k < kGemmSlabs; k++) {
-    if (ctx->gemm_streams[k]) cudaStreamDestroy(ctx->gemm_streams[k]);
-    if (ctx->gemm_join[k]) cudaEventDestroy(ctx->gemm_join[k]);
-  }
-  if (ctx->gemm_fork) cudaEventDestroy(ctx->gemm_fork);
   if (ctx->upload_stream) cudaStreamDestroy(ctx->upload_stream);
   if (ctx->q_ready) cudaEventDestroy(ctx->q_ready);
   if (ctx->upload_fork) cudaEventDestroy(ctx->upload_fork);

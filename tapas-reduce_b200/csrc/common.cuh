@@ -18,7 +18,6 @@ constexpr int kMaxDepth = 19;   // Morton<3, uint64_t>::MaxDepth(), sfc_morton.h
 constexpr int kDepthBits = 5;   // Morton<3, uint64_t>::DepthBits(), sfc_morton.h:154-163
 constexpr int kMinP = 2;
 constexpr int kMaxP = 16;
-constexpr int kGemmSlabs = 4;   // concurrent streams of the FP64 class GEMMs
 
 // ---------------------------------------------------------------------------
 // Error handling: every failure becomes a status code plus a message.
@@ -110,8 +109,12 @@ struct TcState {
   DBuf<int4> items, items_alt;
   DBuf<int2> cls_range;    // per selected class: first sorted pair, pair count
   DBuf<float> ops, Mt, Lt;  // per selected class its FP32 operator rows; FP32 rows of M, L
-  DBuf<double> ops64, Mt64, Lt64;  // FP64 class GEMM (plain form)
-  DBuf<uint8_t> use64;     // FP64 class GEMM: list entries left to the pair kernel
+  // FP64 M2L (plain form): operators, normalised multipoles, one product row per
+  // list entry; its tiles, and their counts and offsets per (list range, class)
+  DBuf<double> ops64, Mt64, rows64;
+  DBuf<int4> items64;
+  DBuf<int32_t> cnt64, off64;
+  DBuf<int2> part64;
   DBuf<int32_t> oflag, opos;  // sharded: owned sorted pairs and their compacted positions
   DBuf<uint8_t> sel, sel2;    // sharded: class selection per sorted / compacted pair
   // tensor-core M2M of the mixed form
@@ -132,7 +135,8 @@ struct TcState {
     pairs64.release(); flag.release(); scan.release(); seg_start.release(); tcflag.release();
     tcid.release(); ntiles.release(); tile_off.release(); items.release(); cls_range.release();
     ops.release(); Mt.release(); Lt.release(); ops64.release();
-    Mt64.release(); Lt64.release(); use64.release(); oflag.release(); opos.release();
+    Mt64.release(); rows64.release(); items64.release(); cnt64.release(); off64.release();
+    part64.release(); oflag.release(); opos.release();
     sel.release(); sel2.release(); ops_tr.release(); tree_list.release();
     iota.release(); tree_items.release(); err.release();
     tr_P = 0;
@@ -217,6 +221,7 @@ struct tapas_b200_ctx {
   int64_t trav_pairs = 0;  // (target, source) pairs the traversal classified
   int list_shift = 1;                   // packed list key = target << shift | source
   bool reference_lists = false;         // keep pairs with empty cells, as the reference visits them
+  bool lists_have_empty = false;        // the current lists were built with reference_lists
   tb::DBuf<int32_t> m2l_off, p2p_off;   // CSR by target cell, ncells+1
   tb::DBuf<int32_t> m2l_tlist, p2p_tlist; // targets having list entries
   int64_t n_m2l_targets = 0, n_p2p_targets = 0;
@@ -257,10 +262,6 @@ struct tapas_b200_ctx {
   uint64_t bh_napprox = 0, bh_ndirect = 0;
 
   tb::HBuf pinned;
-  // FP64 class GEMMs: helper streams (and their fork / join events), made on first use
-  cudaStream_t gemm_streams[tb::kGemmSlabs] = {};
-  cudaEvent_t gemm_join[tb::kGemmSlabs] = {};
-  cudaEvent_t gemm_fork = nullptr;
   // upload of the charges on a side stream while the keys are built and sorted
   cudaStream_t upload_stream = nullptr;
   cudaEvent_t q_ready = nullptr, upload_fork = nullptr;

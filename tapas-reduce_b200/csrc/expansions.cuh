@@ -138,11 +138,45 @@ __device__ __forceinline__ void local_column(int m, double rho, double x, double
   }
 }
 
+template <int P>
+struct Sizes {
+  static constexpr int NT = P * (P + 1) / 2;
+  static constexpr int NY = P * P;
+  static constexpr int R = (NT + 31) / 32;  // coefficients per lane
+};
+
 // (j, k) of coefficient t = j(j+1)/2 + k.
 __device__ __forceinline__ void jk_of(int t, int &j, int &k) {
   j = 0;
   while ((j + 1) * (j + 2) / 2 <= t) j++;
   k = t - j * (j + 1) / 2;
+}
+
+// One source's translation added to lane coefficients (jj[r], kk[r]): the
+// source's M in Mj, the local harmonics of the offset in Y.
+template <int P>
+__device__ __forceinline__ void m2l_accumulate(cd (&acc)[Sizes<P>::R], const int (&jj)[Sizes<P>::R],
+                                               const int (&kk)[Sizes<P>::R], int lane,
+                                               const cd *Mj, const cd *Y) {
+  using S = Sizes<P>;
+#pragma unroll
+  for (int r = 0; r < S::R; r++) {
+    if (lane + 32 * r >= S::NT) continue;
+    const int j = jj[r], k = kk[r];
+    const double Cnm = oddeven(j);
+    for (int n = 0; n < P - j; n++) {
+      const int base = (j + n) * (j + n) + j + n - k;
+      for (int m = -n; m < 0; m++) {
+        const int nms = n * (n + 1) / 2 - m;
+        cmac(acc[r], scal(Cnm, conjd(Mj[nms])), Y[base + m]);
+      }
+      for (int m = 0; m <= n; m++) {
+        const int nms = n * (n + 1) / 2 + m;
+        const double Cnm2 = Cnm * oddeven((k - m) * (k < m) + m);
+        cmac(acc[r], scal(Cnm2, Mj[nms]), Y[base + m]);
+      }
+    }
+  }
 }
 
 }  // namespace tb

@@ -458,6 +458,7 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_sources
     return TAPAS_B200_ERR_ARG;
   }
   ctx->mutual = mutual;
+  ctx->lists_have_empty = ctx->reference_lists;
   cudaStream_t s = ctx->stream;
   ctx->theta = theta;
   ctx->have_lists = false;

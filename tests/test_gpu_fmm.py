@@ -516,3 +516,46 @@ def test_fp32_p2m_per_cell(P, dist, tb, ctx):
     rel = np.linalg.norm(Mmx[ok] - M64[ok], axis=1) / scale[ok]
     assert rel.max() < 1e-6, (rel.max(), np.median(rel))
     assert ctx.tree_info()["max_depth"] >= 6
+
+
+@pytest.mark.parametrize("P", [4, 5, 7, 9, 11, 13, 15, 16])
+def test_fp64_m2l_products_every_order(P, tb, ctx, oracle_mod):
+    """The FP64 M2L's class products (32-pair, 32-output, 16-source blocks:
+    every order ends differently) and its rare classes' pairs against the
+    oracle's L, with the reference's lists (pairs of empty cells have no product
+    row) and without them.  Same bar as the other FP64 expansions."""
+    x, y, z, q = tb.datasets.make("two_gaussians", 1500, 19)
+    o = oracle_mod.Oracle(x, y, z, q, P=P, ncrit=8, theta=0.45)
+    _, oL = o.expansions()
+    oc = o.cells()
+    oo = _cells_by_key(oc)
+    ne = oc["nb"][oo] > 0
+    ctx.partition(x, y, z, q, ncrit=8)
+    ctx.upward(P, tb.FP64)
+    Ls = []
+    for keep in (True, False):
+        ctx.set_reference_lists(keep)
+        ctx.build_lists(0.45)
+        ctx.set_reference_lists(False)
+        ctx.m2l(tb.FP64)
+        ctx.p2p(tb.FP64)
+        ctx.downward(tb.FP64)
+        Ls.append(ctx.expansions()[1])
+    go = _cells_by_key(ctx.cells())
+    assert _rel(Ls[0][go][ne], oL[oo][ne]) < FP64_RTOL
+    assert _rel(Ls[1][go][ne], oL[oo][ne]) < FP64_RTOL
+
+
+def test_fp64_m2l_rows_in_ranges(tb, ctx, oracle_mod):
+    """A list whose product rows exceed the buffer (512 MiB: 247k pairs at P = 16)
+    is evaluated in ranges that cut targets; a pair left out or added twice
+    would show at the 1e-3 level, the truncation error of P = 16, theta = 0.3
+    on this workload is below 1e-5."""
+    x, y, z, q = tb.datasets.make("uniform_cube", 60000, 12)
+    a = ctx.evaluate(x, y, z, q, P=16, ncrit=16, theta=0.3, precision=tb.FP64)
+    assert ctx.list_info()["n_m2l"] > 2 * 987000
+    tg = tb.datasets.sample_targets(len(x), 300)
+    ep, ea = oracle_mod.rel_l2(a[tg], ctx.direct(tg))
+    assert ep < 1e-5 and ea < 1e-5
+    b = ctx.evaluate(x, y, z, q, P=16, ncrit=16, theta=0.3, precision=tb.FP64)
+    assert np.array_equal(a, b)
