@@ -4,6 +4,7 @@
 #include <new>
 
 #include "common.cuh"
+#include "direct.cuh"
 #include "kernels.cuh"
 #include "m2l_tc.cuh"
 #include "traverse.cuh"
@@ -38,46 +39,6 @@ __global__ void widen_idx(const uint32_t *__restrict__ idx, int64_t n, int64_t *
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     out[i] = idx[i];
-}
-
-// FP64 direct sum, field form, one block per target (original indices).
-__global__ void __launch_bounds__(256) direct_kernel(const double *__restrict__ x,
-                                                     const double *__restrict__ y,
-                                                     const double *__restrict__ z,
-                                                     const double *__restrict__ q, int64_t n,
-                                                     const int64_t *__restrict__ tg,
-                                                     double *__restrict__ out) {
-  const int64_t i = tg[blockIdx.x];
-  const double xi = x[i], yi = y[i], zi = z[i];
-  double p = 0, ax = 0, ay = 0, az = 0;
-  for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
-    const double dx = xi - x[j], dy = yi - y[j], dz = zi - z[j];
-    const double R2 = dx * dx + dy * dy + dz * dz;
-    if (R2 != 0) {
-      const double invR = 1.0 / sqrt(R2);
-      const double qr = q[j] * invR;
-      const double s3 = qr * invR * invR;
-      p += qr;
-      ax -= dx * s3;
-      ay -= dy * s3;
-      az -= dz * s3;
-    }
-  }
-  __shared__ double red[4][8];
-  for (int o = 16; o > 0; o >>= 1) {
-    p += __shfl_down_sync(0xffffffffu, p, o);
-    ax += __shfl_down_sync(0xffffffffu, ax, o);
-    ay += __shfl_down_sync(0xffffffffu, ay, o);
-    az += __shfl_down_sync(0xffffffffu, az, o);
-  }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) { red[0][w] = p; red[1][w] = ax; red[2][w] = ay; red[3][w] = az; }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    double s = 0;
-    for (int k = 0; k < 8; k++) s += red[threadIdx.x][k];
-    out[4 * blockIdx.x + threadIdx.x] = s;
-  }
 }
 
 // The non-empty leaves whose ownership mask has bit 1 (their bodies are
@@ -220,6 +181,9 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
   mlp_release(ctx);
   ctx->bh_attr.release();
   ctx->bh_attr32.release();
+  ctx->direct_tg.release();
+  ctx->direct_part.release();
+  ctx->direct_out.release();
   ctx->pinned.release();
   if (ctx->upload_stream) cudaStreamDestroy(ctx->upload_stream);
   if (ctx->q_ready) cudaEventDestroy(ctx->q_ready);
@@ -807,47 +771,39 @@ int tapas_b200_direct(tapas_b200_ctx *ctx, const int64_t *targets, int64_t k, do
     set_error(ctx, "direct: bad target list");
     return TAPAS_B200_ERR_ARG;
   }
-  cudaStream_t s = ctx->stream;
-  int64_t *dt = nullptr;
-  double *dout = nullptr;
-  TB_CUDA(ctx, cudaMallocAsync(&dt, sizeof(int64_t) * k, s));
-  cudaError_t e = cudaMallocAsync(&dout, sizeof(double) * 4 * k, s);
-  if (e != cudaSuccess) {
-    cudaFreeAsync(dt, s);
-    TB_CUDA(ctx, e);
-  }
-  int rc = TAPAS_B200_OK;
-  const cudaMemcpyKind in_kind =
-      mem == TAPAS_B200_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  const cudaMemcpyKind out_kind =
-      mem == TAPAS_B200_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-  std::vector<int64_t> host_check;
   if (mem == TAPAS_B200_HOST) {
     for (int64_t i = 0; i < k; i++)
       if (targets[i] < 0 || targets[i] >= ctx->n) {
         set_error(ctx, "direct: target index %lld out of range", (long long)targets[i]);
-        rc = TAPAS_B200_ERR_ARG;
-        break;
+        return TAPAS_B200_ERR_ARG;
       }
   }
-  if (rc == TAPAS_B200_OK) {
-    e = cudaMemcpyAsync(dt, targets, sizeof(int64_t) * k, in_kind, s);
-    if (e == cudaSuccess) {
-      direct_kernel<<<(unsigned)k, 256, 0, s>>>(ctx->x.p, ctx->y.p, ctx->z.p, ctx->q.p, ctx->n,
-                                                dt, dout);
-      count_launch(ctx);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out4, dout, sizeof(double) * 4 * k, out_kind, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-      set_error(ctx, "direct: %s", cudaGetErrorString(e));
-      rc = TAPAS_B200_ERR_CUDA;
-    }
+  cudaStream_t s = ctx->stream;
+  const int64_t *dt = targets;
+  double *dout = out4;
+  if (mem == TAPAS_B200_HOST) {
+    TB_CUDA(ctx, ctx->direct_tg.ensure(k, s));
+    TB_CUDA(ctx, ctx->direct_out.ensure(4 * k, s));
+    TB_CUDA(ctx, cudaMemcpyAsync(ctx->direct_tg.p, targets, sizeof(int64_t) * k,
+                                 cudaMemcpyHostToDevice, s));
+    dt = ctx->direct_tg.p;
+    dout = ctx->direct_out.p;
   }
-  cudaFreeAsync(dt, s);
-  cudaFreeAsync(dout, s);
-  return rc;
+  // about eight waves of blocks, at least 16 sources per thread
+  const int64_t nb = (k + kDirectTargets - 1) / kDirectTargets;
+  const int64_t waves = ((int64_t)ctx->num_sms * 24 + nb - 1) / nb;
+  const int nsplit = (int)std::max<int64_t>(
+      1, std::min({waves, (int64_t)64, ctx->n / (16 * kDirectThreads)}));
+  TB_CUDA(ctx, ctx->direct_part.ensure((size_t)4 * k * nsplit, s));
+  direct_tiles<<<dim3((unsigned)nb, nsplit), kDirectThreads, 0, s>>>(
+      ctx->x.p, ctx->y.p, ctx->z.p, ctx->q.p, ctx->n, dt, k, nsplit, ctx->direct_part.p);
+  TB_LAUNCH_CHECK(ctx);
+  direct_finish<<<grid_for(4 * k, 256), 256, 0, s>>>(ctx->direct_part.p, k, nsplit, dout);
+  TB_LAUNCH_CHECK(ctx);
+  if (mem == TAPAS_B200_HOST)
+    TB_CUDA(ctx, cudaMemcpyAsync(out4, dout, sizeof(double) * 4 * k, cudaMemcpyDeviceToHost, s));
+  TB_CUDA(ctx, cudaStreamSynchronize(s));
+  return TAPAS_B200_OK;
 }
 
 }  // extern "C"

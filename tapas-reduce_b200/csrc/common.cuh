@@ -261,6 +261,10 @@ struct tapas_b200_ctx {
   bool have_bh_attr = false;
   uint64_t bh_napprox = 0, bh_ndirect = 0;
 
+  // tapas_b200_direct: its targets, partial sums and results
+  tb::DBuf<int64_t> direct_tg;
+  tb::DBuf<double> direct_part, direct_out;
+
   tb::HBuf pinned;
   // upload of the charges on a side stream while the keys are built and sorted
   cudaStream_t upload_stream = nullptr;
@@ -369,6 +373,39 @@ __host__ __device__ inline uint64_t spread3(uint32_t v) {
 __host__ __device__ inline uint64_t finest_key(int ax, int ay, int az) {
   uint64_t k = (spread3((uint32_t)az) << 2) | (spread3((uint32_t)ay) << 1) | spread3((uint32_t)ax);
   return (k << kDepthBits) | (uint64_t)kMaxDepth;
+}
+
+// q / r and 1 / r of kN separations at once, r2 their squares, q their charges;
+// both 0 for r2 = 0 (a body with itself).  The hardware's approximation y of
+// 1 / sqrt(r2) is refined once by the binomial series of (1 - e)^(-1/2),
+// e = 1 - r2 y^2, to third order (1 + e/2 + 3/8 e^2): e is below ~2^-20, so the
+// truncation is below 2^-60 and the result within about an ulp, for 5 FP64
+// operations (measured: rsqrt(r2) takes 10 slots of the FP64 pipe).  Zero,
+// subnormal, infinite and NaN r2, which the approximation flushes or the
+// refinement would turn into NaN, take rsqrt; one branch for all kN, since a
+// branch each would keep their chains from overlapping (4000 targets x 1M
+// bodies: 7.6 ms with a branch per pair).
+template <int kN>
+__device__ __forceinline__ void charge_over_distance(const double (&r2)[kN], const double (&q)[kN],
+                                                     double (&qr)[kN], double (&inv)[kN]) {
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < kN; i++) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2[i]));
+    const double e = fma(-(r2[i] * y), y, 1.0);
+    inv[i] = fma(y, e * fma(e, 0.375, 0.5), y);
+    qr[i] = q[i] * inv[i];
+    odd |= (unsigned)__double2hiint(r2[i]) - 0x00100000u >= 0x7fe00000u;
+  }
+  if (odd) {
+#pragma unroll
+    for (int i = 0; i < kN; i++) {
+      if ((unsigned)__double2hiint(r2[i]) - 0x00100000u < 0x7fe00000u) continue;
+      inv[i] = r2[i] == 0.0 ? 0.0 : rsqrt(r2[i]);
+      qr[i] = r2[i] == 0.0 ? 0.0 : q[i] * inv[i];
+    }
+  }
 }
 
 // The reference's (int) conversion of a double on x86-64 (cvttsd2si):

@@ -25,13 +25,13 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "direct.cuh"
 
 namespace tb {
 namespace {
 
 constexpr int kMaxTargets = 4096;
 constexpr int kSplit = 16;       // blocks per target, each over 1/kSplit of the sources
-constexpr int kNoallocThreads = 256;
 constexpr int kMaxDevices = 64;
 
 // The scratch: per (target, split) the 4 partial sums.
@@ -39,61 +39,6 @@ static __device__ __align__(256) double g_direct_scratch[(size_t)kMaxTargets * k
 
 double *g_scratch_addr[kMaxDevices] = {nullptr};
 std::mutex g_scratch_mutex;
-
-__global__ void __launch_bounds__(kNoallocThreads) direct_partial(
-    const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
-    const double *__restrict__ q, int64_t n, const int64_t *__restrict__ targets,
-    double *__restrict__ scratch) {
-  const int t = blockIdx.x, split = blockIdx.y;
-  const int64_t i = targets[t];
-  const bool ok = i >= 0 && i < n;
-  double p = 0, ax = 0, ay = 0, az = 0;
-  if (ok) {
-    const double xi = x[i], yi = y[i], zi = z[i];
-    for (int64_t j = (int64_t)split * blockDim.x + threadIdx.x; j < n;
-         j += (int64_t)kSplit * blockDim.x) {
-      const double dx = xi - x[j], dy = yi - y[j], dz = zi - z[j];
-      const double R2 = dx * dx + dy * dy + dz * dz;
-      if (R2 != 0) {
-        const double invR = 1.0 / sqrt(R2);
-        const double qr = q[j] * invR;
-        const double s3 = qr * invR * invR;
-        p += qr;
-        ax -= dx * s3;
-        ay -= dy * s3;
-        az -= dz * s3;
-      }
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    p += __shfl_down_sync(0xffffffffu, p, o);
-    ax += __shfl_down_sync(0xffffffffu, ax, o);
-    ay += __shfl_down_sync(0xffffffffu, ay, o);
-    az += __shfl_down_sync(0xffffffffu, az, o);
-  }
-  __shared__ double red[4][kNoallocThreads / 32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) { red[0][w] = p; red[1][w] = ax; red[2][w] = ay; red[3][w] = az; }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    double s = 0;
-    for (int k = 0; k < kNoallocThreads / 32; k++) s += red[threadIdx.x][k];
-    // A target index outside [0, n) yields NaN for that target.
-    scratch[((size_t)t * kSplit + split) * 4 + threadIdx.x] = ok ? s : __longlong_as_double(-1);
-  }
-}
-
-__global__ void direct_finish(const double *__restrict__ scratch, int64_t k,
-                              double *__restrict__ out4) {
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < k * 4;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t t = idx / 4;
-    const int c = (int)(idx % 4);
-    double s = 0;
-    for (int sp = 0; sp < kSplit; sp++) s += scratch[((size_t)t * kSplit + sp) * 4 + c];
-    out4[idx] = s;
-  }
-}
 
 }  // namespace
 }  // namespace tb
@@ -146,11 +91,11 @@ extern "C" int tapas_b200_direct_noalloc(const double *x, const double *y, const
               cudaGetErrorString(e));
     return TAPAS_B200_ERR_CUDA;
   }
-  direct_partial<<<dim3((unsigned)k, kSplit), kNoallocThreads, 0, s>>>(x, y, z, q, n, targets,
-                                                                       scratch);
+  direct_tiles<<<dim3((unsigned)((k + kDirectTargets - 1) / kDirectTargets), kSplit),
+                 kDirectThreads, 0, s>>>(x, y, z, q, n, targets, k, kSplit, scratch);
   e = cudaGetLastError();
   if (e == cudaSuccess) {
-    direct_finish<<<(unsigned)((k * 4 + 255) / 256), 256, 0, s>>>(scratch, k, out4);
+    direct_finish<<<(unsigned)((k * 4 + 255) / 256), 256, 0, s>>>(scratch, k, kSplit, out4);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {

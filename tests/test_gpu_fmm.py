@@ -559,3 +559,28 @@ def test_fp64_m2l_rows_in_ranges(tb, ctx, oracle_mod):
     assert ep < 1e-5 and ea < 1e-5
     b = ctx.evaluate(x, y, z, q, P=16, ncrit=16, theta=0.3, precision=tb.FP64)
     assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (7, 3), (127, 8), (129, 9), (5000, 17), (40001, 1)])
+def test_direct_tile_edges(n, k, tb, ctx, oracle_mod):
+    """Part-filled target tiles, few sources, coincident bodies; the no-alloc
+    form over the same tiles.  Bar as the other direct-sum test."""
+    x, y, z, q = [a.copy() for a in tb.datasets.make("uniform_cube", n, 5)]
+    if n > 6:
+        x[1], y[1], z[1] = x[0], y[0], z[0]  # coincident: their pair adds nothing
+        x[3] = x[2] + 1e-9
+        y[3], z[3] = y[2], z[2]
+    ctx.partition(x, y, z, q, ncrit=64)
+    tg = (np.arange(k) * 7919) % n
+    d = ctx.direct(tg)
+    ref = oracle_mod.direct(x, y, z, q, tg, field=True)
+    assert _rel(d, ref) < 1e-12
+    import torch
+    dev = [torch.from_numpy(a).cuda() for a in (x, y, z, q)]
+    t = torch.from_numpy(tg.astype(np.int64)).cuda()
+    out = torch.zeros((k, 4), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert tb.lib().tapas_b200_direct_noalloc(*[a.data_ptr() for a in dev], n, t.data_ptr(), k,
+                                              out.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert _rel(out.cpu().numpy(), ref) < 1e-12
