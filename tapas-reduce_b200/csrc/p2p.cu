@@ -8,15 +8,14 @@
 //  - warps take target leaves from a global queue ordered by decreasing work
 //    (nt * sum of source bodies), so long interaction lists start first;
 //  - each lane keeps kR targets in registers (kR a template parameter, so no
-//    issue slot is spent on unused target slots); FP64: kR = ceil(nt/32);
-//    mixed: the targets take L = ceil(nt/kR) lanes and the warp holds
-//    G = 32/L copies of them that split the sources, with kR chosen so that
-//    kR/G (time per source) is least;
+//    issue slot is spent on unused target slots): the targets take
+//    L = ceil(nt/kR) lanes and the warp holds G = 32/L copies of them that split
+//    the sources, with kR chosen so that kR/G (time per source) is least;
 //  - source bodies are staged in the warp's shared-memory slice and read as
 //    broadcasts; each target's sum is written once, without atomics.
 //
-// FP64 form: the reference's arithmetic (pot += qi qj / r, acc -= qi qj dX/r^3,
-// r == 0 skipped), 1/r from rsqrt (1 ulp).
+// FP64 form: the reference's sums (pot += qi qj / r, acc -= qi qj dX/r^3, r == 0
+// skipped; the common factor qi at the end), 1/r by charge_over_distance.
 //
 // Mixed form: FP32 arithmetic with results per unit charge.  Positions are
 // kept as FP32 (hi, lo) offsets from the body's leaf centre; a source is moved
@@ -41,10 +40,10 @@
 namespace tb {
 namespace {
 
-constexpr int kWarps = 8;
+constexpr int kWarps = 4;  // FP64 kernel: 4-warp CTAs, 4 per SM (<= 128 registers)
 constexpr int kThreads = 32 * kWarps;
+constexpr int kFp64Blocks = 4;
 constexpr int kStage = 32;   // source bodies staged per warp at a time (one per lane)
-constexpr int kMaxR = 3;     // FP64: targets per lane, leaves up to 96 bodies per pass
 // mixed kernel: 4-warp CTAs, 4 per SM (<= 128 registers, 16 warps per SM), up to
 // 3 targets per lane (leaves of more than 96 bodies take two passes)
 constexpr int kMixedWarps = 4;
@@ -54,13 +53,16 @@ constexpr int kMixedThreads = 32 * kMixedWarps;
 // ---------------------------------------------------------------------------
 // work items: a target leaf with its source list, or a piece of a long list
 // ---------------------------------------------------------------------------
-// A target leaf whose source list holds more than kSplitSources bodies (a big
-// leaf beside a dense region, e.g. the core of a Plummer sphere) is split into
-// consecutive list ranges of about that many sources, so no single warp
-// carries it alone.  A piece writes its partial sums to its own rows of a
-// scratch array; split_reduce adds a leaf's pieces in order, so the result
-// does not depend on which warp finished first.
-constexpr int64_t kSplitSources = 32768;
+// A target leaf with more than piece_pairs body pairs is split into consecutive
+// list ranges of about that many, so no single warp carries it alone: with one
+// item per leaf the last warps ran on while most of the GPU was idle (1M and
+// 300k sphere, FP64: the SMs were busy 60 and 41 % of the kernel's time).  A
+// piece writes its partial sums to its own rows of a scratch array;
+// split_reduce adds a leaf's pieces in order, so the result does not depend on
+// which warp finished first.  piece_pairs is an eighth of a warp's share of all
+// pairs (the tail is then at most that), but at least kMinPiecePairs, below
+// which a piece's own start and its partial rows cost more than the tail.
+constexpr int64_t kMinPiecePairs = 16384;
 
 struct WorkItem {
   int32_t leaf, e0, e1;  // target leaf (cell index) and its list range [e0, e1)
@@ -71,25 +73,28 @@ struct WorkItem {
 __global__ void leaf_pieces(const int32_t *__restrict__ leaves, int64_t nleaves,
                             const int32_t *__restrict__ off, const uint64_t *__restrict__ list,
                             uint64_t src_mask, const int32_t *__restrict__ cnb,
-                            int32_t *__restrict__ kcnt, int32_t *__restrict__ psz) {
+                            int64_t piece_pairs, int32_t *__restrict__ kcnt,
+                            int32_t *__restrict__ psz) {
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nleaves;
        w += (int64_t)gridDim.x * blockDim.x) {
     const int c = leaves[w];
     int64_t ns = 0;
     for (int e = off[c]; e < off[c + 1]; e++) ns += cnb[(int)(list[e] & src_mask)];
-    const int64_t k = ns > kSplitSources ? (ns + kSplitSources - 1) / kSplitSources : 1;
+    const int64_t entries = off[c + 1] - off[c];
+    const int64_t k = max((int64_t)1, min((ns * cnb[c] + piece_pairs - 1) / piece_pairs, entries));
     kcnt[w] = (int32_t)k;
     psz[w] = k > 1 ? (int32_t)(k * cnb[c]) : 0;
   }
 }
 
-// Items of leaf w at koff[w]..: cut its list greedily where the sources
-// reach kSplitSources (at most k pieces; unused slots become empty pieces with
+// Items of leaf w at koff[w]..: cut its list greedily where the pairs reach
+// piece_pairs (at most k pieces; unused slots become empty pieces with
 // zeroed partials).  Work key = nt * sources of the piece, for the queue.
 __global__ void emit_items(const int32_t *__restrict__ leaves, int64_t nleaves,
                            const int32_t *__restrict__ off, const uint64_t *__restrict__ list,
                            uint64_t src_mask, const int32_t *__restrict__ cnb,
-                           const int32_t *__restrict__ kcnt, const int32_t *__restrict__ koff,
+                           int64_t piece_pairs, const int32_t *__restrict__ kcnt,
+                           const int32_t *__restrict__ koff,
                            const int32_t *__restrict__ poff, WorkItem *__restrict__ items,
                            uint64_t *__restrict__ keys, uint32_t *__restrict__ vals,
                            double *__restrict__ part) {
@@ -102,7 +107,7 @@ __global__ void emit_items(const int32_t *__restrict__ leaves, int64_t nleaves,
     int64_t acc = 0;
     for (int e = e0; e < e1; e++) {
       acc += cnb[(int)(list[e] & src_mask)];
-      if ((k > 1 && acc >= kSplitSources && j < k - 1) || e == e1 - 1) {
+      if ((k > 1 && acc * nt >= piece_pairs && j < k - 1) || e == e1 - 1) {
         uint64_t work = (uint64_t)acc * (uint64_t)nt;
         if (work > 0xFFFFFFFFull) work = 0xFFFFFFFFull;
         items[base + j] = WorkItem{c, ea, e + 1, k > 1 ? poff[w] + j * nt : -1};
@@ -129,16 +134,17 @@ __global__ void emit_items(const int32_t *__restrict__ leaves, int64_t nleaves,
 }
 
 // trg rows of split leaves = sum of their pieces' partial rows, in piece order
+// (eight threads per leaf)
 __global__ void split_reduce(const int32_t *__restrict__ leaves, int64_t nleaves,
                              const int32_t *__restrict__ cbeg, const int32_t *__restrict__ cnb,
                              const int32_t *__restrict__ kcnt, const int32_t *__restrict__ poff,
                              const double *__restrict__ part, double *__restrict__ trg) {
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nleaves;
-       w += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; w < nleaves;
+       w += ((int64_t)gridDim.x * blockDim.x) >> 3) {
     const int k = kcnt[w];
     if (k <= 1) continue;
     const int c = leaves[w], nt = cnb[c], b0 = cbeg[c];
-    for (int t = 0; t < nt; t++) {
+    for (int t = threadIdx.x & 7; t < nt; t += 8) {
       double4 acc = make_double4(0, 0, 0, 0);
       for (int j = 0; j < k; j++) {
         const double4 v =
@@ -163,69 +169,159 @@ __device__ __forceinline__ int next_leaf(int *counter, int lane) {
   return __shfl_sync(0xffffffffu, w, 0);
 }
 
+// Shape of a tile of nt <= 128 targets: kR targets per lane, L = ceil(nt/kR)
+// lanes per group, G = 32/L groups that split the sources.  Time per source
+// ~ kR / G: the least of kR = 4, 3, 1 (ties: the larger kR, fewer shared loads
+// and more independent chains per lane).  kR = 2 would fill as many lanes on
+// average (leaves of 16 to 64 bodies: 89 % with or without it), and every
+// variant less leaves more room in the instruction cache, where stalls were
+// half as frequent again as issue with four variants.
+constexpr int kTileTargets = 128;
+__device__ __forceinline__ void tile_shape(int nt, int &R, int &L, int &G) {
+  R = 4;
+  L = (nt + 3) >> 2;
+  G = 32 / L;
+#pragma unroll
+  for (int r = 3; r >= 1; r -= 2) {
+    const int l = (nt + r - 1) / r;
+    if (l > 32) break;
+    const int g = 32 / l;
+    if (r * G < R * g) {
+      R = r;
+      L = l;
+      G = g;
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // FP64
 // ---------------------------------------------------------------------------
+// Lane (g, l) holds targets l, l + L, ... and takes every G-th staged source;
+// the groups' sums are added in group order at the end, so the result is a
+// fixed-order sum.  The source bodies of the item's list range are one stream:
+// the list is read 32 leaves at a time (lane j: entry j's body range and the
+// running count of bodies), and each chunk of 32 consecutive bodies of the
+// stream is staged by a lane each, which finds its leaf by a binary search over
+// the 32 counts with shuffles, so every chunk but a batch's last is full
+// whatever the leaf sizes; the next chunk's loads are issued before the
+// current one is computed.
+//
+// Bound: the FP64 pipe, 18 of its slots per pair (3 separations, 3 for r^2, 5
+// for the refined 1/r, 3 for q/r and q/r^3, 4 sums), 3.55 pairs per clock and SM.
 template <int kR>
-__device__ __forceinline__ void fp64_tile(int lane, int wi, int tb0, int nt, int e0, int e1,
+__device__ __forceinline__ void fp64_tile(int lane, int tb0, int nt, int L, int G, int e0, int e1,
                                           const uint64_t *__restrict__ list, uint64_t mask,
                                           const int32_t *__restrict__ cbeg,
                                           const int32_t *__restrict__ cnb,
                                           const double *__restrict__ sx,
                                           const double *__restrict__ sy,
                                           const double *__restrict__ sz,
-                                          const double *__restrict__ sq, double4 (*src)[32],
+                                          const double *__restrict__ sq, double4 *src,
                                           double4 *__restrict__ out) {
-  double xi[kR], yi[kR], zi[kR], qi[kR], pot[kR], ax[kR], ay[kR], az[kR];
+  const int g = lane / L, tl = lane - g * L;
+  const bool active = g < G;
+  double xi[kR], yi[kR], zi[kR], pot[kR], ax[kR], ay[kR], az[kR];
 #pragma unroll
   for (int r = 0; r < kR; r++) {
-    const int i = lane + 32 * r;
-    const bool v = i < nt;
+    const int i = tl + L * r;
+    const bool v = active && i < nt;
     xi[r] = v ? sx[tb0 + i] : 0.0;
     yi[r] = v ? sy[tb0 + i] : 0.0;
     zi[r] = v ? sz[tb0 + i] : 0.0;
-    qi[r] = v ? sq[tb0 + i] : 0.0;
     pot[r] = ax[r] = ay[r] = az[r] = 0.0;
   }
-  for (int e = e0; e < e1; e++) {
-    const int s = (int)(list[e] & mask);
-    const int sb0 = cbeg[s], ns = cnb[s];
-    for (int chunk = 0; chunk < ns; chunk += 32) {
-      const int cnt = min(32, ns - chunk);
-      __syncwarp();
-      if (lane < cnt) {
-        const int j = sb0 + chunk + lane;
-        src[wi][lane] = make_double4(sx[j], sy[j], sz[j], sq[j]);
-      }
-      __syncwarp();
-      for (int k = 0; k < cnt; k++) {
-        const double4 b = src[wi][k];
+  for (int eb = e0; eb < e1; eb += 32) {
+    int beg = 0, ns = 0;
+    if (eb + lane < e1) {
+      const int s = (int)(list[eb + lane] & mask);
+      beg = cbeg[s];
+      ns = cnb[s];
+    }
+    int upto = ns;  // bodies of the batch's leaves 0 .. lane
 #pragma unroll
-        for (int r = 0; r < kR; r++) {
-          const double dx = xi[r] - b.x, dy = yi[r] - b.y, dz = zi[r] - b.z;
-          const double R2 = dx * dx + dy * dy + dz * dz;
-          if (R2 != 0) {
-            const double invR = rsqrt(R2);
-            const double qq = qi[r] * b.w * invR;
-            const double s3 = invR * invR * qq;
-            pot[r] += qq;
-            ax[r] -= dx * s3;
-            ay[r] -= dy * s3;
-            az[r] -= dz * s3;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, upto, 31);
+    beg -= upto - ns;  // body i of the stream is body beg + i of its leaf's range
+    double4 b = make_double4(0, 0, 0, 0);
+    auto load = [&](int c0) {
+      const int i = c0 + lane;
+      int leaf = 0;  // the first leaf with upto > i
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, upto, leaf + o - 1);
+        if (v <= i) leaf += o;
+      }
+      const int j = __shfl_sync(0xffffffffu, beg, leaf & 31) + i;
+      if (i < total) b = make_double4(sx[j], sy[j], sz[j], sq[j]);
+    };
+    if (total > 0) load(0);
+    for (int c0 = 0; c0 < total; c0 += 32) {
+      const int cnt = min(32, total - c0);
+      __syncwarp();
+      src[lane] = b;
+      __syncwarp();
+      if (c0 + 32 < total) load(c0 + 32);
+      if (!active) continue;
+      // kU sources at a time: at least three separations in flight per lane
+      constexpr int kU = kR == 1 ? 4 : 1, N = kU * kR;
+      for (int k = g; k < cnt; k += kU * G) {
+        double dx[N], dy[N], dz[N], R2[N], q[N], qr[N], inv[N];
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+          const bool in = kU == 1 || k + u * G < cnt;
+          const double4 s = src[in ? k + u * G : k];
+#pragma unroll
+          for (int r = 0; r < kR; r++) {
+            const int i = u * kR + r;
+            dx[i] = xi[r] - s.x;
+            dy[i] = yi[r] - s.y;
+            dz[i] = zi[r] - s.z;
+            R2[i] = dx[i] * dx[i] + dy[i] * dy[i] + dz[i] * dz[i];
+            if (!in) R2[i] = 0.0;  // adds nothing
+            q[i] = s.w;
           }
+        }
+        charge_over_distance(R2, q, qr, inv);
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+          const int r = i % kR;
+          const double s3 = inv[i] * inv[i] * qr[i];
+          pot[r] += qr[i];
+          ax[r] = fma(-dx[i], s3, ax[r]);
+          ay[r] = fma(-dy[i], s3, ay[r]);
+          az[r] = fma(-dz[i], s3, az[r]);
         }
       }
     }
   }
 #pragma unroll
   for (int r = 0; r < kR; r++) {
-    const int i = lane + 32 * r;
-    if (i < nt) out[i] = make_double4(pot[r], ax[r], ay[r], az[r]);
+    const int i = tl + L * r;
+    double4 v = make_double4(pot[r], ax[r], ay[r], az[r]);
+    if (G > 1) {
+      __syncwarp();
+      src[lane] = v;
+      __syncwarp();
+      if (g == 0) {
+        for (int gg = 1; gg < G; gg++) {
+          const double4 o = src[tl + gg * L];
+          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+        }
+      }
+    }
+    if (active && g == 0 && i < nt) {  // the reference's TRG: times the target's charge
+      const double qi = sq[tb0 + i];
+      out[i] = make_double4(qi * v.x, qi * v.y, qi * v.z, qi * v.w);
+    }
   }
+  __syncwarp();
 }
 
-// 3 CTAs of 8 warps per SM (<= 85 registers)
-__global__ void __launch_bounds__(kThreads, 3) p2p_fp64_kernel(
+__global__ void __launch_bounds__(kThreads, kFp64Blocks) p2p_fp64_kernel(
     const uint32_t *__restrict__ order, int64_t nitems, int *__restrict__ counter,
     const WorkItem *__restrict__ items, const uint64_t *__restrict__ list, uint64_t src_mask,
     const int32_t *__restrict__ cbeg, const int32_t *__restrict__ cnb,
@@ -240,17 +336,17 @@ __global__ void __launch_bounds__(kThreads, 3) p2p_fp64_kernel(
     if (it.pbase >= 0 && it.e0 == it.e1) continue;  // unused piece of a split list
     const int c = it.leaf;
     const int tb0 = cbeg[c], nt_all = cnb[c];
-    const int e0 = it.e0, e1 = it.e1;
     double4 *out = item_out(it, tb0, trg, part);
-    for (int tbase = 0; tbase < nt_all; tbase += 32 * kMaxR) {
-      const int nt = min(nt_all - tbase, 32 * kMaxR);
-      const int R = (nt + 31) / 32;
-#define TB_FP64_TILE(RR)                                                                    \
-  fp64_tile<RR>(lane, wi, tb0 + tbase, nt, e0, e1, list, src_mask, cbeg, cnb, sx, sy, sz, sq, \
-                src, out + tbase)
-      if (R == 1) TB_FP64_TILE(1);
-      else if (R == 2) TB_FP64_TILE(2);
-      else TB_FP64_TILE(3);
+    for (int tbase = 0; tbase < nt_all; tbase += kTileTargets) {
+      const int nt = min(nt_all - tbase, kTileTargets);
+      int R, L, G;
+      tile_shape(nt, R, L, G);
+#define TB_FP64_TILE(RR)                                                                         \
+  fp64_tile<RR>(lane, tb0 + tbase, nt, L, G, it.e0, it.e1, list, src_mask, cbeg, cnb, sx, sy, sz, \
+                sq, src[wi], out + tbase)
+      if (R == 4) TB_FP64_TILE(4);
+      else if (R == 3) TB_FP64_TILE(3);
+      else TB_FP64_TILE(1);
 #undef TB_FP64_TILE
     }
   }
@@ -612,8 +708,10 @@ __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
 
 // Builds the P2P work items of the current lists (ctx->p2p_items) and their
 // queue order (ctx->p2p_order: items by decreasing work).
-int p2p_items(tapas_b200_ctx *ctx) {
+int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
   cudaStream_t s = ctx->stream;
+  const int64_t piece_pairs = std::max<int64_t>(
+      kMinPiecePairs, (int64_t)(ctx->n_p2p_int / ((uint64_t)ctx->num_sms * warps_per_sm * 8)));
   int64_t nl = 0;
   const int32_t *leaves = work_leaves(ctx, nl);  // sharded: owned target leaves
   const uint64_t mask = (1ull << ctx->list_shift) - 1;
@@ -622,8 +720,8 @@ int p2p_items(tapas_b200_ctx *ctx) {
   TB_CUDA(ctx, ctx->p2p_psz.ensure(nl + 1, s));
   TB_CUDA(ctx, ctx->p2p_poff.ensure(nl + 1, s));
   leaf_pieces<<<grid_for(nl, 256), 256, 0, s>>>(leaves, nl, ctx->p2p_off.p, ctx->p2p.p,
-                                                 mask, ctx->cnb.p, ctx->p2p_kcnt.p,
-                                                 ctx->p2p_psz.p);
+                                                 mask, ctx->cnb.p, piece_pairs,
+                                                 ctx->p2p_kcnt.p, ctx->p2p_psz.p);
   TB_LAUNCH_CHECK(ctx);
   TB_TRY(scan_exclusive(ctx, ctx->p2p_kcnt.p, ctx->p2p_koff.p, nl, ctx->p2p_koff.p + nl));
   TB_TRY(scan_exclusive(ctx, ctx->p2p_psz.p, ctx->p2p_poff.p, nl, ctx->p2p_poff.p + nl));
@@ -648,7 +746,7 @@ int p2p_items(tapas_b200_ctx *ctx) {
   TB_CUDA(ctx, ctx->p2p_order_alt.ensure(ni + 1, s));
   TB_CUDA(ctx, ctx->p2p_counter.ensure(4, s));
   emit_items<<<grid_for(nl, 256), 256, 0, s>>>(
-      leaves, nl, ctx->p2p_off.p, ctx->p2p.p, mask, ctx->cnb.p, ctx->p2p_kcnt.p,
+      leaves, nl, ctx->p2p_off.p, ctx->p2p.p, mask, ctx->cnb.p, piece_pairs, ctx->p2p_kcnt.p,
       ctx->p2p_koff.p, ctx->p2p_poff.p, reinterpret_cast<WorkItem *>(ctx->p2p_items.p),
       ctx->p2p_wkey.p, ctx->p2p_order.p, ctx->p2p_part.p);
   TB_LAUNCH_CHECK(ctx);
@@ -672,7 +770,7 @@ int p2p_finish(tapas_b200_ctx *ctx) {
   if (!ctx->p2p_split) return TAPAS_B200_OK;
   int64_t nl = 0;
   const int32_t *leaves = work_leaves(ctx, nl);
-  split_reduce<<<grid_for(nl, 256), 256, 0, ctx->stream>>>(
+  split_reduce<<<grid_for(8 * nl, 256), 256, 0, ctx->stream>>>(
       leaves, nl, ctx->cbeg.p, ctx->cnb.p, ctx->p2p_kcnt.p, ctx->p2p_poff.p,
       ctx->p2p_part.p, ctx->trg.p);
   TB_LAUNCH_CHECK(ctx);
@@ -703,7 +801,7 @@ int p2p_fp64(tapas_b200_ctx *ctx) {
   int64_t nl = 0;
   work_leaves(ctx, nl);
   if (nl == 0) return TAPAS_B200_OK;
-  TB_TRY(p2p_items(ctx));
+  TB_TRY(p2p_items(ctx, kFp64Blocks * kWarps));
   const uint64_t mask = (1ull << ctx->list_shift) - 1;
   p2p_fp64_kernel<<<p2p_grid(ctx, kWarps), kThreads, 0, s>>>(
       ctx->p2p_order.p, ctx->p2p_nitems, ctx->p2p_counter.p,
@@ -727,7 +825,7 @@ int p2p_mixed(tapas_b200_ctx *ctx) {
                                                       ctx->sy.p, ctx->sz.p, ctx->sq.p,
                                                       ctx->rel4.p, ctx->rel_lo.p);
   TB_LAUNCH_CHECK(ctx);
-  TB_TRY(p2p_items(ctx));
+  TB_TRY(p2p_items(ctx, 24));
   const uint64_t mask = (1ull << ctx->list_shift) - 1;
   // up to 3 targets per lane; the Kahan pairs in shared memory keep the kernel
   // at 80 registers, 24 warps per SM

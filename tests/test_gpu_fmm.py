@@ -584,3 +584,24 @@ def test_direct_tile_edges(n, k, tb, ctx, oracle_mod):
                                               out.data_ptr(), None) == 0
     torch.cuda.synchronize()
     assert _rel(out.cpu().numpy(), ref) < 1e-12
+
+
+@pytest.mark.parametrize("n,ncrit", [(40, 1), (900, 2), (1500, 9), (3000, 40), (2500, 150),
+                                     (3000, 300), (290, 300), (12000, 600)])
+def test_near_field_tile_shapes(n, ncrit, tb, ctx, oracle_mod):
+    """Leaves of one body up to several hundred: every tile shape (1, 3 or 4
+    targets per lane, sources split over up to 32 lane groups), leaves of more
+    than one tile (128 targets), target lists long enough to be split into
+    pieces, coincident and nearly coincident bodies.  FP64 against the oracle,
+    mixed against FP64, at their bars."""
+    x, y, z, q = [a.copy() for a in tb.datasets.make("two_gaussians", n, 57)]
+    x[1], y[1], z[1] = x[0], y[0], z[0]
+    x[3] = x[2] + 1e-6
+    y[3], z[3] = y[2], z[2]
+    ref = oracle_mod.Oracle(x, y, z, q, P=6, ncrit=ncrit, theta=0.3).result()
+    r64 = ctx.evaluate(x, y, z, q, P=6, ncrit=ncrit, theta=0.3, precision=tb.FP64)
+    assert _rel(r64[:, 0], ref[:, 0]) < FP64_RTOL
+    assert _rel(r64[:, 1:], ref[:, 1:]) < FP64_RTOL
+    rmx = ctx.evaluate(x, y, z, q, P=6, ncrit=ncrit, theta=0.3, precision=tb.MIXED)
+    ep, ea = oracle_mod.rel_l2(rmx, r64)
+    assert ep < 2e-6 and ea < 2e-6
