@@ -676,9 +676,8 @@ int tapas_b200_p2p(tapas_b200_ctx *ctx, int precision) {
 int tapas_b200_traverse(tapas_b200_ctx *ctx, double theta, int mutual, int precision) {
   TB_TRY(check_ctx(ctx));
   TB_TRY(check_precision(ctx, precision));
-  // the mixed form needs the lists grouped by target, not each target's
-  // sources sorted (its M2L regroups the pairs by offset class, its FP32
-  // near field sums in any order)
+  // the mixed form needs the M2L list grouped by target, not each target's
+  // sources sorted (it regroups the pairs by offset class)
   TB_TRY(build_lists(ctx, theta, mutual, precision != TAPAS_B200_MIXED));
   TB_TRY(tapas_b200_m2l(ctx, precision));
   return tapas_b200_p2p(ctx, precision);

@@ -29,8 +29,8 @@
 // the target and source widths) and every separation is at least gap, so one
 // rounding of a coordinate is at most 2^-24 (gap + tw/2 + sw) / gap of the
 // separation; with gap >= (tw/2 + sw) / 3 that is <= 4 * 2^-24 ~ 2.4e-7.
-// Each source leaf is summed in plain FP32 and the partial is Kahan-added into
-// the target's (sum, compensation) pair; the final near field is FP64.
+// Every 64 source bodies are summed in plain FP32 and the partial is added to the
+// target's FP64 sums.
 #include <algorithm>
 #include <cfloat>
 
@@ -43,11 +43,13 @@ namespace {
 constexpr int kWarps = 4;  // FP64 kernel: 4-warp CTAs, 4 per SM (<= 128 registers)
 constexpr int kThreads = 32 * kWarps;
 constexpr int kFp64Blocks = 4;
-constexpr int kStage = 32;   // source bodies staged per warp at a time (one per lane)
-// mixed kernel: 4-warp CTAs, 4 per SM (<= 128 registers, 16 warps per SM), up to
-// 3 targets per lane (leaves of more than 96 bodies take two passes)
+constexpr int kStage = 64;   // mixed: source bodies staged per warp at a time (two per lane)
+// mixed kernel: 4-warp CTAs, up to 4 targets per lane (leaves of more than 128
+// bodies take two passes)
 constexpr int kMixedWarps = 4;
-constexpr int kMixedMaxR = 3;  // most targets per lane of the mixed kernel
+constexpr int kMixedMaxR = 4;
+constexpr int kMixedBlocks = 5;     // CTAs per SM (<= 102 registers)
+constexpr float kNowhere = 1.25e18f;  // coordinate of a chargeless padding source
 constexpr int kMixedThreads = 32 * kMixedWarps;
 
 // ---------------------------------------------------------------------------
@@ -375,49 +377,12 @@ __global__ void __launch_bounds__(256) prepare_rel(
   }
 }
 
-__device__ __forceinline__ void kahan_add(float &sum, float &comp, float v) {
-  const float y = __fsub_rn(v, comp);
-  const float t = __fadd_rn(sum, y);
-  comp = __fsub_rn(__fsub_rn(t, sum), y);
-  sum = t;
-}
-
-// The same on a (sum, compensation) pair held in shared memory.
-__device__ __forceinline__ void kahan_add_sm(float &sum_sm, float &comp_sm, float v) {
-  float sum = sum_sm, comp = comp_sm;
-  kahan_add(sum, comp, v);
-  sum_sm = sum;
-  comp_sm = comp;
-}
-
 // a + b = s + e exactly (Knuth's TwoSum)
 __device__ __forceinline__ float two_sum(float a, float b, float &e) {
   const float s = __fadd_rn(a, b);
   const float bb = __fsub_rn(s, a);
   e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
   return s;
-}
-
-// Shape of a mixed tile of nt targets: kR targets per lane, L = ceil(nt/kR)
-// lanes per group, G = 32/L groups that split the sources.  Time per source
-// ~ kR / G, so pick the kR in 1..kMaxRm that minimises it (ties: the larger
-// kR, fewer shared loads per interaction).  nt <= 32 * kMaxRm.
-template <int kMaxRm>
-__device__ __forceinline__ void mixed_shape(int nt, int &R, int &L, int &G) {
-  R = kMaxRm;
-  L = (nt + kMaxRm - 1) / kMaxRm;
-  G = 32 / L;
-#pragma unroll
-  for (int r = kMaxRm - 1; r >= 1; r--) {
-    const int l = (nt + r - 1) / r;
-    if (l > 32) break;
-    const int g = 32 / l;
-    if (r * G < R * g) {
-      R = r;
-      L = l;
-      G = g;
-    }
-  }
 }
 
 // 1/sqrt(x) for normal x > 0 from the hardware approximation (relative error
@@ -429,72 +394,100 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
   return y;
 }
 
-// A staged source body in the target leaf's frame: FP32 hi part and charge,
-// FP32 lo part.
-struct __align__(16) SrcRec {
-  float4 hi, lo;
+// A source leaf of the current batch: its centre's offset from the target
+// leaf's (FP64 difference as FP32 hi + lo) and whether its box is far enough for
+// plain FP32 coordinates (see above); body i of the batch's stream of source
+// bodies is body b0 + i for the leaf that holds it.
+struct __align__(16) LeafMeta {
+  float hx, hy, hz;
+  int b0;
+  float lx, ly, lz;
+  int far;
 };
 
-// A source leaf of the current batch: body range and centre offset from the
-// target leaf (FP64 difference as FP32 hi + lo).
-struct __align__(16) LeafMeta {
-  int b0, ns;
-  int far;  // the leaf's box is far enough for plain FP32 coordinates (see above)
-  float hx, hy, hz, lx, ly, lz;
+// One warp's shared memory.
+struct __align__(16) MixedWarp {
+  float fx[kStage], fy[kStage], fz[kStage], fq[kStage];  // far: minus coordinates, charge
+  float4 near_hi[kStage], near_lo[kStage];               // near: hi parts and charge, lo parts
+  LeafMeta meta[32];
+  double sum[kMixedMaxR][4][32];   // pot, ax, ay, az per target
+  float lo[kMixedMaxR][3][32];     // the targets' lo parts
 };
 
 // One tile of a target leaf: lane (g, l) = (lane / L, lane % L) holds targets
-// l, l + L, ..., l + (kR-1) L and takes every G-th staged source.
+// l, l + L, ..., l + (kR-1) L and takes its share of the staged sources.
 //
-// The source leaves of the target's list are read 32 at a time: lane j loads
-// list entry j's leaf range and its centre offset (the FP64 difference split
-// into FP32 hi + lo) into the warp's table in shared memory, so the dependent
-// list -> cell loads are paid once per 32 source leaves.  Source bodies move
-// through the warp's shared-memory slice 32 at a time; the next chunk's
-// global loads are issued before the current chunk is computed.
+// The source bodies of the target's list are one stream: the list is read 32
+// leaves at a time (lane j: entry j's body range, the running body count and the
+// centre offset), and 64 consecutive bodies of the stream are staged at a time,
+// two per lane; a lane finds its bodies' leaf by a binary search over the 32
+// counts with shuffles.  Each body is classed far or near and the far ones are
+// stored as coordinate arrays, so that two consecutive sources are one
+// load per coordinate and are evaluated per packed FP32 instruction: 13 packed
+// operations and 2 MUFU per two pairs.  FP32 additions, multiplications and
+// fmas run at the same rate packed or not (measured 112 to 125 lanes per clock
+// and SM either way), so the gain is the issue slots: the pair formula alone
+// reached 8.1 pairs per clock and SM scalar, 9.05 packed, 9.85 being the pipe.
+// With one target per lane the broadcast loads (4 cycles of the shared-memory
+// port each) are the bound at 7.8, hence tiles with as many targets per lane
+// as splitting the sources over lane groups allows.
 template <int kR>
 __device__ __forceinline__ void mixed_tile(
-    int lane, int wi, int tb0, int nt, int L, int G, int e0, int e1, double tcx, double tcy,
-    double tcz, double tw, const uint64_t *__restrict__ list, uint64_t mask,
-    const int32_t *__restrict__ cbeg, const int32_t *__restrict__ cnb,
-    const double *__restrict__ ccen, const double *__restrict__ cmin,
-    const double *__restrict__ cmax, const float4 *__restrict__ rel_hi,
-    const float4 *__restrict__ rel_lo, SrcRec (*ss)[kStage],
-    LeafMeta (*mt)[32], double4 (*red)[32], float (*kc)[kMixedMaxR][8][32],
+    int lane, int tb0, int nt, int L, int G, int e0, int e1, double tcx, double tcy, double tcz,
+    double tw, const uint64_t *__restrict__ list, uint64_t mask, const int32_t *__restrict__ cbeg,
+    const int32_t *__restrict__ cnb, const double *__restrict__ ccen,
+    const double *__restrict__ cmin, const double *__restrict__ cmax,
+    const float4 *__restrict__ rel_hi, const float4 *__restrict__ rel_lo, MixedWarp &sm,
     double4 *__restrict__ out) {
   const int g = lane / L, tl = lane - g * L;
   const bool active = g < G;
-  const int gs = active ? g : kStage;  // idle lanes skip the source loop
   // a source body this far from the target leaf's centre (max norm) is far;
   // the margin covers the FP32 rounding of the test itself
   const float far_body = (float)(tw * (5.0 / 6.0)) * (1.0f + 1e-6f);
-  float txh[kR], tyh[kR], tzh[kR], txl[kR], tyl[kR], tzl[kR];
-  float tp[kR], tx[kR], ty[kR], tz[kR];
-  // the Kahan (sum, compensation) pairs of pot, ax, ay, az per target live in
-  // the warp's shared-memory slice (touched once per source leaf), which keeps
-  // the kernel at 6 CTAs per SM
-  float(*kw)[8][32] = kc[wi];
+  float2 txh[kR], tyh[kR], tzh[kR];  // both halves the target's coordinate
+  float2 tp[kR], tx[kR], ty[kR], tz[kR];  // sums of the even and the odd sources
+  const float2 zero = make_float2(0.f, 0.f);
 #pragma unroll
   for (int r = 0; r < kR; r++) {
     const int t = tl + L * r;
     const bool v = active && t < nt;
     const float4 h = v ? rel_hi[tb0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 l = v ? rel_lo[tb0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
-    txh[r] = h.x; tyh[r] = h.y; tzh[r] = h.z;
-    txl[r] = l.x; tyl[r] = l.y; tzl[r] = l.z;
+    txh[r] = make_float2(h.x, h.x);
+    tyh[r] = make_float2(h.y, h.y);
+    tzh[r] = make_float2(h.z, h.z);
+    sm.lo[r][0][lane] = l.x;
+    sm.lo[r][1][lane] = l.y;
+    sm.lo[r][2][lane] = l.z;
 #pragma unroll
-    for (int k = 0; k < 8; k++) kw[r][k][lane] = 0.f;
-    tp[r] = tx[r] = ty[r] = tz[r] = 0.f;
+    for (int k = 0; k < 4; k++) sm.sum[r][k][lane] = 0.0;
+    tp[r] = tx[r] = ty[r] = tz[r] = zero;
   }
-  LeafMeta *const meta = mt[wi];
+  // far bodies: plain FP32 coordinates in the target frame (relative error of a
+  // separation <= ~2.4e-7), no r = 0 case
+  auto far2 = [&](float2 sx, float2 sy, float2 sz, float2 sq) {
+#pragma unroll
+    for (int r = 0; r < kR; r++) {
+      const float2 dx = __fadd2_rn(txh[r], sx), dy = __fadd2_rn(tyh[r], sy),
+                   dz = __fadd2_rn(tzh[r], sz);
+      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+      const float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+      const float2 qr = __fmul2_rn(sq, ri);
+      const float2 qr3 = __fmul2_rn(__fmul2_rn(qr, ri), ri);
+      tp[r] = __fadd2_rn(tp[r], qr);
+      tx[r] = __ffma2_rn(dx, qr3, tx[r]);
+      ty[r] = __ffma2_rn(dy, qr3, ty[r]);
+      tz[r] = __ffma2_rn(dz, qr3, tz[r]);
+    }
+  };
   for (int eb = e0; eb < e1; eb += 32) {
-    const int nbat = min(32, e1 - eb);
-    __syncwarp();
-    if (lane < nbat) {
+    __syncwarp();  // the previous batch's table is read
+    int ns = 0;
+    LeafMeta m{};
+    if (eb + lane < e1) {
       const int s = (int)(list[eb + lane] & mask);
-      LeafMeta m;
       m.b0 = cbeg[s];
-      m.ns = cnb[s];
+      ns = cnb[s];
       // source frame -> target frame: FP64 centre difference as (hi, lo) floats
       const double dcx = ccen[3 * s] - tcx, dcy = ccen[3 * s + 1] - tcy,
                    dcz = ccen[3 * s + 2] - tcz;
@@ -504,158 +497,128 @@ __device__ __forceinline__ void mixed_tile(
       const double sw = cmax[3 * s] - cmin[3 * s];
       const double gap = fmax(fabs(dcx), fmax(fabs(dcy), fabs(dcz))) - 0.5 * (tw + sw);
       m.far = 3.0 * gap >= 0.5 * tw + sw ? 1 : 0;
-      meta[lane] = m;
     }
-    __syncwarp();
-    // first non-empty source leaf of the batch
-    int j = 0;
-    int ns_j = meta[0].ns;
-    while (ns_j == 0 && ++j < nbat) ns_j = meta[j].ns;
-    if (j >= nbat) continue;
-    int ch = 0;
-    float4 ph = make_float4(0.f, 0.f, 0.f, 0.f), pl = ph;
-    {
-      const int b0 = meta[j].b0;
-      if (lane < min(kStage, ns_j)) {
-        ph = rel_hi[b0 + lane];
-        pl = rel_lo[b0 + lane];
-      }
+    int upto = ns;  // bodies of the batch's leaves 0 .. lane
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
     }
-    while (j < nbat) {
-      const int cnt = min(kStage, ns_j - ch);
-      __syncwarp();
-      // Far bodies first (single floats), then near ones (hi, lo).  A body is
+    const int total = __shfl_sync(0xffffffffu, upto, 31);
+    m.b0 -= upto - ns;
+    sm.meta[lane] = m;
+    for (int c0 = 0; c0 < total; c0 += kStage) {
+      __syncwarp();  // the table is written; the previous chunk is read
+      // Far bodies as single floats, near ones as (hi, lo).  A body is
       // far when its whole leaf is, or when its max-norm distance from the
       // target leaf's centre is at least 5/6 of the leaf width: then every
       // target is >= D - tw/2 away while the coordinates are <= D and tw/2, so
       // one rounding is <= 2^-24 (D + tw/2) / (D - tw/2) <= 4 * 2^-24 of a
       // separation, the leaf rule's bound.
-      int nfar;
-      {
-        const LeafMeta &m = meta[j];
-        float ex = 0.f, ey = 0.f, ez = 0.f, ax = 0.f, ay = 0.f, az = 0.f, lx = 0.f, ly = 0.f,
-              lz = 0.f;
-        bool farb = true;
-        if (lane < cnt) {
-          ax = two_sum(ph.x, m.hx, ex);
-          ay = two_sum(ph.y, m.hy, ey);
-          az = two_sum(ph.z, m.hz, ez);
-          lx = ex + (pl.x + m.lx);
-          ly = ey + (pl.y + m.ly);
-          lz = ez + (pl.z + m.lz);
-          if (!m.far)
-            farb = fmaxf(fabsf(ax + lx), fmaxf(fabsf(ay + ly), fabsf(az + lz))) >= far_body;
+      int nfar = 0, nnear = 0;
+#pragma unroll
+      for (int h = 0; h < kStage / 32; h++) {
+        const int i = c0 + 32 * h + lane;
+        if (c0 + 32 * h >= total) break;  // warp-uniform
+        int leaf = 0;  // the first leaf with upto > i
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const int v = __shfl_sync(0xffffffffu, upto, leaf + o - 1);
+          if (v <= i) leaf += o;
         }
-        const unsigned valid = cnt >= 32 ? 0xffffffffu : ((1u << cnt) - 1u);
-        const unsigned fm = __ballot_sync(0xffffffffu, farb) & valid;
+        const bool valid = i < total;
+        float ax = 0.f, ay = 0.f, az = 0.f, lx = 0.f, ly = 0.f, lz = 0.f, q = 0.f;
+        bool farb = false;
+        if (valid) {
+          const LeafMeta lm = sm.meta[leaf];
+          const float4 ph = rel_hi[lm.b0 + i], pl = rel_lo[lm.b0 + i];
+          float ex, ey, ez;
+          ax = two_sum(ph.x, lm.hx, ex);
+          ay = two_sum(ph.y, lm.hy, ey);
+          az = two_sum(ph.z, lm.hz, ez);
+          lx = ex + (pl.x + lm.lx);
+          ly = ey + (pl.y + lm.ly);
+          lz = ez + (pl.z + lm.lz);
+          q = ph.w;
+          farb = lm.far ||
+                 fmaxf(fabsf(ax + lx), fmaxf(fabsf(ay + ly), fabsf(az + lz))) >= far_body;
+        }
+        const unsigned fm = __ballot_sync(0xffffffffu, farb);
+        const unsigned nm = __ballot_sync(0xffffffffu, valid && !farb);
         const unsigned below = (1u << lane) - 1u;
-        nfar = __popc(fm);
-        if (lane < cnt) {
-          if (farb) {  // one float per coordinate, rounded once
-            ss[wi][__popc(fm & below)].hi = make_float4(ax + lx, ay + ly, az + lz, ph.w);
-          } else {
-            const int k = nfar + __popc(~fm & valid & below);
-            ss[wi][k].hi = make_float4(ax, ay, az, ph.w);
-            ss[wi][k].lo = make_float4(lx, ly, lz, 0.f);
-          }
+        if (farb) {  // one float per coordinate, rounded once
+          const int k = nfar + __popc(fm & below);
+          sm.fx[k] = -(ax + lx);
+          sm.fy[k] = -(ay + ly);
+          sm.fz[k] = -(az + lz);
+          sm.fq[k] = q;
+        } else if (valid) {
+          const int k = nnear + __popc(nm & below);
+          sm.near_hi[k] = make_float4(ax, ay, az, q);
+          sm.near_lo[k] = make_float4(lx, ly, lz, 0.f);
         }
+        nfar += __popc(fm);
+        nnear += __popc(nm);
+      }
+      // an odd last far body is paired with a chargeless one far away
+      if (lane == 0 && (nfar & 1)) {
+        sm.fx[nfar] = sm.fy[nfar] = sm.fz[nfar] = kNowhere;
+        sm.fq[nfar] = 0.f;
       }
       __syncwarp();
-      // next chunk: the rest of this leaf, else the next non-empty leaf of the batch
-      int j2 = j, ch2 = ch + kStage, ns2 = ns_j;
-      const bool leaf_done = ch2 >= ns_j;
-      if (leaf_done) {
-        ch2 = 0;
-        ns2 = 0;
-        while (ns2 == 0 && ++j2 < nbat) ns2 = meta[j2].ns;
-      }
-      if (j2 < nbat) {
-        const int b0 = meta[j2].b0;
-        if (lane < min(kStage, ns2 - ch2)) {
-          ph = rel_hi[b0 + ch2 + lane];
-          pl = rel_lo[b0 + ch2 + lane];
-        }
-      }
-      {
-        // far bodies: plain FP32 coordinates in the target frame (relative
-        // error of a separation <= ~2.4e-7), no r = 0 case
-        auto far_src = [&](int k) {
-          const float4 bh = ss[wi][k].hi;
-#pragma unroll
-          for (int r = 0; r < kR; r++) {
-            const float dx = txh[r] - bh.x, dy = tyh[r] - bh.y, dz = tzh[r] - bh.z;
-            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            const float ri = rsqrt_ftz(r2);
-            const float qr = bh.w * ri;
-            const float qr3 = qr * ri * ri;
-            tp[r] += qr;
-            tx[r] = fmaf(dx, qr3, tx[r]);
-            ty[r] = fmaf(dy, qr3, ty[r]);
-            tz[r] = fmaf(dz, qr3, tz[r]);
-          }
-        };
-        if (G == 1) {
-          // one group takes every source: unit stride, fixed offsets
-#pragma unroll 4
-          for (int k = active ? 0 : nfar; k < nfar; k++) far_src(k);
-        } else {
-#pragma unroll 2
-          for (int k = gs; k < nfar; k += G) far_src(k);
-        }
-      }
-      if (nfar < cnt) {
+      if (active) {
+        // loops short enough for the instruction cache nearest the scheduler: with
+        // three or four targets a lane has that many independent chains anyway
+#pragma unroll(kR == 1 ? 2 : 1)
+        for (int k = 2 * g; k < nfar; k += 2 * G)
+          far2(*reinterpret_cast<const float2 *>(sm.fx + k),
+               *reinterpret_cast<const float2 *>(sm.fy + k),
+               *reinterpret_cast<const float2 *>(sm.fz + k),
+               *reinterpret_cast<const float2 *>(sm.fq + k));
         // near bodies: separations from (hi, lo) coordinates
-        // two sources in flight: their rsqrt latencies overlap
-#pragma unroll 2
-        for (int k = nfar + gs; k < cnt; k += G) {
-          const float4 bh = ss[wi][k].hi;
-          const float4 bl = ss[wi][k].lo;
+#pragma unroll(kR == 1 ? 2 : 1)
+        for (int k = g; k < nnear; k += G) {
+          const float4 bh = sm.near_hi[k];
+          const float4 bl = sm.near_lo[k];
 #pragma unroll
           for (int r = 0; r < kR; r++) {
-            const float dx = (txh[r] - bh.x) + (txl[r] - bl.x);
-            const float dy = (tyh[r] - bh.y) + (tyl[r] - bl.y);
-            const float dz = (tzh[r] - bh.z) + (tzl[r] - bl.z);
+            const float dx = (txh[r].x - bh.x) + (sm.lo[r][0][lane] - bl.x);
+            const float dy = (tyh[r].x - bh.y) + (sm.lo[r][1][lane] - bl.y);
+            const float dz = (tzh[r].x - bh.z) + (sm.lo[r][2][lane] - bl.z);
             const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             const float ri = r2 >= FLT_MIN ? rsqrt_ftz(r2) : 0.f;
             const float qr = bh.w * ri;
             const float qr3 = qr * ri * ri;
-            tp[r] += qr;
-            tx[r] = fmaf(dx, qr3, tx[r]);
-            ty[r] = fmaf(dy, qr3, ty[r]);
-            tz[r] = fmaf(dz, qr3, tz[r]);
+            tp[r].x += qr;
+            tx[r].x = fmaf(dx, qr3, tx[r].x);
+            ty[r].x = fmaf(dy, qr3, ty[r].x);
+            tz[r].x = fmaf(dz, qr3, tz[r].x);
           }
         }
       }
-      if (leaf_done) {
-        // one source leaf summed in FP32: Kahan-add it into the target's sums
+      // a chunk is summed in FP32 and added to the target's FP64 sums
 #pragma unroll
-        for (int r = 0; r < kR; r++) {
-          kahan_add_sm(kw[r][0][lane], kw[r][1][lane], tp[r]);
-          kahan_add_sm(kw[r][2][lane], kw[r][3][lane], tx[r]);
-          kahan_add_sm(kw[r][4][lane], kw[r][5][lane], ty[r]);
-          kahan_add_sm(kw[r][6][lane], kw[r][7][lane], tz[r]);
-          tp[r] = tx[r] = ty[r] = tz[r] = 0.f;
-        }
+      for (int r = 0; r < kR; r++) {
+        sm.sum[r][0][lane] += (double)(tp[r].x + tp[r].y);
+        sm.sum[r][1][lane] += (double)(tx[r].x + tx[r].y);
+        sm.sum[r][2][lane] += (double)(ty[r].x + ty[r].y);
+        sm.sum[r][3][lane] += (double)(tz[r].x + tz[r].y);
+        tp[r] = tx[r] = ty[r] = tz[r] = zero;
       }
-      j = j2;
-      ch = ch2;
-      ns_j = ns2;
     }
   }
-  __syncwarp();
+  double4 *red = reinterpret_cast<double4 *>(sm.near_hi);  // the sources are done with
 #pragma unroll
   for (int r = 0; r < kR; r++) {
-    const float *k = &kw[r][0][lane];
-    double4 v = make_double4((double)k[0] - (double)k[32], -((double)k[64] - (double)k[96]),
-                             -((double)k[128] - (double)k[160]),
-                             -((double)k[192] - (double)k[224]));
+    double4 v = make_double4(sm.sum[r][0][lane], -sm.sum[r][1][lane], -sm.sum[r][2][lane],
+                             -sm.sum[r][3][lane]);
     if (G > 1) {
       __syncwarp();
-      red[wi][lane] = v;
+      red[lane] = v;
       __syncwarp();
       if (g == 0) {
         for (int gg = 1; gg < G; gg++) {
-          const double4 o = red[wi][tl + gg * L];
+          const double4 o = red[tl + gg * L];
           v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
         }
       }
@@ -663,9 +626,10 @@ __device__ __forceinline__ void mixed_tile(
     const int t = tl + L * r;
     if (active && g == 0 && t < nt) out[t] = v;
   }
+  __syncwarp();  // the next tile reuses the warp's shared memory
 }
 
-template <int kMaxRm, int kBlocks>
+template <int kBlocks>
 __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
     const uint32_t *__restrict__ order, int64_t nitems, int *__restrict__ counter,
     const WorkItem *__restrict__ items, const uint64_t *__restrict__ list, uint64_t src_mask,
@@ -673,11 +637,7 @@ __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
     const double *__restrict__ ccen, const double *__restrict__ cmin,
     const double *__restrict__ cmax, const float4 *__restrict__ rel_hi,
     const float4 *__restrict__ rel_lo, double *__restrict__ trg, double *__restrict__ part) {
-  static_assert(kMaxRm <= kMixedMaxR, "targets per lane");
-  __shared__ SrcRec ss[kMixedWarps][kStage];
-  __shared__ LeafMeta mt[kMixedWarps][32];
-  __shared__ double4 red[kMixedWarps][32];
-  __shared__ float kc[kMixedWarps][kMixedMaxR][8][32];
+  __shared__ MixedWarp sm[kMixedWarps];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   for (;;) {
     const int w = next_leaf(counter, lane);
@@ -690,17 +650,16 @@ __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
     double4 *out = item_out(it, tb0, trg, part);
     const double tcx = ccen[3 * c], tcy = ccen[3 * c + 1], tcz = ccen[3 * c + 2];
     const double tw = cmax[3 * c] - cmin[3 * c];
-    for (int tbase = 0; tbase < nt_all; tbase += 32 * kMaxRm) {
-      const int nt = min(nt_all - tbase, 32 * kMaxRm);
+    for (int tbase = 0; tbase < nt_all; tbase += kTileTargets) {
+      const int nt = min(nt_all - tbase, kTileTargets);
       int R, L, G;
-      mixed_shape<kMaxRm>(nt, R, L, G);
-#define TB_MIXED_TILE(RR)                                                                     \
-  mixed_tile<RR>(lane, wi, tb0 + tbase, nt, L, G, e0, e1, tcx, tcy, tcz, tw, list, src_mask, \
-                 cbeg, cnb, ccen, cmin, cmax, rel_hi, rel_lo, ss, mt, red, kc, out + tbase)
-      if (R == 1) TB_MIXED_TILE(1);
-      else if (R == 2) TB_MIXED_TILE(2);
-      else if (kMaxRm == 3 || R == 3) TB_MIXED_TILE(3);
-      else TB_MIXED_TILE(kMaxRm);
+      tile_shape(nt, R, L, G);
+#define TB_MIXED_TILE(RR)                                                                        \
+  mixed_tile<RR>(lane, tb0 + tbase, nt, L, G, e0, e1, tcx, tcy, tcz, tw, list, src_mask, cbeg,  \
+                 cnb, ccen, cmin, cmax, rel_hi, rel_lo, sm[wi], out + tbase)
+      if (R == 4) TB_MIXED_TILE(4);
+      else if (R == 3) TB_MIXED_TILE(3);
+      else TB_MIXED_TILE(1);
 #undef TB_MIXED_TILE
     }
   }
@@ -825,11 +784,9 @@ int p2p_mixed(tapas_b200_ctx *ctx) {
                                                       ctx->sy.p, ctx->sz.p, ctx->sq.p,
                                                       ctx->rel4.p, ctx->rel_lo.p);
   TB_LAUNCH_CHECK(ctx);
-  TB_TRY(p2p_items(ctx, 24));
+  TB_TRY(p2p_items(ctx, kMixedBlocks * kMixedWarps));
   const uint64_t mask = (1ull << ctx->list_shift) - 1;
-  // up to 3 targets per lane; the Kahan pairs in shared memory keep the kernel
-  // at 80 registers, 24 warps per SM
-  p2p_mixed_kernel<3, 6><<<p2p_grid(ctx, kMixedWarps), kMixedThreads, 0, s>>>(
+  p2p_mixed_kernel<kMixedBlocks><<<p2p_grid(ctx, kMixedWarps), kMixedThreads, 0, s>>>(
       ctx->p2p_order.p, ctx->p2p_nitems, ctx->p2p_counter.p,
       reinterpret_cast<const WorkItem *>(ctx->p2p_items.p), ctx->p2p.p, mask, ctx->cbeg.p,
       ctx->cnb.p, ctx->ccen.p, ctx->cmin.p, ctx->cmax.p, ctx->rel4.p, ctx->rel_lo.p,

@@ -344,6 +344,16 @@ __global__ void __launch_bounds__(kSegWarps * 32) sort_segments(
       continue;
     }
     const int np = pow2_at_least(len);
+    if (np <= 32) {  // in registers, a lane an entry
+      uint32_t v = lane < len ? src[a0 + lane] : 0xFFFFFFFFu;
+      for (int k = 2; k <= np; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, v, j);
+          v = ((lane & j) == 0) == ((lane & k) == 0) ? min(v, o) : max(v, o);
+        }
+      if (lane < len) out[a0 + lane] = th | v;
+      continue;
+    }
     for (int i = lane; i < np; i += 32) a[i] = i < len ? src[a0 + i] : 0xFFFFFFFFu;
     __syncwarp();
     bitonic_sort<false>(a, np, lane, 32);
@@ -444,7 +454,7 @@ int sort_list_sources(tapas_b200_ctx *ctx) {
   return sort_list_sources(ctx, 1);
 }
 
-int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_sources) {
+int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sources) {
   if (!ctx->have_tree) {
     set_error(ctx, "build_lists: no tree (call partition first)");
     return TAPAS_B200_ERR_STATE;
@@ -600,7 +610,7 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_sources
         scatter_by_target<<<grid_for(n, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
             L.p, n, ctx->list_cnt.p, ctx->list_src.p);
         TB_LAUNCH_CHECK(ctx);
-        if (!sort_sources) {
+        if (w == 0 && !sort_m2l_sources) {
           // grouped by target only; sort_list_sources() completes the order
           // when a caller needs it
           pack_segments<<<grid_for(C, kSegWarps, ctx->num_sms * 8), kSegWarps * 32, 0, s>>>(
