@@ -6,7 +6,7 @@
 //                   body, a non-leaf the mass and mass-weighted centre of its 8
 //                   children summed in index order (leaves with more bodies,
 //                   ncrit > 1, use the same formula over their bodies).
-//  bh_walk_kernel   interact + ComputeForce (bh.cc:135-153, 192-224): each
+//  bh_walk64, bh_walk32   interact + ComputeForce (bh.cc:135-153, 192-224): each
 //                   body walks the tree depth first from the root, children
 //                   visited 0..7 like the sample's recursion; a warp's 32
 //                   bodies (consecutive in Morton order) share one bounded
@@ -14,10 +14,14 @@
 //                   accepted when width / |centre - body| < theta; a leaf is
 //                   summed body by body (the body itself included, as in the
 //                   sample).
-// The FP64 form uses separately rounded operations in the sample's order, so
-// it reproduces the sample bit for bit; the FP32 form ("mixed") walks with FP32
-// positions and FP32 copies of the FP64 cell moments.
+// The FP64 form rounds as the sample does, operation by operation in the
+// sample's order, so it reproduces the sample bit for bit; the FP32 form
+// ("mixed") takes the same decisions and sums FP32 terms of FP32 positions and
+// FP32 copies of the FP64 cell moments.
+#include <cfloat>
+
 #include "common.cuh"
+#include "primitives.cuh"
 
 namespace tb {
 namespace {
@@ -66,151 +70,113 @@ __global__ void bh_upward_level(int64_t a, int64_t cnt, const int32_t *__restric
   }
 }
 
-// ComputeForce (bh.cc:135-153), FP64, the sample's rounding order.
-__device__ __forceinline__ void force64(double px, double py, double pz, double ax, double ay,
-                                        double az, double aw, double eps2, double4 &o) {
-  const double dx = __dsub_rn(ax, px), dy = __dsub_rn(ay, py), dz = __dsub_rn(az, pz);
-  double R2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-  R2 = __dadd_rn(__dadd_rn(R2, __dmul_rn(dz, dz)), eps2);
-  const double invR = __ddiv_rn(1.0, __dsqrt_rn(R2));
-  const double invR3 = __dmul_rn(__dmul_rn(invR, invR), invR);
-  o.x = __dadd_rn(o.x, __dmul_rn(__dmul_rn(dx, invR3), aw));
-  o.y = __dadd_rn(o.y, __dmul_rn(__dmul_rn(dy, invR3), aw));
-  o.z = __dadd_rn(o.z, __dmul_rn(__dmul_rn(dz, invR3), aw));
-  o.w = __dadd_rn(o.w, __dmul_rn(invR, aw));
-}
-
-__device__ __forceinline__ void force32(float px, float py, float pz, float ax, float ay, float az,
-                                        float aw, float eps2, float4 &o) {
-  const float dx = ax - px, dy = ay - py, dz = az - pz;
-  const float R2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-  const float invR = rsqrtf(R2);
-  const float wr = aw * invR;
-  const float wr3 = wr * invR * invR;
-  o.x = fmaf(dx, wr3, o.x);
-  o.y = fmaf(dy, wr3, o.y);
-  o.z = fmaf(dz, wr3, o.z);
-  o.w += wr;
-}
-
-struct BhTree {
-  const int32_t *leaf, *nb, *beg, *child;
-  const double *cmin, *cmax, *ccen;
+// What the walks read of a cell, packed per walk: centre and squared width, and
+// {first child, -1}, or for a leaf {its bodies, their number}: the first body
+// of the FP64 walk, the first pair of the FP32 walk's body pairs.
+struct BhCells {
+  const double4 *geo;
+  const int2 *meta;
+  const double *cmin, *cmax, *ccen;  // the acceptance test inside its band
 };
 
-// One walk per warp over the union of its 32 bodies' walks.  The warp keeps
-// one stack of (cell, lanes that reach it); at each popped cell the lanes in
-// its mask do what their own walk does there (sum a leaf, accept the cell, or
-// open it), and the cell's children are pushed for the lanes that opened it.
-// Every lane's walk is a depth-first walk with children 0..7 of a subtree of
-// the union's, so a lane meets its cells in its own order, takes the sample's
-// decisions and sums its interactions in the sample's order; the warp reads
-// each cell and each leaf body once for all its lanes, and the bodies, in
-// Morton order, share most of their walks.
-constexpr int kWalkWarps = 4;
-template <bool kFp64>
-__global__ void __launch_bounds__(32 * kWalkWarps) bh_walk_kernel(
-    BhTree T, int64_t n, const double *__restrict__ sx, const double *__restrict__ sy,
-    const double *__restrict__ sz, const double *__restrict__ sm, const double4 *__restrict__ attr,
-    const float4 *__restrict__ attr32, const float4 *__restrict__ pos32, double theta,
-    double eps2, double *__restrict__ out, unsigned long long *__restrict__ counters) {
-  __shared__ int scell[kWalkWarps][kStack];
-  __shared__ unsigned smask[kWalkWarps][kStack];
-  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  const double theta2 = __dmul_rn(theta, theta);
-  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = b < n;
-  unsigned long long napprox = 0, ndirect = 0, overflow = 0;
-  const double px = valid ? sx[b] : 0.0, py = valid ? sy[b] : 0.0, pz = valid ? sz[b] : 0.0;
-  double4 o64 = make_double4(0, 0, 0, 0);
-  float4 o32 = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 p32 = (kFp64 || !valid) ? make_float4(0.f, 0.f, 0.f, 0.f) : pos32[b];
-  const unsigned lanes = __ballot_sync(0xffffffffu, valid);
-  int sp = 0;  // the same in every lane
-  if (lanes) {
-    if (lane == 0) {
-      scell[wi][0] = 0;
-      smask[wi][0] = lanes;
-    }
-    sp = 1;
-    __syncwarp();
+// 1/x of the rounded sqrt(r2), each correctly rounded, as the sample computes it
+// (bh.cc:148-149), from the hardware's approximation: refined to about an ulp
+// (the series of charge_over_distance), then one residual step each for the square
+// root and the reciprocal (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990): the residuals are exact in an
+// fma, so the results differ from the rounded exact ones only where those lie
+// within ~2^-104 of a rounding boundary.  12 FP64 operations where the two
+// library sequences take about 57 slots of the FP64 pipe.
+// kN at once, with one branch for all: a branch each would keep their chains
+// from overlapping.
+template <int kN>
+__device__ __forceinline__ void rounded_inv_sqrt(const double (&r2)[kN], double (&inv)[kN]) {
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < kN; i++) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2[i]));
+    const double e = fma(-(r2[i] * y), y, 1.0);
+    y = fma(y, e * fma(e, 0.375, 0.5), y);
+    const double g = r2[i] * y;
+    const double s = fma(fma(-g, g, r2[i]), 0.5 * y, g);
+    inv[i] = fma(y, fma(-s, y, 1.0), y);
+    // outside 2^-767 .. 2^768 the residuals could underflow
+    odd |= (unsigned)__double2hiint(r2[i]) - 0x10000000u >= 0x60000000u;
   }
-  while (sp > 0) {
-    --sp;
-    const int c = scell[wi][sp];
-    const unsigned m = smask[wi][sp];
-    __syncwarp();  // read before a push reuses the slot
-    const bool mine = (m >> lane) & 1u;
-    if (T.leaf[c]) {
-      if (mine) {
-        const int nb = T.nb[c], b0 = T.beg[c];
-        for (int i = 0; i < nb; i++) {
-          const int j = b0 + i;
-          if (kFp64) force64(px, py, pz, sx[j], sy[j], sz[j], sm[j], eps2, o64);
-          else {
-            const float4 q = pos32[j];
-            force32(p32.x, p32.y, p32.z, q.x, q.y, q.z, q.w, (float)eps2, o32);
-          }
-        }
-        ndirect += (unsigned)nb;
-      }
-      continue;
-    }
-    bool open = false;
-    if (mine) {
-      // the sample's MAC: cell width / |centre - body| < theta
-      const double dx = __dsub_rn(px, T.ccen[3 * c]), dy = __dsub_rn(py, T.ccen[3 * c + 1]),
-                   dz = __dsub_rn(pz, T.ccen[3 * c + 2]);
-      double R = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-      R = __dadd_rn(R, __dmul_rn(dz, dz));
-      const double s = __dsub_rn(T.cmax[3 * c], T.cmin[3 * c]);
-      // The sample evaluates fl(s / fl(sqrt(R))) < theta.  That value is
-      // s/sqrt(R) within ~2.3 ulp, and s^2 against theta^2 R below within
-      // ~4 ulp, so outside a relative band of 1e-13 around theta^2 R the
-      // squared test decides the same way without the square root and the
-      // division; inside it the sample's own operations decide.
-      const double s2 = __dmul_rn(s, s), t2R = __dmul_rn(theta2, R);
-      bool accept;
-      if (s2 < __dmul_rn(t2R, 1.0 - 1e-13)) accept = true;
-      else if (s2 > __dmul_rn(t2R, 1.0 + 1e-13)) accept = false;
-      else accept = __ddiv_rn(s, __dsqrt_rn(R)) < theta;
-      if (accept) {
-        if (kFp64) {
-          const double4 a = attr[c];
-          force64(px, py, pz, a.x, a.y, a.z, a.w, eps2, o64);
-        } else {
-          const float4 a = attr32[c];
-          force32(p32.x, p32.y, p32.z, a.x, a.y, a.z, a.w, (float)eps2, o32);
-        }
-        napprox++;
-      } else {
-        open = true;
-      }
-    }
-    const unsigned om = __ballot_sync(0xffffffffu, open);
-    if (om) {
-      if (sp + 8 > kStack) {
-        if (mine) overflow = 1;
-        break;
-      }
-      // children 7..0 from the bottom up, so child 0 is popped first
-      if (lane < 8) {
-        scell[wi][sp + lane] = T.child[c] + 7 - lane;
-        smask[wi][sp + lane] = om;
-      }
-      sp += 8;
-      __syncwarp();
+  if (odd) {
+#pragma unroll
+    for (int i = 0; i < kN; i++)
+      if ((unsigned)__double2hiint(r2[i]) - 0x10000000u >= 0x60000000u)
+        inv[i] = __ddiv_rn(1.0, __dsqrt_rn(r2[i]));
+  }
+}
+
+// The sample's acceptance test fl(width / fl(|centre - body|)) < theta.  That
+// quotient is width / distance within ~2.3 ulp and d below is s^2 - theta^2 R
+// within ~5 ulp of s^2, so outside a relative band of 2^-42 (2.3e-13) the sign
+// of d decides the same way without the square root and the division; inside
+// it (and for d not finite) the sample's own operations decide.  The band is
+// tested on the high words: 8 slots of the FP64 pipe per test.
+__device__ __forceinline__ bool bh_accept(const BhCells &T, int c, const double4 &g, double px,
+                                          double py, double pz, double theta, double theta2) {
+  const double dx = px - g.x, dy = py - g.y, dz = pz - g.z;
+  const double R = fma(dz, dz, fma(dy, dy, dx * dx));
+  const double d = fma(-theta2, R, g.w);
+  const int hd = __double2hiint(d);
+  const int lo = max(__double2hiint(g.w) - (42 << 20), 0);
+  if ((unsigned)((hd & 0x7fffffff) - lo) < (unsigned)(0x7ff00000 - lo)) return hd < 0;
+  const double ex = __dsub_rn(px, T.ccen[3 * c]), ey = __dsub_rn(py, T.ccen[3 * c + 1]),
+               ez = __dsub_rn(pz, T.ccen[3 * c + 2]);
+  double R2 = __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey));
+  R2 = __dadd_rn(R2, __dmul_rn(ez, ez));
+  const double s = __dsub_rn(T.cmax[3 * c], T.cmin[3 * c]);
+  return __ddiv_rn(s, __dsqrt_rn(R2)) < theta;
+}
+
+// What the acceptance test gives for all bodies of a warp at once, from their
+// bounding box: 1 every body accepts the cell, 2 every body opens it, 0 neither is
+// certain.  The nearest and farthest squared distances of the box to the centre
+// bound the bodies' own; the margin of 1e-12 is far above the rounding on
+// either side and the exact test's band, so a certain answer is every body's.
+struct BodyBox {
+  double lo[3], hi[3];
+};
+__device__ __forceinline__ BodyBox body_box(bool valid, double px, double py, double pz) {
+  BodyBox b;
+  const double p[3] = {px, py, pz}, inf = __longlong_as_double(0x7ff0000000000000ll);
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    b.lo[d] = valid ? p[d] : inf;
+    b.hi[d] = valid ? p[d] : -inf;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      b.lo[d] = fmin(b.lo[d], __shfl_xor_sync(0xffffffffu, b.lo[d], o));
+      b.hi[d] = fmax(b.hi[d], __shfl_xor_sync(0xffffffffu, b.hi[d], o));
     }
   }
-  if (valid) {
-    double4 *o = reinterpret_cast<double4 *>(out) + b;
-    *o = kFp64 ? o64 : make_double4((double)o32.x, (double)o32.y, (double)o32.z, (double)o32.w);
+  return b;
+}
+__device__ __forceinline__ int box_accept(const BodyBox &b, const double4 &g, double theta2) {
+  const double c[3] = {g.x, g.y, g.z};
+  double near2 = 0, far2 = 0;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const double u = b.lo[d] - c[d], v = c[d] - b.hi[d];  // > 0: the box is beyond c
+    const double n = fmax(fmax(u, v), 0.0), f = fmax(-u, -v);
+    near2 = fma(n, n, near2);
+    far2 = fma(f, f, far2);
   }
-  for (int s = 16; s > 0; s >>= 1) {
-    napprox += __shfl_down_sync(0xffffffffu, napprox, s);
-    ndirect += __shfl_down_sync(0xffffffffu, ndirect, s);
-    overflow |= __shfl_down_sync(0xffffffffu, overflow, s);
-  }
+  if (g.w < theta2 * near2 * (1.0 - 1e-12)) return 1;
+  if (g.w > theta2 * far2 * (1.0 + 1e-12)) return 2;
+  return 0;
+}
+
+constexpr int kWalk32Warps = 4;  // FP32 walk: warps per block
+
+__device__ __forceinline__ void add_counts(int lane, unsigned long long napprox,
+                                           unsigned long long ndirect, bool overflow,
+                                           unsigned long long *__restrict__ counters) {
   if (lane == 0) {
     if (napprox) atomicAdd(counters + 0, napprox);
     if (ndirect) atomicAdd(counters + 1, ndirect);
@@ -218,18 +184,468 @@ __global__ void __launch_bounds__(32 * kWalkWarps) bh_walk_kernel(
   }
 }
 
-__global__ void bh_to_fp32(int64_t ncells, const double4 *__restrict__ attr,
-                           float4 *__restrict__ attr32, int64_t n, const double *__restrict__ sx,
-                           const double *__restrict__ sy, const double *__restrict__ sz,
-                           const double *__restrict__ sm, float4 *__restrict__ pos32) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ncells + n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    if (i < ncells) {
-      const double4 a = attr[i];
-      attr32[i] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
-    } else {
-      const int64_t b = i - ncells;
-      pos32[b] = make_float4((float)sx[b], (float)sy[b], (float)sz[b], (float)sm[b]);
+// FP64: one walk per warp over the union of its 32 bodies' walks.  Opening a
+// cell classes its eight children by eight lanes with the bodies' box, tests
+// the uncertain ones body by body, and pushes each child with the lanes that
+// accept it and the lanes that open it (leaves with the lanes that reach them).
+// Popped depth first, children 0..7, the accepted cells and leaf bodies form a
+// list; entry k of the list is held by lane k (index and lane mask), and when
+// 32 are there their moments or bodies are loaded by a lane each and every lane
+// adds the terms of its own entries in list order.  A lane's entries in the list
+// are its own walk's, in its own walk's order, so it takes the sample's
+// decisions and sums the sample's terms in the sample's order, bit for bit.
+//
+// Why so: 32 bodies' union walk is long and small sets have few warps (20k
+// bodies: 625, one per scheduler), so the time is one warp's chain of dependent
+// loads and FP64 sequences; here a chain step serves eight cells, 32 loads or
+// four terms instead of one.  One warp per block, so that few warps spread
+// evenly over the SMs.  20k bodies, ncrit 1: 0.82 ms; 2.39 ms with one cell and
+// one term at a time, 1.68 ms without the box's tests.
+__global__ void __launch_bounds__(32) bh_walk64(
+    BhCells T, int64_t n, const double *__restrict__ sx, const double *__restrict__ sy,
+    const double *__restrict__ sz, const double *__restrict__ sm,
+    const double4 *__restrict__ attr, double theta, double eps2, double *__restrict__ out,
+    unsigned long long *__restrict__ counters) {
+  // stack entry: {cell, -first child, accepting lanes, opening lanes} or, a
+  // leaf, {first body, bodies, lanes, 0}
+  __shared__ int4 stack[kStack];
+  __shared__ double4 data[32];
+  const int lane = threadIdx.x;
+  const double theta2 = __dmul_rn(theta, theta);
+  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = b < n;
+  const double px = valid ? sx[b] : 0.0, py = valid ? sy[b] : 0.0, pz = valid ? sz[b] : 0.0;
+  double4 o = make_double4(0, 0, 0, 0);
+  unsigned long long napprox = 0, ndirect = 0;
+  bool overflow = false;
+  const unsigned lanes = __ballot_sync(0xffffffffu, valid);
+  if (lanes == 0) return;
+
+  const BodyBox box = body_box(valid, px, py, pz);
+
+  int count = 0;       // list entries
+  int idx = 0;         // this lane's entry: body, or ~cell
+  unsigned mask = 0;   // and the lanes that add it
+  auto flush = [&]() {
+    __syncwarp();
+    double4 v = make_double4(0, 0, 0, 0);
+    if (lane < count) v = idx >= 0 ? make_double4(sx[idx], sy[idx], sz[idx], sm[idx]) : attr[~idx];
+    else mask = 0;
+    data[lane] = v;
+    __syncwarp();
+#pragma unroll 1
+    for (int k = 0; k < count; k += 4) {
+      // ComputeForce (bh.cc:135-153), the sample's rounding order
+      double dx[4], dy[4], dz[4], w[4], R2[4], inv[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const double4 a = data[k + i];
+        dx[i] = __dsub_rn(a.x, px);
+        dy[i] = __dsub_rn(a.y, py);
+        dz[i] = __dsub_rn(a.z, pz);
+        w[i] = a.w;
+        R2[i] = __dadd_rn(__dmul_rn(dx[i], dx[i]), __dmul_rn(dy[i], dy[i]));
+        R2[i] = __dadd_rn(__dadd_rn(R2[i], __dmul_rn(dz[i], dz[i])), eps2);
+      }
+      rounded_inv_sqrt(R2, inv);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const bool mine = (__shfl_sync(0xffffffffu, mask, k + i) >> lane) & 1u;
+        const double inv3 = __dmul_rn(__dmul_rn(inv[i], inv[i]), inv[i]);
+        const double tx = __dmul_rn(__dmul_rn(dx[i], inv3), w[i]),
+                     ty = __dmul_rn(__dmul_rn(dy[i], inv3), w[i]),
+                     tz = __dmul_rn(__dmul_rn(dz[i], inv3), w[i]), tw = __dmul_rn(inv[i], w[i]);
+        if (mine) {
+          o.x = __dadd_rn(o.x, tx);
+          o.y = __dadd_rn(o.y, ty);
+          o.z = __dadd_rn(o.z, tz);
+          o.w = __dadd_rn(o.w, tw);
+        }
+      }
+    }
+    count = 0;
+  };
+
+  int sp = 1;
+  {
+    const int2 m = T.meta[0];
+    int4 e = make_int4(m.x, m.y, (int)lanes, 0);
+    if (m.y < 0) {
+      const bool acc = valid && bh_accept(T, 0, T.geo[0], px, py, pz, theta, theta2);
+      const unsigned am = __ballot_sync(0xffffffffu, acc);
+      e = make_int4(0, -m.x, (int)am, (int)(lanes & ~am));
+    }
+    if (lane == 0) stack[0] = e;
+    __syncwarp();
+  }
+  while (sp > 0) {
+    const int4 e = stack[--sp];
+    if (e.y >= 0) {  // a leaf's bodies
+      ndirect += (unsigned long long)e.y * __popc(e.z);
+      for (int done = 0; done < e.y;) {
+        const int take = min(32 - count, e.y - done), at = lane - count;
+        if (at >= 0 && at < take) {
+          idx = e.x + done + at;
+          mask = (unsigned)e.z;
+        }
+        done += take;
+        count += take;
+        if (count == 32) flush();
+      }
+      continue;
+    }
+    if (e.z) {
+      napprox += __popc(e.z);
+      if (lane == count) {
+        idx = ~e.x;
+        mask = (unsigned)e.z;
+      }
+      if (++count == 32) flush();
+    }
+    if (e.w) {
+      if (sp + 8 > kStack) {
+        overflow = true;
+        break;
+      }
+      const int ch = -e.y, c = ch + (lane & 7);
+      const int2 m = T.meta[c];
+      const double4 g = T.geo[c];
+      const int kind = m.y < 0 ? box_accept(box, g, theta2) : 3;  // 3: a leaf
+      // this lane's child (lanes 0..7): accepting and opening lanes
+      unsigned am = kind == 1 ? (unsigned)e.w : 0u, om = kind == 2 ? (unsigned)e.w : 0u;
+      unsigned todo = __ballot_sync(0xffffffffu, kind == 0) & 0xffu;
+      while (todo) {
+        const int i = __ffs(todo) - 1;
+        todo &= todo - 1;
+        double4 gi;
+        gi.x = __shfl_sync(0xffffffffu, g.x, i);
+        gi.y = __shfl_sync(0xffffffffu, g.y, i);
+        gi.z = __shfl_sync(0xffffffffu, g.z, i);
+        gi.w = __shfl_sync(0xffffffffu, g.w, i);
+        const bool acc = bh_accept(T, ch + i, gi, px, py, pz, theta, theta2);
+        const unsigned a = __ballot_sync(0xffffffffu, acc) & (unsigned)e.w;
+        if (lane == i) {
+          am = a;
+          om = (unsigned)e.w & ~a;
+        }
+      }
+      // every lane has read the popped entries (the ballots); child 7 at the bottom
+      const bool push = lane < 8 && m.y != 0;  // not an empty leaf
+      const unsigned pushes = __ballot_sync(0xffffffffu, push);
+      if (push)
+        stack[sp + __popc(pushes >> (lane + 1))] =
+            m.y > 0 ? make_int4(m.x, m.y, e.w, 0) : make_int4(c, -m.x, (int)am, (int)om);
+      sp += __popc(pushes);
+      __syncwarp();
+    }
+  }
+  if (!overflow) flush();
+  if (valid) reinterpret_cast<double4 *>(out)[b] = o;
+  add_counts(lane, napprox, ndirect, overflow, counters);
+}
+
+// 1/sqrt(x): the hardware approximation for x >= FLT_MIN (kNormal), else rsqrtf.
+template <bool kNormal>
+__device__ __forceinline__ float inv_sqrt32(float x) {
+  if (!kNormal) return rsqrtf(x);
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// FP32: the same union walk and decisions (the acceptance test stays FP64), but
+// a body's terms are added in any order (FP32 sums).  The stack holds opened
+// cells only.  Four of them are opened at a time, a lane per child: the bodies'
+// box decides for all bodies where it can, the uncertain children are tested
+// body by body; leaf children and accepted children go to two lists with the
+// lanes that add them.  32 listed leaves are evaluated as one stream of body
+// pairs, 32 pairs at a time loaded by a lane each into shared memory whatever
+// leaf they belong to, then added leaf by leaf by the lanes that reach it; 32
+// listed cells make 16 pairs with a mask per cell, 1/r replaced by 0 for the
+// lanes that do not accept it.
+// Leaf bodies are stored as pairs {x0,x1,y0,y1},{z0,z1,m0,m1}, each leaf starting
+// a pair (an odd leaf's last one is padded with a massless copy of its first
+// body), and a packed FP32 instruction evaluates two: 13 packed operations and 2
+// MUFU per pair.  Bound: FP32 pipe (62 %) and issue (62 %); the union holds 1.37
+// times the bodies' own leaf bodies (a simulated 400k Plummer sphere: 73 % of
+// the lanes add a listed body).  4M Plummer, ncrit 32: 35.3 ms; 66.5 ms with a
+// test per lane and cell and the leaves evaluated where they are met, from global
+// memory (4.4 slots per issue waiting for loads), 53.1 ms with the lists but a test
+// per lane and a mask per source.
+// kNormal: eps2 is a normal FP32 number, so no squared distance is below it.
+constexpr float kNowhere = 1.25e18f;  // coordinate of a padding source
+constexpr int kOpen = 4;              // cells opened at a time
+constexpr int kStack32 = 640;         // > 28 pending cells x 19 levels + 32
+
+struct __align__(16) Walk32Warp {
+  double4 geo[32];
+  float4 a[32], b[32];  // pairs of sources {x0,x1,y0,y1}, {z0,z1,m0,m1}
+  uint2 m[16];          // listed cells: the lanes that add either
+  int2 leaf[64];        // {first pair, pairs}
+  int cell[64];
+  unsigned leaf_m[64], cell_m[64];  // and the lanes that add them
+  int2 stack[kStack32];             // {first child, lanes that opened the cell}
+};
+
+template <bool kNormal>
+__global__ void __launch_bounds__(32 * kWalk32Warps, 6) bh_walk32(
+    BhCells T, int64_t n, const double *__restrict__ sx, const double *__restrict__ sy,
+    const double *__restrict__ sz, const float4 *__restrict__ attr32,
+    const float4 *__restrict__ pairs, double theta, float eps2, double *__restrict__ out,
+    unsigned long long *__restrict__ counters) {
+  __shared__ Walk32Warp warps[kWalk32Warps];
+  const int lane = threadIdx.x & 31;
+  Walk32Warp &S = warps[threadIdx.x >> 5];
+  const unsigned me = 1u << lane, below = me - 1;
+  const double theta2 = __dmul_rn(theta, theta);
+  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = b < n;
+  const double px = valid ? sx[b] : 0.0, py = valid ? sy[b] : 0.0, pz = valid ? sz[b] : 0.0;
+  const float fx = -(float)px, fy = -(float)py, fz = -(float)pz;
+  const float2 nx = make_float2(fx, fx), ny = make_float2(fy, fy), nz = make_float2(fz, fz);
+  const float2 e2 = make_float2(eps2, eps2);
+  float2 ox = make_float2(0.f, 0.f), oy = ox, oz = ox, ow = ox;
+  unsigned long long napprox = 0, ndirect = 0;  // this lane's cells' and leaves'
+  bool overflow = false;
+  const unsigned lanes = __ballot_sync(0xffffffffu, valid);
+  if (lanes == 0) return;
+  const BodyBox box = body_box(valid, px, py, pz);
+
+  // adds a pair of sources; a source whose flag is false adds nothing
+  auto add_pair = [&](const float4 &u, const float4 &v, bool t0, bool t1) {
+    const float2 dx = __fadd2_rn(make_float2(u.x, u.y), nx),
+                 dy = __fadd2_rn(make_float2(u.z, u.w), ny),
+                 dz = __fadd2_rn(make_float2(v.x, v.y), nz);
+    const float2 R2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+    const float i0 = inv_sqrt32<kNormal>(R2.x), i1 = inv_sqrt32<kNormal>(R2.y);
+    const float2 inv = make_float2(t0 ? i0 : 0.f, t1 ? i1 : 0.f);
+    const float2 wr = __fmul2_rn(make_float2(v.z, v.w), inv);
+    const float2 wr3 = __fmul2_rn(__fmul2_rn(wr, inv), inv);
+    ox = __ffma2_rn(dx, wr3, ox);
+    oy = __ffma2_rn(dy, wr3, oy);
+    oz = __ffma2_rn(dz, wr3, oz);
+    ow = __fadd2_rn(ow, wr);
+  };
+
+  int nleaf = 0, ncell = 0;  // listed
+  auto flush_leaves = [&]() {  // the last 32 listed, or all
+    __syncwarp();
+    const int base = max(0, nleaf - 32), cnt = nleaf - base;
+    int2 l = make_int2(0, 0);
+    unsigned lm = 0;
+    if (lane < cnt) {
+      l = S.leaf[base + lane];
+      lm = S.leaf_m[base + lane];
+    }
+    nleaf = base;
+    int upto = l.y;  // pairs of the leaves 0 .. lane
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, upto, 31);
+    const int first = l.x - (upto - l.y);  // pair i of the stream is pair first + i
+    int e = 0, at = 0;                     // the stream's next leaf and pair
+    for (int c0 = 0; c0 < total; c0 += 32) {
+      const int i = c0 + lane;
+      int k = 0;  // the first leaf with upto > i
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, upto, k + o - 1);
+        if (v <= i) k += o;
+      }
+      const int64_t p = __shfl_sync(0xffffffffu, first, k) + i;
+      if (i < total) {
+        S.a[lane] = __ldg(pairs + 2 * p);
+        S.b[lane] = __ldg(pairs + 2 * p + 1);
+      }
+      __syncwarp();
+      const int end = min(c0 + 32, total);
+      while (at < end) {
+        const int ue = __shfl_sync(0xffffffffu, upto, e);
+        const unsigned m = __shfl_sync(0xffffffffu, lm, e);
+        const int stop = min(ue, end);
+        if (m & me) {
+#pragma unroll 2
+          for (int q = at - c0; q < stop - c0; q++) add_pair(S.a[q], S.b[q], true, true);
+        }
+        at = stop;
+        if (at == ue) e++;
+      }
+      __syncwarp();
+    }
+  };
+  auto flush_cells = [&]() {  // the last 32 listed, or all
+    __syncwarp();
+    const int base = max(0, ncell - 32), cnt = ncell - base;
+    int cell = 0;
+    unsigned cm = 0, m = 0;
+    float4 c = make_float4(kNowhere, kNowhere, kNowhere, 0.f);
+    bool odd = false;
+    if (lane < cnt) {
+      cell = S.cell[base + lane];
+      cm = S.cell_m[base + lane];
+      const float4 v = attr32[cell];
+      // a centre that is not finite (no net mass) must reach its own lanes only
+      odd = !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) <= FLT_MAX);
+      if (!odd) {
+        c = v;
+        m = cm;
+      }
+    }
+    ncell = base;
+    const int half = lane & 1;
+    float *pa = reinterpret_cast<float *>(&S.a[lane >> 1]) + half;
+    float *pb = reinterpret_cast<float *>(&S.b[lane >> 1]) + half;
+    pa[0] = c.x;
+    pa[2] = c.y;
+    pb[0] = c.z;
+    pb[2] = c.w;
+    reinterpret_cast<unsigned *>(&S.m[lane >> 1])[half] = m;
+    __syncwarp();
+#pragma unroll 2
+    for (int k = 0; k < (cnt + 1) >> 1; k++) {
+      const uint2 w = S.m[k];
+      add_pair(S.a[k], S.b[k], (w.x & me) != 0, (w.y & me) != 0);
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, odd);
+    while (todo) {
+      const int k = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const float4 v = attr32[__shfl_sync(0xffffffffu, cell, k)];
+      if (__shfl_sync(0xffffffffu, cm, k) & me) {
+        const float dx = v.x + fx, dy = v.y + fy, dz = v.z + fz;
+        const float inv = inv_sqrt32<kNormal>(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2))));
+        const float wr = v.w * inv, wr3 = wr * inv * inv;
+        ox.x = fmaf(dx, wr3, ox.x);
+        oy.x = fmaf(dy, wr3, oy.x);
+        oz.x = fmaf(dz, wr3, oz.x);
+        ow.x += wr;
+      }
+    }
+    __syncwarp();
+  };
+
+  // A round classes this lane's cell c (if has), with record {m, g} and the lanes
+  // reach that opened its parent.
+  int sp = 0;
+  auto round = [&](bool has, int c, int2 m, const double4 &g, unsigned reach) {
+    const bool is_leaf = has && m.y > 0;
+    int kind = has && m.y < 0 ? box_accept(box, g, theta2) : 3;
+    unsigned todo = __ballot_sync(0xffffffffu, kind == 0);
+    if (kind == 0) S.geo[lane] = g;
+    const unsigned leaves = __ballot_sync(0xffffffffu, is_leaf);
+    if (is_leaf) {
+      const int k = nleaf + __popc(leaves & below);
+      S.leaf[k] = make_int2(m.x, (m.y + 1) >> 1);
+      S.leaf_m[k] = reach;
+      ndirect += (unsigned long long)m.y * __popc(reach);
+    }
+    nleaf += __popc(leaves);
+    __syncwarp();
+    unsigned am = kind == 1 ? reach : 0u, om = kind == 2 ? reach : 0u;
+    while (todo) {  // uncertain: every body's own test
+      const int i = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int ci = __shfl_sync(0xffffffffu, c, i);
+      const bool acc = bh_accept(T, ci, S.geo[i], px, py, pz, theta, theta2);
+      const unsigned a = __ballot_sync(0xffffffffu, acc);
+      if (lane == i) {
+        am = a & reach;
+        om = reach & ~a;
+      }
+    }
+    const unsigned accs = __ballot_sync(0xffffffffu, am != 0),
+                   opens = __ballot_sync(0xffffffffu, om != 0);
+    if (am) {
+      const int k = ncell + __popc(accs & below);
+      S.cell[k] = c;
+      S.cell_m[k] = am;
+      napprox += __popc(am);
+    }
+    ncell += __popc(accs);
+    if (om) S.stack[sp + __popc(opens & below)] = make_int2(m.x, (int)om);
+    sp += __popc(opens);
+    if (nleaf >= 32) flush_leaves();
+    if (ncell >= 32) flush_cells();
+    __syncwarp();
+  };
+  round(lane == 0, 0, T.meta[0], T.geo[0], lanes);
+  while (sp > 0) {
+    const int take = min(kOpen, sp);
+    sp -= take;
+    if (sp + 8 * kOpen > kStack32) {
+      overflow = true;
+      break;
+    }
+    const bool has = (lane >> 3) < take;
+    const int2 e = has ? S.stack[sp + (lane >> 3)] : make_int2(0, 0);
+    const int c = e.x + (lane & 7);
+    int2 m = make_int2(0, 0);
+    double4 g = make_double4(0, 0, 0, 0);
+    if (has) {
+      m = __ldg(T.meta + c);
+      g = T.geo[c];
+    }
+    __syncwarp();  // the popped entries are read
+    round(has, c, m, g, (unsigned)e.y);
+  }
+  while (nleaf) flush_leaves();
+  while (ncell) flush_cells();
+  if (valid)
+    reinterpret_cast<double4 *>(out)[b] =
+        make_double4((double)(ox.x + ox.y), (double)(oy.x + oy.y), (double)(oz.x + oz.y),
+                     (double)(ow.x + ow.y));
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    napprox += __shfl_xor_sync(0xffffffffu, napprox, s);
+    ndirect += __shfl_xor_sync(0xffffffffu, ndirect, s);
+  }
+  add_counts(lane, napprox, ndirect, overflow, counters);
+}
+
+// Body pairs of a leaf (0 for other cells), for the FP32 walk's pair offsets.
+__global__ void bh_pair_counts(int64_t ncells, const int32_t *__restrict__ cleaf,
+                               const int32_t *__restrict__ cnb, int32_t *__restrict__ cnt) {
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
+       c += (int64_t)gridDim.x * blockDim.x)
+    cnt[c] = cleaf[c] ? (cnb[c] + 1) >> 1 : 0;
+}
+
+// The walk's cell records; with pair_off (FP32 walk) also the FP32 moments and
+// the leaves' body pairs, eight threads per cell.
+__global__ void __launch_bounds__(256) bh_pack(
+    int64_t ncells, const int32_t *__restrict__ cleaf, const int32_t *__restrict__ cnb,
+    const int32_t *__restrict__ cbeg, const int32_t *__restrict__ cchild,
+    const double *__restrict__ cmin, const double *__restrict__ cmax,
+    const double *__restrict__ ccen, const double4 *__restrict__ attr,
+    const int32_t *__restrict__ pair_off, const double *__restrict__ sx,
+    const double *__restrict__ sy, const double *__restrict__ sz, const double *__restrict__ sm,
+    double4 *__restrict__ geo, int2 *__restrict__ meta, float4 *__restrict__ attr32,
+    float4 *__restrict__ pairs) {
+  const int sub = threadIdx.x & 7;
+  for (int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; c < ncells;
+       c += ((int64_t)gridDim.x * blockDim.x) >> 3) {
+    const bool is_leaf = cleaf[c] != 0;
+    const int nb = cnb[c], b0 = cbeg[c];
+    if (sub == 0) {
+      const double s = __dsub_rn(cmax[3 * c], cmin[3 * c]);
+      geo[c] = make_double4(ccen[3 * c], ccen[3 * c + 1], ccen[3 * c + 2], __dmul_rn(s, s));
+      meta[c] = is_leaf ? make_int2(pair_off ? pair_off[c] : b0, nb) : make_int2(cchild[c], -1);
+      if (pair_off) {
+        const double4 a = attr[c];
+        attr32[c] = make_float4((float)a.x, (float)a.y, (float)a.z, (float)a.w);
+      }
+    }
+    if (!pair_off || !is_leaf) continue;
+    for (int k = sub; k < (nb + 1) >> 1; k += 8) {
+      const int i = b0 + 2 * k;
+      const bool two = 2 * k + 1 < nb;
+      const int j = two ? i + 1 : b0;
+      float4 *o = pairs + 2 * ((int64_t)pair_off[c] + k);
+      o[0] = make_float4((float)sx[i], (float)sx[j], (float)sy[i], (float)sy[j]);
+      o[1] = make_float4((float)sz[i], (float)sz[j], (float)sm[i], two ? (float)sm[j] : 0.f);
     }
   }
 }
@@ -269,24 +685,37 @@ int bh_interact(tapas_b200_ctx *ctx, double theta, double eps2, int precision) {
   const int64_t n = ctx->n, C = ctx->ncells;
   TB_CUDA(ctx, ctx->counters.ensure(8, s));
   TB_CUDA(ctx, cudaMemsetAsync(ctx->counters.p, 0, 8 * sizeof(unsigned long long), s));
-  BhTree T{ctx->cleaf.p, ctx->cnb.p, ctx->cbeg.p, ctx->cchild.p, ctx->cmin.p, ctx->cmax.p,
-           ctx->ccen.p};
+  const bool fp64 = precision == TAPAS_B200_FP64;
+  TB_CUDA(ctx, ctx->trav_geo.ensure(C + 1, s));
+  TB_CUDA(ctx, ctx->trav_meta.ensure(C + 1, s));
   PhaseTimer t(ctx, &ctx->timings.p2p);
-  const int grid = (int)((n + 32 * kWalkWarps - 1) / (32 * kWalkWarps));
-  if (precision == TAPAS_B200_FP64) {
-    bh_walk_kernel<true><<<grid, 32 * kWalkWarps, 0, s>>>(T, n, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->sq.p,
-                                              ctx->bh_attr.p, nullptr, nullptr, theta, eps2,
-                                              ctx->trg.p, ctx->counters.p);
-  } else {
+  const int32_t *pair_off = nullptr;
+  if (!fp64) {
+    TB_CUDA(ctx, ctx->flag.ensure(C + 1, s));
+    TB_CUDA(ctx, ctx->flag_scan.ensure(C + 1, s));
     TB_CUDA(ctx, ctx->bh_attr32.ensure(C + 1, s));
-    TB_CUDA(ctx, ctx->rel4.ensure(n, s));
-    bh_to_fp32<<<grid_for(C + n, 256), 256, 0, s>>>(C, ctx->bh_attr.p, ctx->bh_attr32.p, n,
-                                                     ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->sq.p,
-                                                     ctx->rel4.p);
+    TB_CUDA(ctx, ctx->rel4.ensure(n + C + 2, s));  // two per pair, at most (n + leaves) / 2 pairs
+    bh_pair_counts<<<grid_for(C, 256), 256, 0, s>>>(C, ctx->cleaf.p, ctx->cnb.p, ctx->flag.p);
     TB_LAUNCH_CHECK(ctx);
-    bh_walk_kernel<false><<<grid, 32 * kWalkWarps, 0, s>>>(T, n, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->sq.p,
-                                               ctx->bh_attr.p, ctx->bh_attr32.p, ctx->rel4.p,
-                                               theta, eps2, ctx->trg.p, ctx->counters.p);
+    TB_TRY(scan_exclusive(ctx, ctx->flag.p, ctx->flag_scan.p, C, nullptr));
+    pair_off = ctx->flag_scan.p;
+  }
+  bh_pack<<<grid_for(8 * C, 256), 256, 0, s>>>(
+      C, ctx->cleaf.p, ctx->cnb.p, ctx->cbeg.p, ctx->cchild.p, ctx->cmin.p, ctx->cmax.p,
+      ctx->ccen.p, ctx->bh_attr.p, pair_off, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->sq.p,
+      ctx->trav_geo.p, ctx->trav_meta.p, ctx->bh_attr32.p, ctx->rel4.p);
+  TB_LAUNCH_CHECK(ctx);
+  const BhCells T{ctx->trav_geo.p, ctx->trav_meta.p, ctx->cmin.p, ctx->cmax.p, ctx->ccen.p};
+  if (fp64) {
+    bh_walk64<<<(unsigned)((n + 31) / 32), 32, 0, s>>>(T, n, ctx->sx.p, ctx->sy.p, ctx->sz.p,
+                                                       ctx->sq.p, ctx->bh_attr.p, theta, eps2,
+                                                       ctx->trg.p, ctx->counters.p);
+  } else {
+    constexpr int kThreads = 32 * kWalk32Warps;
+    auto walk = (float)eps2 >= FLT_MIN ? bh_walk32<true> : bh_walk32<false>;
+    walk<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(
+        T, n, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->bh_attr32.p, ctx->rel4.p, theta, (float)eps2,
+        ctx->trg.p, ctx->counters.p);
   }
   TB_LAUNCH_CHECK(ctx);
   unsigned long long *h = reinterpret_cast<unsigned long long *>(ctx->pinned.p);

@@ -56,3 +56,52 @@ def test_bh_fp32_and_accuracy(tb, ctx):
     ef = np.sqrt(np.sum((r64[tg, :3] - d[:, :3]) ** 2) / np.sum(d[:, :3] ** 2))
     ep = np.sqrt(np.sum((r64[tg, 3] - d[:, 3]) ** 2) / np.sum(d[:, 3] ** 2))
     assert ef < 1e-2 and ep < 1e-2
+
+
+@pytest.mark.parametrize("ncrit", [1, 3, 70])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 200, 3001])
+def test_bh_walk_edges(n, ncrit, tb, ctx, oracle_mod):
+    """Part-filled warps, a root that is a leaf, odd and even leaves, lists that
+    end part-filled: FP64 bit-exact with the oracle, the FP32 walk with the
+    same interaction counts and within its 1e-5 bar."""
+    x, y, z, m = tb.datasets.make("plummer", n, 83)
+    r = ctx.bh_evaluate(x, y, z, m, ncrit=ncrit, theta=0.6, eps2=1e-6, precision=tb.FP64)
+    ref, cnt = oracle_mod.barnes_hut(x, y, z, m, ncrit=ncrit, theta=0.6, eps2=1e-6)
+    np.testing.assert_array_equal(r, ref)
+    assert ctx.bh_counts() == (int(cnt[0]), int(cnt[1]))
+    r32 = ctx.bh_evaluate(x, y, z, m, ncrit=ncrit, theta=0.6, eps2=1e-6, precision=tb.MIXED)
+    assert ctx.bh_counts() == (int(cnt[0]), int(cnt[1]))
+    num, den = np.linalg.norm(r32 - r, axis=0), np.linalg.norm(r, axis=0)
+    assert np.all(num <= 1e-5 * den)
+
+
+@pytest.mark.parametrize("eps2", [1e-40, 0.0])
+def test_bh_walk_softening_below_fp32(eps2, tb, ctx, oracle_mod):
+    """A softening that is no normal FP32 number: every body meets itself at
+    that distance, so the accelerations' and potentials' finiteness follows
+    1/sqrt(eps2) in either precision (zero: not finite)."""
+    x, y, z, m = tb.datasets.make("uniform_cube", 500, 84)
+    r = ctx.bh_evaluate(x, y, z, m, ncrit=4, theta=0.5, eps2=eps2, precision=tb.FP64)
+    ref, _ = oracle_mod.barnes_hut(x, y, z, m, ncrit=4, theta=0.5, eps2=eps2)
+    np.testing.assert_array_equal(r, ref)
+    r32 = ctx.bh_evaluate(x, y, z, m, ncrit=4, theta=0.5, eps2=eps2, precision=tb.MIXED)
+    if eps2 > 0:  # 1/sqrt(1e-40) = 1e20 is an FP32 number, and dominates the potential
+        ok = np.isfinite(r32[:, 3])
+        assert ok.all()
+        assert np.linalg.norm(r32[:, 3] - r[:, 3]) <= 1e-5 * np.linalg.norm(r[:, 3])
+    else:
+        assert not np.isfinite(r32[:, :3]).any()
+
+
+def test_bh_massless_cells(tb, ctx, oracle_mod):
+    """A far cluster without mass has no centre (0/0): the bodies that accept one
+    of its cells get NaN, as in the sample; all others stay finite, in both
+    precisions (an FP32 lane must not feel a cell that only its neighbours
+    accept)."""
+    x, y, z, m = [a.copy() for a in tb.datasets.make("uniform_cube", 3000, 85)]
+    m[(x > 0.2) & (x < 0.5) & (y > 0)] = 0.0
+    r = ctx.bh_evaluate(x, y, z, m, ncrit=4, theta=0.3, eps2=1e-6, precision=tb.FP64)
+    ref, _ = oracle_mod.barnes_hut(x, y, z, m, ncrit=4, theta=0.3, eps2=1e-6)
+    np.testing.assert_array_equal(r, ref)
+    r32 = ctx.bh_evaluate(x, y, z, m, ncrit=4, theta=0.3, eps2=1e-6, precision=tb.MIXED)
+    assert np.array_equal(np.isnan(r32), np.isnan(r))
