@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <string>
@@ -55,8 +56,8 @@ struct DBuf {
   // Ensures room for n elements; contents are NOT preserved unless keep.
   cudaError_t ensure(size_t n, cudaStream_t s, bool keep = false, size_t used = 0) {
     if (n <= cap) return cudaSuccess;
-    size_t nc = cap ? cap : 1024;
-    while (nc < n) nc += nc / 2 + 1024;
+    // a half more than before, or an eighth more than needed
+    const size_t nc = std::max(cap + cap / 2, n + n / 8) + 1024;
     T *q = nullptr;
     cudaError_t e = cudaMalloc(&q, nc * sizeof(T));
     if (e != cudaSuccess) return e;
@@ -186,7 +187,8 @@ struct tapas_b200_ctx {
   tb::DBuf<double> cmin, cmax, ccen;    // 3 doubles per cell (x,y,z interleaved)
   tb::DBuf<double4> trav_geo;          // traversal: per cell {centre, MAC radius for this theta}
   tb::DBuf<int2> trav_meta;            // traversal: per cell {nb, first child or -1 for a leaf}
-  tb::DBuf<int32_t> flag, flag_scan;    // per-level scratch
+  tb::DBuf<int2> tree_nodes;            // per non-leaf cell {first body, cell}
+  tb::DBuf<int32_t> flag, flag_scan;    // per-cell scratch
   tb::DBuf<int32_t> leaf_list;          // indices of non-empty leaves
   // mixed L2P, body-parallel: per evaluated leaf its FP32 local expansion and
   // (centre, width); per body its leaf's ordinal (-1: not evaluated here)
@@ -218,6 +220,7 @@ struct tapas_b200_ctx {
   int mutual = 0;                       // lists of the last build_lists came from a mutual traversal
   uint64_t n_p2p_int = 0;
   int trav_iters = 0;
+  int trav_blocks = 0;     // blocks of the traversal kernel the GPU holds at once
   int64_t trav_pairs = 0;  // (target, source) pairs the traversal classified
   int list_shift = 1;                   // packed list key = target << shift | source
   bool reference_lists = false;         // keep pairs with empty cells, as the reference visits them

@@ -374,6 +374,12 @@ size_t scatter_smem_bytes() {
 
 }  // namespace
 
+int scan_rows(tapas_b200_ctx *ctx, uint32_t *rows, int nrows, int ncols, uint32_t *totals) {
+  radix_scan_rows<<<nrows, 1024, 0, ctx->stream>>>(rows, ncols, totals);
+  TB_LAUNCH_CHECK(ctx);
+  return TAPAS_B200_OK;
+}
+
 int radix_sort(tapas_b200_ctx *ctx, uint64_t *&keys, uint64_t *&keys_alt, uint32_t *&vals,
                uint32_t *&vals_alt, int64_t n, int begin_bit, int end_bit) {
   if (n <= 1) return TAPAS_B200_OK;

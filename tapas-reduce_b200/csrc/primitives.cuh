@@ -8,6 +8,9 @@ namespace tb {
 int scan_exclusive(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
                    int32_t *d_total);
 
+// Exclusive scan of each row of rows[nrows][ncols] in place; totals[row] = its sum.
+int scan_rows(tapas_b200_ctx *ctx, uint32_t *rows, int nrows, int ncols, uint32_t *totals);
+
 // Stable LSD radix sort on key bits [begin_bit, end_bit).  Keys (and values,
 // if vals is non-null) are sorted between the two buffers; on return `keys`
 // and `vals` point at the sorted data (the pointers are swapped per pass).

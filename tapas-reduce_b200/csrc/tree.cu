@@ -1,5 +1,5 @@
 // Octree construction on the GPU: bounding cube, Morton keys, key sort, body
-// permutation and the level-by-level cell build.
+// permutation and the cell build.
 //
 // Follows cpp/include/tapas/hot/buildtree.h (SamplingOctree) on one rank:
 //  - bbox_*:        the constructor's box, :72-87, including its scalar
@@ -8,10 +8,11 @@
 //                   sfc_morton.h:387-402.
 //  - radix sort:    SortByKeys, common.h:249-273 (stable here; the reference's
 //                   std::sort leaves equal keys in unspecified order).
-//  - build_level:   GenerateCell, :388-459: a cell's bodies are the sorted
-//                   range [lower_bound(k), lower_bound(GetNext(k))); it is a
-//                   leaf iff nb <= ncrit; non-leaves get all 8 children.  Cells
-//                   are stored breadth first, level after level.
+//  - count_nonleaves, list_nonleaves, build_children: GenerateCell, :388-459: a
+//                   cell's bodies are the sorted range [lower_bound(k),
+//                   lower_bound(GetNext(k))); it is a leaf iff nb <= ncrit;
+//                   non-leaves get all 8 children.  Cells are stored breadth
+//                   first, level after level; all levels are built at once.
 // Layout in HBM: bodies SoA FP64 (x,y,z,q) in input and sorted order; keys
 // u64; cells SoA (key, range, parent, first child, leaf, 3x min/max/center).
 #include <algorithm>
@@ -66,13 +67,27 @@ __global__ void __launch_bounds__(kBlock) bbox_partial(const double *__restrict_
   }
 }
 
-__global__ void bbox_final(const double *__restrict__ part, int nparts, double *__restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double lo = part[0], hi = part[1];
-    for (int i = 1; i < nparts; i++) {
-      lo = fmin(lo, part[2 * i]);
-      hi = fmax(hi, part[2 * i + 1]);
-    }
+// The box over the blocks' boxes, one block (a single thread's chain of loads
+// took 28 us for 400 boxes).
+__global__ void __launch_bounds__(kBlock) bbox_final(const double *__restrict__ part, int nparts,
+                                                     double *__restrict__ out) {
+  double lo = part[0], hi = part[1];
+  for (int i = threadIdx.x; i < nparts; i += kBlock) {
+    lo = fmin(lo, part[2 * i]);
+    hi = fmax(hi, part[2 * i + 1]);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  __shared__ double sl[kBlock / 32], sh[kBlock / 32];
+  if ((threadIdx.x & 31) == 0) {
+    sl[threadIdx.x >> 5] = lo;
+    sh[threadIdx.x >> 5] = hi;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kBlock / 32; w++) { lo = fmin(lo, sl[w]); hi = fmax(hi, sh[w]); }
     out[0] = lo;
     out[1] = hi;
   }
@@ -148,12 +163,125 @@ __global__ void init_root(int64_t n, int ncrit, const double *__restrict__ box,
   }
 }
 
-// split flag of each cell of a level
-__global__ void level_flags(const int32_t *__restrict__ cleaf, int64_t a, int64_t cnt,
-                            int32_t *__restrict__ flag) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
-       i += (int64_t)gridDim.x * blockDim.x)
-    flag[i] = cleaf[a + i] ? 0 : 1;
+// ---------------------------------------------------------------------------
+// Cells of all levels at once.  With the keys sorted, body i begins a cell of
+// every level below the one it shares with body i - 1, and that cell holds more
+// than ncrit bodies iff body i + ncrit is still in it, so the non-leaf cells
+// body i begins are those of levels a + 1 .. b, a and b being the levels i
+// shares with i - 1 and with i + ncrit (at most kMaxDepth - 1: cells of the
+// deepest level are leaves).  Counting them per level and tile of bodies, a
+// scan and one read-back give every level's size; each non-leaf cell's rank in
+// its level is its order by first body, and its eight children are the cells
+// 1 + 8q .. 8 + 8q for its rank q over all levels, level after level.  (Level by
+// level, every level cost six launches and a host round trip: 20k bodies at
+// ncrit 1, 18 levels, 0.67 ms.)
+// ---------------------------------------------------------------------------
+constexpr int kTreeSteps = 8;                       // bodies per thread
+constexpr int kTreeTile = kBlock * kTreeSteps;      // bodies per block
+constexpr int kTreeLevels = kMaxDepth;              // levels that can have non-leaf cells
+
+// Levels two body keys share: 0 (the root only) .. kMaxDepth (equal keys).
+__device__ __forceinline__ int shared_levels(uint64_t x, uint64_t y) {
+  const uint64_t v = (x ^ y) >> kDepthBits;
+  if (v == 0) return kMaxDepth;
+  return (3 * kMaxDepth - 1 - (63 - __clzll((long long)v))) / 3;
+}
+
+// Levels (a, b] of the non-leaf cells that body i begins (none if a >= b).
+__device__ __forceinline__ void begun_levels(const uint64_t *__restrict__ keys, int64_t n,
+                                             int ncrit, int64_t i, int &a, int &b) {
+  a = 0;
+  b = -1;
+  if (i >= n || i + ncrit >= n) return;
+  const uint64_t k = keys[i];
+  b = min(shared_levels(k, keys[i + ncrit]), kMaxDepth - 1);
+  a = i == 0 ? -1 : shared_levels(keys[i - 1], k);
+}
+
+// Calls f(level, lanes that begin a non-leaf cell there) for the levels any of
+// the warp's 32 bodies begins one at.
+template <class F>
+__device__ __forceinline__ void each_begun_level(int a, int b, F f) {
+  if (!__any_sync(0xffffffffu, a < b)) return;
+  const int lo = __reduce_min_sync(0xffffffffu, a < b ? a + 1 : kMaxDepth),
+            hi = __reduce_max_sync(0xffffffffu, a < b ? b : -1);
+  for (int l = lo; l <= hi; l++) f(l, __ballot_sync(0xffffffffu, a < l && l <= b));
+}
+
+// Non-leaf cells begun per level (row) and tile (column).
+__global__ void __launch_bounds__(kBlock) count_nonleaves(const uint64_t *__restrict__ keys,
+                                                          int64_t n, int ncrit, int ntiles,
+                                                          uint32_t *__restrict__ cnt) {
+  __shared__ uint32_t tot[kTreeLevels];
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < kTreeLevels) tot[threadIdx.x] = 0;
+  __syncthreads();
+  uint32_t mine = 0;  // lane l: level l's
+  const int64_t base = (int64_t)blockIdx.x * kTreeTile + (threadIdx.x >> 5) * (32 * kTreeSteps);
+  for (int s = 0; s < kTreeSteps; s++) {
+    int a, b;
+    begun_levels(keys, n, ncrit, base + 32 * s + lane, a, b);
+    each_begun_level(a, b, [&](int l, unsigned m) {
+      if (lane == l) mine += __popc(m);
+    });
+  }
+  if (lane < kTreeLevels && mine) atomicAdd(&tot[lane], mine);
+  __syncthreads();
+  if (threadIdx.x < kTreeLevels) cnt[(size_t)threadIdx.x * ntiles + blockIdx.x] = tot[threadIdx.x];
+}
+
+// First rank (over all levels) of the non-leaf cells of each level.
+struct LevelRanks {
+  int32_t first[kTreeLevels + 1];
+};
+
+// node[q] = {first body, cell} of the non-leaf cell of rank q.
+__global__ void __launch_bounds__(kBlock) list_nonleaves(const uint64_t *__restrict__ keys,
+                                                         int64_t n, int ncrit, int ntiles,
+                                                         const uint32_t *__restrict__ before,
+                                                         LevelRanks ranks,
+                                                         int2 *__restrict__ node) {
+  __shared__ uint32_t warp_cnt[kBlock / 32][kTreeLevels];
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int64_t base = (int64_t)blockIdx.x * kTreeTile + wi * (32 * kTreeSteps);
+  int a[kTreeSteps], b[kTreeSteps];
+  uint32_t mine = 0;
+#pragma unroll
+  for (int s = 0; s < kTreeSteps; s++) {
+    begun_levels(keys, n, ncrit, base + 32 * s + lane, a[s], b[s]);
+    each_begun_level(a[s], b[s], [&](int l, unsigned m) {
+      if (lane == l) mine += __popc(m);
+    });
+  }
+  if (lane < kTreeLevels) warp_cnt[wi][lane] = mine;
+  __syncthreads();
+  // lane l: non-leaf cells of level l begun before this warp's next body
+  uint32_t run = 0;
+  if (lane < kTreeLevels) {
+    run = before[(size_t)lane * ntiles + blockIdx.x];
+    for (int w = 0; w < wi; w++) run += warp_cnt[w][lane];
+  }
+#pragma unroll
+  for (int s = 0; s < kTreeSteps; s++) {
+    const int64_t i = base + 32 * s + lane;
+    // upto: cells of the level above begun by bodies 0 .. i
+    int upto = 0, prev = -2;
+    each_begun_level(a[s], b[s], [&](int l, unsigned m) {
+      if (l != prev + 1 && l > 0) upto = (int)__shfl_sync(0xffffffffu, run, l - 1);
+      prev = l;
+      const int incl = (int)__shfl_sync(0xffffffffu, run, l) + __popc(m & ((2u << lane) - 1));
+      if ((m >> lane) & 1u) {
+        int cell = 0;
+        if (l > 0) {
+          const int oct = (int)(keys[i] >> (kDepthBits + 3 * (kMaxDepth - l))) & 7;
+          cell = 1 + 8 * (ranks.first[l - 1] + upto - 1) + oct;
+        }
+        node[ranks.first[l] + incl - 1] = make_int2((int)i, cell);
+      }
+      upto = incl;
+      if (lane == l) run += __popc(m);
+    });
+  }
 }
 
 __device__ __forceinline__ int64_t lower_bound_u64(const uint64_t *__restrict__ a, int64_t lo,
@@ -165,49 +293,67 @@ __device__ __forceinline__ int64_t lower_bound_u64(const uint64_t *__restrict__ 
   return lo;
 }
 
-// One thread per child of the non-leaf cells of level [a, a+cnt).
+// One thread per child of the non-leaf cells (rank q, octant o: cell 1 + 8q + o).
 __global__ void __launch_bounds__(kBlock) build_children(
-    int64_t a, int64_t cnt, int64_t child_base, const int32_t *__restrict__ flag,
-    const int32_t *__restrict__ flag_scan, const uint64_t *__restrict__ keys, int ncrit,
+    int64_t nnode, LevelRanks ranks, const int2 *__restrict__ node,
+    const uint64_t *__restrict__ keys, int64_t n, int ncrit, const double *__restrict__ box,
     uint64_t *__restrict__ ckey, int32_t *__restrict__ cbeg, int32_t *__restrict__ cnb,
     int32_t *__restrict__ cparent, int32_t *__restrict__ cchild, int32_t *__restrict__ cleaf,
     int32_t *__restrict__ clevel, double *__restrict__ cmin, double *__restrict__ cmax,
     double *__restrict__ ccen) {
-  const int64_t total = cnt * 8;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t li = t >> 3;   // cell within the level
-    const int ci = (int)(t & 7);
-    if (!flag[li]) continue;
-    const int64_t p = a + li;
-    const int64_t c = child_base + 8 * (int64_t)flag_scan[li] + ci;
-    if (ci == 0) cchild[p] = (int32_t)c;
-    const uint64_t pk = ckey[p];
-    const uint64_t k = key_child(pk, ci);
-    const int64_t pb = cbeg[p], pe = pb + cnb[p];
-    const int64_t rb = lower_bound_u64(keys, pb, pe, k);
-    const int64_t re = lower_bound_u64(keys, rb, pe, key_next(k));
-    const int nb = (int)(re - rb);
-    const int depth = key_depth(k);
+  const int64_t total = 8 * nnode, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); t0 < total;
+       t0 += stride) {  // warp-uniform: the lanes of a node exchange their bounds
+    const int64_t t = t0 + (threadIdx.x & 31);
+    const bool in = t < total;
+    const int64_t q = in ? t >> 3 : 0;
+    const int o = (int)(t & 7);
+    const int2 nd = node[q];
+    int level = 0;  // of the parent
+    while (q >= ranks.first[level + 1]) level++;
+    const int shift = kDepthBits + 3 * (kMaxDepth - level);
+    const uint64_t pk = (keys[nd.x] >> shift << shift) | (uint64_t)level;
+    const uint64_t k = key_child(pk, o);
+    // this child's end: the first body of the next one, or beyond the parent
+    const uint64_t next = o < 7 ? key_child(pk, o + 1) : key_next(pk);
+    int64_t lo = nd.x, hi = lo + ncrit + 1;  // the parent holds more than ncrit bodies
+    while (hi < n && keys[hi] < next) {
+      const int64_t w = hi - lo;
+      lo = hi;
+      hi += 2 * w;
+    }
+    const int64_t re = lower_bound_u64(keys, lo, min(hi, n), next);
+    const int64_t rprev = __shfl_up_sync(0xffffffffu, re, 1, 8);
+    const int64_t rb = o == 0 ? nd.x : rprev;
+    if (!in) continue;
+    const int64_t c = 1 + t;
+    if (o == 0) cchild[nd.y] = (int32_t)c;
+    const int nb = (int)(re - rb), depth = level + 1;
+    // Leaf iff nb <= ncrit.  Cells at the deepest key level are leaves too:
+    // the reference's child-key shift is undefined there.
+    const bool leaf = nb <= ncrit || depth >= kMaxDepth;
     ckey[c] = k;
     cbeg[c] = (int32_t)rb;
     cnb[c] = nb;
-    cparent[c] = (int32_t)p;
-    cchild[c] = -1;
-    // Leaf iff nb <= ncrit.  Cells at the deepest key level are leaves too:
-    // the reference's child-key shift is undefined there.
-    cleaf[c] = (nb <= ncrit || depth >= kMaxDepth) ? 1 : 0;
+    cparent[c] = nd.y;
+    if (leaf) cchild[c] = -1;  // else its own children's thread writes it
+    cleaf[c] = leaf ? 1 : 0;
     clevel[c] = depth;
-    // Region: parent's box halved once (CalcRegion, sfc_morton.h:536-557).
+    // Region: the root's box halved once per level (CalcRegion, sfc_morton.h:536-557).
+    double mn[3] = {box[0], box[0], box[0]}, mx[3] = {box[1], box[1], box[1]};
+    for (int l = 1; l <= depth; l++) {
+      const int ci = (int)(k >> (kDepthBits + 3 * (kMaxDepth - l))) & 7;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const double mid = dadd(mx[d], mn[d]) / 2;
+        if ((ci >> d) & 1) mn[d] = mid; else mx[d] = mid;
+      }
+    }
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      const double mn = cmin[3 * p + d], mx = cmax[3 * p + d];
-      const double mid = dadd(mx, mn) / 2;
-      double lo, hi;
-      if ((ci >> d) & 1) { lo = mid; hi = mx; } else { lo = mn; hi = mid; }
-      cmin[3 * c + d] = lo;
-      cmax[3 * c + d] = hi;
-      ccen[3 * c + d] = dadd(hi, lo) / 2;
+      cmin[3 * c + d] = mn[d];
+      cmax[3 * c + d] = mx[d];
+      ccen[3 * c + d] = dadd(mx[d], mn[d]) / 2;
     }
   }
 }
@@ -264,19 +410,18 @@ int leaf_depth_histogram(tapas_b200_ctx *ctx, int nbins, int64_t *out) {
   return TAPAS_B200_OK;
 }
 
-int ensure_cells(tapas_b200_ctx *ctx, int64_t need, int64_t used) {
+int ensure_cells(tapas_b200_ctx *ctx, int64_t need) {
   cudaStream_t s = ctx->stream;
-  if ((size_t)need <= ctx->ckey.cap) return TAPAS_B200_OK;
-  TB_CUDA(ctx, ctx->ckey.ensure(need, s, true, used));
-  TB_CUDA(ctx, ctx->cbeg.ensure(need, s, true, used));
-  TB_CUDA(ctx, ctx->cnb.ensure(need, s, true, used));
-  TB_CUDA(ctx, ctx->cparent.ensure(need, s, true, used));
-  TB_CUDA(ctx, ctx->cchild.ensure(need, s, true, used));
-  TB_CUDA(ctx, ctx->cleaf.ensure(need, s, true, used));
-  TB_CUDA(ctx, ctx->clevel.ensure(need, s, true, used));
-  TB_CUDA(ctx, ctx->cmin.ensure(3 * need, s, true, 3 * used));
-  TB_CUDA(ctx, ctx->cmax.ensure(3 * need, s, true, 3 * used));
-  TB_CUDA(ctx, ctx->ccen.ensure(3 * need, s, true, 3 * used));
+  TB_CUDA(ctx, ctx->ckey.ensure(need, s));
+  TB_CUDA(ctx, ctx->cbeg.ensure(need, s));
+  TB_CUDA(ctx, ctx->cnb.ensure(need, s));
+  TB_CUDA(ctx, ctx->cparent.ensure(need, s));
+  TB_CUDA(ctx, ctx->cchild.ensure(need, s));
+  TB_CUDA(ctx, ctx->cleaf.ensure(need, s));
+  TB_CUDA(ctx, ctx->clevel.ensure(need, s));
+  TB_CUDA(ctx, ctx->cmin.ensure(3 * need, s));
+  TB_CUDA(ctx, ctx->cmax.ensure(3 * need, s));
+  TB_CUDA(ctx, ctx->ccen.ensure(3 * need, s));
   return TAPAS_B200_OK;
 }
 
@@ -308,7 +453,7 @@ int build_tree(tapas_b200_ctx *ctx, int ncrit) {
     TB_CUDA(ctx, ctx->scratch_d.ensure(2 * nparts + 2, s));
     bbox_partial<<<nparts, kBlock, 0, s>>>(ctx->x.p, ctx->y.p, ctx->z.p, n, ctx->scratch_d.p);
     TB_LAUNCH_CHECK(ctx);
-    bbox_final<<<1, 32, 0, s>>>(ctx->scratch_d.p, nparts, ctx->bbox.p);
+    bbox_final<<<1, kBlock, 0, s>>>(ctx->scratch_d.p, nparts, ctx->bbox.p);
     TB_LAUNCH_CHECK(ctx);
     keys_kernel<<<grid_for(n, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
         ctx->x.p, ctx->y.p, ctx->z.p, ctx->q_pending ? nullptr : ctx->q.p, n, ctx->bbox.p,
@@ -335,49 +480,53 @@ int build_tree(tapas_b200_ctx *ctx, int ncrit) {
     TB_LAUNCH_CHECK(ctx);
   }
   PhaseTimer t(ctx, &ctx->timings.tree);
-  // Level-by-level build.  Estimate capacity: ~ 8/7 * 8 * n / ncrit cells.
-  int64_t est = 64 + (int64_t)(2.5 * 8.0 * (double)n / (double)std::max(ncrit, 1));
-  TB_TRY(ensure_cells(ctx, est, 0));
-  TB_CUDA(ctx, ctx->pinned.ensure(64));
+  const int ntiles = (int)((n + kTreeTile - 1) / kTreeTile);
+  TB_CUDA(ctx, ctx->sort_hist.ensure((size_t)kTreeLevels * (ntiles + 1), s));
+  uint32_t *cnt = ctx->sort_hist.p, *d_total = cnt + (size_t)kTreeLevels * ntiles;
+  TB_CUDA(ctx, ctx->pinned.ensure(256));
+  count_nonleaves<<<ntiles, kBlock, 0, s>>>(ctx->keys.p, n, ncrit, ntiles, cnt);
+  TB_LAUNCH_CHECK(ctx);
+  TB_TRY(scan_rows(ctx, cnt, kTreeLevels, ntiles, d_total));
+  uint32_t *h_total = reinterpret_cast<uint32_t *>(ctx->pinned.p);
+  TB_CUDA(ctx, cudaMemcpyAsync(h_total, d_total, kTreeLevels * sizeof(uint32_t),
+                               cudaMemcpyDeviceToHost, s));
+  TB_CUDA(ctx, cudaStreamSynchronize(s));
+  LevelRanks ranks;
+  int64_t nnode = 0;
+  int depth = 0;
+  ctx->level_off.assign(1, 0);
+  ctx->level_off.push_back(1);
+  for (int l = 0; l < kTreeLevels; l++) {
+    ranks.first[l] = (int32_t)nnode;
+    nnode += h_total[l];
+    if (nnode > (int64_t)0x0FFFFFFF) {
+      set_error(ctx, "tree build: more than 2^31 cells");
+      return TAPAS_B200_ERR_CAPACITY;
+    }
+    if (h_total[l]) {
+      depth = l + 1;
+      ctx->level_off.push_back(1 + 8 * nnode);
+    }
+  }
+  ranks.first[kTreeLevels] = (int32_t)nnode;
+  ctx->ncells = 1 + 8 * nnode;
+  ctx->max_depth = depth;
+  TB_TRY(ensure_cells(ctx, ctx->ncells));
   init_root<<<1, 32, 0, s>>>(n, ncrit, ctx->bbox.p, ctx->ckey.p, ctx->cbeg.p, ctx->cnb.p,
                              ctx->cparent.p, ctx->cchild.p, ctx->cleaf.p, ctx->clevel.p,
                              ctx->cmin.p, ctx->cmax.p, ctx->ccen.p);
   TB_LAUNCH_CHECK(ctx);
-  ctx->level_off.assign(1, 0);
-  ctx->level_off.push_back(1);
-  int64_t a = 0, cnt = 1;
-  int depth = 0;
-  int32_t *h_total = reinterpret_cast<int32_t *>(ctx->pinned.p);
-  while (true) {
-    TB_CUDA(ctx, ctx->flag.ensure(cnt + 1, s));
-    TB_CUDA(ctx, ctx->flag_scan.ensure(cnt + 1, s));
-    level_flags<<<grid_for(cnt, kBlock), kBlock, 0, s>>>(ctx->cleaf.p, a, cnt, ctx->flag.p);
+  if (nnode > 0) {
+    TB_CUDA(ctx, ctx->tree_nodes.ensure(nnode, s));
+    list_nonleaves<<<ntiles, kBlock, 0, s>>>(ctx->keys.p, n, ncrit, ntiles, cnt, ranks,
+                                             ctx->tree_nodes.p);
     TB_LAUNCH_CHECK(ctx);
-    TB_TRY(scan_exclusive(ctx, ctx->flag.p, ctx->flag_scan.p, cnt, ctx->flag_scan.p + cnt));
-    TB_CUDA(ctx, cudaMemcpyAsync(h_total, ctx->flag_scan.p + cnt, sizeof(int32_t),
-                                 cudaMemcpyDeviceToHost, s));
-    TB_CUDA(ctx, cudaStreamSynchronize(s));
-    const int64_t nsplit = *h_total;
-    if (nsplit == 0) break;
-    const int64_t child_base = a + cnt;
-    const int64_t nchild = 8 * nsplit;
-    TB_TRY(ensure_cells(ctx, child_base + nchild, child_base));
-    build_children<<<grid_for(cnt * 8, kBlock, ctx->num_sms * 32), kBlock, 0, s>>>(
-        a, cnt, child_base, ctx->flag.p, ctx->flag_scan.p, ctx->keys.p, ncrit, ctx->ckey.p,
+    build_children<<<grid_for(8 * nnode, kBlock, ctx->num_sms * 32), kBlock, 0, s>>>(
+        nnode, ranks, ctx->tree_nodes.p, ctx->keys.p, n, ncrit, ctx->bbox.p, ctx->ckey.p,
         ctx->cbeg.p, ctx->cnb.p, ctx->cparent.p, ctx->cchild.p, ctx->cleaf.p, ctx->clevel.p,
         ctx->cmin.p, ctx->cmax.p, ctx->ccen.p);
     TB_LAUNCH_CHECK(ctx);
-    a = child_base;
-    cnt = nchild;
-    depth++;
-    ctx->level_off.push_back(a + cnt);
-    if (depth > kMaxDepth) {
-      set_error(ctx, "tree build exceeded the maximum key depth");
-      return TAPAS_B200_ERR_CAPACITY;
-    }
   }
-  ctx->ncells = a + cnt;
-  ctx->max_depth = depth;
   // Non-empty leaves (the P2M / L2P / P2P work units).
   const int64_t C = ctx->ncells;
   TB_CUDA(ctx, ctx->flag.ensure(C + 1, s));
