@@ -26,6 +26,8 @@
 // every decision matches the reference bit for bit; the lists are therefore
 // equal as sets.  They are then sorted by (target, source) so the evaluation
 // order, and so every result, is deterministic.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "primitives.cuh"
@@ -44,6 +46,23 @@ struct TravCells {
   const int2 *meta;
 };
 
+// State of a traversal, in device memory; the host reads it once at the end.
+struct TravState {
+  // sizes at the start of the step `cur`: frontier (in buffer cur & 1), lists
+  unsigned long long nfront, m2l, p2p;
+  unsigned long long inter;    // P2P body pairs of the finished steps
+  unsigned long long visited;  // pairs classified in them
+  int steps;                   // finished steps
+  int stop;                    // 1: a buffer was too small for step `steps`
+  // what that step reserved, for the host to size the buffers by
+  unsigned long long need_front, need_m2l, need_p2p;
+  // reservations: step k uses set k % 3 and clears the next step's, whose last
+  // readers (step k - 2) are behind the barrier before step k
+  unsigned long long cnt[3][4];  // next frontier, M2L, P2P, body pairs
+};
+constexpr int kTravStateAt = 16;  // in ctx->counters
+static_assert(sizeof(TravState) <= (64 - kTravStateAt) * sizeof(unsigned long long), "counters");
+
 // The traversal's cell records for this theta, with the reference's
 // operations in its order for R (max over the widths, halve, * 1.00001,
 // / theta), computed once per traversal instead of twice per visited pair.
@@ -51,7 +70,13 @@ __global__ void trav_cells(int64_t ncells, const double *__restrict__ mn,
                            const double *__restrict__ mx, const double *__restrict__ cen,
                            const int32_t *__restrict__ nb, const int32_t *__restrict__ leaf,
                            const int32_t *__restrict__ child, double theta,
-                           double4 *__restrict__ geo, int2 *__restrict__ meta) {
+                           double4 *__restrict__ geo, int2 *__restrict__ meta,
+                           int2 *__restrict__ front, TravState *__restrict__ st) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {  // the traversal starts with (root, root)
+    front[0] = make_int2(0, 0);
+    *st = TravState{};
+    st->nfront = 1;
+  }
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ncells;
        i += (int64_t)gridDim.x * blockDim.x) {
     double w = 0;
@@ -74,136 +99,174 @@ constexpr int kSelfSplit = 36;  // child pairs (i, j), i <= j, of a cell with it
 static_assert(kBlock <= 256, "packed per-block counts hold at most 256 threads");
 static_assert(kSelfSplit * kBlock < (1 << 14), "frontier count field is 14 bits");
 
-// counters: [0] next frontier size, [1] m2l size, [2] p2p size,
-//           [3] p2p body-pair interactions, [4] overflow bits (1: a list,
-//           2: the next frontier; [0] still counts the frontier's full size)
-// Slots in the three outputs are reserved once per block (one atomic per
-// counter per block), the block's threads taking consecutive slots.
-__global__ void __launch_bounds__(kBlock) dtt_step(TravCells c, const int2 *__restrict__ front,
-                                                   int64_t nfront, int2 *__restrict__ next,
-                                                   int64_t next_cap, uint64_t *__restrict__ m2l,
-                                                   int64_t m2l_cap, uint64_t *__restrict__ p2p,
-                                                   int64_t p2p_cap,
-                                                   unsigned long long *__restrict__ counters,
-                                                   int prune_empty, int mutual) {
+struct TravBufs {
+  int2 *front[2];
+  long long front_cap[2];
+  uint64_t *m2l, *p2p;
+  long long m2l_cap, p2p_cap;
+};
+
+constexpr int kMaxSteps = 4 * (kMaxDepth + 2);
+
+// The whole breadth-first traversal in one cooperative launch: every step
+// classifies the pairs of the current frontier and appends to the two lists
+// and the next frontier, and a grid-wide barrier ends it.  Slots in the three
+// outputs are reserved once per block (one atomic per counter per block), the
+// block's threads taking consecutive slots.  A step that finds a buffer too
+// small ends the kernel without having counted; the host enlarges the buffer
+// and starts it again from that step.  (A launch and a host round trip per step
+// took about 20 us each, 9 to 25 times.)
+__global__ void __launch_bounds__(kBlock) dtt_steps(TravCells c, TravBufs bufs, TravState *st,
+                                                    int prune_empty, int mutual) {
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
   __shared__ uint32_t wsum[kWarpsPerBlock];
   __shared__ unsigned long long wint[kWarpsPerBlock];
   __shared__ unsigned long long bbase[3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nfront;
-       base += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = base + threadIdx.x;
-    int kind = 0;  // 0 none, 1 m2l, 2 p2p, 3 split target, 4 split source, 5 split both
-    int t = 0, s = 0, split_child = 0;
-    unsigned long long inter = 0;
-    if (i < nfront) {
-      const int2 pr = front[i];
-      t = pr.x;
-      s = pr.y;
-      const int2 mt = c.meta[t], ms = c.meta[s];
-      // An empty cell (and so all of its descendants) contributes nothing as a
-      // source and receives nothing used later as a target.
-      if (!prune_empty || (mt.x != 0 && ms.x != 0)) {
-        const double4 gt = c.geo[t], gs = c.geo[s];
-        const double dx = __dsub_rn(gt.x, gs.x);
-        const double dy = __dsub_rn(gt.y, gs.y);
-        const double dz = __dsub_rn(gt.z, gs.z);
-        double R2 = __dadd_rn(0.0, __dmul_rn(dx, dx));
-        R2 = __dadd_rn(R2, __dmul_rn(dy, dy));
-        R2 = __dadd_rn(R2, __dmul_rn(dz, dz));
-        const double Ri = gt.w, Rj = gs.w;
-        const double RR = __dadd_rn(Ri, Rj);
-        const bool lt = mt.y < 0, ls = ms.y < 0;
-        if (R2 > __dmul_rn(RR, RR)) {
-          kind = 1;
-        } else if (lt && ls) {
-          if (mt.x > 0 && ms.x > 0) {
-            kind = 2;
-            // body pairs evaluated: both directions of a mutual pair of two leaves
-            inter = (unsigned long long)mt.x * (unsigned long long)ms.x;
-            if (mutual && t != s) inter *= 2;
+  int64_t nfront = (int64_t)st->nfront;
+  unsigned long long n_m2l = st->m2l, n_p2p = st->p2p, n_int = st->inter, visited = st->visited;
+  int step = st->steps;
+  while (nfront > 0 && step < kMaxSteps) {
+    const int2 *front = bufs.front[step & 1];
+    int2 *next = bufs.front[(step & 1) ^ 1];
+    const int64_t next_cap = bufs.front_cap[(step & 1) ^ 1];
+    unsigned long long *counters = st->cnt[step % 3];
+    if (blockIdx.x == 0 && threadIdx.x < 4) st->cnt[(step + 1) % 3][threadIdx.x] = 0;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nfront;
+         base += (int64_t)gridDim.x * blockDim.x) {
+      const int64_t i = base + threadIdx.x;
+      int kind = 0;  // 0 none, 1 m2l, 2 p2p, 3 split target, 4 split source, 5 split both
+      int t = 0, s = 0, split_child = 0;
+      unsigned long long inter = 0;
+      if (i < nfront) {
+        const int2 pr = __ldcg(front + i);
+        t = pr.x;
+        s = pr.y;
+        const int2 mt = c.meta[t], ms = c.meta[s];
+        // An empty cell (and so all of its descendants) contributes nothing as a
+        // source and receives nothing used later as a target.
+        if (!prune_empty || (mt.x != 0 && ms.x != 0)) {
+          const double4 gt = c.geo[t], gs = c.geo[s];
+          const double dx = __dsub_rn(gt.x, gs.x);
+          const double dy = __dsub_rn(gt.y, gs.y);
+          const double dz = __dsub_rn(gt.z, gs.z);
+          double R2 = __dadd_rn(0.0, __dmul_rn(dx, dx));
+          R2 = __dadd_rn(R2, __dmul_rn(dy, dy));
+          R2 = __dadd_rn(R2, __dmul_rn(dz, dz));
+          const double Ri = gt.w, Rj = gs.w;
+          const double RR = __dadd_rn(Ri, Rj);
+          const bool lt = mt.y < 0, ls = ms.y < 0;
+          if (R2 > __dmul_rn(RR, RR)) {
+            kind = 1;
+          } else if (lt && ls) {
+            if (mt.x > 0 && ms.x > 0) {
+              kind = 2;
+              // body pairs evaluated: both directions of a mutual pair of two leaves
+              inter = (unsigned long long)mt.x * (unsigned long long)ms.x;
+              if (mutual && t != s) inter *= 2;
+            }
+          } else if (ls) {
+            kind = 3;
+          } else if (lt) {
+            kind = 4;
+          } else if (mutual && t == s) {
+            kind = 5;
+          } else {
+            kind = (Ri >= Rj) ? 3 : 4;
           }
-        } else if (ls) {
-          kind = 3;
-        } else if (lt) {
-          kind = 4;
-        } else if (mutual && t == s) {
-          kind = 5;
-        } else {
-          kind = (Ri >= Rj) ? 3 : 4;
+          split_child = kind == 3 ? mt.y : ms.y;
         }
-        split_child = kind == 3 ? mt.y : ms.y;
       }
-    }
-    const uint32_t mine = (kind == 1 ? 1u : 0u) | (kind == 2 ? 1u << 9 : 0u) |
-                          (kind == 3 || kind == 4 ? 8u << 18 : 0u) |
-                          (kind == 5 ? (uint32_t)kSelfSplit << 18 : 0u);
-    uint32_t incl = mine;
+      const uint32_t mine = (kind == 1 ? 1u : 0u) | (kind == 2 ? 1u << 9 : 0u) |
+                            (kind == 3 || kind == 4 ? 8u << 18 : 0u) |
+                            (kind == 5 ? (uint32_t)kSelfSplit << 18 : 0u);
+      uint32_t incl = mine;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    unsigned long long w = inter;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-    if (lane == 31) wsum[warp] = incl;
-    if (lane == 0) wint[warp] = w;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t run = 0;
-      unsigned long long tot = 0;
-#pragma unroll
-      for (int k = 0; k < kWarpsPerBlock; k++) {
-        const uint32_t v = wsum[k];
-        wsum[k] = run;
-        run += v;
-        tot += wint[k];
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
       }
-      const uint32_t n1 = run & 511u, n2 = (run >> 9) & 511u, n3 = run >> 18;
-      bbase[0] = n1 ? atomicAdd(counters + 1, (unsigned long long)n1) : 0;
-      bbase[1] = n2 ? atomicAdd(counters + 2, (unsigned long long)n2) : 0;
-      bbase[2] = n3 ? atomicAdd(counters + 0, (unsigned long long)n3) : 0;
-      if (tot) atomicAdd(counters + 3, tot);
-    }
-    __syncthreads();
-    const uint32_t off = wsum[warp] + incl - mine;
-    if (kind == 1) {
-      const unsigned long long dst = bbase[0] + (off & 511u);
-      if ((int64_t)dst < m2l_cap) m2l[dst] = ((uint64_t)(uint32_t)t << 32) | (uint32_t)s;
-      else atomicOr(counters + 4, 1ull);
-    } else if (kind == 2) {
-      const unsigned long long dst = bbase[1] + ((off >> 9) & 511u);
-      if ((int64_t)dst < p2p_cap) p2p[dst] = ((uint64_t)(uint32_t)t << 32) | (uint32_t)s;
-      else atomicOr(counters + 4, 1ull);
-    } else if (kind == 5) {
-      const unsigned long long dst = bbase[2] + (off >> 18);
-      if ((int64_t)(dst + kSelfSplit) <= next_cap) {
-        int2 *o = next + dst;
-        int k = 0;
-        for (int a = 0; a < 8; a++)
-          for (int b2 = a; b2 < 8; b2++) o[k++] = make_int2(split_child + a, split_child + b2);
-      } else {
-        atomicOr(counters + 4, 2ull);
-      }
-    } else if (kind >= 3) {
-      const unsigned long long dst = bbase[2] + (off >> 18);
-      if ((int64_t)(dst + 8) <= next_cap) {
-        int4 *o4 = reinterpret_cast<int4 *>(next + dst);  // dst is even (8 and 36 are)
-        if (kind == 3) {
+      unsigned long long w = inter;
 #pragma unroll
-          for (int k = 0; k < 8; k += 2)
-            o4[k / 2] = make_int4(split_child + k, s, split_child + k + 1, s);
-        } else {
+      for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+      if (lane == 31) wsum[warp] = incl;
+      if (lane == 0) wint[warp] = w;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        uint32_t run = 0;
+        unsigned long long tot = 0;
 #pragma unroll
-          for (int k = 0; k < 8; k += 2)
-            o4[k / 2] = make_int4(t, split_child + k, t, split_child + k + 1);
+        for (int k = 0; k < kWarpsPerBlock; k++) {
+          const uint32_t v = wsum[k];
+          wsum[k] = run;
+          run += v;
+          tot += wint[k];
         }
-      } else {
-        atomicOr(counters + 4, 2ull);
+        const uint32_t n1 = run & 511u, n2 = (run >> 9) & 511u, n3 = run >> 18;
+        bbase[0] = n_m2l + (n1 ? atomicAdd(counters + 1, (unsigned long long)n1) : 0);
+        bbase[1] = n_p2p + (n2 ? atomicAdd(counters + 2, (unsigned long long)n2) : 0);
+        bbase[2] = n3 ? atomicAdd(counters + 0, (unsigned long long)n3) : 0;
+        if (tot) atomicAdd(counters + 3, tot);
       }
+      __syncthreads();
+      const uint32_t off = wsum[warp] + incl - mine;
+      if (kind == 1) {
+        const unsigned long long dst = bbase[0] + (off & 511u);
+        if ((int64_t)dst < bufs.m2l_cap) bufs.m2l[dst] = ((uint64_t)(uint32_t)t << 32) | (uint32_t)s;
+      } else if (kind == 2) {
+        const unsigned long long dst = bbase[1] + ((off >> 9) & 511u);
+        if ((int64_t)dst < bufs.p2p_cap) bufs.p2p[dst] = ((uint64_t)(uint32_t)t << 32) | (uint32_t)s;
+      } else if (kind == 5) {
+        const unsigned long long dst = bbase[2] + (off >> 18);
+        if ((int64_t)(dst + kSelfSplit) <= next_cap) {
+          int2 *o = next + dst;
+          int k = 0;
+          for (int a = 0; a < 8; a++)
+            for (int b2 = a; b2 < 8; b2++) o[k++] = make_int2(split_child + a, split_child + b2);
+        }
+      } else if (kind >= 3) {
+        const unsigned long long dst = bbase[2] + (off >> 18);
+        if ((int64_t)(dst + 8) <= next_cap) {
+          int4 *o4 = reinterpret_cast<int4 *>(next + dst);  // dst is even (8 and 36 are)
+          if (kind == 3) {
+#pragma unroll
+            for (int k = 0; k < 8; k += 2)
+              o4[k / 2] = make_int4(split_child + k, s, split_child + k + 1, s);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 8; k += 2)
+              o4[k / 2] = make_int4(t, split_child + k, t, split_child + k + 1);
+          }
+        }
+      }
+      __syncthreads();  // wsum / bbase are rewritten by the next round
     }
-    __syncthreads();  // wsum / bbase are rewritten by the next round
+    grid.sync();
+    const unsigned long long f = __ldcg(counters + 0), m = n_m2l + __ldcg(counters + 1),
+                             p = n_p2p + __ldcg(counters + 2);
+    if ((int64_t)f > next_cap || (int64_t)m > bufs.m2l_cap || (int64_t)p > bufs.p2p_cap) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->stop = 1;
+        st->need_front = f;
+        st->need_m2l = m;
+        st->need_p2p = p;
+      }
+      break;
+    }
+    n_int += __ldcg(counters + 3);
+    visited += (unsigned long long)nfront;
+    nfront = (int64_t)f;
+    n_m2l = m;
+    n_p2p = p;
+    step++;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->nfront = (unsigned long long)nfront;
+    st->m2l = n_m2l;
+    st->p2p = n_p2p;
+    st->inter = n_int;
+    st->visited = visited;
+    st->steps = step;
   }
 }
 
@@ -475,69 +538,78 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
   const int64_t C = ctx->ncells;
   TB_CUDA(ctx, ctx->trav_geo.ensure(C + 1, s));
   TB_CUDA(ctx, ctx->trav_meta.ensure(C + 1, s));
-  trav_cells<<<grid_for(C, kBlock), kBlock, 0, s>>>(C, ctx->cmin.p, ctx->cmax.p, ctx->ccen.p,
-                                                    ctx->cnb.p, ctx->cleaf.p, ctx->cchild.p, theta,
-                                                    ctx->trav_geo.p, ctx->trav_meta.p);
-  TB_LAUNCH_CHECK(ctx);
-  const TravCells cv{ctx->trav_geo.p, ctx->trav_meta.p};
-  TB_CUDA(ctx, ctx->counters.ensure(8, s));
-  TB_CUDA(ctx, ctx->pinned.ensure(256));
+  TB_CUDA(ctx, ctx->counters.ensure(64, s));
+  TB_CUDA(ctx, ctx->pinned.ensure(512));
+  // First sizes: a list entry per cell and near or far neighbour of a
+  // volume-filling tree for small trees, of a surface for large ones; a list that
+  // outgrows its buffer is met below, and the buffers stay for the next call.
+  auto room = [&](int64_t per_cell, int64_t large, int64_t extra) {
+    return (size_t)(std::min(per_cell * C, large * C + extra) + 4096);
+  };
+  TB_CUDA(ctx, ctx->front_a.ensure(room(64, 16, 2000000), s));
+  TB_CUDA(ctx, ctx->front_b.ensure(room(64, 16, 2000000), s));
+  TB_CUDA(ctx, ctx->m2l.ensure(room(128, 40, 4000000), s));
+  TB_CUDA(ctx, ctx->p2p.ensure(room(64, 24, 2000000), s));
   unsigned long long *hc = reinterpret_cast<unsigned long long *>(ctx->pinned.p);
   TB_CUDA(ctx, cudaMemsetAsync(ctx->counters.p, 0, 8 * sizeof(unsigned long long), s));
+  TravState *st = reinterpret_cast<TravState *>(ctx->counters.p + kTravStateAt);
+  trav_cells<<<grid_for(C, kBlock), kBlock, 0, s>>>(
+      C, ctx->cmin.p, ctx->cmax.p, ctx->ccen.p, ctx->cnb.p, ctx->cleaf.p, ctx->cchild.p, theta,
+      ctx->trav_geo.p, ctx->trav_meta.p, ctx->front_a.p, st);
+  TB_LAUNCH_CHECK(ctx);
+  const TravCells cv{ctx->trav_geo.p, ctx->trav_meta.p};
   {
     PhaseTimer tm(ctx, &ctx->timings.traverse);
-    TB_CUDA(ctx, ctx->front_a.ensure(1024, s));
-    const int2 root = make_int2(0, 0);
-    TB_CUDA(ctx, cudaMemcpyAsync(ctx->front_a.p, &root, sizeof(int2), cudaMemcpyHostToDevice, s));
-    int64_t nfront = 1, n_m2l = 0, n_p2p = 0, visited = 0;
-    unsigned long long n_int = 0;
-    int iters = 0;
-    unsigned long long *hset = hc + 16;  // counter values restored before a step
-    while (nfront > 0) {
-      visited += nfront;
-      // Each visited pair adds at most one M2L or P2P pair; the next frontier
-      // gets 2 * nfront slots first, and a step that needs more is run again
-      // with the size its reservations counted.
-      TB_CUDA(ctx, ctx->m2l.ensure(n_m2l + nfront, s, true, n_m2l));
-      TB_CUDA(ctx, ctx->p2p.ensure(n_p2p + nfront, s, true, n_p2p));
-      TB_CUDA(ctx, ctx->front_b.ensure(std::max<int64_t>(2 * nfront, 1024), s));
-      for (int attempt = 0;; attempt++) {
-        hset[0] = 0;
-        hset[1] = (unsigned long long)n_m2l;
-        hset[2] = (unsigned long long)n_p2p;
-        hset[3] = n_int;
-        hset[4] = 0;
-        TB_CUDA(ctx, cudaMemcpyAsync(ctx->counters.p, hset, 5 * sizeof(unsigned long long),
-                                     cudaMemcpyHostToDevice, s));
-        dtt_step<<<grid_for(nfront, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
-            cv, ctx->front_a.p, nfront, ctx->front_b.p, (int64_t)ctx->front_b.cap, ctx->m2l.p,
-            (int64_t)ctx->m2l.cap, ctx->p2p.p, (int64_t)ctx->p2p.cap, ctx->counters.p,
-            ctx->reference_lists ? 0 : 1, mutual);
-        TB_LAUNCH_CHECK(ctx);
-        TB_CUDA(ctx, cudaMemcpyAsync(hc, ctx->counters.p, 5 * sizeof(unsigned long long),
-                                     cudaMemcpyDeviceToHost, s));
-        TB_CUDA(ctx, cudaStreamSynchronize(s));
-        if (hc[4] & 1) {
-          set_error(ctx, "traversal: work list capacity exceeded");
-          return TAPAS_B200_ERR_CAPACITY;
-        }
-        if (!(hc[4] & 2)) break;
-        if (attempt > 0) {
-          set_error(ctx, "traversal: frontier capacity exceeded after resizing");
-          return TAPAS_B200_ERR_CAPACITY;
-        }
-        TB_CUDA(ctx, ctx->front_b.ensure((size_t)hc[0], s));
-      }
-      nfront = (int64_t)hc[0];
-      n_m2l = (int64_t)hc[1];
-      n_p2p = (int64_t)hc[2];
-      n_int = hc[3];
-      std::swap(ctx->front_a, ctx->front_b);
-      if (++iters > 4 * (kMaxDepth + 2)) {
-        set_error(ctx, "traversal did not terminate within its iteration bound");
+    if (ctx->trav_blocks == 0) {
+      int per_sm = 0;
+      TB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dtt_steps, kBlock, 0));
+      ctx->trav_blocks = std::max(1, per_sm) * ctx->num_sms;
+    }
+    // few blocks for a small tree: the barrier costs more than their work
+    const int blocks =
+        (int)std::min<int64_t>(ctx->trav_blocks, std::max<int64_t>(32, C * 8 / kBlock));
+    TravState *h = reinterpret_cast<TravState *>(hc + 16);
+    for (int attempt = 0;; attempt++) {
+      TravBufs bufs{{ctx->front_a.p, ctx->front_b.p},
+                    {(long long)ctx->front_a.cap, (long long)ctx->front_b.cap},
+                    ctx->m2l.p,
+                    ctx->p2p.p,
+                    (long long)ctx->m2l.cap,
+                    (long long)ctx->p2p.cap};
+      TravCells cells = cv;
+      int prune = ctx->reference_lists ? 0 : 1, mut = mutual;
+      TravState *state = st;
+      void *args[] = {&cells, &bufs, &state, &prune, &mut};
+      TB_CUDA(ctx, cudaLaunchCooperativeKernel(reinterpret_cast<void *>(dtt_steps), dim3(blocks),
+                                               dim3(kBlock), args, 0, s));
+      count_launch(ctx);
+      TB_CUDA(ctx, cudaMemcpyAsync(h, st, sizeof(TravState), cudaMemcpyDeviceToHost, s));
+      TB_CUDA(ctx, cudaStreamSynchronize(s));
+      if (!h->stop) break;
+      if (attempt > 3 * kMaxSteps) {
+        set_error(ctx, "traversal: frontier capacity exceeded after resizing");
         return TAPAS_B200_ERR_CAPACITY;
       }
+      tb::DBuf<int2> &next = (h->steps & 1) ? ctx->front_a : ctx->front_b;
+      if (h->need_front > next.cap)
+        TB_CUDA(ctx, next.ensure(h->need_front + h->need_front / 2, s));
+      if (h->need_m2l > ctx->m2l.cap)
+        TB_CUDA(ctx, ctx->m2l.ensure(h->need_m2l + h->need_m2l / 2, s, true, h->m2l));
+      if (h->need_p2p > ctx->p2p.cap)
+        TB_CUDA(ctx, ctx->p2p.ensure(h->need_p2p + h->need_p2p / 2, s, true, h->p2p));
+      h->stop = 0;
+      for (auto &set : h->cnt)
+        for (auto &v : set) v = 0;
+      TB_CUDA(ctx, cudaMemcpyAsync(st, h, sizeof(TravState), cudaMemcpyHostToDevice, s));
     }
+    if (h->nfront > 0) {
+      set_error(ctx, "traversal did not terminate within its iteration bound");
+      return TAPAS_B200_ERR_CAPACITY;
+    }
+    int64_t n_m2l = (int64_t)h->m2l, n_p2p = (int64_t)h->p2p;
+    const unsigned long long n_int = h->inter;
+    const int64_t visited = (int64_t)h->visited;
+    const int iters = h->steps;
     ctx->n_m2l_visited = n_m2l;
     ctx->n_p2p_visited = n_p2p;
     if (mutual) {
