@@ -89,6 +89,16 @@ __global__ void leaf_pieces(const int32_t *__restrict__ leaves, int64_t nleaves,
   }
 }
 
+// Queue key of an item of that many body pairs: decreasing work in steps of an
+// eighth of an octave, so that one radix pass orders the queue (exact order took
+// four, 12 launches, and shortens the tail by nothing that shows).
+__device__ __forceinline__ uint64_t work_key(uint64_t work) {
+  if (work == 0) return 255;
+  const int e = 63 - __clzll((long long)work);  // work in [2^e, 2^(e+1))
+  const int f = (int)((e >= 3 ? work >> (e - 3) : work << (3 - e)) & 7);
+  return 255 - min(255, 8 * max(e - 4, 0) + f);
+}
+
 // Items of leaf w at koff[w]..: cut its list greedily where the pairs reach
 // piece_pairs (at most k pieces; unused slots become empty pieces with
 // zeroed partials).  Work key = nt * sources of the piece, for the queue.
@@ -110,10 +120,8 @@ __global__ void emit_items(const int32_t *__restrict__ leaves, int64_t nleaves,
     for (int e = e0; e < e1; e++) {
       acc += cnb[(int)(list[e] & src_mask)];
       if ((k > 1 && acc * nt >= piece_pairs && j < k - 1) || e == e1 - 1) {
-        uint64_t work = (uint64_t)acc * (uint64_t)nt;
-        if (work > 0xFFFFFFFFull) work = 0xFFFFFFFFull;
         items[base + j] = WorkItem{c, ea, e + 1, k > 1 ? poff[w] + j * nt : -1};
-        keys[base + j] = 0xFFFFFFFFull - work;  // ascending sort -> decreasing work
+        keys[base + j] = work_key((uint64_t)acc * (uint64_t)nt);
         vals[base + j] = (uint32_t)(base + j);
         j++;
         ea = e + 1;
@@ -122,13 +130,13 @@ __global__ void emit_items(const int32_t *__restrict__ leaves, int64_t nleaves,
     }
     if (e1 == e0) {  // no list: one empty item still writes the leaf's zero sums
       items[base] = WorkItem{c, e0, e0, -1};
-      keys[base] = 0xFFFFFFFFull;
+      keys[base] = work_key(0);
       vals[base] = (uint32_t)base;
       j = 1;
     }
     for (; j < k; j++) {  // unused pieces: empty, zero partials
       items[base + j] = WorkItem{c, e1, e1, poff[w] + j * nt};
-      keys[base + j] = 0xFFFFFFFFull;
+      keys[base + j] = work_key(0);
       vals[base + j] = (uint32_t)(base + j);
       for (int t = 0; t < 4 * nt; t++) part[4 * ((int64_t)poff[w] + (int64_t)j * nt) + t] = 0.0;
     }
@@ -711,7 +719,7 @@ int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
   TB_LAUNCH_CHECK(ctx);
   uint64_t *k = ctx->p2p_wkey.p, *ka = ctx->p2p_wkey_alt.p;
   uint32_t *v = ctx->p2p_order.p, *va = ctx->p2p_order_alt.p;
-  TB_TRY(radix_sort(ctx, k, ka, v, va, ni, 0, 32));
+  TB_TRY(radix_sort(ctx, k, ka, v, va, ni, 0, 8));
   if (v != ctx->p2p_order.p) {
     std::swap(ctx->p2p_order.p, ctx->p2p_order_alt.p);
     std::swap(ctx->p2p_order.cap, ctx->p2p_order_alt.cap);
