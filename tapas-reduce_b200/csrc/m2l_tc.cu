@@ -603,21 +603,28 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
+// Executed by the whole warp with warp-uniform operands; `leader` is nonzero in
+// the one lane that issues.  (Under a branch to that lane the operands live in
+// per-lane registers, and moving them to the uniform ones cost 107 cycles per MMA.)
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
+                                          uint32_t idesc, uint32_t accumulate, uint32_t leader) {
   const uint32_t z = 0;
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+      "setp.ne.b32 q, %9, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z),
-        "r"(z), "r"(z));
+        "r"(z), "r"(z), "r"(leader));
 }
 
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
+__device__ __forceinline__ void umma_commit(uint64_t *bar, uint32_t leader) {
   asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(bar))
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          smem_u32(bar)),
+      "r"(leader)
       : "memory");
 }
 
@@ -706,7 +713,8 @@ __device__ __forceinline__ bool wait_phase(uint64_t *bar, uint32_t parity, volat
 // rows, both K-major core matrices.
 template <int P, bool kDense = false>
 __device__ __forceinline__ void issue_chunk_mmas(uint32_t dcol, uint32_t a_hi, uint32_t a_lo,
-                                                 uint32_t b_hi, uint32_t b_lo, int kc, int nr) {
+                                                 uint32_t b_hi, uint32_t b_lo, int kc, int nr,
+                                                 uint32_t leader) {
   using S = TcShape<P, kDense>;
   const uint32_t LBO = 128;                  // adjacent k-cores
   const uint32_t SBO = (S::KC / 4) * 128;    // adjacent 8-row groups
@@ -727,9 +735,9 @@ __device__ __forceinline__ void issue_chunk_mmas(uint32_t dcol, uint32_t a_hi, u
       const uint64_t bh = umma_desc(b_hi + boff, LBO, SBO);
       const uint64_t bl = umma_desc(b_lo + boff, LBO, SBO);
       const uint32_t d = dcol + (uint32_t)n0;
-      umma_tf32(d, ah, bh, idesc, acc);
-      umma_tf32(d, al, bh, idesc, 1u);
-      umma_tf32(d, ah, bl, idesc, 1u);
+      umma_tf32(d, ah, bh, idesc, acc, leader);
+      umma_tf32(d, al, bh, idesc, 1u, leader);
+      umma_tf32(d, ah, bl, idesc, 1u, leader);
     }
   }
 }
@@ -748,20 +756,24 @@ constexpr int kEpiWarps = 8;       //   column half (warp - 8) / 4)
 constexpr int kMmaWarp = 16;       // warp 16: TMEM allocation, MMA issue (lane 0)
 constexpr int kSplitWarp0 = 17;    // warps 17-24: split the staged rows into hi + lo
 constexpr int kSplitThreads = 256;
-constexpr int kThreadsTc = 32 * 25;
+constexpr int kSplitGroups = 4;    //   in groups of two warps, each its own ring stages
+constexpr int kSplitGroup = kSplitThreads / kSplitGroups;
+constexpr int kBulkWarp = 25;      // warp 25: the operators' bulk copies
+constexpr int kThreadsTc = 32 * 26;
 
 // Persistent CTA over the tiles blockIdx.x, blockIdx.x + gridDim.x, ...,
 // warp-specialised; the roles meet only at mbarriers:
 //  - producers (warps 0-7) walk the (tile, k-chunk) steps through an NS-stage
 //    ring: every producer cp.async-copies its share of the 128 gathered
 //    multipole rows (A, FP32; lanes of a warp cover whole row segments) and
-//    arrives on landed[stage] when they have landed; thread 0 bulk-copies
+//    arrives on landed[stage] when they have landed; warp 25 bulk-copies
 //    the operator rows the chunk reaches (B, contiguous, split into TF32 hi
 //    and lo when they were built), which complete on landed[stage] too.  A
 //    stage is refilled after the MMAs that read it commit to empty[stage].
-//  - the split warps (17-24) wait for landed[stage], split the multipole
-//    rows into TF32 hi + lo in place and arrive on full[stage].
-//  - the MMA thread (warp 16, lane 0) waits for full[stage], issues the
+//  - the split warps (17-24), two per group of stages, wait for landed[stage],
+//    split the multipole rows into TF32 hi + lo in place and arrive on
+//    full[stage].
+//  - the MMA warp (16) waits for full[stage]; one lane issues the
 //    chunk's 3xTF32 MMAs into one of TBUF TMEM accumulators and commits them
 //    to empty[stage]; after a tile's last chunk it commits to tfull[buffer].
 //  - the epilogue warps (8-15) wait for tfull[buffer], read the accumulator
@@ -794,7 +806,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
   if (tid == 0) {
     for (int i = 0; i < NS; i++) {
       mbar_init(&landed[i], kProdThreads + 1);
-      mbar_init(&full[i], kSplitThreads);
+      mbar_init(&full[i], kSplitGroup);
       mbar_init(&empty[i], 1);
     }
     for (int b = 0; b < 2; b++) {
@@ -839,25 +851,32 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
     constexpr int RPP = (kProdThreads / 32) * RPW;
     constexpr int NRT = kNTile / RPP;
     const int apiece = (tid & 31) / RPW, arow0 = (tid >> 5) * RPW + (tid & 31) % RPW;
-    int cur_src[NRT], nxt_src[NRT];
-    int cur_cls = 0, nxt_cls = 0;
-    auto fetch = [&](int64_t jt) {
-      nxt_cls = 0;
-      TileItem it;
-      it.len = 0;
-      it.start = 0;
-      if (jt < ntiles) {
-        it = item_of(jt);
-        nxt_cls = it.cls;
-      }
+    // The sources of the next tile are found by a chain of dependent loads
+    // (item, sorted pair, list entry), one link per step or tile, so that no
+    // link waits for the one before (all three in one place stalled the
+    // copies for about 2000 cycles per tile).
+    int cur_src[NRT];
+    uint64_t nxt_pair[NRT];  // list entries of tile jt + 1 (~0: no row)
+    uint32_t nxt_idx[NRT];   // and their indices
+    TileItem ahead = {0, 0, 0, 0};  // item of tile jt + 1, then jt + 2
+    auto item_or_none = [&](int64_t jt) {
+      return jt < ntiles ? item_of(jt) : TileItem{0, 0, 0, 0};
+    };
+    auto find_idx = [&](const TileItem &it) {
 #pragma unroll
       for (int i = 0; i < NRT; i++) {
         const int row = arow0 + i * RPP;
-        nxt_src[i] = row < it.len ? (int)(list[sorted_vals[it.start + row]] & mask) : -1;
+        nxt_idx[i] = row < it.len ? sorted_vals[it.start + row] : 0xFFFFFFFFu;
       }
     };
-    fetch(0);
-    int64_t issued = 0;
+    auto find_pairs = [&]() {
+#pragma unroll
+      for (int i = 0; i < NRT; i++)
+        nxt_pair[i] = nxt_idx[i] != 0xFFFFFFFFu ? list[nxt_idx[i]] : ~0ull;
+    };
+    find_idx(item_or_none(0));
+    find_pairs();
+    ahead = item_or_none(1);
     for (int64_t step = 0; step < nsteps; step++) {
       const int st = (int)(step % NS);
       if (step >= NS &&
@@ -867,19 +886,10 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
       const int kc = (int)(step % S::NKC);
       if (kc == 0) {
 #pragma unroll
-        for (int i = 0; i < NRT; i++) cur_src[i] = nxt_src[i];
-        cur_cls = nxt_cls;
+        for (int i = 0; i < NRT; i++)
+          cur_src[i] = nxt_pair[i] != ~0ull ? (int)(nxt_pair[i] & mask) : -1;
       }
       float *sA_hi = base + (size_t)st * S::STAGE_FLOATS;
-      float *sB_hi = sA_hi + 2 * kNTile * S::KC;
-      if (tid == 0) {
-        // the chunk's operator rows (the ones it reaches), TF32 hi and lo
-        const size_t boff = (size_t)cur_cls * 2 * S::OPS_FLOATS + (size_t)co_sh[kc];
-        const uint32_t bbytes = (uint32_t)(nr_sh[kc] * S::KC * sizeof(float));
-        mbar_expect_tx(&landed[st], 2 * bbytes);
-        bulk_copy(sB_hi, ops + boff, bbytes, &landed[st]);
-        bulk_copy(sB_hi + S::NPAD * S::KC, ops + boff + S::OPS_FLOATS, bbytes, &landed[st]);
-      }
 #pragma unroll
       for (int i = 0; i < NRT; i++) {
         const int row = arow0 + i * RPP;
@@ -890,65 +900,106 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
         cp_async16(sA_hi + o, Mt + aoff, have ? 16u : 0u);
       }
       cp_async_arrive_noinc(&landed[st]);
-      issued = step + 1;
-      // the next tile's sources (a chain of dependent loads), after this
-      // tile's first copies are on their way
-      if (kc == 0) fetch(jt + 1);
+      if (kc == 0) {
+        find_idx(ahead);
+        ahead = item_or_none(jt + 2);
+      }
+      static_assert(S::NKC >= 2, "one link of the chain per step");
+      if (kc == 1) find_pairs();
     }
     cp_async_wait_all();
-    if (tid == 0 && *abort) {
-      // bulk copies of steps the MMA thread may not have consumed: let them land
+  } else if (warp == kBulkWarp) {
+    // ---------------- operator copies ----------------
+    // per step the operator rows the chunk reaches, TF32 hi and lo; the warp
+    // walks the steps together (uniform operands), one lane issues
+    int64_t issued = 0;
+    int cls = 0, nxt_cls = ntiles > 0 ? item_of(0).cls : 0;
+    for (int64_t step = 0; step < nsteps; step++) {
+      const int st = (int)(step % NS);
+      if (step >= NS &&
+          !__all_sync(0xffffffffu, wait_phase(&empty[st], (uint32_t)((step / NS - 1) & 1), abort,
+                                              wait_limit)))
+        break;
+      const int kc = (int)(step % S::NKC);
+      if (kc == 0) {
+        cls = nxt_cls;
+        if (step / S::NKC + 1 < ntiles) nxt_cls = item_of(step / S::NKC + 1).cls;
+      }
+      if (lane == 0) {
+        float *sB_hi = base + (size_t)st * S::STAGE_FLOATS + 2 * kNTile * S::KC;
+        const size_t boff = (size_t)cls * 2 * S::OPS_FLOATS + (size_t)co_sh[kc];
+        const uint32_t bbytes = (uint32_t)(nr_sh[kc] * S::KC * sizeof(float));
+        mbar_expect_tx(&landed[st], 2 * bbytes);
+        bulk_copy(sB_hi, ops + boff, bbytes, &landed[st]);
+        bulk_copy(sB_hi + S::NPAD * S::KC, ops + boff + S::OPS_FLOATS, bbytes, &landed[st]);
+      }
+      __syncwarp();
+      issued = step + 1;
+    }
+    if (lane == 0 && *abort) {
+      // bulk copies of steps that may not have been consumed: let them land
       for (int64_t s = issued > NS ? issued - NS : 0; s < issued; s++) {
         const long long t0 = clock64();
-        while (!mbar_try_wait(&full[s % NS], (uint32_t)((s / NS) & 1)) &&
+        while (!mbar_try_wait(&landed[s % NS], (uint32_t)((s / NS) & 1)) &&
                clock64() - t0 < 200000000LL) {
         }
       }
     }
   } else if (warp == kMmaWarp) {
     // ---------------- MMA issue ----------------
-    if (lane == 0) {
-      for (int64_t jt = 0; jt < ntiles && !*abort; jt++) {
-        const int b = NB == 2 ? (int)(jt & 1) : 0;
-        const int64_t use_b = NB == 2 ? (jt >> 1) : jt;
-        if (use_b >= 1 && !wait_phase(&tempty[b], (uint32_t)((use_b - 1) & 1), abort, wait_limit)) break;
-        tc_fence_after();
-        const uint32_t dcol = tmem + (uint32_t)(b * S::BSTRIDE);
-        bool ok = true;
-        for (int kc = 0; kc < S::NKC; kc++) {
-          const int64_t step = jt * S::NKC + kc;
-          const int st = (int)(step % NS);
-          if (!wait_phase(&full[st], (uint32_t)((step / NS) & 1), abort, wait_limit)) {
-            ok = false;
-            break;
-          }
-          fence_async_smem();  // the cp.async rows are visible to the tensor core
-          tc_fence_after();
-          float *sA_hi = base + (size_t)st * S::STAGE_FLOATS;
-          float *sA_lo = sA_hi + kNTile * S::KC;
-          float *sB_hi = sA_lo + kNTile * S::KC;
-          float *sB_lo = sB_hi + S::NPAD * S::KC;
-          issue_chunk_mmas<P, kDense>(dcol, smem_u32(sA_hi), smem_u32(sA_lo), smem_u32(sB_hi),
-                                      smem_u32(sB_lo), kc, nr_sh[kc]);
-          umma_commit(&empty[st]);
-        }
-        if (!ok) break;
-        umma_commit(&tfull[b]);
+    // the whole warp walks the steps (uniform control flow), one lane issues
+    uint32_t leader;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(leader));
+    bool ok = true;
+    for (int64_t jt = 0; jt < ntiles && ok; jt++) {
+      const int b = NB == 2 ? (int)(jt & 1) : 0;
+      const int64_t use_b = NB == 2 ? (jt >> 1) : jt;
+      if (use_b >= 1)
+        ok = __all_sync(0xffffffffu, wait_phase(&tempty[b], (uint32_t)((use_b - 1) & 1), abort,
+                                                wait_limit));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t dcol = tmem + (uint32_t)(b * S::BSTRIDE);
+#pragma unroll
+      for (int kc = 0; kc < S::NKC; kc++) {
+        const int64_t step = jt * S::NKC + kc;
+        const int st = (int)(step % NS);
+        if (ok)
+          ok = __all_sync(0xffffffffu, wait_phase(&full[st], (uint32_t)((step / NS) & 1), abort,
+                                                  wait_limit));
+        if (!ok) continue;
+        tc_fence_after();  // (the split warps made their rows visible to the tensor core)
+        const uint32_t sA_hi = smem_u32(base) + (uint32_t)(st * S::STAGE_FLOATS * sizeof(float));
+        const uint32_t sA_lo = sA_hi + kNTile * S::KC * sizeof(float);
+        const uint32_t sB_hi = sA_lo + kNTile * S::KC * sizeof(float);
+        const uint32_t sB_lo = sB_hi + S::NPAD * S::KC * sizeof(float);
+        issue_chunk_mmas<P, kDense>(dcol, sA_hi, sA_lo, sB_hi, sB_lo, kc, S::nrows(kc), leader);
+        umma_commit(&empty[st], leader);
       }
-      // every MMA issued so far has completed before TMEM is freed
-      umma_commit(&fin);
-      const long long t0 = clock64();
-      while (!mbar_try_wait(&fin, 0) && clock64() - t0 < 400000000LL) {
-      }
+      if (ok) umma_commit(&tfull[b], leader);
+    }
+    // every MMA issued so far has completed before TMEM is freed
+    umma_commit(&fin, leader);
+    const long long t0 = clock64();
+    while (!mbar_try_wait(&fin, 0) && clock64() - t0 < 400000000LL) {
     }
     __syncwarp();
   } else if (warp >= kSplitWarp0) {
     // ---------------- split ----------------
     // once a stage's FP32 multipole rows (and its operator rows, split when
-    // they were built) have landed, the 256 threads split the multipole rows
-    // into TF32 hi + lo in place (16 bytes at a time), then arrive on
-    // full[stage]
-    const int t = tid - kSplitWarp0 * 32;
+    // they were built) have landed, a group of 64 threads splits the multipole
+    // rows into TF32 hi + lo in place (16 bytes at a time), then arrives on
+    // full[stage].  Each ring stage belongs to one group: a stage's wait, split
+    // and proxy fence are a chain of about 900 cycles whatever the number of
+    // threads, so all of them on every stage held the ring to that.  (A group
+    // must see every phase of its stages' barriers in order: a wait for a phase
+    // whose predecessor has not completed would return at once, its parity being
+    // the one before that.)
+    const int t = (tid - kSplitWarp0 * 32) % kSplitGroup;
     auto split4 = [](float *hi_p, float *lo_p) {
       const float4 x = *reinterpret_cast<const float4 *>(hi_p);
       float4 hi, lo;
@@ -959,15 +1010,16 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
       *reinterpret_cast<float4 *>(hi_p) = hi;
       *reinterpret_cast<float4 *>(lo_p) = lo;
     };
+    const int group = (tid - kSplitWarp0 * 32) / kSplitGroup;
     for (int64_t step = 0; step < nsteps; step++) {
       const int st = (int)(step % NS);
-      const int kc = (int)(step % S::NKC);
+      if (st % kSplitGroups != group) continue;
       if (!wait_phase(&landed[st], (uint32_t)((step / NS) & 1), abort, wait_limit)) break;
       float *sA_hi = base + (size_t)st * S::STAGE_FLOATS;
       float *sA_lo = sA_hi + kNTile * S::KC;
 #pragma unroll
-      for (int i = 0; i < (kNTile * S::KC) / (4 * kSplitThreads); i++) {
-        const int o = 4 * (t + i * kSplitThreads);
+      for (int i = 0; i < (kNTile * S::KC) / (4 * kSplitGroup); i++) {
+        const int o = 4 * (t + i * kSplitGroup);
         split4(sA_hi + o, sA_lo + o);
       }
       fence_async_smem();  // the split rows are visible to the tensor core
@@ -983,21 +1035,26 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
     const int h = (warp - kEpiWarp0) >> 2;
     constexpr int NG = (S::NPAD + 31) / 32;
     float *xb = base + (size_t)NS * S::STAGE_FLOATS + (warp - kEpiWarp0) * 32 * S::EPI_STRIDE;
-    int tg = -1, tg_next = -1;  // target of this lane's pair, this tile and the next
-    auto load_target = [&](int64_t jt) {
-      TileItem it;
-      it.len = 0;
-      it.start = 0;
-      if (jt < ntiles) it = item_of(jt);
-      const int p = q * 32 + lane;
-      return p < it.len ? (int)(list[sorted_vals[it.start + p]] >> shift) : -1;
+    // Target of this lane's pair; the chain item -> sorted pair -> list entry runs
+    // one link per tile ahead, as the producers'.
+    const int prow = q * 32 + lane;
+    auto item_or_none = [&](int64_t jt) {
+      return jt < ntiles ? item_of(jt) : TileItem{0, 0, 0, 0};
     };
-    tg_next = load_target(0);
+    auto find_idx = [&](const TileItem &it) {
+      return prow < it.len ? sorted_vals[it.start + prow] : 0xFFFFFFFFu;
+    };
+    auto find_pair = [&](uint32_t e) { return e != 0xFFFFFFFFu ? list[e] : ~0ull; };
+    uint64_t pair1 = find_pair(find_idx(item_or_none(0)));  // of tile jt, then jt + 1
+    uint32_t idx2 = find_idx(item_or_none(1));              // of tile jt + 1, then jt + 2
+    TileItem item3 = item_or_none(2);                       // of tile jt + 2, then jt + 3
     for (int64_t jt = 0; jt < ntiles; jt++) {
       const int b = NB == 2 ? (int)(jt & 1) : 0;
       const int64_t use_b = NB == 2 ? (jt >> 1) : jt;
-      tg = tg_next;
-      tg_next = load_target(jt + 1);
+      const int tg = pair1 != ~0ull ? (int)(pair1 >> shift) : -1;
+      pair1 = find_pair(idx2);
+      idx2 = find_idx(item3);
+      item3 = item_or_none(jt + 3);
       if (!wait_phase(&tfull[b], (uint32_t)(use_b & 1), abort, wait_limit)) break;
       tc_fence_after();
 #pragma unroll 1
