@@ -173,6 +173,7 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
   for (auto *b : {&ctx->p2p_order, &ctx->p2p_order_alt}) b->release();
   for (auto *b : {&ctx->p2p_kcnt, &ctx->p2p_koff, &ctx->p2p_psz, &ctx->p2p_poff}) b->release();
   ctx->p2p_counter.release();
+  ctx->p2p_key.release();
   ctx->p2p_items.release();
   ctx->p2p_part.release();
   for (auto *b : {&ctx->l2p_body_leaf}) b->release();

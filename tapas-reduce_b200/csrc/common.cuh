@@ -238,6 +238,7 @@ struct tapas_b200_ctx {
   tb::DBuf<uint64_t> p2p_wkey, p2p_wkey_alt;  // P2P work order: keys
   tb::DBuf<uint32_t> p2p_order, p2p_order_alt;  // target leaves by decreasing work
   tb::DBuf<int> p2p_counter;            // P2P work-queue head
+  tb::DBuf<uint8_t> p2p_key;            // per leaf: queue key of its whole list
   tb::DBuf<int4> p2p_items;             // P2P work items (leaf, list range, partial rows)
   tb::DBuf<int32_t> p2p_kcnt, p2p_koff, p2p_psz, p2p_poff;  // per leaf: pieces, partial rows
   tb::DBuf<double> p2p_part;            // partial sums of pieces of split leaves

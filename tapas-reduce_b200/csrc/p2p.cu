@@ -44,10 +44,10 @@ constexpr int kWarps = 4;  // FP64 kernel: 4-warp CTAs, 4 per SM (<= 128 registe
 constexpr int kThreads = 32 * kWarps;
 constexpr int kFp64Blocks = 4;
 constexpr int kStage = 64;   // mixed: source bodies staged per warp at a time (two per lane)
-// mixed kernel: 4-warp CTAs, up to 4 targets per lane (leaves of more than 128
+// mixed kernel: 4-warp CTAs, up to 3 targets per lane (leaves of more than 96
 // bodies take two passes)
 constexpr int kMixedWarps = 4;
-constexpr int kMixedMaxR = 4;
+constexpr int kMixedMaxR = 3;
 constexpr int kMixedBlocks = 5;     // CTAs per SM (<= 102 registers)
 constexpr float kNowhere = 1.25e18f;  // coordinate of a chargeless padding source
 constexpr int kMixedThreads = 32 * kMixedWarps;
@@ -71,24 +71,6 @@ struct WorkItem {
   int32_t pbase;         // -1: writes trg directly; else first row of its partials
 };
 
-// per non-empty leaf w: pieces k (>= 1) and partial rows (k * nt when split)
-__global__ void leaf_pieces(const int32_t *__restrict__ leaves, int64_t nleaves,
-                            const int32_t *__restrict__ off, const uint64_t *__restrict__ list,
-                            uint64_t src_mask, const int32_t *__restrict__ cnb,
-                            int64_t piece_pairs, int32_t *__restrict__ kcnt,
-                            int32_t *__restrict__ psz) {
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nleaves;
-       w += (int64_t)gridDim.x * blockDim.x) {
-    const int c = leaves[w];
-    int64_t ns = 0;
-    for (int e = off[c]; e < off[c + 1]; e++) ns += cnb[(int)(list[e] & src_mask)];
-    const int64_t entries = off[c + 1] - off[c];
-    const int64_t k = max((int64_t)1, min((ns * cnb[c] + piece_pairs - 1) / piece_pairs, entries));
-    kcnt[w] = (int32_t)k;
-    psz[w] = k > 1 ? (int32_t)(k * cnb[c]) : 0;
-  }
-}
-
 // Queue key of an item of that many body pairs: decreasing work in steps of an
 // eighth of an octave, so that one radix pass orders the queue (exact order took
 // four, 12 launches, and shortens the tail by nothing that shows).
@@ -99,14 +81,42 @@ __device__ __forceinline__ uint64_t work_key(uint64_t work) {
   return 255 - min(255, 8 * max(e - 4, 0) + f);
 }
 
+// per non-empty leaf w (eight threads): its work key, pieces k (>= 1) and partial
+// rows (k * nt when split)
+__global__ void __launch_bounds__(256) leaf_pieces(
+    const int32_t *__restrict__ leaves, int64_t nleaves, const int32_t *__restrict__ off,
+    const uint64_t *__restrict__ list, uint64_t src_mask, const int32_t *__restrict__ cnb,
+    int64_t piece_pairs, uint8_t *__restrict__ wkey, int32_t *__restrict__ kcnt,
+    int32_t *__restrict__ psz) {
+  const int sub = threadIdx.x & 7;
+  const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 3;
+  for (int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >> 3; w0 < nleaves;
+       w0 += stride) {  // warp-uniform
+    const int64_t w = w0 + ((threadIdx.x & 31) >> 3);
+    const bool in = w < nleaves;
+    const int c = in ? leaves[w] : 0;
+    const int e0 = off[c], e1 = in ? off[c + 1] : e0;
+    int64_t ns = 0;
+    for (int e = e0 + sub; e < e1; e += 8) ns += cnb[(int)(list[e] & src_mask)];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) ns += __shfl_xor_sync(0xffffffffu, ns, o);
+    if (!in || sub != 0) continue;
+    const int64_t entries = e1 - e0;
+    const int64_t k = max((int64_t)1, min((ns * cnb[c] + piece_pairs - 1) / piece_pairs, entries));
+    wkey[w] = (uint8_t)work_key((uint64_t)ns * (uint64_t)cnb[c]);
+    kcnt[w] = (int32_t)k;
+    psz[w] = k > 1 ? (int32_t)(k * cnb[c]) : 0;
+  }
+}
+
 // Items of leaf w at koff[w]..: cut its list greedily where the pairs reach
 // piece_pairs (at most k pieces; unused slots become empty pieces with
 // zeroed partials).  Work key = nt * sources of the piece, for the queue.
 __global__ void emit_items(const int32_t *__restrict__ leaves, int64_t nleaves,
                            const int32_t *__restrict__ off, const uint64_t *__restrict__ list,
                            uint64_t src_mask, const int32_t *__restrict__ cnb,
-                           int64_t piece_pairs, const int32_t *__restrict__ kcnt,
-                           const int32_t *__restrict__ koff,
+                           int64_t piece_pairs, const uint8_t *__restrict__ wkey,
+                           const int32_t *__restrict__ kcnt, const int32_t *__restrict__ koff,
                            const int32_t *__restrict__ poff, WorkItem *__restrict__ items,
                            uint64_t *__restrict__ keys, uint32_t *__restrict__ vals,
                            double *__restrict__ part) {
@@ -115,24 +125,24 @@ __global__ void emit_items(const int32_t *__restrict__ leaves, int64_t nleaves,
     const int c = leaves[w];
     const int e0 = off[c], e1 = off[c + 1], k = kcnt[w], nt = cnb[c];
     const int base = koff[w];
+    if (k == 1) {  // the whole list (an empty one still writes the leaf's zero sums)
+      items[base] = WorkItem{c, e0, e1, -1};
+      keys[base] = wkey[w];
+      vals[base] = (uint32_t)base;
+      continue;
+    }
     int j = 0, ea = e0;
     int64_t acc = 0;
     for (int e = e0; e < e1; e++) {
       acc += cnb[(int)(list[e] & src_mask)];
-      if ((k > 1 && acc * nt >= piece_pairs && j < k - 1) || e == e1 - 1) {
-        items[base + j] = WorkItem{c, ea, e + 1, k > 1 ? poff[w] + j * nt : -1};
+      if ((acc * nt >= piece_pairs && j < k - 1) || e == e1 - 1) {
+        items[base + j] = WorkItem{c, ea, e + 1, poff[w] + j * nt};
         keys[base + j] = work_key((uint64_t)acc * (uint64_t)nt);
         vals[base + j] = (uint32_t)(base + j);
         j++;
         ea = e + 1;
         acc = 0;
       }
-    }
-    if (e1 == e0) {  // no list: one empty item still writes the leaf's zero sums
-      items[base] = WorkItem{c, e0, e0, -1};
-      keys[base] = work_key(0);
-      vals[base] = (uint32_t)base;
-      j = 1;
     }
     for (; j < k; j++) {  // unused pieces: empty, zero partials
       items[base + j] = WorkItem{c, e1, e1, poff[w] + j * nt};
@@ -144,18 +154,19 @@ __global__ void emit_items(const int32_t *__restrict__ leaves, int64_t nleaves,
 }
 
 // trg rows of split leaves = sum of their pieces' partial rows, in piece order
-// (eight threads per leaf)
+// (a warp per leaf, the rows' loads in flight together)
 __global__ void split_reduce(const int32_t *__restrict__ leaves, int64_t nleaves,
                              const int32_t *__restrict__ cbeg, const int32_t *__restrict__ cnb,
                              const int32_t *__restrict__ kcnt, const int32_t *__restrict__ poff,
                              const double *__restrict__ part, double *__restrict__ trg) {
-  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; w < nleaves;
-       w += ((int64_t)gridDim.x * blockDim.x) >> 3) {
+  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nleaves;
+       w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const int k = kcnt[w];
     if (k <= 1) continue;
     const int c = leaves[w], nt = cnb[c], b0 = cbeg[c];
-    for (int t = threadIdx.x & 7; t < nt; t += 8) {
+    for (int t = threadIdx.x & 31; t < nt; t += 32) {
       double4 acc = make_double4(0, 0, 0, 0);
+#pragma unroll 8
       for (int j = 0; j < k; j++) {
         const double4 v =
             reinterpret_cast<const double4 *>(part)[(int64_t)poff[w] + (int64_t)j * nt + t];
@@ -179,20 +190,22 @@ __device__ __forceinline__ int next_leaf(int *counter, int lane) {
   return __shfl_sync(0xffffffffu, w, 0);
 }
 
-// Shape of a tile of nt <= 128 targets: kR targets per lane, L = ceil(nt/kR)
-// lanes per group, G = 32/L groups that split the sources.  Time per source
-// ~ kR / G: the least of kR = 4, 3, 1 (ties: the larger kR, fewer shared loads
-// and more independent chains per lane).  kR = 2 would fill as many lanes on
-// average (leaves of 16 to 64 bodies: 89 % with or without it), and every
-// variant less leaves more room in the instruction cache, where stalls were
-// half as frequent again as issue with four variants.
-constexpr int kTileTargets = 128;
+// Shape of a tile of nt targets: kR targets per lane, L = ceil(nt/kR) lanes per
+// group, G = 32/L groups that split the sources.  Time per source ~ kR / G: the
+// least of the kernel's three kR (ties: the larger kR, fewer shared loads and
+// more independent chains per lane).  Three, because every variant takes room in
+// the instruction cache, where stalls were half as frequent again as issue with
+// four.  FP64 uses 4, 3, 1 (89 % of the lanes on leaves of 16 to 64 bodies);
+// the mixed kernel 3, 2, 1 (87 %): a fourth target's registers cost it more than
+// the lanes (1M Plummer 1.83 against 1.93 ms, 16M sphere 26.4 against 26.7).
+template <int kR0, int kR1>
 __device__ __forceinline__ void tile_shape(int nt, int &R, int &L, int &G) {
-  R = 4;
-  L = (nt + 3) >> 2;
+  R = kR0;
+  L = (nt + kR0 - 1) / kR0;
   G = 32 / L;
 #pragma unroll
-  for (int r = 3; r >= 1; r -= 2) {
+  for (int i = 0; i < 2; i++) {
+    const int r = i == 0 ? kR1 : 1;
     const int l = (nt + r - 1) / r;
     if (l > 32) break;
     const int g = 32 / l;
@@ -347,10 +360,10 @@ __global__ void __launch_bounds__(kThreads, kFp64Blocks) p2p_fp64_kernel(
     const int c = it.leaf;
     const int tb0 = cbeg[c], nt_all = cnb[c];
     double4 *out = item_out(it, tb0, trg, part);
-    for (int tbase = 0; tbase < nt_all; tbase += kTileTargets) {
-      const int nt = min(nt_all - tbase, kTileTargets);
+    for (int tbase = 0; tbase < nt_all; tbase += 128) {
+      const int nt = min(nt_all - tbase, 128);
       int R, L, G;
-      tile_shape(nt, R, L, G);
+      tile_shape<4, 3>(nt, R, L, G);
 #define TB_FP64_TILE(RR)                                                                         \
   fp64_tile<RR>(lane, tb0 + tbase, nt, L, G, it.e0, it.e1, list, src_mask, cbeg, cnb, sx, sy, sz, \
                 sq, src[wi], out + tbase)
@@ -658,15 +671,15 @@ __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
     double4 *out = item_out(it, tb0, trg, part);
     const double tcx = ccen[3 * c], tcy = ccen[3 * c + 1], tcz = ccen[3 * c + 2];
     const double tw = cmax[3 * c] - cmin[3 * c];
-    for (int tbase = 0; tbase < nt_all; tbase += kTileTargets) {
-      const int nt = min(nt_all - tbase, kTileTargets);
+    for (int tbase = 0; tbase < nt_all; tbase += 32 * kMixedMaxR) {
+      const int nt = min(nt_all - tbase, 32 * kMixedMaxR);
       int R, L, G;
-      tile_shape(nt, R, L, G);
+      tile_shape<3, 2>(nt, R, L, G);
 #define TB_MIXED_TILE(RR)                                                                        \
   mixed_tile<RR>(lane, tb0 + tbase, nt, L, G, e0, e1, tcx, tcy, tcz, tw, list, src_mask, cbeg,  \
                  cnb, ccen, cmin, cmax, rel_hi, rel_lo, sm[wi], out + tbase)
-      if (R == 4) TB_MIXED_TILE(4);
-      else if (R == 3) TB_MIXED_TILE(3);
+      if (R == 3) TB_MIXED_TILE(3);
+      else if (R == 2) TB_MIXED_TILE(2);
       else TB_MIXED_TILE(1);
 #undef TB_MIXED_TILE
     }
@@ -686,9 +699,10 @@ int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
   TB_CUDA(ctx, ctx->p2p_koff.ensure(nl + 1, s));
   TB_CUDA(ctx, ctx->p2p_psz.ensure(nl + 1, s));
   TB_CUDA(ctx, ctx->p2p_poff.ensure(nl + 1, s));
-  leaf_pieces<<<grid_for(nl, 256), 256, 0, s>>>(leaves, nl, ctx->p2p_off.p, ctx->p2p.p,
-                                                 mask, ctx->cnb.p, piece_pairs,
-                                                 ctx->p2p_kcnt.p, ctx->p2p_psz.p);
+  TB_CUDA(ctx, ctx->p2p_key.ensure(nl + 1, s));
+  leaf_pieces<<<grid_for(8 * nl, 256), 256, 0, s>>>(leaves, nl, ctx->p2p_off.p, ctx->p2p.p, mask,
+                                                    ctx->cnb.p, piece_pairs, ctx->p2p_key.p,
+                                                    ctx->p2p_kcnt.p, ctx->p2p_psz.p);
   TB_LAUNCH_CHECK(ctx);
   TB_TRY(scan_exclusive(ctx, ctx->p2p_kcnt.p, ctx->p2p_koff.p, nl, ctx->p2p_koff.p + nl));
   TB_TRY(scan_exclusive(ctx, ctx->p2p_psz.p, ctx->p2p_poff.p, nl, ctx->p2p_poff.p + nl));
@@ -713,8 +727,8 @@ int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
   TB_CUDA(ctx, ctx->p2p_order_alt.ensure(ni + 1, s));
   TB_CUDA(ctx, ctx->p2p_counter.ensure(4, s));
   emit_items<<<grid_for(nl, 256), 256, 0, s>>>(
-      leaves, nl, ctx->p2p_off.p, ctx->p2p.p, mask, ctx->cnb.p, piece_pairs, ctx->p2p_kcnt.p,
-      ctx->p2p_koff.p, ctx->p2p_poff.p, reinterpret_cast<WorkItem *>(ctx->p2p_items.p),
+      leaves, nl, ctx->p2p_off.p, ctx->p2p.p, mask, ctx->cnb.p, piece_pairs, ctx->p2p_key.p,
+      ctx->p2p_kcnt.p, ctx->p2p_koff.p, ctx->p2p_poff.p, reinterpret_cast<WorkItem *>(ctx->p2p_items.p),
       ctx->p2p_wkey.p, ctx->p2p_order.p, ctx->p2p_part.p);
   TB_LAUNCH_CHECK(ctx);
   uint64_t *k = ctx->p2p_wkey.p, *ka = ctx->p2p_wkey_alt.p;
@@ -737,7 +751,7 @@ int p2p_finish(tapas_b200_ctx *ctx) {
   if (!ctx->p2p_split) return TAPAS_B200_OK;
   int64_t nl = 0;
   const int32_t *leaves = work_leaves(ctx, nl);
-  split_reduce<<<grid_for(8 * nl, 256), 256, 0, ctx->stream>>>(
+  split_reduce<<<grid_for(32 * nl, 256), 256, 0, ctx->stream>>>(
       leaves, nl, ctx->cbeg.p, ctx->cnb.p, ctx->p2p_kcnt.p, ctx->p2p_poff.p,
       ctx->p2p_part.p, ctx->trg.p);
   TB_LAUNCH_CHECK(ctx);
