@@ -159,6 +159,7 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
   ctx->counters.release();
   ctx->trav_geo.release();
   ctx->tree_nodes.release();
+  ctx->tree_cnt.release();
   ctx->body_pack.release();
   ctx->trav_meta.release();
   ctx->list_src.release();

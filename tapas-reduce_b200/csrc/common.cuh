@@ -187,6 +187,7 @@ struct tapas_b200_ctx {
   tb::DBuf<double> cmin, cmax, ccen;    // 3 doubles per cell (x,y,z interleaved)
   tb::DBuf<double4> trav_geo;          // traversal: per cell {centre, MAC radius for this theta}
   tb::DBuf<int2> trav_meta;            // traversal: per cell {nb, first child or -1 for a leaf}
+  tb::DBuf<uint32_t> tree_cnt;          // non-leaf cells per level and tile of bodies
   tb::DBuf<int2> tree_nodes;            // per non-leaf cell {first body, cell}
   tb::DBuf<int32_t> flag, flag_scan;    // per-cell scratch
   tb::DBuf<int32_t> leaf_list;          // indices of non-empty leaves

@@ -52,6 +52,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int *smem_warp, int &total
 __global__ void __launch_bounds__(kScanThreads) scan_tiles(const int32_t *__restrict__ in,
                                                            int32_t *__restrict__ out, int64_t n,
                                                            int32_t *__restrict__ block_sums) {
+  // block_sums: per block its sum (for one block, the total); may be null
   __shared__ int sw[33];
   const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
   int v[kScanItems];
@@ -83,21 +84,17 @@ __global__ void __launch_bounds__(kScanThreads) scan_add(int32_t *__restrict__ o
   }
 }
 
-// Sum of the last input and last output element = total.
-__global__ void scan_total(const int32_t *in, const int32_t *out, int64_t n, int32_t *total) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *total = n > 0 ? out[n - 1] + in[n - 1] : 0;
-}
-
 }  // namespace
 
 // Scan of in[0..n) into out using scratch[scratch_off..) for the block sums of
-// this level and the levels below (recursive reduce-then-scan).
+// this level and the levels below (recursive reduce-then-scan); the last level's
+// one block writes the total.
 static int scan_level(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
-                      size_t scratch_off) {
+                      size_t scratch_off, int32_t *d_total) {
   cudaStream_t s = ctx->stream;
   const int64_t nb = (n + kScanTile - 1) / kScanTile;
   if (nb == 1) {
-    scan_tiles<<<1, kScanThreads, 0, s>>>(in, out, n, nullptr);
+    scan_tiles<<<1, kScanThreads, 0, s>>>(in, out, n, d_total);
     TB_LAUNCH_CHECK(ctx);
     return TAPAS_B200_OK;
   }
@@ -105,7 +102,7 @@ static int scan_level(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int6
   int32_t *offs = sums + nb + 32;
   scan_tiles<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, sums);
   TB_LAUNCH_CHECK(ctx);
-  TB_TRY(scan_level(ctx, sums, offs, nb, scratch_off + 2 * (size_t)nb + 64));
+  TB_TRY(scan_level(ctx, sums, offs, nb, scratch_off + 2 * (size_t)nb + 64, d_total));
   scan_add<<<(unsigned)nb, kScanThreads, 0, s>>>(out, n, offs);
   TB_LAUNCH_CHECK(ctx);
   return TAPAS_B200_OK;
@@ -130,12 +127,7 @@ int scan_exclusive(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t
     m = nb;
   }
   TB_CUDA(ctx, ctx->scan_tmp.ensure(need, s));
-  TB_TRY(scan_level(ctx, in, out, n, 0));
-  if (d_total) {
-    scan_total<<<1, 32, 0, s>>>(in, out, n, d_total);
-    TB_LAUNCH_CHECK(ctx);
-  }
-  return TAPAS_B200_OK;
+  return scan_level(ctx, in, out, n, 0, d_total);
 }
 
 // ---------------------------------------------------------------------------
@@ -367,12 +359,153 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(
   }
 }
 
+// The whole sort of at most kSortTile elements by one block, in shared memory: a
+// pass ranks and places the tile as radix_scatter does.  (Up to 4096 elements
+// the passes' three launches each were the time: 24 for 57 key bits, 0.14 ms.)
+template <bool kHasVals>
+__global__ void __launch_bounds__(kSortThreads) radix_block(
+    const uint64_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
+    uint64_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int n, int begin_bit,
+    int end_bit) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint32_t *wcnt = reinterpret_cast<uint32_t *>(smem_raw);
+  uint32_t *tstart = wcnt + kSortWarps * kRadix;
+  uint64_t *skeys = reinterpret_cast<uint64_t *>(tstart + 2 * kRadix);
+  uint32_t *svals = reinterpret_cast<uint32_t *>(skeys + kSortTile);
+  __shared__ uint32_t ws[kRadix / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const int first = warp * (32 * kSortItems) + lane;  // this thread's elements: + 32 it
+  uint64_t k[kSortItems];
+  uint32_t v[kSortItems];
+#pragma unroll
+  for (int it = 0; it < kSortItems; it++) {
+    const int g = first + 32 * it;
+    k[it] = g < n ? keys_in[g] : ~0ull;
+    if (kHasVals) v[it] = g < n ? vals_in[g] : 0u;
+  }
+  for (int shift = begin_bit; shift < end_bit; shift += kRadixBits) {
+    for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads) wcnt[i] = 0;
+    __syncthreads();
+    uint32_t rank[kSortItems];
+#pragma unroll
+    for (int it = 0; it < kSortItems; it++) {
+      const bool valid = first + 32 * it < n;
+      const uint32_t d = digit_of(k[it], shift);
+      unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+      for (int b = 0; b < kRadixBits; b++) {
+        const bool bit = (d >> b) & 1u;
+        const unsigned bb = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? bb : ~bb;
+      }
+      rank[it] = 0;
+      if (valid) {
+        const uint32_t before = wcnt[warp * kRadix + d];
+        rank[it] = before + __popc(peers & lt_mask);
+        __syncwarp(peers);
+        if (lane == __ffs(peers) - 1) wcnt[warp * kRadix + d] = before + __popc(peers);
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    uint32_t sum = 0, incl = 0;
+    if (threadIdx.x < kRadix) {
+#pragma unroll
+      for (int w = 0; w < kSortWarps; w++) {
+        const uint32_t c = wcnt[w * kRadix + threadIdx.x];
+        wcnt[w * kRadix + threadIdx.x] = sum;
+        sum += c;
+      }
+      incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      if (lane == 31) ws[warp] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x < kRadix) {
+      uint32_t base = 0;
+      for (int w = 0; w < warp; w++) base += ws[w];
+      tstart[threadIdx.x] = base + incl - sum;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < kSortItems; it++) {
+      if (first + 32 * it >= n) continue;
+      const uint32_t d = digit_of(k[it], shift);
+      const uint32_t pos = tstart[d] + wcnt[warp * kRadix + d] + rank[it];
+      skeys[pos] = k[it];
+      if (kHasVals) svals[pos] = v[it];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < kSortItems; it++) {
+      const int g = first + 32 * it;
+      if (g >= n) continue;
+      k[it] = skeys[g];
+      if (kHasVals) v[it] = svals[g];
+    }
+  }
+#pragma unroll
+  for (int it = 0; it < kSortItems; it++) {
+    const int g = first + 32 * it;
+    if (g >= n) continue;
+    keys_out[g] = k[it];
+    if (kHasVals) vals_out[g] = v[it];
+  }
+}
+
+// Completes the order of elements sorted on the bits from low_bits up: the run of
+// elements that agree there is put in order of all its bits by the thread of its
+// first element (stable insertion); *longest becomes at least the length of
+// any run too long for that, which is left as it is.
+__global__ void __launch_bounds__(256) order_runs(uint64_t *__restrict__ keys,
+                                                  uint32_t *__restrict__ vals, int64_t n,
+                                                  int low_bits, int max_run,
+                                                  int *__restrict__ longest) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i + 1 < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    // only high bits are compared: a thread of another run may be reordering the
+    // neighbours' low ones
+    const uint64_t h = keys[i] >> low_bits;
+    if (keys[i + 1] >> low_bits != h || (i > 0 && keys[i - 1] >> low_bits == h)) continue;
+    int64_t e = i + 2;
+    while (e < n && e - i <= max_run && keys[e] >> low_bits == h) e++;
+    if (e - i > max_run) {
+      atomicMax(longest, (int)(e - i));
+      continue;
+    }
+    for (int64_t a = i + 1; a < e; a++) {
+      const uint64_t k = keys[a];
+      const uint32_t v = vals[a];
+      int64_t b = a;
+      for (; b > i && keys[b - 1] > k; b--) {
+        keys[b] = keys[b - 1];
+        vals[b] = vals[b - 1];
+      }
+      keys[b] = k;
+      vals[b] = v;
+    }
+  }
+}
+
 size_t scatter_smem_bytes() {
   return sizeof(uint32_t) * (kSortWarps * kRadix + 2 * kRadix) + sizeof(uint64_t) * kSortTile +
          sizeof(uint32_t) * kSortTile;
 }
 
 }  // namespace
+
+int order_equal_runs(tapas_b200_ctx *ctx, uint64_t *keys, uint32_t *vals, int64_t n, int low_bits,
+                     int max_run, int *longest) {
+  order_runs<<<grid_for(n, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(keys, vals, n, low_bits,
+                                                                         max_run, longest);
+  TB_LAUNCH_CHECK(ctx);
+  return TAPAS_B200_OK;
+}
 
 int scan_rows(tapas_b200_ctx *ctx, uint32_t *rows, int nrows, int ncols, uint32_t *totals) {
   radix_scan_rows<<<nrows, 1024, 0, ctx->stream>>>(rows, ncols, totals);
@@ -388,6 +521,18 @@ int radix_sort(tapas_b200_ctx *ctx, uint64_t *&keys, uint64_t *&keys_alt, uint32
     return TAPAS_B200_ERR_ARG;
   }
   cudaStream_t s = ctx->stream;
+  if (n <= kSortTile) {
+    const size_t smem = scatter_smem_bytes();
+    auto kernel = vals ? radix_block<true> : radix_block<false>;
+    TB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+    kernel<<<1, kSortThreads, smem, s>>>(keys, vals, keys_alt, vals_alt, (int)n, begin_bit,
+                                         end_bit);
+    TB_LAUNCH_CHECK(ctx);
+    std::swap(keys, keys_alt);
+    if (vals) std::swap(vals, vals_alt);
+    return TAPAS_B200_OK;
+  }
   const int ntiles = (int)((n + kSortTile - 1) / kSortTile);
   TB_CUDA(ctx, ctx->sort_hist.ensure((size_t)kRadix * ntiles + kRadix, s));
   uint32_t *hist = ctx->sort_hist.p;

@@ -17,4 +17,10 @@ int scan_rows(tapas_b200_ctx *ctx, uint32_t *rows, int nrows, int ncols, uint32_
 int radix_sort(tapas_b200_ctx *ctx, uint64_t *&keys, uint64_t *&keys_alt, uint32_t *&vals,
                uint32_t *&vals_alt, int64_t n, int begin_bit, int end_bit);
 
+// After a radix sort on the bits from low_bits up only: orders every run of keys
+// equal there by all bits (stable), except runs of more than max_run, of which
+// *longest (device, 0 before) is raised to a length above max_run.
+int order_equal_runs(tapas_b200_ctx *ctx, uint64_t *keys, uint32_t *vals, int64_t n, int low_bits,
+                     int max_run, int *longest);
+
 }  // namespace tb

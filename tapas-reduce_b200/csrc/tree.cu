@@ -176,6 +176,14 @@ __global__ void init_root(int64_t n, int ncrit, const double *__restrict__ box,
 // level, every level cost six launches and a host round trip: 20k bodies at
 // ncrit 1, 18 levels, 0.67 ms.)
 // ---------------------------------------------------------------------------
+// The body sort takes the 40 highest of the 57 key bits (13 of 19 levels; five radix
+// passes instead of eight) and orders the few bodies that agree there by
+// insertion; more than kMaxRun of them in one place (1 in 10^4 of the root's
+// width) and the sort is run on all bits instead, which the read-back of the
+// level sizes tells.
+constexpr int kSortLow = kDepthBits + 3 * kMaxDepth - 40;
+constexpr int kMaxRun = 32;
+
 constexpr int kTreeSteps = 8;                       // bodies per thread
 constexpr int kTreeTile = kBlock * kTreeSteps;      // bodies per block
 constexpr int kTreeLevels = kMaxDepth;              // levels that can have non-leaf cells
@@ -460,14 +468,22 @@ int build_tree(tapas_b200_ctx *ctx, int ncrit) {
         ctx->keys.p, ctx->idx.p, ctx->body_pack.p);
     TB_LAUNCH_CHECK(ctx);
   }
-  {
-    PhaseTimer t(ctx, &ctx->timings.sort);
+  const int ntiles = (int)((n + kTreeTile - 1) / kTreeTile);
+  // counts per level and tile, level totals, longest unordered run
+  TB_CUDA(ctx, ctx->tree_cnt.ensure((size_t)kTreeLevels * (ntiles + 1) + 1, s));
+  uint32_t *cnt = ctx->tree_cnt.p, *d_total = cnt + (size_t)kTreeLevels * ntiles;
+  int *d_longest = reinterpret_cast<int *>(d_total + kTreeLevels);
+  // Sorts on the key bits from `low` up (bits 4..0, the depth, are 19 for every
+  // body), completes the order, and gathers the bodies.
+  auto sort_bodies = [&](int low) -> int {
     uint64_t *k = ctx->keys.p, *ka = ctx->keys_alt.p;
     uint32_t *v = ctx->idx.p, *va = ctx->idx_alt.p;
-    // Depth bits (4..0) are 19 for every body key; sort on bits 5..61.
-    TB_TRY(radix_sort(ctx, k, ka, v, va, n, kDepthBits, kDepthBits + 3 * kMaxDepth));
+    TB_TRY(radix_sort(ctx, k, ka, v, va, n, low, kDepthBits + 3 * kMaxDepth));
     if (k != ctx->keys.p) { std::swap(ctx->keys.p, ctx->keys_alt.p); std::swap(ctx->keys.cap, ctx->keys_alt.cap); }
     if (v != ctx->idx.p) { std::swap(ctx->idx.p, ctx->idx_alt.p); std::swap(ctx->idx.cap, ctx->idx_alt.cap); }
+    TB_CUDA(ctx, cudaMemsetAsync(d_longest, 0, sizeof(int), s));
+    if (low > kDepthBits)
+      TB_TRY(order_equal_runs(ctx, ctx->keys.p, ctx->idx.p, n, low, kMaxRun, d_longest));
     if (ctx->q_pending) {  // the charges' copy ran alongside the keys and the sort
       TB_CUDA(ctx, cudaStreamWaitEvent(s, ctx->q_ready, 0));
       pack_charges<<<grid_for(n, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(ctx->q.p, n,
@@ -478,19 +494,27 @@ int build_tree(tapas_b200_ctx *ctx, int ncrit) {
     gather_bodies<<<grid_for(n, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
         ctx->body_pack.p, ctx->idx.p, n, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->sq.p);
     TB_LAUNCH_CHECK(ctx);
+    return TAPAS_B200_OK;
+  };
+  {
+    PhaseTimer t(ctx, &ctx->timings.sort);
+    TB_TRY(sort_bodies(kSortLow));
   }
   PhaseTimer t(ctx, &ctx->timings.tree);
-  const int ntiles = (int)((n + kTreeTile - 1) / kTreeTile);
-  TB_CUDA(ctx, ctx->sort_hist.ensure((size_t)kTreeLevels * (ntiles + 1), s));
-  uint32_t *cnt = ctx->sort_hist.p, *d_total = cnt + (size_t)kTreeLevels * ntiles;
   TB_CUDA(ctx, ctx->pinned.ensure(256));
-  count_nonleaves<<<ntiles, kBlock, 0, s>>>(ctx->keys.p, n, ncrit, ntiles, cnt);
-  TB_LAUNCH_CHECK(ctx);
-  TB_TRY(scan_rows(ctx, cnt, kTreeLevels, ntiles, d_total));
   uint32_t *h_total = reinterpret_cast<uint32_t *>(ctx->pinned.p);
-  TB_CUDA(ctx, cudaMemcpyAsync(h_total, d_total, kTreeLevels * sizeof(uint32_t),
-                               cudaMemcpyDeviceToHost, s));
-  TB_CUDA(ctx, cudaStreamSynchronize(s));
+  for (bool complete = false;;) {
+    count_nonleaves<<<ntiles, kBlock, 0, s>>>(ctx->keys.p, n, ncrit, ntiles, cnt);
+    TB_LAUNCH_CHECK(ctx);
+    TB_TRY(scan_rows(ctx, cnt, kTreeLevels, ntiles, d_total));
+    TB_CUDA(ctx, cudaMemcpyAsync(h_total, d_total, (kTreeLevels + 1) * sizeof(uint32_t),
+                                 cudaMemcpyDeviceToHost, s));
+    TB_CUDA(ctx, cudaStreamSynchronize(s));
+    if (h_total[kTreeLevels] == 0 || complete) break;
+    // many bodies in one cell of level 13: sort on all bits
+    complete = true;
+    TB_TRY(sort_bodies(kDepthBits));
+  }
   LevelRanks ranks;
   int64_t nnode = 0;
   int depth = 0;

@@ -605,3 +605,53 @@ def test_near_field_tile_shapes(n, ncrit, tb, ctx, oracle_mod):
     rmx = ctx.evaluate(x, y, z, q, P=6, ncrit=ncrit, theta=0.3, precision=tb.MIXED)
     ep, ea = oracle_mod.rel_l2(rmx, r64)
     assert ep < 2e-6 and ea < 2e-6
+
+
+def _check_tree(tb, ctx, oracle_mod, x, y, z, q, ncrit):
+    o = oracle_mod.Oracle(x, y, z, q, P=2, ncrit=ncrit, theta=5.0)
+    info = ctx.partition(x, y, z, q, ncrit=ncrit)
+    oi, ok, _ = o.bodies()
+    gi, gk = ctx.sorted_bodies()
+    assert np.array_equal(gk, ok)
+    assert np.array_equal(gi, oi)
+    oc, gc = o.cells(), ctx.cells()
+    go, oo = _cells_by_key(gc), _cells_by_key(oc)
+    for name, ours in (("key", "key"), ("leaf", "leaf"), ("nb", "nb"), ("center", "center"),
+                       ("width", "width")):
+        assert np.array_equal(gc[ours][go], oc[name][oo]), name
+    assert np.array_equal(gc["bbeg"][go].astype(np.int64), oc["bid"][oo])
+    # breadth first, children after their parent, eight in a row
+    assert info["n_cells"] == len(gc["key"])
+    level = gc["key"] & np.uint64(31)
+    assert np.all(np.diff(level.astype(np.int64)) >= 0)
+    inner = np.flatnonzero(gc["leaf"] == 0)
+    for k in range(8):
+        assert np.array_equal(gc["parent"][gc["child0"][inner] + k], inner)
+    assert np.all(gc["child0"][gc["leaf"] != 0] == -1)
+
+
+@pytest.mark.parametrize("n,ncrit", [(2047, 1), (2048, 7), (2049, 300), (4096, 1), (4097, 2),
+                                     (6145, 16), (33, 32), (300, 299)])
+def test_tree_all_levels_at_once(n, ncrit, tb, ctx, oracle_mod):
+    """Body counts around the counting pass's warps and blocks and the one-block
+    sort's limit, few and many levels, against the oracle's tree, bit for bit."""
+    x, y, z, q = tb.datasets.make("two_gaussians" if n % 2 else "uniform_cube", n, 91)
+    _check_tree(tb, ctx, oracle_mod, x, y, z, q, ncrit)
+
+
+@pytest.mark.parametrize("n", [1500, 9000])
+@pytest.mark.parametrize("longest", [3, 31, 33])
+def test_tree_bodies_close_in_one_cell(n, longest, tb, ctx, oracle_mod):
+    """Clusters far smaller than a cell of level 13: the sort orders runs of up to
+    32 such bodies after its high key bits and starts over on all bits for a
+    longer one; some bodies coincide (equal keys stay in input order)."""
+    x, y, z, q = [a.copy() for a in tb.datasets.make("uniform_cube", n, 92)]
+    rng = np.random.default_rng(5)
+    for k, at in enumerate(range(0, n - longest, n // 7)):
+        m = longest if k == 3 else 1 + k % 3
+        idx = rng.permutation(n)[:m]
+        for a, c in ((x, 0.3), (y, -0.2), (z, 0.6)):
+            a[idx] = c + 0.1 * k + 3e-6 * rng.random(m)
+        if m > 1:
+            x[idx[1]], y[idx[1]], z[idx[1]] = x[idx[0]], y[idx[0]], z[idx[0]]
+    _check_tree(tb, ctx, oracle_mod, x, y, z, q, 4)
