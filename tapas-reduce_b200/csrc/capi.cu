@@ -167,7 +167,6 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
   ctx->L.release();
   ctx->op_m2m.release();
   ctx->op_l2l.release();
-  ctx->op_part.release();
   // mixed-form state: near-field offsets, P2P work items, tensor-core M2L
   for (auto *b : {&ctx->rel4, &ctx->rel_lo}) b->release();
   for (auto *b : {&ctx->p2p_wkey, &ctx->p2p_wkey_alt}) b->release();

@@ -256,7 +256,6 @@ struct tapas_b200_ctx {
   tb::DBuf<double2> M, L;               // ncells x nterm complex FP64
   tb::DBuf<double> op_m2m, op_l2l;      // per level: child<->parent translation operators
   int level_ops_P = 0;                  // order the operators were built for (0: none)
-  tb::DBuf<double> op_part;             // M2M of small levels: per-octant partial products
 
   tb::Mlp *mlp = nullptr;               // learned chooser network, if created
 

@@ -602,246 +602,224 @@ __global__ void __launch_bounds__(kThreads) l2p32_bodies(
 //   L2L:  L[children_i] (16NT) += Tdn_l (16NT x 2NT) . L[parent_i]
 // are one FP64 GEMM per level over the level's non-leaf cells i.  The
 // operators are built from one representative parent of the level with the
-// reference's formulas, one thread per (target, source) block; M2M rows of degree j read only source degrees <= j
-// and L2L rows of degree j only source degrees >= j, and the GEMM skips the
-// zero ranges this leaves.
+// reference's formulas, one thread per (target, source) pair; M2M rows of
+// degree j read only source degrees <= j and L2L rows of degree j only source
+// degrees >= j, and the operators are stored without the zero ranges this leaves.
 // ---------------------------------------------------------------------------
 constexpr int kMaxLevels = kMaxDepth + 1;
 struct LevelFirstChild {
   int64_t c0[kMaxLevels];  // first cell of level l + 1 (child 0 of the level's first parent)
 };
 
-__host__ __device__ __forceinline__ int degree_of(int t) {
-  int j = 0;
-  while ((j + 1) * (j + 2) / 2 <= t) j++;
-  return j;
-}
+constexpr int kOutBlock = 32;  // outputs of one block of an operator
+constexpr int kStep = 16;      // sources of one block of an operator
 
-// The real 2 x 2 block mapping a source coefficient to a target one when
-// out = a * src + b * conj(src):
+// A level operator: per octant the blocks of 32 outputs in order, each with its
+// source blocks of 16 from first(b) on, stored in the multiplication's order
+// (dmma_m16n8k16): for each 8 outputs f and half h of a lane's four sources, the
+// two doubles of each lane.
+template <int P, bool kUp>
+struct LevelOp {
+  static constexpr int NT = P * (P + 1) / 2;
+  static constexpr int K = 2 * NT;
+  static constexpr int NB = (K + kOutBlock - 1) / kOutBlock;
+  __host__ __device__ static constexpr int degree(int t) {
+    int j = 0;
+    while ((j + 1) * (j + 2) / 2 <= t) j++;
+    return j;
+  }
+  __host__ __device__ static constexpr int first(int b) {
+    if (kUp) return 0;
+    const int j = degree(b * (kOutBlock / 2));
+    return j * (j + 1) / kStep;
+  }
+  __host__ __device__ static constexpr int steps(int b) {
+    if (!kUp) return (K + kStep - 1) / kStep - first(b);
+    const int last = (b + 1) * (kOutBlock / 2) - 1;
+    const int j = degree(last < NT ? last : NT - 1);
+    return ((j + 1) * (j + 2) + kStep - 1) / kStep;
+  }
+  __host__ __device__ static constexpr int blocks(int b) {  // blocks before output block b
+    int s = 0;
+    for (int i = 0; i < b; i++) s += steps(i);
+    return s;
+  }
+  static constexpr int NBLK = blocks(NB);                          // per octant
+  static constexpr size_t OCTANT = (size_t)NBLK * kOutBlock * kStep;  // doubles
+};
+
+// One block of the grid (levels with children, 8 octants, parts): its share of
+// one (level, octant) operator.  Entry (target (j,k), source (j',k')) collects
+// the terms of the reference's loops that read that source: M2M (:165-206) with
+// n = j - j' and m = k - k' (source as is) or m = k + k' (conjugated); L2L
+// (:309-345) with n = j' and m = k' (as is) or m = -k' (conjugated).  The real
+// 2 x 2 block of out = a * src + b * conj(src):
 //   [Re out]   [a.x + b.x   b.y - a.y] [Re src]
 //   [Im out] = [a.y + b.y   a.x - b.x] [Im src]
-// stored transposed (operators are kept K x R, column k of the map
-// contiguous): colre / colim point at the target's two rows in the source's
-// real / imaginary column.
-__device__ __forceinline__ void store_block(double *colre, double *colim, cd a, cd b) {
-  *reinterpret_cast<double2 *>(colre) = make_double2(a.x + b.x, a.y + b.y);
-  *reinterpret_cast<double2 *>(colim) = make_double2(b.y - a.y, a.x - b.x);
-}
-
-// grid (levels with children, 8 octants, 2: M2M / L2L); every entry of the
-// operators is written.  Entry (target (j,k), source (j',k')) collects the
-// terms of the reference's loops that read that source: M2M (:165-206) with
-// n = j - j' and m = k - k' (source as is) or m = k + k' (conjugated); L2L
-// (:309-345) with n = j' and m = k' (as is) or m = -k' (conjugated).
-template <int P>
-__global__ void __launch_bounds__(256) build_translation_ops(
-    LevelFirstChild lf, const int32_t *__restrict__ cparent, const double *__restrict__ ccen,
-    double *__restrict__ op_up, double *__restrict__ op_dn) {
+template <int P, bool kUp>
+__global__ void __launch_bounds__(256) build_level_op(LevelFirstChild lf,
+                                                      const int32_t *__restrict__ cparent,
+                                                      const double *__restrict__ ccen,
+                                                      double *__restrict__ ops) {
   using S = Sizes<P>;
-  constexpr int NT2 = 2 * S::NT;
+  using O = LevelOp<P, kUp>;
   __shared__ cd Y[S::NY];
+  __shared__ short blk_out[O::NBLK], blk_step[O::NBLK];
   const int l = blockIdx.x, o = blockIdx.y;
-  const bool up = blockIdx.z == 0;
   const int64_t cj = lf.c0[l] + o;
   const int p = cparent[cj];
   const double dx = ccen[3 * p] - ccen[3 * cj], dy = ccen[3 * p + 1] - ccen[3 * cj + 1],
                dz = ccen[3 * p + 2] - ccen[3 * cj + 2];
   // M2M translates by parent - child, L2L by child - parent
-  const Sph sp = up ? sph_of(dx, dy, dz) : sph_of(-dx, -dy, -dz);
+  const Sph sp = kUp ? sph_of(dx, dy, dz) : sph_of(-dx, -dy, -dz);
   if (threadIdx.x < P) multipole_column<P>(threadIdx.x, sp.r, sp.x, sp.y, sp.ei, Y);
+  if (threadIdx.x >= 32 && threadIdx.x < 32 + O::NB) {
+    const int b = threadIdx.x - 32;
+    const int at = O::blocks(b);
+    for (int i = 0; i < O::steps(b); i++) {
+      blk_out[at + i] = (short)b;
+      blk_step[at + i] = (short)(O::first(b) + i);
+    }
+  }
   __syncthreads();
-  for (int e = threadIdx.x; e < S::NT * S::NT; e += blockDim.x) {
-    const int u = e / S::NT, t = e - u * S::NT;  // consecutive threads: consecutive targets
-    int j, k, jp, kp;
-    jk_of(t, j, k);
-    jk_of(u, jp, kp);
+  double2 *op = reinterpret_cast<double2 *>(ops + ((size_t)l * 8 + o) * O::OCTANT);
+  constexpr int kPairs = (kOutBlock / 2) * (kStep / 2);
+  for (int idx = blockIdx.z * blockDim.x + threadIdx.x; idx < O::NBLK * kPairs;
+       idx += gridDim.z * blockDim.x) {
+    const int blk = idx / kPairs, in = idx - blk * kPairs;
+    const int lo = in >> 3, li = in & 7;  // complex target, source within the block
+    const int t = blk_out[blk] * (kOutBlock / 2) + lo, u = blk_step[blk] * (kStep / 2) + li;
     cd a{0, 0}, b{0, 0};
-    if (up) {
-      const int n = j - jp;
-      if (n >= 0) {
-        if (kp >= 1) {
-          const int m = k - kp;
-          if (m >= -n && m <= n) {
-            const double sgn = ((m >= 0) ? 1.0 : oddeven(m)) * oddeven(n);
-            a = scal(sgn, Y[n * n + n - m]);
+    if (t < S::NT && u < S::NT) {
+      int j, k, jp, kp;
+      jk_of(t, j, k);
+      jk_of(u, jp, kp);
+      if (kUp) {
+        const int n = j - jp;
+        if (n >= 0) {
+          if (kp >= 1) {
+            const int m = k - kp;
+            if (m >= -n && m <= n) {
+              const double sgn = ((m >= 0) ? 1.0 : oddeven(m)) * oddeven(n);
+              a = scal(sgn, Y[n * n + n - m]);
+            }
           }
+          const int m = k + kp;
+          if (m <= n) b = scal(oddeven(k + n + m), Y[n * n + n - m]);
         }
-        const int m = k + kp;
-        if (m <= n) b = scal(oddeven(k + n + m), Y[n * n + n - m]);
+      } else {
+        const int n = jp;
+        if (n >= j) {
+          const int base = (n - j) * (n - j) + n - j - k;
+          if (kp >= 1 && kp <= n - j - k) b = scal(oddeven(k), Y[base - kp]);
+          if (n - j >= abs(kp - k)) a = scal(oddeven((kp - k) * (kp < k)), Y[base + kp]);
+        }
       }
-      // K = 16 NT sources (child o's at o * 2NT), R = 2NT targets
-      double *c0 = op_up + (size_t)l * NT2 * 8 * NT2 + (size_t)(o * NT2 + 2 * u) * NT2 + 2 * t;
-      store_block(c0, c0 + NT2, a, b);
-    } else {
-      const int n = jp;
-      if (n >= j) {
-        const int base = (n - j) * (n - j) + n - j - k;
-        if (kp >= 1 && kp <= n - j - k) b = scal(oddeven(k), Y[base - kp]);
-        if (n - j >= abs(kp - k)) a = scal(oddeven((kp - k) * (kp < k)), Y[base + kp]);
-      }
-      // K = 2NT sources, R = 16 NT targets (child o's at o * 2NT)
-      double *c0 = op_dn + (size_t)l * 8 * NT2 * NT2 + (size_t)(2 * u) * (8 * NT2) + o * NT2 + 2 * t;
-      store_block(c0, c0 + 8 * NT2, a, b);
     }
+    const int f = lo >> 2, g = (2 * lo) & 7;
+    double2 *dst = op + (((size_t)blk * 4 + f) * 2 + (li & 1)) * 32 + 4 * g + (li >> 1);
+    dst[0] = make_double2(a.x + b.x, b.y - a.y);
+    dst[4] = make_double2(a.y + b.y, a.x - b.x);
   }
 }
 
-// One level's translation GEMM.  Column i is the level's i-th non-leaf cell:
-// its children are cells c0 + 8i .. c0 + 8i + 7, its index cparent[c0 + 8i].
-struct LevelGemm {
-  const double *At; // operator, transposed: K x R, row k = the map's column k
-  int R, K, nt2;    // nt2 = 2 NT
-  int up;           // 1: M2M (C = A B), 0: L2L (C += A B)
-  int split;        // M2M only: blockIdx.z = octant, partial products to `part`
-  int64_t c0, ncols;
-  const int32_t *cparent;
-  double *X;        // M (up) or L (down) as doubles, nt2 per cell
-  double *part;     // split: [8][ncols][R]
-};
-
-constexpr int kGM = 64, kGN = 64, kGK = 16;  // level_gemm tiling
-constexpr int kLThreads = 128;     // level_gemm: four warps
-constexpr int kLStride = kGM + 4;  // level_gemm shared-memory row stride (doubles)
-
-// One FP64 tensor-core MMA (m8n8k4): d (8 x 8) += a (8 x 4) b (4 x 8).  Lane l
-// holds a[l / 4][l % 4], b[l % 4][l / 4] and d[l / 4][2 (l % 4) + {0, 1}].
-__device__ __forceinline__ void dmma_m8n8k4(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
-// 64 x 64 output tile per block of four warps, each warp a 32 x 32 quadrant
-// as 4 x 4 FP64 MMAs (m8n8k4) per k-step of 4.  A tiles (operator rows) are
-// copied as they lie (k-major), B tiles (one column per source cell) one
-// column per thread; rows of both are padded to 68 doubles so that every
-// fragment load of a warp is conflict-free.  The next 16-source chunk is
-// loaded into registers while the current one is multiplied from shared
-// memory (two buffers, one barrier per chunk).  Every output is a fixed-order
-// sum, so the result does not depend on the grid.
-__global__ void __launch_bounds__(kLThreads, 3) level_gemm(LevelGemm g) {
-  __shared__ __align__(16) double As[2][kGK][kLStride];
-  __shared__ __align__(16) double Bs[2][kGK][kLStride];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int r0 = blockIdx.y * kGM;
-  const int64_t n0 = (int64_t)blockIdx.x * kGN;
-  const int wm = 32 * (w & 1), wn = 32 * (w >> 1);  // the warp's quadrant
-  const int fr = lane >> 2, fk = lane & 3;            // fragment row / k of this lane
-  // A loads: rows r0 + 2 (tid & 31) (+1), sources (tid >> 5) + 4x, x < 4
-  const int am = 2 * (tid & 31), ak = tid >> 5;
-  const bool arow_ok = r0 + am < g.R;  // R even: the pair is valid together
-  // B loads: column tid & 63, sources 8 (tid >> 6) .. +7
-  const int bn = tid & 63, bk = 8 * (tid >> 6);
-  const int64_t bcol_i = n0 + bn;
-  const bool bcol_ok = bcol_i < g.ncols;
-  const double *bcol = nullptr;
-  if (bcol_ok) {
-    const int64_t child0 = g.c0 + 8 * bcol_i;
-    const int64_t cell = g.up ? child0 : (int64_t)g.cparent[child0];
-    bcol = g.X + cell * g.nt2;
+// One level's translation GEMM on the FP64 tensor cores.  A block takes 32 of
+// the level's non-leaf cells (c0 + 8i .. c0 + 8i + 7 are cell i's children) and
+// one block of 32 outputs, a warp per octant: 32 x 32 x 16 steps with both
+// operands read from L2 / L1 straight into MMA fragments (four lanes read 128
+// contiguous bytes of a cell's row; the operator is stored in fragment order).
+// L2L: each warp adds into its octant's child.  M2M: the eight octants'
+// products are added in octant order through shared memory.  Every output is a
+// fixed-order sum, so the result does not depend on the grid.  Bound: the FP64
+// pipe; small levels by the chain of a few steps and the launch.
+template <int P, bool kUp>
+__global__ void __launch_bounds__(kUp ? 256 : 64, kUp ? 1 : 6) level_gemm(const double *__restrict__ ops, int64_t c0,
+                                                     int64_t ncols,
+                                                     const int32_t *__restrict__ cparent,
+                                                     double *__restrict__ X) {
+  using O = LevelOp<P, kUp>;
+  extern __shared__ __align__(16) double red[];  // M2M: [octant][cell][output]
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int o = blockIdx.z * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t i0 = (int64_t)blockIdx.x * 32;
+  const int b = blockIdx.y;
+  const double2 *src[4];
+#pragma unroll
+  for (int m = 0; m < 4; m++) {  // the last cell again beyond the level's end
+    const int64_t child0 = c0 + 8 * min(i0 + g + 8 * m, ncols - 1);
+    const int64_t cell = kUp ? child0 + o : (int64_t)cparent[child0];
+    src[m] = reinterpret_cast<const double2 *>(X + cell * O::K) + 2 * t;
   }
-  // source ranges holding the tile's nonzero operator columns
-  int seg0, nseg, seg_len, seg_k0;
-  if (g.up) {
-    const int tmax = (min(r0 + kGM, g.R) - 1) / 2;
-    const int jm = degree_of(tmax);
-    seg0 = g.split ? (int)blockIdx.z : 0;
-    nseg = g.split ? 1 : 8;
-    seg_len = min(g.nt2, (jm + 1) * (jm + 2));
-    seg_k0 = 0;
-  } else {
-    const int rs = r0 % g.nt2;
-    int kstart = 0;
-    if (rs + kGM <= g.nt2) {
-      const int j = degree_of(rs / 2);
-      kstart = j * (j + 1);
+  int at = 0;
+  for (int i = 0; i < b; i++) at += O::steps(i);
+  const double2 *op =
+      reinterpret_cast<const double2 *>(ops + (size_t)o * O::OCTANT) + (size_t)at * 256 + lane;
+  double acc[2][4][4];
+#pragma unroll
+  for (int m = 0; m < 2; m++)
+#pragma unroll
+    for (int f = 0; f < 4; f++)
+#pragma unroll
+      for (int x = 0; x < 4; x++) acc[m][f][x] = 0;
+  const int s1 = O::first(b) + O::steps(b);
+  for (int s = O::first(b); s < s1; s++) {
+    double a[2][8];
+    // rows hold K = P(P+1) doubles: the last step's pairs beyond them are zero
+    const bool in0 = s * kStep + 4 * t < O::K, in1 = s * kStep + 4 * t + 2 < O::K;
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const double2 zero = make_double2(0.0, 0.0);
+      const double2 u = in0 ? src[m][8 * s] : zero, v = in1 ? src[m][8 * s + 1] : zero;
+      double *d = a[m >> 1] + (m & 1);
+      d[0] = u.x;
+      d[2] = u.y;
+      d[4] = v.x;
+      d[6] = v.y;
     }
-    seg0 = 0;
-    nseg = 1;
-    seg_k0 = kstart;
-    seg_len = g.nt2 - kstart;
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+      const double2 u = __ldg(op + f * 64), v = __ldg(op + f * 64 + 32);
+#pragma unroll
+      for (int m = 0; m < 2; m++) dmma_m16n8k16(acc[m][f], a[m], u.x, u.y, v.x, v.y);
+    }
+    op += 256;
   }
-  const int cps = (seg_len + kGK - 1) / kGK;  // chunks per segment
-  const int nchunks = nseg * cps;
-  double2 av[4], bv[4];
-  auto load_chunk = [&](int c) {
-    const int sg = seg0 + c / cps, kc = (c % cps) * kGK;
-    const int kseg = seg_k0 + sg * g.nt2;  // first source of the segment
+  if (kUp) {
 #pragma unroll
-    for (int x = 0; x < 4; x++) {
-      const int kk = kc + ak + 4 * x;
-      av[x] = (kk < seg_len && arow_ok)
-                  ? *reinterpret_cast<const double2 *>(g.At + (size_t)(kseg + kk) * g.R + r0 + am)
-                  : make_double2(0, 0);
-      const int kb = kc + bk + 2 * x;  // even; seg_len is even
-      bv[x] = (kb < seg_len && bcol_ok) ? *reinterpret_cast<const double2 *>(bcol + kseg + kb)
-                                        : make_double2(0, 0);
-    }
-  };
-  double acc[4][4][2];
+    for (int f = 0; f < 4; f++)
 #pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0;
-  if (nchunks > 0) load_chunk(0);
-  for (int c = 0; c < nchunks; c++) {
-    const int buf = c & 1;
-#pragma unroll
-    for (int x = 0; x < 4; x++) {
-      *reinterpret_cast<double2 *>(&As[buf][ak + 4 * x][am]) = av[x];
-      Bs[buf][bk + 2 * x][bn] = bv[x].x;
-      Bs[buf][bk + 2 * x + 1][bn] = bv[x].y;
-    }
+      for (int m = 0; m < 4; m++)
+        *reinterpret_cast<double2 *>(red + ((o * 32 + g + 8 * m) * 32 + 8 * f + 2 * t)) =
+            make_double2(acc[m >> 1][f][2 * (m & 1)], acc[m >> 1][f][2 * (m & 1) + 1]);
     __syncthreads();
-    if (c + 1 < nchunks) load_chunk(c + 1);
+    for (int e = threadIdx.x; e < 32 * 16; e += 256) {
+      const int row = e >> 4, col = 2 * (e & 15);
+      if (i0 + row >= ncols || b * kOutBlock + col >= O::K) continue;
+      double2 v = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int k0 = 0; k0 < kGK; k0 += 4) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[buf][k0 + fk][wm + 8 * i + fr];
-#pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[buf][k0 + fk][wn + 8 * j + fr];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) dmma_m8n8k4(acc[i][j], a[i], b[j]);
+      for (int q = 0; q < 8; q++) {
+        const double2 w = *reinterpret_cast<const double2 *>(red + (q * 32 + row) * 32 + col);
+        v.x += w.x;
+        v.y += w.y;
+      }
+      *reinterpret_cast<double2 *>(X + (int64_t)cparent[c0 + 8 * (i0 + row)] * O::K +
+                                   b * kOutBlock + col) = v;
     }
-  }
+  } else {
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
+    for (int m = 0; m < 4; m++) {
+      const int64_t i = i0 + g + 8 * m;
+      if (i >= ncols) continue;
+      double *dst = X + (c0 + 8 * i + o) * O::K + b * kOutBlock + 2 * t;
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int64_t ci = n0 + wn + 8 * j + 2 * fk + e;
-      if (ci >= g.ncols) continue;
-      const int64_t child0 = g.c0 + 8 * ci;
-      double *ccol;
-      if (g.split) ccol = g.part + ((int64_t)blockIdx.z * g.ncols + ci) * g.R;
-      else ccol = g.X + (g.up ? (int64_t)g.cparent[child0] : child0) * g.nt2;
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int row = r0 + wm + 8 * i + fr;
-        if (row >= g.R) continue;
-        if (g.up) ccol[row] = acc[i][j][e];
-        else ccol[row] += acc[i][j][e];
+      for (int f = 0; f < 4; f++) {
+        if (b * kOutBlock + 8 * f + 2 * t >= O::K) continue;
+        double2 *d = reinterpret_cast<double2 *>(dst + 8 * f);
+        const double2 w = *d;
+        *d = make_double2(w.x + acc[m >> 1][f][2 * (m & 1)],
+                          w.y + acc[m >> 1][f][2 * (m & 1) + 1]);
       }
     }
-  }
-}
-
-// Split M2M: M[parent_i] = sum over octants o = 0..7, in that order, of part[o][i].
-__global__ void sum_octant_parts(const double *__restrict__ part, int64_t ncols, int R,
-                                 int64_t c0, const int32_t *__restrict__ cparent, int nt2,
-                                 double *__restrict__ X) {
-  const int64_t total = ncols * R;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t ci = e / R;
-    const int row = (int)(e - ci * R);
-    double v = 0;
-#pragma unroll
-    for (int o = 0; o < 8; o++) v += part[(o * ncols + ci) * R + row];
-    X[(int64_t)cparent[c0 + 8 * ci] * nt2 + row] = v;
   }
 }
 
@@ -849,7 +827,6 @@ __global__ void sum_octant_parts(const double *__restrict__ part, int64_t ncols,
 // children).
 template <int P>
 int build_level_ops(tapas_b200_ctx *ctx, int &nlev, LevelFirstChild &lf) {
-  using S = Sizes<P>;
   cudaStream_t s = ctx->stream;
   nlev = 0;
   for (int l = 0; l + 2 < (int)ctx->level_off.size() && l < kMaxLevels; l++) {
@@ -858,48 +835,33 @@ int build_level_ops(tapas_b200_ctx *ctx, int &nlev, LevelFirstChild &lf) {
     nlev = l + 1;
   }
   if (nlev == 0) return TAPAS_B200_OK;
-  const size_t per = (size_t)(2 * S::NT) * (16 * S::NT);  // doubles per level, either op
-  TB_CUDA(ctx, ctx->op_m2m.ensure(per * nlev, s));
-  TB_CUDA(ctx, ctx->op_l2l.ensure(per * nlev, s));
-  build_translation_ops<P><<<dim3(nlev, 8, 2), 256, 0, s>>>(lf, ctx->cparent.p, ctx->ccen.p,
-                                                           ctx->op_m2m.p, ctx->op_l2l.p);
+  using Up = LevelOp<P, true>;
+  using Dn = LevelOp<P, false>;
+  TB_CUDA(ctx, ctx->op_m2m.ensure(8 * Up::OCTANT * nlev, s));
+  TB_CUDA(ctx, ctx->op_l2l.ensure(8 * Dn::OCTANT * nlev, s));
+  // enough blocks to fill the GPU, each building its harmonics table again
+  const dim3 grid(nlev, 8, std::max(1, 2 * ctx->num_sms / (8 * nlev)));
+  build_level_op<P, true><<<grid, 256, 0, s>>>(lf, ctx->cparent.p, ctx->ccen.p, ctx->op_m2m.p);
+  TB_LAUNCH_CHECK(ctx);
+  build_level_op<P, false><<<grid, 256, 0, s>>>(lf, ctx->cparent.p, ctx->ccen.p, ctx->op_l2l.p);
   TB_LAUNCH_CHECK(ctx);
   return TAPAS_B200_OK;
 }
 
-template <int P>
-int level_translate(tapas_b200_ctx *ctx, int l, const LevelFirstChild &lf, bool up) {
-  using S = Sizes<P>;
+template <int P, bool kUp>
+int level_translate(tapas_b200_ctx *ctx, int l, const LevelFirstChild &lf) {
+  using O = LevelOp<P, kUp>;
   const int64_t ncols = (ctx->level_off[l + 2] - ctx->level_off[l + 1]) / 8;
   if (ncols <= 0) return TAPAS_B200_OK;
-  const size_t per = (size_t)(2 * S::NT) * (16 * S::NT);
-  LevelGemm g;
-  g.At = (up ? ctx->op_m2m.p : ctx->op_l2l.p) + per * l;
-  g.R = up ? 2 * S::NT : 16 * S::NT;
-  g.K = up ? 16 * S::NT : 2 * S::NT;
-  g.nt2 = 2 * S::NT;
-  g.up = up ? 1 : 0;
-  g.c0 = lf.c0[l];
-  g.ncols = ncols;
-  g.cparent = ctx->cparent.p;
-  g.X = reinterpret_cast<double *>(up ? ctx->M.p : ctx->L.p);
-  g.part = nullptr;
-  dim3 grid((unsigned)((ncols + kGN - 1) / kGN), (unsigned)((g.R + kGM - 1) / kGM));
-  // A level too small to fill the GPU splits M2M's eight octant products
-  // over blocks and adds them afterwards in octant order.
-  g.split = (up && (int64_t)grid.x * grid.y < 2 * ctx->num_sms) ? 1 : 0;
-  if (g.split) {
-    TB_CUDA(ctx, ctx->op_part.ensure((size_t)8 * ncols * g.R, ctx->stream));
-    g.part = ctx->op_part.p;
-    grid.z = 8;
-  }
-  level_gemm<<<grid, kLThreads, 0, ctx->stream>>>(g);
+  const dim3 grid((unsigned)((ncols + 31) / 32), O::NB, kUp ? 1 : 4);
+  const int smem = kUp ? 8 * 32 * 32 * (int)sizeof(double) : 0;
+  if (kUp)
+    TB_CUDA(ctx, cudaFuncSetAttribute(level_gemm<P, kUp>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  level_gemm<P, kUp><<<grid, kUp ? 256 : 64, smem, ctx->stream>>>(
+      (kUp ? ctx->op_m2m.p : ctx->op_l2l.p) + 8 * O::OCTANT * l, lf.c0[l], ncols, ctx->cparent.p,
+      reinterpret_cast<double *>(kUp ? ctx->M.p : ctx->L.p));
   TB_LAUNCH_CHECK(ctx);
-  if (g.split) {
-    sum_octant_parts<<<grid_for(ncols * g.R, 256), 256, 0, ctx->stream>>>(
-        g.part, ncols, g.R, g.c0, g.cparent, g.nt2, g.X);
-    TB_LAUNCH_CHECK(ctx);
-  }
   return TAPAS_B200_OK;
 }
 
@@ -934,7 +896,7 @@ int m2m_P(tapas_b200_ctx *ctx) {
   LevelFirstChild lf;
   TB_TRY(build_level_ops<P>(ctx, nlev, lf));
   ctx->level_ops_P = P;
-  for (int lev = nlev - 1; lev >= 0; lev--) TB_TRY(level_translate<P>(ctx, lev, lf, true));
+  for (int lev = nlev - 1; lev >= 0; lev--) TB_TRY((level_translate<P, true>(ctx, lev, lf)));
   return TAPAS_B200_OK;
 }
 
@@ -946,7 +908,7 @@ int fp64_m2m_levels_P(tapas_b200_ctx *ctx, int max_levels) {
   TB_TRY(build_level_ops<P>(ctx, nlev, lf));  // the upward pass builds them for this tree
   ctx->level_ops_P = P;
   for (int lev = std::min(nlev, max_levels) - 1; lev >= 0; lev--)
-    TB_TRY(level_translate<P>(ctx, lev, lf, true));
+    TB_TRY((level_translate<P, true>(ctx, lev, lf)));
   return TAPAS_B200_OK;
 }
 
@@ -1007,7 +969,7 @@ int downward_P(tapas_b200_ctx *ctx, bool l2p_f32) {
         nlev = l + 1;
       }
     }
-    for (int lev = 0; lev < nlev; lev++) TB_TRY(level_translate<P>(ctx, lev, lf, false));
+    for (int lev = 0; lev < nlev; lev++) TB_TRY((level_translate<P, false>(ctx, lev, lf)));
   }
   PhaseTimer t(ctx, &ctx->timings.l2p);
   int64_t nl = 0;

@@ -152,6 +152,21 @@ __device__ __forceinline__ void jk_of(int t, int &j, int &k) {
   k = t - j * (j + 1) / 2;
 }
 
+// d (16 x 8) += a (16 x 16) b (16 x 8), FP64 tensor cores.  Lane l (g = l / 4,
+// t = l % 4) holds a[g + 8 (i & 1)][k], b[k][g] with k the lane's (i / 2)th,
+// resp. ith, of its four, and d[g][2t + {0,1}], d[g + 8][2t + {0,1}].  The
+// instruction's k = t + 4i is renamed 4t + i here for both operands, which
+// leaves the sum over k unchanged and makes a lane's four values contiguous.
+__device__ __forceinline__ void dmma_m16n8k16(double (&d)[4], const double (&a)[8], double b0,
+                                              double b1, double b2, double b3) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, "
+      "{%4, %5, %6, %7, %8, %9, %10, %11}, {%12, %13, %14, %15}, {%0, %1, %2, %3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]),
+        "d"(b0), "d"(b1), "d"(b2), "d"(b3));
+}
+
 // One source's translation added to lane coefficients (jj[r], kk[r]): the
 // source's M in Mj, the local harmonics of the offset in Y.
 template <int P>
