@@ -936,11 +936,7 @@ int m2l_P(tapas_b200_ctx *ctx) {
 
 template <int P>
 int m2l_pairs_P(tapas_b200_ctx *ctx) {
-  using S = Sizes<P>;
   cudaStream_t s = ctx->stream;
-  const int64_t C = ctx->ncells;
-  TB_CUDA(ctx, ctx->L.ensure((size_t)C * S::NT, s));
-  TB_CUDA(ctx, cudaMemsetAsync(ctx->L.p, 0, sizeof(double2) * (size_t)C * S::NT, s));
   PhaseTimer t(ctx, &ctx->timings.m2l_fp64);
   const int64_t np = ctx->m2l_npairs;
   if (np > 0) {

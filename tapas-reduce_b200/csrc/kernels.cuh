@@ -19,8 +19,8 @@ int fp64_m2m_levels(tapas_b200_ctx *ctx, int max_levels);
 // each target's sum in list order; P = 2, 3 by the warp-per-target kernel.
 int m2l_fp64(tapas_b200_ctx *ctx);
 int m2l_fp64_cells(tapas_b200_ctx *ctx);
-// L zeroed, then the FP64 M2L of the pairs at list indices pairs[0..npairs)
-// added into it (atomics: the order of a target's sums is not fixed).
+// The FP64 M2L of the pairs at list indices pairs[0..npairs) added into L
+// (atomics: the order of a target's sums is not fixed).
 int m2l_fp64_pairs(tapas_b200_ctx *ctx, const uint32_t *pairs, int64_t npairs);
 int downward_fp64(tapas_b200_ctx *ctx);
 // FP64 L2L, then L2P in FP32 added to the near field.

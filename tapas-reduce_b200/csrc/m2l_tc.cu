@@ -337,28 +337,32 @@ struct TileItem {
   int32_t pad;
 };
 
+// One warp per class.
 __global__ void build_tiles(const int32_t *__restrict__ seg_start, int64_t nseg, int64_t n,
                             const int32_t *__restrict__ tcflag, const int32_t *__restrict__ tcid,
                             const int32_t *__restrict__ tile_off,
                             const uint64_t *__restrict__ keys, KeyPack kp,
                             uint64_t *__restrict__ tc_keys, TileItem *__restrict__ items,
                             int2 *__restrict__ cls_range, int *__restrict__ tc_pairs) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nseg;
-       c += (int64_t)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nseg;
+       c += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     if (!tcflag[c]) continue;
     const int64_t b = seg_start[c], e = (c + 1 < nseg) ? seg_start[c + 1] : n;
     const int id = tcid[c];
-    tc_keys[id] = kp.wide(keys[b]);
-    cls_range[id] = make_int2((int)b, (int)(e - b));
-    atomicAdd(tc_pairs, (int)(e - b));
-    int64_t o = tile_off[c];
-    for (int64_t p = b; p < e; p += kNTile, o++) {
+    if (lane == 0) {
+      tc_keys[id] = kp.wide(keys[b]);
+      cls_range[id] = make_int2((int)b, (int)(e - b));
+      atomicAdd(tc_pairs, (int)(e - b));
+    }
+    const int64_t o = tile_off[c];
+    for (int64_t k = lane; b + k * kNTile < e; k += 32) {
       TileItem it;
       it.cls = id;
-      it.start = (int32_t)p;
-      it.len = (int32_t)min((int64_t)kNTile, e - p);
+      it.start = (int32_t)(b + k * kNTile);
+      it.len = (int32_t)min((int64_t)kNTile, e - it.start);
       it.pad = 0;
-      items[o] = it;
+      items[o + k] = it;
     }
   }
 }
@@ -531,7 +535,8 @@ __global__ void __launch_bounds__(256) normalize_M(int64_t ncells, const int32_t
   }
 }
 
-// Per cell c (one warp each): L[c][t] += Lt[c][t] / w^(j+1) (j = degree of t).
+// Per cell c (one warp each): L[c][t] = Lt[c][t] / w^(j+1) (j = degree of t), 0 for
+// an empty cell.
 template <int P>
 __global__ void __launch_bounds__(256) add_scaled_L(int64_t ncells, const int32_t *__restrict__ cnb,
                                                     const double *__restrict__ cmin,
@@ -552,18 +557,21 @@ __global__ void __launch_bounds__(256) add_scaled_L(int64_t ncells, const int32_
   }
   const int64_t nw = (int64_t)gridDim.x * 8;
   for (int64_t c = (int64_t)blockIdx.x * 8 + wi; c < ncells; c += nw) {
-    if (cnb[c] == 0) continue;  // warp-uniform
+    const bool live = cnb[c] > 0;  // warp-uniform
     __syncwarp();
-    if (lane <= P) pw[wi][lane] = pow(cmax[3 * c] - cmin[3 * c], -lane);
+    if (live && lane <= P) pw[wi][lane] = pow(cmax[3 * c] - cmin[3 * c], -lane);
     __syncwarp();
 #pragma unroll
     for (int r = 0; r < kSlots; r++) {
       const int t = lane + 32 * r;
       if (t >= S::NT) continue;
-      const double sc = pw[wi][deg[r] + 1];
-      const float2 lt = *reinterpret_cast<const float2 *>(Lt + c * S::KP + 2 * t);
-      const double2 o = L[c * S::NT + t];
-      L[c * S::NT + t] = make_double2(o.x + (double)lt.x * sc, o.y + (double)lt.y * sc);
+      double2 v = make_double2(0.0, 0.0);
+      if (live) {
+        const double sc = pw[wi][deg[r] + 1];
+        const float2 lt = *reinterpret_cast<const float2 *>(Lt + c * S::KP + 2 * t);
+        v = make_double2((double)lt.x * sc, (double)lt.y * sc);
+      }
+      L[c * S::NT + t] = v;
     }
   }
 }
@@ -1265,7 +1273,7 @@ int m2l_classes(tapas_b200_ctx *ctx, size_t op_bytes, int64_t min_pairs, M2LClas
   TB_CUDA(ctx, T.items.ensure((size_t)(nitems + 1) * sizeof(TileItem) / 16 + 1, s));
   TB_CUDA(ctx, T.err.ensure(4, s));
   TB_CUDA(ctx, cudaMemsetAsync(T.err.p, 0, 4 * sizeof(int), s));
-  build_tiles<<<grid_for(nseg, 256), 256, 0, s>>>(T.seg_start.p, nseg, n, T.tcflag.p, T.tcid.p,
+  build_tiles<<<grid_for(32 * nseg, 256), 256, 0, s>>>(T.seg_start.p, nseg, n, T.tcflag.p, T.tcid.p,
                                                    T.tile_off.p, T.keys.p, kp, T.tc_keys.p,
                                                    reinterpret_cast<TileItem *>(T.items.p),
                                                    T.cls_range.p, T.err.p + 1);
@@ -1333,8 +1341,9 @@ int m2l_tc_P(tapas_b200_ctx *ctx) {
     std::swap(T.items.cap, T.items_alt.cap);
   }
   setup_timer.reset();
-  // 5. FP64 part (rare classes) writes L; the GEMM adds into Lt
-  TB_TRY(m2l_fp64_pairs(ctx, T.pairs64.p, n64));
+  // 5. the GEMM adds into Lt, L is written from it, the rare classes' pairs are
+  // added to L
+  TB_CUDA(ctx, ctx->L.ensure((size_t)C * S::NT, s));
   if (nitems > 0) {
     PhaseTimer t(ctx, &ctx->timings.m2l_tc);
     const TileItem *it = reinterpret_cast<const TileItem *>(T.items.p);
@@ -1351,6 +1360,7 @@ int m2l_tc_P(tapas_b200_ctx *ctx) {
   add_scaled_L<P><<<grid_for(C, 8, ctx->num_sms * 8), 256, 0, s>>>(
       C, ctx->cnb.p, ctx->cmin.p, ctx->cmax.p, T.Lt.p, ctx->L.p);
   TB_LAUNCH_CHECK(ctx);
+  TB_TRY(m2l_fp64_pairs(ctx, T.pairs64.p, n64));
   TB_CUDA(ctx, cudaMemcpyAsync(h, T.err.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   TB_CUDA(ctx, cudaStreamSynchronize(s));
   ctx->n_m2l_tc = h[1];
