@@ -91,13 +91,15 @@ __global__ void trav_cells(int64_t ncells, const double *__restrict__ mn,
   }
 }
 
-// Per-thread output counts packed in one word for the block scan: M2L pairs
-// in bits 0-8, P2P pairs in bits 9-17, new frontier pairs in bits 18-31
-// (at most 256, 256 and 36 * 256 per block; 36 for a mutual self split).
+// Per-thread output counts packed in one word for the block scan: M2L pairs in
+// bits 0-15, P2P pairs in bits 16-31, new frontier pairs (8 per split, 36 for a
+// mutual self split) from bit 32.
 constexpr int kWarpsPerBlock = kBlock / 32;
+constexpr int kPerThread = 4;
 constexpr int kSelfSplit = 36;  // child pairs (i, j), i <= j, of a cell with itself
-static_assert(kBlock <= 256, "packed per-block counts hold at most 256 threads");
-static_assert(kSelfSplit * kBlock < (1 << 14), "frontier count field is 14 bits");
+constexpr int kP2pAt = 16, kFrontAt = 32;
+constexpr unsigned long long kCountMask = 0xffff;
+static_assert(kBlock * kPerThread <= (int)kCountMask, "packed per-block counts");
 
 struct TravBufs {
   int2 *front[2];
@@ -119,7 +121,7 @@ constexpr int kMaxSteps = 4 * (kMaxDepth + 2);
 __global__ void __launch_bounds__(kBlock) dtt_steps(TravCells c, TravBufs bufs, TravState *st,
                                                     int prune_empty, int mutual) {
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  __shared__ uint32_t wsum[kWarpsPerBlock];
+  __shared__ unsigned long long wsum[kWarpsPerBlock];
   __shared__ unsigned long long wint[kWarpsPerBlock];
   __shared__ unsigned long long bbase[3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -132,111 +134,125 @@ __global__ void __launch_bounds__(kBlock) dtt_steps(TravCells c, TravBufs bufs, 
     const int64_t next_cap = bufs.front_cap[(step & 1) ^ 1];
     unsigned long long *counters = st->cnt[step % 3];
     if (blockIdx.x == 0 && threadIdx.x < 4) st->cnt[(step + 1) % 3][threadIdx.x] = 0;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nfront;
-         base += (int64_t)gridDim.x * blockDim.x) {
-      const int64_t i = base + threadIdx.x;
-      int kind = 0;  // 0 none, 1 m2l, 2 p2p, 3 split target, 4 split source, 5 split both
-      int t = 0, s = 0, split_child = 0;
-      unsigned long long inter = 0;
-      if (i < nfront) {
-        const int2 pr = __ldcg(front + i);
-        t = pr.x;
-        s = pr.y;
+    // A block takes kPerThread pairs per thread at a time when there are enough for
+    // all blocks: the three barriers and the reservations' latency per round were
+    // most of the time.
+    const int per = nfront > (int64_t)gridDim.x * kBlock ? kPerThread : 1;
+    for (int64_t base = (int64_t)blockIdx.x * kBlock * per; base < nfront;
+         base += (int64_t)gridDim.x * kBlock * per) {
+      int kind[kPerThread];  // 0 none, 1 m2l, 2 p2p, 3 split target, 4 split source, 5 split both
+      int2 pair[kPerThread];
+      int child[kPerThread];
+      unsigned long long mine = 0, inter = 0;
+#pragma unroll
+      for (int q = 0; q < kPerThread; q++) {
+        kind[q] = 0;
+        const int64_t i = base + q * kBlock + threadIdx.x;
+        if (q >= per || i >= nfront) continue;
+        pair[q] = __ldcg(front + i);
+        const int t = pair[q].x, s = pair[q].y;
         const int2 mt = c.meta[t], ms = c.meta[s];
         // An empty cell (and so all of its descendants) contributes nothing as a
         // source and receives nothing used later as a target.
-        if (!prune_empty || (mt.x != 0 && ms.x != 0)) {
-          const double4 gt = c.geo[t], gs = c.geo[s];
-          const double dx = __dsub_rn(gt.x, gs.x);
-          const double dy = __dsub_rn(gt.y, gs.y);
-          const double dz = __dsub_rn(gt.z, gs.z);
-          double R2 = __dadd_rn(0.0, __dmul_rn(dx, dx));
-          R2 = __dadd_rn(R2, __dmul_rn(dy, dy));
-          R2 = __dadd_rn(R2, __dmul_rn(dz, dz));
-          const double Ri = gt.w, Rj = gs.w;
-          const double RR = __dadd_rn(Ri, Rj);
-          const bool lt = mt.y < 0, ls = ms.y < 0;
-          if (R2 > __dmul_rn(RR, RR)) {
-            kind = 1;
-          } else if (lt && ls) {
-            if (mt.x > 0 && ms.x > 0) {
-              kind = 2;
-              // body pairs evaluated: both directions of a mutual pair of two leaves
-              inter = (unsigned long long)mt.x * (unsigned long long)ms.x;
-              if (mutual && t != s) inter *= 2;
-            }
-          } else if (ls) {
-            kind = 3;
-          } else if (lt) {
-            kind = 4;
-          } else if (mutual && t == s) {
-            kind = 5;
-          } else {
-            kind = (Ri >= Rj) ? 3 : 4;
+        if (prune_empty && (mt.x == 0 || ms.x == 0)) continue;
+        const double4 gt = c.geo[t], gs = c.geo[s];
+        const double dx = __dsub_rn(gt.x, gs.x);
+        const double dy = __dsub_rn(gt.y, gs.y);
+        const double dz = __dsub_rn(gt.z, gs.z);
+        double R2 = __dadd_rn(0.0, __dmul_rn(dx, dx));
+        R2 = __dadd_rn(R2, __dmul_rn(dy, dy));
+        R2 = __dadd_rn(R2, __dmul_rn(dz, dz));
+        const double Ri = gt.w, Rj = gs.w;
+        const double RR = __dadd_rn(Ri, Rj);
+        const bool lt = mt.y < 0, ls = ms.y < 0;
+        int kd;
+        if (R2 > __dmul_rn(RR, RR)) {
+          kd = 1;
+        } else if (lt && ls) {
+          kd = 0;
+          if (mt.x > 0 && ms.x > 0) {
+            kd = 2;
+            // body pairs evaluated: both directions of a mutual pair of two leaves
+            inter += (unsigned long long)mt.x * (unsigned long long)ms.x *
+                     (mutual && t != s ? 2 : 1);
           }
-          split_child = kind == 3 ? mt.y : ms.y;
+        } else if (ls) {
+          kd = 3;
+        } else if (lt) {
+          kd = 4;
+        } else if (mutual && t == s) {
+          kd = 5;
+        } else {
+          kd = (Ri >= Rj) ? 3 : 4;
         }
+        kind[q] = kd;
+        child[q] = kd == 3 ? mt.y : ms.y;
+        mine += kd == 0   ? 0ull
+                : kd == 1 ? 1ull
+                : kd == 2 ? 1ull << kP2pAt
+                : kd == 5 ? (unsigned long long)kSelfSplit << kFrontAt
+                          : 8ull << kFrontAt;
       }
-      const uint32_t mine = (kind == 1 ? 1u : 0u) | (kind == 2 ? 1u << 9 : 0u) |
-                            (kind == 3 || kind == 4 ? 8u << 18 : 0u) |
-                            (kind == 5 ? (uint32_t)kSelfSplit << 18 : 0u);
-      uint32_t incl = mine;
+      unsigned long long incl = mine;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
       }
-      unsigned long long w = inter;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+      for (int o = 16; o > 0; o >>= 1) inter += __shfl_xor_sync(0xffffffffu, inter, o);
       if (lane == 31) wsum[warp] = incl;
-      if (lane == 0) wint[warp] = w;
+      if (lane == 0) wint[warp] = inter;
       __syncthreads();
       if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        unsigned long long tot = 0;
+        unsigned long long run = 0, tot = 0;
 #pragma unroll
         for (int k = 0; k < kWarpsPerBlock; k++) {
-          const uint32_t v = wsum[k];
+          const unsigned long long v = wsum[k];
           wsum[k] = run;
           run += v;
           tot += wint[k];
         }
-        const uint32_t n1 = run & 511u, n2 = (run >> 9) & 511u, n3 = run >> 18;
-        bbase[0] = n_m2l + (n1 ? atomicAdd(counters + 1, (unsigned long long)n1) : 0);
-        bbase[1] = n_p2p + (n2 ? atomicAdd(counters + 2, (unsigned long long)n2) : 0);
-        bbase[2] = n3 ? atomicAdd(counters + 0, (unsigned long long)n3) : 0;
+        const unsigned long long n1 = run & kCountMask, n2 = (run >> kP2pAt) & kCountMask,
+                                 n3 = run >> kFrontAt;
+        bbase[0] = n_m2l + (n1 ? atomicAdd(counters + 1, n1) : 0);
+        bbase[1] = n_p2p + (n2 ? atomicAdd(counters + 2, n2) : 0);
+        bbase[2] = n3 ? atomicAdd(counters + 0, n3) : 0;
         if (tot) atomicAdd(counters + 3, tot);
       }
       __syncthreads();
-      const uint32_t off = wsum[warp] + incl - mine;
-      if (kind == 1) {
-        const unsigned long long dst = bbase[0] + (off & 511u);
-        if ((int64_t)dst < bufs.m2l_cap) bufs.m2l[dst] = ((uint64_t)(uint32_t)t << 32) | (uint32_t)s;
-      } else if (kind == 2) {
-        const unsigned long long dst = bbase[1] + ((off >> 9) & 511u);
-        if ((int64_t)dst < bufs.p2p_cap) bufs.p2p[dst] = ((uint64_t)(uint32_t)t << 32) | (uint32_t)s;
-      } else if (kind == 5) {
-        const unsigned long long dst = bbase[2] + (off >> 18);
-        if ((int64_t)(dst + kSelfSplit) <= next_cap) {
-          int2 *o = next + dst;
-          int k = 0;
-          for (int a = 0; a < 8; a++)
-            for (int b2 = a; b2 < 8; b2++) o[k++] = make_int2(split_child + a, split_child + b2);
-        }
-      } else if (kind >= 3) {
-        const unsigned long long dst = bbase[2] + (off >> 18);
-        if ((int64_t)(dst + 8) <= next_cap) {
-          int4 *o4 = reinterpret_cast<int4 *>(next + dst);  // dst is even (8 and 36 are)
-          if (kind == 3) {
+      const unsigned long long off = wsum[warp] + incl - mine;
+      int64_t at_m2l = (int64_t)(bbase[0] + (off & kCountMask)),
+              at_p2p = (int64_t)(bbase[1] + ((off >> kP2pAt) & kCountMask)),
+              at_next = (int64_t)(bbase[2] + (off >> kFrontAt));
 #pragma unroll
-            for (int k = 0; k < 8; k += 2)
-              o4[k / 2] = make_int4(split_child + k, s, split_child + k + 1, s);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 8; k += 2)
-              o4[k / 2] = make_int4(t, split_child + k, t, split_child + k + 1);
+      for (int q = 0; q < kPerThread; q++) {
+        if (kind[q] == 0) continue;
+        const int t = pair[q].x, s = pair[q].y, ch = child[q];
+        const uint64_t packed = ((uint64_t)(uint32_t)t << 32) | (uint32_t)s;
+        if (kind[q] == 1) {
+          if (at_m2l < bufs.m2l_cap) bufs.m2l[at_m2l] = packed;
+          at_m2l++;
+        } else if (kind[q] == 2) {
+          if (at_p2p < bufs.p2p_cap) bufs.p2p[at_p2p] = packed;
+          at_p2p++;
+        } else if (kind[q] == 5) {
+          if (at_next + kSelfSplit <= next_cap) {
+            int2 *o = next + at_next;
+            int k = 0;
+            for (int a = 0; a < 8; a++)
+              for (int b2 = a; b2 < 8; b2++) o[k++] = make_int2(ch + a, ch + b2);
           }
+          at_next += kSelfSplit;
+        } else {
+          if (at_next + 8 <= next_cap) {
+            int4 *o4 = reinterpret_cast<int4 *>(next + at_next);  // even: 8 and 36 are
+#pragma unroll
+            for (int k = 0; k < 8; k += 2)
+              o4[k / 2] = kind[q] == 3 ? make_int4(ch + k, s, ch + k + 1, s)
+                                       : make_int4(t, ch + k, t, ch + k + 1);
+          }
+          at_next += 8;
         }
       }
       __syncthreads();  // wsum / bbase are rewritten by the next round
