@@ -694,7 +694,7 @@ int bh_interact(tapas_b200_ctx *ctx, double theta, double eps2, int precision) {
     TB_CUDA(ctx, ctx->flag.ensure(C + 1, s));
     TB_CUDA(ctx, ctx->flag_scan.ensure(C + 1, s));
     TB_CUDA(ctx, ctx->bh_attr32.ensure(C + 1, s));
-    TB_CUDA(ctx, ctx->rel4.ensure(n + C + 2, s));  // two per pair, at most (n + leaves) / 2 pairs
+    TB_CUDA(ctx, ctx->bh_pairs.ensure(n + C + 2, s));  // two per pair, at most (n + leaves) / 2 pairs
     bh_pair_counts<<<grid_for(C, 256), 256, 0, s>>>(C, ctx->cleaf.p, ctx->cnb.p, ctx->flag.p);
     TB_LAUNCH_CHECK(ctx);
     TB_TRY(scan_exclusive(ctx, ctx->flag.p, ctx->flag_scan.p, C, nullptr));
@@ -703,7 +703,7 @@ int bh_interact(tapas_b200_ctx *ctx, double theta, double eps2, int precision) {
   bh_pack<<<grid_for(8 * C, 256), 256, 0, s>>>(
       C, ctx->cleaf.p, ctx->cnb.p, ctx->cbeg.p, ctx->cchild.p, ctx->cmin.p, ctx->cmax.p,
       ctx->ccen.p, ctx->bh_attr.p, pair_off, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->sq.p,
-      ctx->trav_geo.p, ctx->trav_meta.p, ctx->bh_attr32.p, ctx->rel4.p);
+      ctx->trav_geo.p, ctx->trav_meta.p, ctx->bh_attr32.p, ctx->bh_pairs.p);
   TB_LAUNCH_CHECK(ctx);
   const BhCells T{ctx->trav_geo.p, ctx->trav_meta.p, ctx->cmin.p, ctx->cmax.p, ctx->ccen.p};
   if (fp64) {
@@ -714,7 +714,7 @@ int bh_interact(tapas_b200_ctx *ctx, double theta, double eps2, int precision) {
     constexpr int kThreads = 32 * kWalk32Warps;
     auto walk = (float)eps2 >= FLT_MIN ? bh_walk32<true> : bh_walk32<false>;
     walk<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-        T, n, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->bh_attr32.p, ctx->rel4.p, theta, (float)eps2,
+        T, n, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->bh_attr32.p, ctx->bh_pairs.p, theta, (float)eps2,
         ctx->trg.p, ctx->counters.p);
   }
   TB_LAUNCH_CHECK(ctx);

@@ -168,7 +168,6 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
   ctx->op_m2m.release();
   ctx->op_l2l.release();
   // mixed-form state: near-field offsets, P2P work items, tensor-core M2L
-  for (auto *b : {&ctx->rel4, &ctx->rel_lo}) b->release();
   for (auto *b : {&ctx->p2p_wkey, &ctx->p2p_wkey_alt}) b->release();
   for (auto *b : {&ctx->p2p_order, &ctx->p2p_order_alt}) b->release();
   for (auto *b : {&ctx->p2p_kcnt, &ctx->p2p_koff, &ctx->p2p_psz, &ctx->p2p_poff}) b->release();
@@ -183,6 +182,7 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
   mlp_release(ctx);
   ctx->bh_attr.release();
   ctx->bh_attr32.release();
+  ctx->bh_pairs.release();
   ctx->direct_tg.release();
   ctx->direct_part.release();
   ctx->direct_out.release();

@@ -234,8 +234,6 @@ struct tapas_b200_ctx {
   int P = 0;
   int precision = TAPAS_B200_FP64;       // of the expansion passes (set by upward)
   int near_precision = TAPAS_B200_FP64;  // of the last P2P: FP64 sums carry q_i, mixed do not
-  tb::DBuf<float4> rel4;                // mixed: hi part of (x,y,z) - c_leaf, and q, FP32
-  tb::DBuf<float4> rel_lo;              // mixed: lo part of (x,y,z) - c_leaf, FP32
   tb::DBuf<uint64_t> p2p_wkey, p2p_wkey_alt;  // P2P work order: keys
   tb::DBuf<uint32_t> p2p_order, p2p_order_alt;  // target leaves by decreasing work
   tb::DBuf<int> p2p_counter;            // P2P work-queue head
@@ -262,6 +260,7 @@ struct tapas_b200_ctx {
   // ---- Barnes-Hut ----
   tb::DBuf<double4> bh_attr;            // per cell: mass-weighted centre (x,y,z) and mass
   tb::DBuf<float4> bh_attr32;           // FP32 copy for the FP32 walk
+  tb::DBuf<float4> bh_pairs;            // FP32 walk: the leaves' bodies in pairs
   bool have_bh_attr = false;
   uint64_t bh_napprox = 0, bh_ndirect = 0;
 

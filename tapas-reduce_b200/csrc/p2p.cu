@@ -17,11 +17,10 @@
 // FP64 form: the reference's sums (pot += qi qj / r, acc -= qi qj dX/r^3, r == 0
 // skipped; the common factor qi at the end), 1/r by charge_over_distance.
 //
-// Mixed form: FP32 arithmetic with results per unit charge.  Positions are
-// kept as FP32 (hi, lo) offsets from the body's leaf centre; a source is moved
-// into the target leaf's frame with an error-free sum (TwoSum) of its hi part
-// and the FP64 centre difference, so the separation x_i - x_j is formed from
-// ~47-bit operands and rounds once.  1/r is the hardware rsqrt (its error is far below
+// Mixed form: FP32 arithmetic with results per unit charge.  Targets and sources
+// are taken into the target leaf's frame by an FP64 subtraction (its pipe is idle
+// here) and kept as FP32 (hi, lo) parts, so the separation x_i - x_j is formed
+// from ~48-bit operands and rounds once.  1/r is the hardware rsqrt (its error is far below
 // the near field's summation error, so no Newton step).
 // A source leaf whose box is far enough from the target's box skips the lo
 // parts.  In the target frame a source coordinate is at most gap + tw/2 + sw
@@ -397,34 +396,6 @@ __global__ void __launch_bounds__(kThreads, kFp64Blocks) p2p_fp64_kernel(
 // ---------------------------------------------------------------------------
 // mixed
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) prepare_rel(
-    const int32_t *__restrict__ leaves, int64_t nleaves, const int32_t *__restrict__ cbeg,
-    const int32_t *__restrict__ cnb, const double *__restrict__ ccen,
-    const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
-    const double *__restrict__ sq, float4 *__restrict__ rel_hi, float4 *__restrict__ rel_lo) {
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (w >= nleaves) return;
-  const int c = leaves[w];
-  const int b0 = cbeg[c], nb = cnb[c];
-  const double cx = ccen[3 * c], cy = ccen[3 * c + 1], cz = ccen[3 * c + 2];
-  for (int b = lane; b < nb; b += 32) {
-    const int i = b0 + b;
-    const double rx = sx[i] - cx, ry = sy[i] - cy, rz = sz[i] - cz;
-    const float hx = (float)rx, hy = (float)ry, hz = (float)rz;
-    rel_hi[i] = make_float4(hx, hy, hz, (float)sq[i]);
-    rel_lo[i] = make_float4((float)(rx - hx), (float)(ry - hy), (float)(rz - hz), 0.f);
-  }
-}
-
-// a + b = s + e exactly (Knuth's TwoSum)
-__device__ __forceinline__ float two_sum(float a, float b, float &e) {
-  const float s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-  return s;
-}
-
 // 1/sqrt(x) for normal x > 0 from the hardware approximation (relative error
 // below 2^-22.9), without the denormal rescaling rsqrtf adds; callers treat
 // x < FLT_MIN (a separation below ~1e-19) as coincident bodies.
@@ -434,15 +405,11 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
   return y;
 }
 
-// A source leaf of the current batch: its centre's offset from the target
-// leaf's (FP64 difference as FP32 hi + lo) and whether its box is far enough for
-// plain FP32 coordinates (see above); body i of the batch's stream of source
-// bodies is body b0 + i for the leaf that holds it.
-struct __align__(16) LeafMeta {
-  float hx, hy, hz;
-  int b0;
-  float lx, ly, lz;
-  int far;
+// A source leaf of the current batch: body i of the batch's stream of source
+// bodies is body b0 + i for the leaf that holds it; far: its box is far enough
+// for plain FP32 coordinates (see above).
+struct __align__(8) LeafMeta {
+  int b0, far;
 };
 
 // One warp's shared memory.
@@ -458,8 +425,8 @@ struct __align__(16) MixedWarp {
 // l, l + L, ..., l + (kR-1) L and takes its share of the staged sources.
 //
 // The source bodies of the target's list are one stream: the list is read 32
-// leaves at a time (lane j: entry j's body range, the running body count and the
-// centre offset), and 64 consecutive bodies of the stream are staged at a time,
+// leaves at a time (lane j: entry j's body range and the running body count), and
+// 64 consecutive bodies of the stream are staged at a time,
 // two per lane; a lane finds its bodies' leaf by a binary search over the 32
 // counts with shuffles.  Each body is classed far or near and the far ones are
 // stored as coordinate arrays, so that two consecutive sources are one
@@ -477,8 +444,8 @@ __device__ __forceinline__ void mixed_tile(
     double tw, const uint64_t *__restrict__ list, uint64_t mask, const int32_t *__restrict__ cbeg,
     const int32_t *__restrict__ cnb, const double *__restrict__ ccen,
     const double *__restrict__ cmin, const double *__restrict__ cmax,
-    const float4 *__restrict__ rel_hi, const float4 *__restrict__ rel_lo, MixedWarp &sm,
-    double4 *__restrict__ out) {
+    const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
+    const double *__restrict__ sq, MixedWarp &sm, double4 *__restrict__ out) {
   const int g = lane / L, tl = lane - g * L;
   const bool active = g < G;
   // a source body this far from the target leaf's centre (max norm) is far;
@@ -491,14 +458,15 @@ __device__ __forceinline__ void mixed_tile(
   for (int r = 0; r < kR; r++) {
     const int t = tl + L * r;
     const bool v = active && t < nt;
-    const float4 h = v ? rel_hi[tb0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 l = v ? rel_lo[tb0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
-    txh[r] = make_float2(h.x, h.x);
-    tyh[r] = make_float2(h.y, h.y);
-    tzh[r] = make_float2(h.z, h.z);
-    sm.lo[r][0][lane] = l.x;
-    sm.lo[r][1][lane] = l.y;
-    sm.lo[r][2][lane] = l.z;
+    const double dx = v ? sx[tb0 + t] - tcx : 0.0, dy = v ? sy[tb0 + t] - tcy : 0.0,
+                 dz = v ? sz[tb0 + t] - tcz : 0.0;
+    const float hx = (float)dx, hy = (float)dy, hz = (float)dz;
+    txh[r] = make_float2(hx, hx);
+    tyh[r] = make_float2(hy, hy);
+    tzh[r] = make_float2(hz, hz);
+    sm.lo[r][0][lane] = (float)(dx - hx);
+    sm.lo[r][1][lane] = (float)(dy - hy);
+    sm.lo[r][2][lane] = (float)(dz - hz);
 #pragma unroll
     for (int k = 0; k < 4; k++) sm.sum[r][k][lane] = 0.0;
     tp[r] = tx[r] = ty[r] = tz[r] = zero;
@@ -528,11 +496,8 @@ __device__ __forceinline__ void mixed_tile(
       const int s = (int)(list[eb + lane] & mask);
       m.b0 = cbeg[s];
       ns = cnb[s];
-      // source frame -> target frame: FP64 centre difference as (hi, lo) floats
       const double dcx = ccen[3 * s] - tcx, dcy = ccen[3 * s + 1] - tcy,
                    dcz = ccen[3 * s + 2] - tcz;
-      m.hx = (float)dcx; m.hy = (float)dcy; m.hz = (float)dcz;
-      m.lx = (float)(dcx - m.hx); m.ly = (float)(dcy - m.hy); m.lz = (float)(dcz - m.hz);
       // boxes separated by gap along the farthest axis: every pair is >= gap apart
       const double sw = cmax[3 * s] - cmin[3 * s];
       const double gap = fmax(fabs(dcx), fmax(fabs(dcy), fabs(dcz))) - 0.5 * (tw + sw);
@@ -567,35 +532,36 @@ __device__ __forceinline__ void mixed_tile(
           if (v <= i) leaf += o;
         }
         const bool valid = i < total;
-        float ax = 0.f, ay = 0.f, az = 0.f, lx = 0.f, ly = 0.f, lz = 0.f, q = 0.f;
+        // position in the target leaf's frame: the FP64 difference, rounded once
+        double dx = 0.0, dy = 0.0, dz = 0.0;
+        float hx = 0.f, hy = 0.f, hz = 0.f, q = 0.f;
         bool farb = false;
         if (valid) {
           const LeafMeta lm = sm.meta[leaf];
-          const float4 ph = rel_hi[lm.b0 + i], pl = rel_lo[lm.b0 + i];
-          float ex, ey, ez;
-          ax = two_sum(ph.x, lm.hx, ex);
-          ay = two_sum(ph.y, lm.hy, ey);
-          az = two_sum(ph.z, lm.hz, ez);
-          lx = ex + (pl.x + lm.lx);
-          ly = ey + (pl.y + lm.ly);
-          lz = ez + (pl.z + lm.lz);
-          q = ph.w;
-          farb = lm.far ||
-                 fmaxf(fabsf(ax + lx), fmaxf(fabsf(ay + ly), fabsf(az + lz))) >= far_body;
+          const int j = lm.b0 + i;
+          dx = sx[j] - tcx;
+          dy = sy[j] - tcy;
+          dz = sz[j] - tcz;
+          q = (float)sq[j];
+          hx = (float)dx;
+          hy = (float)dy;
+          hz = (float)dz;
+          farb = lm.far || fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz))) >= far_body;
         }
         const unsigned fm = __ballot_sync(0xffffffffu, farb);
         const unsigned nm = __ballot_sync(0xffffffffu, valid && !farb);
         const unsigned below = (1u << lane) - 1u;
-        if (farb) {  // one float per coordinate, rounded once
+        if (farb) {
           const int k = nfar + __popc(fm & below);
-          sm.fx[k] = -(ax + lx);
-          sm.fy[k] = -(ay + ly);
-          sm.fz[k] = -(az + lz);
+          sm.fx[k] = -hx;
+          sm.fy[k] = -hy;
+          sm.fz[k] = -hz;
           sm.fq[k] = q;
         } else if (valid) {
           const int k = nnear + __popc(nm & below);
-          sm.near_hi[k] = make_float4(ax, ay, az, q);
-          sm.near_lo[k] = make_float4(lx, ly, lz, 0.f);
+          sm.near_hi[k] = make_float4(hx, hy, hz, q);
+          sm.near_lo[k] =
+              make_float4((float)(dx - hx), (float)(dy - hy), (float)(dz - hz), 0.f);
         }
         nfar += __popc(fm);
         nnear += __popc(nm);
@@ -675,8 +641,9 @@ __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
     const WorkItem *__restrict__ items, const uint64_t *__restrict__ list, uint64_t src_mask,
     const int32_t *__restrict__ cbeg, const int32_t *__restrict__ cnb,
     const double *__restrict__ ccen, const double *__restrict__ cmin,
-    const double *__restrict__ cmax, const float4 *__restrict__ rel_hi,
-    const float4 *__restrict__ rel_lo, double *__restrict__ trg, double *__restrict__ part) {
+    const double *__restrict__ cmax, const double *__restrict__ sx,
+    const double *__restrict__ sy, const double *__restrict__ sz, const double *__restrict__ sq,
+    double *__restrict__ trg, double *__restrict__ part) {
   __shared__ MixedWarp sm[kMixedWarps];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   for (;;) {
@@ -696,7 +663,7 @@ __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
       tile_shape<3, 2>(nt, R, L, G);
 #define TB_MIXED_TILE(RR)                                                                        \
   mixed_tile<RR>(lane, tb0 + tbase, nt, L, G, e0, e1, tcx, tcy, tcz, tw, list, src_mask, cbeg,  \
-                 cnb, ccen, cmin, cmax, rel_hi, rel_lo, sm[wi], out + tbase)
+                 cnb, ccen, cmin, cmax, sx, sy, sz, sq, sm[wi], out + tbase)
       if (R == 3) TB_MIXED_TILE(3);
       else if (R == 2) TB_MIXED_TILE(2);
       else TB_MIXED_TILE(1);
@@ -817,21 +784,13 @@ int p2p_mixed(tapas_b200_ctx *ctx) {
   int64_t nw = 0;
   work_leaves(ctx, nw);
   if (nw == 0) return TAPAS_B200_OK;
-  const int64_t nl = ctx->n_nonempty_leaves;  // every source leaf needs its offsets
-  TB_CUDA(ctx, ctx->rel4.ensure(ctx->n, s));
-  TB_CUDA(ctx, ctx->rel_lo.ensure(ctx->n, s));
-  prepare_rel<<<(unsigned)((nl + 7) / 8), 256, 0, s>>>(ctx->leaf_list.p, nl, ctx->cbeg.p,
-                                                      ctx->cnb.p, ctx->ccen.p, ctx->sx.p,
-                                                      ctx->sy.p, ctx->sz.p, ctx->sq.p,
-                                                      ctx->rel4.p, ctx->rel_lo.p);
-  TB_LAUNCH_CHECK(ctx);
   TB_TRY(p2p_items(ctx, kMixedBlocks * kMixedWarps));
   const uint64_t mask = (1ull << ctx->list_shift) - 1;
   p2p_mixed_kernel<kMixedBlocks><<<p2p_grid(ctx, kMixedWarps), kMixedThreads, 0, s>>>(
       ctx->p2p_order.p, ctx->p2p_nitems, ctx->p2p_counter.p,
       reinterpret_cast<const WorkItem *>(ctx->p2p_items.p), ctx->p2p.p, mask, ctx->cbeg.p,
-      ctx->cnb.p, ctx->ccen.p, ctx->cmin.p, ctx->cmax.p, ctx->rel4.p, ctx->rel_lo.p,
-      ctx->trg.p, ctx->p2p_part.p);
+      ctx->cnb.p, ctx->ccen.p, ctx->cmin.p, ctx->cmax.p, ctx->sx.p, ctx->sy.p, ctx->sz.p,
+      ctx->sq.p, ctx->trg.p, ctx->p2p_part.p);
   TB_LAUNCH_CHECK(ctx);
   return p2p_finish(ctx);
 }
