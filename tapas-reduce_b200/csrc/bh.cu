@@ -172,11 +172,14 @@ __device__ __forceinline__ int box_accept(const BodyBox &b, const double4 &g, do
   return 0;
 }
 
-constexpr int kWalk32Warps = 4;  // FP32 walk: warps per block
-
 __device__ __forceinline__ void add_counts(int lane, unsigned long long napprox,
                                            unsigned long long ndirect, bool overflow,
                                            unsigned long long *__restrict__ counters) {
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    napprox += __shfl_xor_sync(0xffffffffu, napprox, s);
+    ndirect += __shfl_xor_sync(0xffffffffu, ndirect, s);
+  }
   if (lane == 0) {
     if (napprox) atomicAdd(counters + 0, napprox);
     if (ndirect) atomicAdd(counters + 1, ndirect);
@@ -184,32 +187,159 @@ __device__ __forceinline__ void add_counts(int lane, unsigned long long napprox,
   }
 }
 
+// Opens a cell for the lanes `reach`: its eight children (from ch on) are classed
+// by eight lanes with the bodies' box, the uncertain ones tested body by body, and
+// each is pushed, child 7 first, with the lanes that accept it and the lanes that
+// open it (a leaf with `reach`; empty leaves are left out).  Returns the new
+// stack height; the warp is converged before and after.
+__device__ __forceinline__ int push_children(const BhCells &T, int ch, unsigned reach,
+                                             const BodyBox &box, int lane, double px, double py,
+                                             double pz, double theta, double theta2, int4 *stack,
+                                             int sp) {
+  const int c = ch + (lane & 7);
+  const int2 m = T.meta[c];
+  const double4 g = T.geo[c];
+  const int kind = m.y < 0 ? box_accept(box, g, theta2) : 3;  // 3: a leaf
+  // this lane's child (lanes 0..7): accepting and opening lanes
+  unsigned am = kind == 1 ? reach : 0u, om = kind == 2 ? reach : 0u;
+  unsigned todo = __ballot_sync(0xffffffffu, kind == 0) & 0xffu;
+  while (todo) {
+    const int i = __ffs(todo) - 1;
+    todo &= todo - 1;
+    double4 gi;
+    gi.x = __shfl_sync(0xffffffffu, g.x, i);
+    gi.y = __shfl_sync(0xffffffffu, g.y, i);
+    gi.z = __shfl_sync(0xffffffffu, g.z, i);
+    gi.w = __shfl_sync(0xffffffffu, g.w, i);
+    const bool acc = bh_accept(T, ch + i, gi, px, py, pz, theta, theta2);
+    const unsigned a = __ballot_sync(0xffffffffu, acc) & reach;
+    if (lane == i) {
+      am = a;
+      om = reach & ~a;
+    }
+  }
+  // every lane has read the popped entries (the ballots); child 7 at the bottom
+  const bool push = lane < 8 && m.y != 0;  // not an empty leaf
+  const unsigned pushes = __ballot_sync(0xffffffffu, push);
+  if (push)
+    stack[sp + __popc(pushes >> (lane + 1))] =
+        m.y > 0 ? make_int4(m.x, m.y, (int)reach, 0) : make_int4(c, -m.x, (int)am, (int)om);
+  __syncwarp();
+  return sp + __popc(pushes);
+}
+
+// A warp's walk: the stack, and the accepted cells and leaves in walk order.
+struct __align__(16) Walk {
+  // {cell, -first child, accepting lanes, opening lanes} or, a leaf, {first body
+  // or pair, bodies, lanes, 0}
+  int4 stack[kStack];
+  int2 list[64];  // {first body or pair, bodies} or {~cell, -1}
+  unsigned list_lanes[64];
+};
+
+// One step of a warp's walk: pops the entries from the top down to the first that
+// opens, appends the accepted cells and the leaves among them to the list (at
+// most 31 long before), and opens that one.  False: the stack would overflow.
+// napprox and ndirect count the interactions of the entries this lane popped.
+__device__ __forceinline__ bool walk_step(const BhCells &T, Walk &S, const BodyBox &box, int lane,
+                                          double px, double py, double pz, double theta,
+                                          double theta2, int &sp, int &count,
+                                          unsigned long long &napprox,
+                                          unsigned long long &ndirect) {
+  int4 e = make_int4(0, 0, 0, 0);
+  if (lane < sp) e = S.stack[sp - 1 - lane];
+  const bool leaf = e.y >= 0;
+  const unsigned opens = __ballot_sync(0xffffffffu, !leaf && e.w != 0);
+  const int top = opens ? __ffs(opens) : min(sp, 32);
+  const bool add = lane < top && e.z != 0;
+  const unsigned adds = __ballot_sync(0xffffffffu, add);
+  if (add) {
+    const int k = count + __popc(adds & ((1u << lane) - 1));
+    S.list[k] = leaf ? make_int2(e.x, e.y) : make_int2(~e.x, -1);
+    S.list_lanes[k] = (unsigned)e.z;
+    if (leaf) ndirect += (unsigned long long)e.y * __popc(e.z);
+    else napprox += __popc(e.z);
+  }
+  count += __popc(adds);
+  sp -= top;
+  __syncwarp();
+  if (opens) {
+    const int ch = -__shfl_sync(0xffffffffu, e.y, top - 1);
+    const unsigned reach = __shfl_sync(0xffffffffu, e.w, top - 1);
+    if (sp + 8 > kStack) return false;
+    sp = push_children(T, ch, reach, box, lane, px, py, pz, theta, theta2, S.stack, sp);
+  }
+  return true;
+}
+
+// Puts the root on a walk's empty stack.
+__device__ __forceinline__ void walk_start(const BhCells &T, Walk &S, int lane, unsigned lanes,
+                                           double px, double py, double pz, double theta,
+                                           double theta2) {
+  const int2 m = T.meta[0];
+  int4 e = make_int4(m.x, m.y, (int)lanes, 0);
+  if (m.y < 0) {
+    const bool acc = (lanes >> lane & 1) && bh_accept(T, 0, T.geo[0], px, py, pz, theta, theta2);
+    const unsigned am = __ballot_sync(0xffffffffu, acc);
+    e = make_int4(0, -m.x, (int)am, (int)(lanes & ~am));
+  }
+  if (lane == 0) S.stack[0] = e;
+  __syncwarp();
+}
+
+// Drops the list's first 32 entries.
+__device__ __forceinline__ void walk_shift(Walk &S, int lane, int &count) {
+  count -= 32;
+  if (lane < count) {
+    S.list[lane] = S.list[lane + 32];
+    S.list_lanes[lane] = S.list_lanes[lane + 32];
+  }
+  __syncwarp();
+}
+
+// The inclusive sums of v over the lanes, and the first lane whose sum is above i.
+__device__ __forceinline__ int lane_sums(int lane, int v) {
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, s);
+    if (lane >= s) v += u;
+  }
+  return v;
+}
+__device__ __forceinline__ int lane_above(int sums, int i) {
+  int k = 0;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1)
+    if (__shfl_sync(0xffffffffu, sums, k + s - 1) <= i) k += s;
+  return k;
+}
+
 // FP64: one walk per warp over the union of its 32 bodies' walks.  Opening a
 // cell classes its eight children by eight lanes with the bodies' box, tests
 // the uncertain ones body by body, and pushes each child with the lanes that
 // accept it and the lanes that open it (leaves with the lanes that reach them).
-// Popped depth first, children 0..7, the accepted cells and leaf bodies form a
-// list; entry k of the list is held by lane k (index and lane mask), and when
-// 32 are there their moments or bodies are loaded by a lane each and every lane
-// adds the terms of its own entries in list order.  A lane's entries in the list
-// are its own walk's, in its own walk's order, so it takes the sample's
-// decisions and sums the sample's terms in the sample's order, bit for bit.
+// Popped depth first, children 0..7, the accepted cells and the leaves form a
+// list; 32 entries at a time, their moments and bodies are loaded by a lane each
+// and every lane adds the terms of its own entries in list order.  A lane's
+// entries in the list are its own walk's, in its own walk's order, so it takes
+// the sample's decisions and sums the sample's terms in the sample's order, bit
+// for bit.
 //
 // Why so: 32 bodies' union walk is long and small sets have few warps (20k
 // bodies: 625, one per scheduler), so the time is one warp's chain of dependent
-// loads and FP64 sequences; here a chain step serves eight cells, 32 loads or
-// four terms instead of one.  One warp per block, so that few warps spread
-// evenly over the SMs.  20k bodies, ncrit 1: 0.82 ms; 2.39 ms with one cell and
-// one term at a time, 1.68 ms without the box's tests.
+// loads and FP64 sequences; here a chain step serves up to 32 popped entries,
+// eight opened cells, 32 loads or four terms instead of one.  One warp per block,
+// so that few warps spread evenly over the SMs.  20k bodies, ncrit 1: 0.69 ms;
+// 0.81 ms with one entry popped at a time, 2.39 ms with one cell and one term at
+// a time, 1.68 ms without the box's tests.
 __global__ void __launch_bounds__(32) bh_walk64(
     BhCells T, int64_t n, const double *__restrict__ sx, const double *__restrict__ sy,
     const double *__restrict__ sz, const double *__restrict__ sm,
     const double4 *__restrict__ attr, double theta, double eps2, double *__restrict__ out,
     unsigned long long *__restrict__ counters) {
-  // stack entry: {cell, -first child, accepting lanes, opening lanes} or, a
-  // leaf, {first body, bodies, lanes, 0}
-  __shared__ int4 stack[kStack];
+  __shared__ Walk S;
   __shared__ double4 data[32];
+  __shared__ unsigned data_lanes[32];
   const int lane = threadIdx.x;
   const double theta2 = __dmul_rn(theta, theta);
   const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -223,123 +353,77 @@ __global__ void __launch_bounds__(32) bh_walk64(
 
   const BodyBox box = body_box(valid, px, py, pz);
 
-  int count = 0;       // list entries
-  int idx = 0;         // this lane's entry: body, or ~cell
-  unsigned mask = 0;   // and the lanes that add it
-  auto flush = [&]() {
-    __syncwarp();
-    double4 v = make_double4(0, 0, 0, 0);
-    if (lane < count) v = idx >= 0 ? make_double4(sx[idx], sy[idx], sz[idx], sm[idx]) : attr[~idx];
-    else mask = 0;
-    data[lane] = v;
-    __syncwarp();
+  // Adds the terms of the first `count` (<= 32) list entries.
+  auto flush = [&](int count) {
+    int2 r = make_int2(0, 0);
+    unsigned rm = 0;
+    if (lane < count) {
+      r = S.list[lane];
+      rm = S.list_lanes[lane];
+    }
+    const int terms = r.y >= 0 ? r.y : 1;
+    const int upto = lane_sums(lane, terms);
+    const int total = __shfl_sync(0xffffffffu, upto, 31);
+    for (int c0 = 0; c0 < total; c0 += 32) {
+      const int i = c0 + lane, k = lane_above(upto, i);
+      const int p = __shfl_sync(0xffffffffu, r.x, k);
+      const int p0 = __shfl_sync(0xffffffffu, upto - terms, k);
+      const unsigned m = __shfl_sync(0xffffffffu, rm, k);
+      double4 v = make_double4(0, 0, 0, 0);
+      if (i < total) {
+        const int j = p + (i - p0);
+        v = p >= 0 ? make_double4(sx[j], sy[j], sz[j], sm[j]) : attr[~p];
+      }
+      data[lane] = v;
+      data_lanes[lane] = i < total ? m : 0u;
+      __syncwarp();
+      const int end = min(32, total - c0);
 #pragma unroll 1
-    for (int k = 0; k < count; k += 4) {
-      // ComputeForce (bh.cc:135-153), the sample's rounding order
-      double dx[4], dy[4], dz[4], w[4], R2[4], inv[4];
+      for (int q = 0; q < end; q += 4) {
+        // ComputeForce (bh.cc:135-153), the sample's rounding order
+        double dx[4], dy[4], dz[4], w[4], R2[4], inv[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const double4 a = data[k + i];
-        dx[i] = __dsub_rn(a.x, px);
-        dy[i] = __dsub_rn(a.y, py);
-        dz[i] = __dsub_rn(a.z, pz);
-        w[i] = a.w;
-        R2[i] = __dadd_rn(__dmul_rn(dx[i], dx[i]), __dmul_rn(dy[i], dy[i]));
-        R2[i] = __dadd_rn(__dadd_rn(R2[i], __dmul_rn(dz[i], dz[i])), eps2);
-      }
-      rounded_inv_sqrt(R2, inv);
+        for (int i = 0; i < 4; i++) {
+          const double4 a = data[q + i];
+          dx[i] = __dsub_rn(a.x, px);
+          dy[i] = __dsub_rn(a.y, py);
+          dz[i] = __dsub_rn(a.z, pz);
+          w[i] = a.w;
+          R2[i] = __dadd_rn(__dmul_rn(dx[i], dx[i]), __dmul_rn(dy[i], dy[i]));
+          R2[i] = __dadd_rn(__dadd_rn(R2[i], __dmul_rn(dz[i], dz[i])), eps2);
+        }
+        rounded_inv_sqrt(R2, inv);
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const bool mine = (__shfl_sync(0xffffffffu, mask, k + i) >> lane) & 1u;
-        const double inv3 = __dmul_rn(__dmul_rn(inv[i], inv[i]), inv[i]);
-        const double tx = __dmul_rn(__dmul_rn(dx[i], inv3), w[i]),
-                     ty = __dmul_rn(__dmul_rn(dy[i], inv3), w[i]),
-                     tz = __dmul_rn(__dmul_rn(dz[i], inv3), w[i]), tw = __dmul_rn(inv[i], w[i]);
-        if (mine) {
-          o.x = __dadd_rn(o.x, tx);
-          o.y = __dadd_rn(o.y, ty);
-          o.z = __dadd_rn(o.z, tz);
-          o.w = __dadd_rn(o.w, tw);
+        for (int i = 0; i < 4; i++) {
+          const double inv3 = __dmul_rn(__dmul_rn(inv[i], inv[i]), inv[i]);
+          const double tx = __dmul_rn(__dmul_rn(dx[i], inv3), w[i]),
+                       ty = __dmul_rn(__dmul_rn(dy[i], inv3), w[i]),
+                       tz = __dmul_rn(__dmul_rn(dz[i], inv3), w[i]), tw = __dmul_rn(inv[i], w[i]);
+          if (data_lanes[q + i] >> lane & 1u) {
+            o.x = __dadd_rn(o.x, tx);
+            o.y = __dadd_rn(o.y, ty);
+            o.z = __dadd_rn(o.z, tz);
+            o.w = __dadd_rn(o.w, tw);
+          }
         }
       }
-    }
-    count = 0;
-  };
-
-  int sp = 1;
-  {
-    const int2 m = T.meta[0];
-    int4 e = make_int4(m.x, m.y, (int)lanes, 0);
-    if (m.y < 0) {
-      const bool acc = valid && bh_accept(T, 0, T.geo[0], px, py, pz, theta, theta2);
-      const unsigned am = __ballot_sync(0xffffffffu, acc);
-      e = make_int4(0, -m.x, (int)am, (int)(lanes & ~am));
-    }
-    if (lane == 0) stack[0] = e;
-    __syncwarp();
-  }
-  while (sp > 0) {
-    const int4 e = stack[--sp];
-    if (e.y >= 0) {  // a leaf's bodies
-      ndirect += (unsigned long long)e.y * __popc(e.z);
-      for (int done = 0; done < e.y;) {
-        const int take = min(32 - count, e.y - done), at = lane - count;
-        if (at >= 0 && at < take) {
-          idx = e.x + done + at;
-          mask = (unsigned)e.z;
-        }
-        done += take;
-        count += take;
-        if (count == 32) flush();
-      }
-      continue;
-    }
-    if (e.z) {
-      napprox += __popc(e.z);
-      if (lane == count) {
-        idx = ~e.x;
-        mask = (unsigned)e.z;
-      }
-      if (++count == 32) flush();
-    }
-    if (e.w) {
-      if (sp + 8 > kStack) {
-        overflow = true;
-        break;
-      }
-      const int ch = -e.y, c = ch + (lane & 7);
-      const int2 m = T.meta[c];
-      const double4 g = T.geo[c];
-      const int kind = m.y < 0 ? box_accept(box, g, theta2) : 3;  // 3: a leaf
-      // this lane's child (lanes 0..7): accepting and opening lanes
-      unsigned am = kind == 1 ? (unsigned)e.w : 0u, om = kind == 2 ? (unsigned)e.w : 0u;
-      unsigned todo = __ballot_sync(0xffffffffu, kind == 0) & 0xffu;
-      while (todo) {
-        const int i = __ffs(todo) - 1;
-        todo &= todo - 1;
-        double4 gi;
-        gi.x = __shfl_sync(0xffffffffu, g.x, i);
-        gi.y = __shfl_sync(0xffffffffu, g.y, i);
-        gi.z = __shfl_sync(0xffffffffu, g.z, i);
-        gi.w = __shfl_sync(0xffffffffu, g.w, i);
-        const bool acc = bh_accept(T, ch + i, gi, px, py, pz, theta, theta2);
-        const unsigned a = __ballot_sync(0xffffffffu, acc) & (unsigned)e.w;
-        if (lane == i) {
-          am = a;
-          om = (unsigned)e.w & ~a;
-        }
-      }
-      // every lane has read the popped entries (the ballots); child 7 at the bottom
-      const bool push = lane < 8 && m.y != 0;  // not an empty leaf
-      const unsigned pushes = __ballot_sync(0xffffffffu, push);
-      if (push)
-        stack[sp + __popc(pushes >> (lane + 1))] =
-            m.y > 0 ? make_int4(m.x, m.y, e.w, 0) : make_int4(c, -m.x, (int)am, (int)om);
-      sp += __popc(pushes);
       __syncwarp();
     }
+  };
+
+  int sp = 1, count = 0;
+  walk_start(T, S, lane, lanes, px, py, pz, theta, theta2);
+  while (sp > 0) {
+    if (!walk_step(T, S, box, lane, px, py, pz, theta, theta2, sp, count, napprox, ndirect)) {
+      overflow = true;
+      break;
+    }
+    if (count >= 32) {
+      flush(32);
+      walk_shift(S, lane, count);
+    }
   }
-  if (!overflow) flush();
+  if (!overflow) flush(count);
   if (valid) reinterpret_cast<double4 *>(out)[b] = o;
   add_counts(lane, napprox, ndirect, overflow, counters);
 }
@@ -353,255 +437,141 @@ __device__ __forceinline__ float inv_sqrt32(float x) {
   return y;
 }
 
-// FP32: the same union walk and decisions (the acceptance test stays FP64), but
-// a body's terms are added in any order (FP32 sums).  The stack holds opened
-// cells only.  Four of them are opened at a time, a lane per child: the bodies'
-// box decides for all bodies where it can, the uncertain children are tested
-// body by body; leaf children and accepted children go to two lists with the
-// lanes that add them.  32 listed leaves are evaluated as one stream of body
-// pairs, 32 pairs at a time loaded by a lane each into shared memory whatever
-// leaf they belong to, then added leaf by leaf by the lanes that reach it; 32
-// listed cells make 16 pairs with a mask per cell, 1/r replaced by 0 for the
-// lanes that do not accept it.
+// FP32: the same union walk, decisions and order (the acceptance test stays
+// FP64).  Accepted cells and leaves form one list in walk order, appended for all
+// the stack's top entries down to the first that opens at once.  32 entries are
+// evaluated as one stream of slots, a slot a pair of leaf bodies or of cells: 32
+// slots at a time are loaded by a lane each, whatever entry they belong to, into
+// shared memory with the lanes that add each half, then evaluated by all lanes.
 // Leaf bodies are stored as pairs {x0,x1,y0,y1},{z0,z1,m0,m1}, each leaf starting
 // a pair (an odd leaf's last one is padded with a massless copy of its first
-// body), and a packed FP32 instruction evaluates two: 13 packed operations and 2
-// MUFU per pair.  Bound: FP32 pipe (62 %) and issue (62 %); the union holds 1.37
-// times the bodies' own leaf bodies (a simulated 400k Plummer sphere: 73 % of
-// the lanes add a listed body).  4M Plummer, ncrit 32: 35.3 ms; 66.5 ms with a
-// test per lane and cell and the leaves evaluated where they are met, from global
-// memory (4.4 slots per issue waiting for loads), 53.1 ms with the lists but a test
-// per lane and a mask per source.
+// body).  A slot's terms are evaluated by packed FP32 instructions, then added one
+// after the other: an FP32 sum of 10^4 terms of one sign is rounded by 3e-5
+// somewhere, and only the walk's own order rounds it where this form always has.
+// Bound: issue slots and FP32 pipe; the union holds 1.37 times the bodies' own leaf
+// bodies (a simulated 400k Plummer sphere: 73 % of the lanes add a listed body).
+// 4M Plummer, ncrit 32: 41.4 ms; 66.5 ms with a cell or a body at a time; 43.7 ms as
+// four warps to a block, whose slowest holds the others' places; 57.2 ms with one
+// entry popped and evaluated at a time.
 // kNormal: eps2 is a normal FP32 number, so no squared distance is below it.
-constexpr float kNowhere = 1.25e18f;  // coordinate of a padding source
-constexpr int kOpen = 4;              // cells opened at a time
-constexpr int kStack32 = 640;         // > 28 pending cells x 19 levels + 32
-
-struct __align__(16) Walk32Warp {
-  double4 geo[32];
-  float4 a[32], b[32];  // pairs of sources {x0,x1,y0,y1}, {z0,z1,m0,m1}
-  uint2 m[16];          // listed cells: the lanes that add either
-  int2 leaf[64];        // {first pair, pairs}
-  int cell[64];
-  unsigned leaf_m[64], cell_m[64];  // and the lanes that add them
-  int2 stack[kStack32];             // {first child, lanes that opened the cell}
-};
+constexpr int kSlots = 4;  // slots evaluated at once: 41.4 ms; 2: 42.5 ms
 
 template <bool kNormal>
-__global__ void __launch_bounds__(32 * kWalk32Warps, 6) bh_walk32(
+__global__ void __launch_bounds__(32, 32) bh_walk32(
     BhCells T, int64_t n, const double *__restrict__ sx, const double *__restrict__ sy,
     const double *__restrict__ sz, const float4 *__restrict__ attr32,
     const float4 *__restrict__ pairs, double theta, float eps2, double *__restrict__ out,
     unsigned long long *__restrict__ counters) {
-  __shared__ Walk32Warp warps[kWalk32Warps];
-  const int lane = threadIdx.x & 31;
-  Walk32Warp &S = warps[threadIdx.x >> 5];
-  const unsigned me = 1u << lane, below = me - 1;
+  __shared__ Walk S;
+  __shared__ BodyBox box;  // kept here: the registers are needed
+  // staged slots {x0,x1,y0,y1}, {z0,z1,m0,m1} and the lanes that add their halves
+  __shared__ float4 slot_a[32], slot_b[32];
+  __shared__ uint2 slot_lanes[32];
+  const int lane = threadIdx.x;
+  const unsigned me = 1u << lane;
   const double theta2 = __dmul_rn(theta, theta);
   const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = b < n;
   const double px = valid ? sx[b] : 0.0, py = valid ? sy[b] : 0.0, pz = valid ? sz[b] : 0.0;
   const float fx = -(float)px, fy = -(float)py, fz = -(float)pz;
-  const float2 nx = make_float2(fx, fx), ny = make_float2(fy, fy), nz = make_float2(fz, fz);
-  const float2 e2 = make_float2(eps2, eps2);
-  float2 ox = make_float2(0.f, 0.f), oy = ox, oz = ox, ow = ox;
-  unsigned long long napprox = 0, ndirect = 0;  // this lane's cells' and leaves'
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  unsigned long long napprox = 0, ndirect = 0;
   bool overflow = false;
   const unsigned lanes = __ballot_sync(0xffffffffu, valid);
   if (lanes == 0) return;
-  const BodyBox box = body_box(valid, px, py, pz);
-
-  // adds a pair of sources; a source whose flag is false adds nothing
-  auto add_pair = [&](const float4 &u, const float4 &v, bool t0, bool t1) {
-    const float2 dx = __fadd2_rn(make_float2(u.x, u.y), nx),
-                 dy = __fadd2_rn(make_float2(u.z, u.w), ny),
-                 dz = __fadd2_rn(make_float2(v.x, v.y), nz);
-    const float2 R2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-    const float i0 = inv_sqrt32<kNormal>(R2.x), i1 = inv_sqrt32<kNormal>(R2.y);
-    const float2 inv = make_float2(t0 ? i0 : 0.f, t1 ? i1 : 0.f);
-    const float2 wr = __fmul2_rn(make_float2(v.z, v.w), inv);
-    const float2 wr3 = __fmul2_rn(__fmul2_rn(wr, inv), inv);
-    ox = __ffma2_rn(dx, wr3, ox);
-    oy = __ffma2_rn(dy, wr3, oy);
-    oz = __ffma2_rn(dz, wr3, oz);
-    ow = __fadd2_rn(ow, wr);
-  };
-
-  int nleaf = 0, ncell = 0;  // listed
-  auto flush_leaves = [&]() {  // the last 32 listed, or all
+  {
+    const BodyBox bx = body_box(valid, px, py, pz);
+    if (lane == 0) box = bx;
     __syncwarp();
-    const int base = max(0, nleaf - 32), cnt = nleaf - base;
-    int2 l = make_int2(0, 0);
-    unsigned lm = 0;
-    if (lane < cnt) {
-      l = S.leaf[base + lane];
-      lm = S.leaf_m[base + lane];
+  }
+
+  // Evaluates the first `count` (<= 32) list entries.
+  auto flush = [&](int count) {
+    int2 r = make_int2(0, 0);
+    unsigned rm = 0;
+    if (lane < count) {
+      r = S.list[lane];
+      rm = S.list_lanes[lane];
     }
-    nleaf = base;
-    int upto = l.y;  // pairs of the leaves 0 .. lane
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, upto, o);
-      if (lane >= o) upto += v;
-    }
+    // a run of cells is taken in pairs: the second one's slot is the first one's
+    const unsigned cells = __ballot_sync(0xffffffffu, r.y < 0);
+    const int before = lane ? __clz(~(cells << (32 - lane))) : 0;  // cells just below
+    const int slots = r.y >= 0 ? (r.y + 1) >> 1 : (before & 1) ^ 1;
+    const int upto = lane_sums(lane, slots);
     const int total = __shfl_sync(0xffffffffu, upto, 31);
-    const int first = l.x - (upto - l.y);  // pair i of the stream is pair first + i
-    int e = 0, at = 0;                     // the stream's next leaf and pair
     for (int c0 = 0; c0 < total; c0 += 32) {
-      const int i = c0 + lane;
-      int k = 0;  // the first leaf with upto > i
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, upto, k + o - 1);
-        if (v <= i) k += o;
-      }
-      const int64_t p = __shfl_sync(0xffffffffu, first, k) + i;
+      const int i = c0 + lane, k = lane_above(upto, i);
+      const int p = __shfl_sync(0xffffffffu, r.x, k);
+      const int p0 = __shfl_sync(0xffffffffu, upto - slots, k);
+      const unsigned m0 = __shfl_sync(0xffffffffu, rm, k);
+      const int pn = __shfl_sync(0xffffffffu, r.x, (k + 1) & 31);
+      const unsigned mn = __shfl_sync(0xffffffffu, rm, (k + 1) & 31);
       if (i < total) {
-        S.a[lane] = __ldg(pairs + 2 * p);
-        S.b[lane] = __ldg(pairs + 2 * p + 1);
-      }
-      __syncwarp();
-      const int end = min(c0 + 32, total);
-      while (at < end) {
-        const int ue = __shfl_sync(0xffffffffu, upto, e);
-        const unsigned m = __shfl_sync(0xffffffffu, lm, e);
-        const int stop = min(ue, end);
-        if (m & me) {
-#pragma unroll 2
-          for (int q = at - c0; q < stop - c0; q++) add_pair(S.a[q], S.b[q], true, true);
+        if (p >= 0) {
+          const float4 *src = pairs + 2 * ((int64_t)p + (i - p0));
+          slot_a[lane] = __ldg(src);
+          slot_b[lane] = __ldg(src + 1);
+          slot_lanes[lane] = make_uint2(m0, m0);
+        } else {
+          const bool two = k < 31 && (cells >> (k + 1) & 1);
+          const float4 u = __ldg(attr32 + ~p);
+          const float4 v = two ? __ldg(attr32 + ~pn) : u;
+          slot_a[lane] = make_float4(u.x, v.x, u.y, v.y);
+          slot_b[lane] = make_float4(u.z, v.z, u.w, v.w);
+          slot_lanes[lane] = make_uint2(m0, two ? mn : 0u);
         }
-        at = stop;
-        if (at == ue) e++;
+      } else {
+        slot_lanes[lane] = make_uint2(0u, 0u);  // whatever the slot holds
+      }
+      __syncwarp();
+      const int end = min(32, total - c0);
+#pragma unroll 1
+      for (int q0 = 0; q0 < end; q0 += kSlots)
+#pragma unroll
+      for (int q = q0; q < q0 + kSlots; q++) {
+        const float4 u = slot_a[q], v = slot_b[q];
+        const uint2 m = slot_lanes[q];
+        const float2 dx = __fadd2_rn(make_float2(u.x, u.y), make_float2(fx, fx)),
+                     dy = __fadd2_rn(make_float2(u.z, u.w), make_float2(fy, fy)),
+                     dz = __fadd2_rn(make_float2(v.x, v.y), make_float2(fz, fz));
+        const float2 R2 = __ffma2_rn(
+            dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, make_float2(eps2, eps2))));
+        const float2 inv = make_float2(inv_sqrt32<kNormal>(R2.x), inv_sqrt32<kNormal>(R2.y));
+        const float2 wr = __fmul2_rn(make_float2(v.z, v.w), inv);
+        const float2 wr3 = __fmul2_rn(__fmul2_rn(wr, inv), inv);
+        if (m.x & me) {
+          o.x = fmaf(dx.x, wr3.x, o.x);
+          o.y = fmaf(dy.x, wr3.x, o.y);
+          o.z = fmaf(dz.x, wr3.x, o.z);
+          o.w = __fadd_rn(o.w, wr.x);
+        }
+        if (m.y & me) {
+          o.x = fmaf(dx.y, wr3.y, o.x);
+          o.y = fmaf(dy.y, wr3.y, o.y);
+          o.z = fmaf(dz.y, wr3.y, o.z);
+          o.w = __fadd_rn(o.w, wr.y);
+        }
       }
       __syncwarp();
     }
-  };
-  auto flush_cells = [&]() {  // the last 32 listed, or all
-    __syncwarp();
-    const int base = max(0, ncell - 32), cnt = ncell - base;
-    int cell = 0;
-    unsigned cm = 0, m = 0;
-    float4 c = make_float4(kNowhere, kNowhere, kNowhere, 0.f);
-    bool odd = false;
-    if (lane < cnt) {
-      cell = S.cell[base + lane];
-      cm = S.cell_m[base + lane];
-      const float4 v = attr32[cell];
-      // a centre that is not finite (no net mass) must reach its own lanes only
-      odd = !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) <= FLT_MAX);
-      if (!odd) {
-        c = v;
-        m = cm;
-      }
-    }
-    ncell = base;
-    const int half = lane & 1;
-    float *pa = reinterpret_cast<float *>(&S.a[lane >> 1]) + half;
-    float *pb = reinterpret_cast<float *>(&S.b[lane >> 1]) + half;
-    pa[0] = c.x;
-    pa[2] = c.y;
-    pb[0] = c.z;
-    pb[2] = c.w;
-    reinterpret_cast<unsigned *>(&S.m[lane >> 1])[half] = m;
-    __syncwarp();
-#pragma unroll 2
-    for (int k = 0; k < (cnt + 1) >> 1; k++) {
-      const uint2 w = S.m[k];
-      add_pair(S.a[k], S.b[k], (w.x & me) != 0, (w.y & me) != 0);
-    }
-    unsigned todo = __ballot_sync(0xffffffffu, odd);
-    while (todo) {
-      const int k = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const float4 v = attr32[__shfl_sync(0xffffffffu, cell, k)];
-      if (__shfl_sync(0xffffffffu, cm, k) & me) {
-        const float dx = v.x + fx, dy = v.y + fy, dz = v.z + fz;
-        const float inv = inv_sqrt32<kNormal>(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2))));
-        const float wr = v.w * inv, wr3 = wr * inv * inv;
-        ox.x = fmaf(dx, wr3, ox.x);
-        oy.x = fmaf(dy, wr3, oy.x);
-        oz.x = fmaf(dz, wr3, oz.x);
-        ow.x += wr;
-      }
-    }
-    __syncwarp();
   };
 
-  // A round classes this lane's cell c (if has), with record {m, g} and the lanes
-  // reach that opened its parent.
-  int sp = 0;
-  auto round = [&](bool has, int c, int2 m, const double4 &g, unsigned reach) {
-    const bool is_leaf = has && m.y > 0;
-    int kind = has && m.y < 0 ? box_accept(box, g, theta2) : 3;
-    unsigned todo = __ballot_sync(0xffffffffu, kind == 0);
-    if (kind == 0) S.geo[lane] = g;
-    const unsigned leaves = __ballot_sync(0xffffffffu, is_leaf);
-    if (is_leaf) {
-      const int k = nleaf + __popc(leaves & below);
-      S.leaf[k] = make_int2(m.x, (m.y + 1) >> 1);
-      S.leaf_m[k] = reach;
-      ndirect += (unsigned long long)m.y * __popc(reach);
-    }
-    nleaf += __popc(leaves);
-    __syncwarp();
-    unsigned am = kind == 1 ? reach : 0u, om = kind == 2 ? reach : 0u;
-    while (todo) {  // uncertain: every body's own test
-      const int i = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const int ci = __shfl_sync(0xffffffffu, c, i);
-      const bool acc = bh_accept(T, ci, S.geo[i], px, py, pz, theta, theta2);
-      const unsigned a = __ballot_sync(0xffffffffu, acc);
-      if (lane == i) {
-        am = a & reach;
-        om = reach & ~a;
-      }
-    }
-    const unsigned accs = __ballot_sync(0xffffffffu, am != 0),
-                   opens = __ballot_sync(0xffffffffu, om != 0);
-    if (am) {
-      const int k = ncell + __popc(accs & below);
-      S.cell[k] = c;
-      S.cell_m[k] = am;
-      napprox += __popc(am);
-    }
-    ncell += __popc(accs);
-    if (om) S.stack[sp + __popc(opens & below)] = make_int2(m.x, (int)om);
-    sp += __popc(opens);
-    if (nleaf >= 32) flush_leaves();
-    if (ncell >= 32) flush_cells();
-    __syncwarp();
-  };
-  round(lane == 0, 0, T.meta[0], T.geo[0], lanes);
+  int sp = 1, count = 0;
+  walk_start(T, S, lane, lanes, px, py, pz, theta, theta2);
   while (sp > 0) {
-    const int take = min(kOpen, sp);
-    sp -= take;
-    if (sp + 8 * kOpen > kStack32) {
+    if (!walk_step(T, S, box, lane, px, py, pz, theta, theta2, sp, count, napprox, ndirect)) {
       overflow = true;
       break;
     }
-    const bool has = (lane >> 3) < take;
-    const int2 e = has ? S.stack[sp + (lane >> 3)] : make_int2(0, 0);
-    const int c = e.x + (lane & 7);
-    int2 m = make_int2(0, 0);
-    double4 g = make_double4(0, 0, 0, 0);
-    if (has) {
-      m = __ldg(T.meta + c);
-      g = T.geo[c];
+    if (count >= 32) {
+      flush(32);
+      walk_shift(S, lane, count);
     }
-    __syncwarp();  // the popped entries are read
-    round(has, c, m, g, (unsigned)e.y);
   }
-  while (nleaf) flush_leaves();
-  while (ncell) flush_cells();
+  if (!overflow) flush(count);
   if (valid)
     reinterpret_cast<double4 *>(out)[b] =
-        make_double4((double)(ox.x + ox.y), (double)(oy.x + oy.y), (double)(oz.x + oz.y),
-                     (double)(ow.x + ow.y));
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) {
-    napprox += __shfl_xor_sync(0xffffffffu, napprox, s);
-    ndirect += __shfl_xor_sync(0xffffffffu, ndirect, s);
-  }
+        make_double4((double)o.x, (double)o.y, (double)o.z, (double)o.w);
   add_counts(lane, napprox, ndirect, overflow, counters);
 }
 
@@ -711,11 +681,10 @@ int bh_interact(tapas_b200_ctx *ctx, double theta, double eps2, int precision) {
                                                        ctx->sq.p, ctx->bh_attr.p, theta, eps2,
                                                        ctx->trg.p, ctx->counters.p);
   } else {
-    constexpr int kThreads = 32 * kWalk32Warps;
     auto walk = (float)eps2 >= FLT_MIN ? bh_walk32<true> : bh_walk32<false>;
-    walk<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-        T, n, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->bh_attr32.p, ctx->bh_pairs.p, theta, (float)eps2,
-        ctx->trg.p, ctx->counters.p);
+    walk<<<(unsigned)((n + 31) / 32), 32, 0, s>>>(T, n, ctx->sx.p, ctx->sy.p, ctx->sz.p,
+                                                  ctx->bh_attr32.p, ctx->bh_pairs.p, theta,
+                                                  (float)eps2, ctx->trg.p, ctx->counters.p);
   }
   TB_LAUNCH_CHECK(ctx);
   unsigned long long *h = reinterpret_cast<unsigned long long *>(ctx->pinned.p);
