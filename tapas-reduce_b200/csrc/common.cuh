@@ -213,7 +213,7 @@ struct tapas_b200_ctx {
   tb::DBuf<int2> front_a, front_b;      // (target, source) pairs
   tb::DBuf<uint64_t> m2l, p2p;          // (target << 32 | source)
   tb::DBuf<uint64_t> list_alt;
-  tb::DBuf<int32_t> list_cnt;           // list ordering: per-target counts, cursors, long segments
+  tb::DBuf<int32_t> list_cnt;           // list ordering: per-target counts of both lists, long segments
   tb::DBuf<uint32_t> list_src;          // list ordering: sources grouped by target
   tb::DBuf<unsigned long long> counters; // [next, m2l, p2p, p2p_interactions, overflow]
   int64_t n_m2l = 0, n_p2p = 0;         // directed pairs in the lists
@@ -236,7 +236,7 @@ struct tapas_b200_ctx {
   int near_precision = TAPAS_B200_FP64;  // of the last P2P: FP64 sums carry q_i, mixed do not
   tb::DBuf<uint64_t> p2p_wkey, p2p_wkey_alt;  // P2P work order: keys
   tb::DBuf<uint32_t> p2p_order, p2p_order_alt;  // target leaves by decreasing work
-  tb::DBuf<int> p2p_counter;            // P2P work-queue head
+  tb::DBuf<int> p2p_counter;            // P2P work-queue head, item and piece-row totals
   tb::DBuf<uint8_t> p2p_key;            // per leaf: queue key of its whole list
   tb::DBuf<int4> p2p_items;             // P2P work items (leaf, list range, partial rows)
   tb::DBuf<int32_t> p2p_kcnt, p2p_koff, p2p_psz, p2p_poff;  // per leaf: pieces, partial rows

@@ -1252,16 +1252,15 @@ int m2l_classes(tapas_b200_ctx *ctx, size_t op_bytes, int64_t min_pairs, M2LClas
                                                               T.tcflag.p, T.ntiles.p);
     TB_LAUNCH_CHECK(ctx);
   }
-  TB_TRY(scan_exclusive(ctx, T.tcflag.p, T.tcid.p, nseg, T.tcid.p + nseg));
-  TB_TRY(scan_exclusive(ctx, T.ntiles.p, T.tile_off.p, nseg, T.tile_off.p + nseg));
-  TB_CUDA(ctx, cudaMemsetAsync(T.err.p + 3, 0, sizeof(int), s));
+  // their totals and the FP64 pairs' count: err 5 .. 7 (7 is zero since the start)
+  const int32_t *const in[2] = {T.tcflag.p, T.ntiles.p};
+  int32_t *const out[2] = {T.tcid.p, T.tile_off.p};
+  int32_t *const tot[2] = {T.err.p + 5, T.err.p + 6};
+  TB_TRY(scan_exclusive2(ctx, in, out, nseg, tot, nullptr));
   mark_fp64_pairs<<<grid_for(n, 256, ctx->num_sms * 16), 256, 0, s>>>(
-      T.scan.p, T.flag.p, T.tcflag.p, T.keys.p, kp, T.vals.p, n, T.pairs64.p, T.err.p + 3);
+      T.scan.p, T.flag.p, T.tcflag.p, T.keys.p, kp, T.vals.p, n, T.pairs64.p, T.err.p + 7);
   TB_LAUNCH_CHECK(ctx);
-  TB_CUDA(ctx, cudaMemcpyAsync(h, T.tcid.p + nseg, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  TB_CUDA(ctx, cudaMemcpyAsync(h + 1, T.tile_off.p + nseg, sizeof(int32_t),
-                               cudaMemcpyDeviceToHost, s));
-  TB_CUDA(ctx, cudaMemcpyAsync(h + 2, T.err.p + 3, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  TB_CUDA(ctx, cudaMemcpyAsync(h, T.err.p + 5, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   TB_CUDA(ctx, cudaStreamSynchronize(s));
   const int64_t ntc = h[0], nitems = h[1], n64 = h[2];
   ctx->tc_classes = ntc;
@@ -1271,8 +1270,6 @@ int m2l_classes(tapas_b200_ctx *ctx, size_t op_bytes, int64_t min_pairs, M2LClas
   TB_CUDA(ctx, T.tc_keys.ensure(ntc + 1, s));
   TB_CUDA(ctx, T.cls_range.ensure(ntc + 1, s));
   TB_CUDA(ctx, T.items.ensure((size_t)(nitems + 1) * sizeof(TileItem) / 16 + 1, s));
-  TB_CUDA(ctx, T.err.ensure(4, s));
-  TB_CUDA(ctx, cudaMemsetAsync(T.err.p, 0, 4 * sizeof(int), s));
   build_tiles<<<grid_for(32 * nseg, 256), 256, 0, s>>>(T.seg_start.p, nseg, n, T.tcflag.p, T.tcid.p,
                                                    T.tile_off.p, T.keys.p, kp, T.tc_keys.p,
                                                    reinterpret_cast<TileItem *>(T.items.p),

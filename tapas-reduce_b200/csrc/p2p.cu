@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(256) leaf_pieces(
     const int32_t *__restrict__ leaves, int64_t nleaves, const int32_t *__restrict__ off,
     const uint64_t *__restrict__ list, uint64_t src_mask, const int32_t *__restrict__ cnb,
     int64_t piece_pairs, uint8_t *__restrict__ wkey, int32_t *__restrict__ kcnt,
-    int32_t *__restrict__ psz) {
+    int32_t *__restrict__ psz, int *__restrict__ counter) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;  // the queue's head
   const int sub = threadIdx.x & 7;
   const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 3;
   for (int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >> 3; w0 < nleaves;
@@ -686,16 +687,19 @@ int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
   TB_CUDA(ctx, ctx->p2p_psz.ensure(nl + 1, s));
   TB_CUDA(ctx, ctx->p2p_poff.ensure(nl + 1, s));
   TB_CUDA(ctx, ctx->p2p_key.ensure(nl + 1, s));
+  TB_CUDA(ctx, ctx->p2p_counter.ensure(4, s));
   leaf_pieces<<<grid_for(8 * nl, 256), 256, 0, s>>>(leaves, nl, ctx->p2p_off.p, ctx->p2p.p, mask,
                                                     ctx->cnb.p, piece_pairs, ctx->p2p_key.p,
-                                                    ctx->p2p_kcnt.p, ctx->p2p_psz.p);
+                                                    ctx->p2p_kcnt.p, ctx->p2p_psz.p,
+                                                    ctx->p2p_counter.p);
   TB_LAUNCH_CHECK(ctx);
-  TB_TRY(scan_exclusive(ctx, ctx->p2p_kcnt.p, ctx->p2p_koff.p, nl, ctx->p2p_koff.p + nl));
-  TB_TRY(scan_exclusive(ctx, ctx->p2p_psz.p, ctx->p2p_poff.p, nl, ctx->p2p_poff.p + nl));
+  const int32_t *const in[2] = {ctx->p2p_kcnt.p, ctx->p2p_psz.p};
+  int32_t *const out[2] = {ctx->p2p_koff.p, ctx->p2p_poff.p};
+  int32_t *const tot[2] = {ctx->p2p_counter.p + 1, ctx->p2p_counter.p + 2};
+  TB_TRY(scan_exclusive2(ctx, in, out, nl, tot, nullptr));
   TB_CUDA(ctx, ctx->pinned.ensure(256));
   int32_t *h = reinterpret_cast<int32_t *>(ctx->pinned.p);
-  TB_CUDA(ctx, cudaMemcpyAsync(h, ctx->p2p_koff.p + nl, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  TB_CUDA(ctx, cudaMemcpyAsync(h + 1, ctx->p2p_poff.p + nl, sizeof(int32_t),
+  TB_CUDA(ctx, cudaMemcpyAsync(h, ctx->p2p_counter.p + 1, 2 * sizeof(int32_t),
                                cudaMemcpyDeviceToHost, s));
   TB_CUDA(ctx, cudaStreamSynchronize(s));
   const int64_t ni = h[0], npart = h[1];
@@ -711,7 +715,6 @@ int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
   TB_CUDA(ctx, ctx->p2p_wkey_alt.ensure(ni + 1, s));
   TB_CUDA(ctx, ctx->p2p_order.ensure(ni + 1, s));
   TB_CUDA(ctx, ctx->p2p_order_alt.ensure(ni + 1, s));
-  TB_CUDA(ctx, ctx->p2p_counter.ensure(4, s));
   emit_items<<<grid_for(8 * nl, 256), 256, 0, s>>>(
       leaves, nl, ctx->p2p_off.p, ctx->p2p.p, mask, ctx->cnb.p, piece_pairs, ctx->p2p_key.p,
       ctx->p2p_kcnt.p, ctx->p2p_koff.p, ctx->p2p_poff.p, reinterpret_cast<WorkItem *>(ctx->p2p_items.p),
@@ -728,7 +731,6 @@ int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
     std::swap(ctx->p2p_wkey.p, ctx->p2p_wkey_alt.p);
     std::swap(ctx->p2p_wkey.cap, ctx->p2p_wkey_alt.cap);
   }
-  TB_CUDA(ctx, cudaMemsetAsync(ctx->p2p_counter.p, 0, sizeof(int), s));
   return TAPAS_B200_OK;
 }
 

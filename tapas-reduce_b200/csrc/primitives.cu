@@ -49,11 +49,18 @@ __device__ __forceinline__ int block_excl_scan(int v, int *smem_warp, int &total
   return r;
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_tiles(const int32_t *__restrict__ in,
-                                                           int32_t *__restrict__ out, int64_t n,
-                                                           int32_t *__restrict__ block_sums) {
-  // block_sums: per block its sum (for one block, the total); may be null
+// Up to two arrays of the same length scanned by one launch (blockIdx.y).
+struct ScanPair {
+  const int32_t *in[2];
+  int32_t *out[2];
+  int32_t *sums[2];  // per block its sum (for one block, the total); may be null
+  unsigned long long *mx[2];  // raised to the largest value; may be null
+};
+
+__global__ void __launch_bounds__(kScanThreads) scan_tiles(ScanPair p, int64_t n) {
   __shared__ int sw[33];
+  const int32_t *__restrict__ in = p.in[blockIdx.y];
+  int32_t *__restrict__ out = p.out[blockIdx.y];
   const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
   int v[kScanItems];
   int s = 0;
@@ -71,13 +78,20 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles(const int32_t *__rest
     if (g < n) out[g] = off;
     off += v[i];
   }
-  if (threadIdx.x == 0 && block_sums) block_sums[blockIdx.x] = total;
+  if (threadIdx.x == 0 && p.sums[blockIdx.y]) p.sums[blockIdx.y][blockIdx.x] = total;
+  if (p.mx[blockIdx.y]) {
+    int m = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) m = max(m, v[i]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(p.mx[blockIdx.y], (unsigned long long)m);
+  }
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_add(int32_t *__restrict__ out, int64_t n,
-                                                         const int32_t *__restrict__ block_offs) {
+__global__ void __launch_bounds__(kScanThreads) scan_add(ScanPair p, int64_t n) {
+  int32_t *__restrict__ out = p.out[blockIdx.y];
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
-  const int add = block_offs[blockIdx.x];
+  const int add = p.sums[blockIdx.y][blockIdx.x];
   for (int i = threadIdx.x; i < kScanTile; i += blockDim.x) {
     int64_t g = base + i;
     if (g < n) out[g] += add;
@@ -86,33 +100,41 @@ __global__ void __launch_bounds__(kScanThreads) scan_add(int32_t *__restrict__ o
 
 }  // namespace
 
-// Scan of in[0..n) into out using scratch[scratch_off..) for the block sums of
-// this level and the levels below (recursive reduce-then-scan); the last level's
-// one block writes the total.
-static int scan_level(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
-                      size_t scratch_off, int32_t *d_total) {
+// Scan of k arrays (p.sums: their totals) using scratch[scratch_off..) for the
+// block sums of this level and the levels below (recursive reduce-then-scan); the
+// last level's one block writes the total.
+static int scan_level(tapas_b200_ctx *ctx, const ScanPair &p, int k, int64_t n,
+                      size_t scratch_off) {
   cudaStream_t s = ctx->stream;
   const int64_t nb = (n + kScanTile - 1) / kScanTile;
   if (nb == 1) {
-    scan_tiles<<<1, kScanThreads, 0, s>>>(in, out, n, d_total);
+    scan_tiles<<<dim3(1, k), kScanThreads, 0, s>>>(p, n);
     TB_LAUNCH_CHECK(ctx);
     return TAPAS_B200_OK;
   }
-  int32_t *sums = ctx->scan_tmp.p + scratch_off;
-  int32_t *offs = sums + nb + 32;
-  scan_tiles<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, sums);
+  ScanPair tiles = p, below{}, add = p;
+  for (int y = 0; y < k; y++) {
+    int32_t *sums = ctx->scan_tmp.p + scratch_off + (size_t)y * (2 * (size_t)nb + 64);
+    int32_t *offs = sums + nb + 32;
+    tiles.sums[y] = sums;
+    below.in[y] = sums;
+    below.out[y] = offs;
+    below.sums[y] = p.sums[y];
+    add.sums[y] = offs;
+  }
+  scan_tiles<<<dim3((unsigned)nb, k), kScanThreads, 0, s>>>(tiles, n);
   TB_LAUNCH_CHECK(ctx);
-  TB_TRY(scan_level(ctx, sums, offs, nb, scratch_off + 2 * (size_t)nb + 64, d_total));
-  scan_add<<<(unsigned)nb, kScanThreads, 0, s>>>(out, n, offs);
+  TB_TRY(scan_level(ctx, below, k, nb, scratch_off + (size_t)k * (2 * (size_t)nb + 64)));
+  scan_add<<<dim3((unsigned)nb, k), kScanThreads, 0, s>>>(add, n);
   TB_LAUNCH_CHECK(ctx);
   return TAPAS_B200_OK;
 }
 
-int scan_exclusive(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
-                   int32_t *d_total) {
+static int scan_arrays(tapas_b200_ctx *ctx, const ScanPair &p, int k, int64_t n) {
   cudaStream_t s = ctx->stream;
   if (n <= 0) {
-    if (d_total) TB_CUDA(ctx, cudaMemsetAsync(d_total, 0, sizeof(int32_t), s));
+    for (int y = 0; y < k; y++)
+      if (p.sums[y]) TB_CUDA(ctx, cudaMemsetAsync(p.sums[y], 0, sizeof(int32_t), s));
     return TAPAS_B200_OK;
   }
   if (n > (int64_t)0x7FFFFFFF) {
@@ -126,8 +148,29 @@ int scan_exclusive(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t
     need += 2 * (size_t)nb + 64;
     m = nb;
   }
-  TB_CUDA(ctx, ctx->scan_tmp.ensure(need, s));
-  return scan_level(ctx, in, out, n, 0, d_total);
+  TB_CUDA(ctx, ctx->scan_tmp.ensure(k * need, s));
+  return scan_level(ctx, p, k, n, 0);
+}
+
+int scan_exclusive(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
+                   int32_t *d_total) {
+  ScanPair p{};
+  p.in[0] = in;
+  p.out[0] = out;
+  p.sums[0] = d_total;
+  return scan_arrays(ctx, p, 1, n);
+}
+
+int scan_exclusive2(tapas_b200_ctx *ctx, const int32_t *const in[2], int32_t *const out[2],
+                    int64_t n, int32_t *const d_total[2], unsigned long long *const d_max[2]) {
+  ScanPair p{};
+  for (int y = 0; y < 2; y++) {
+    p.in[y] = in[y];
+    p.out[y] = out[y];
+    p.sums[y] = d_total[y];
+    p.mx[y] = d_max ? d_max[y] : nullptr;
+  }
+  return scan_arrays(ctx, p, 2, n);
 }
 
 // ---------------------------------------------------------------------------

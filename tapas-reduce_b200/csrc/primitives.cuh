@@ -8,6 +8,12 @@ namespace tb {
 int scan_exclusive(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
                    int32_t *d_total);
 
+// The same for two arrays of n values with one set of launches: half the launches
+// where the scans are short.  d_max (or an entry of it) may be null; else *d_max[y]
+// is raised to array y's largest value.  No output may be another array's input.
+int scan_exclusive2(tapas_b200_ctx *ctx, const int32_t *const in[2], int32_t *const out[2],
+                    int64_t n, int32_t *const d_total[2], unsigned long long *const d_max[2]);
+
 // Exclusive scan of each row of rows[nrows][ncols] in place; totals[row] = its sum.
 int scan_rows(tapas_b200_ctx *ctx, uint32_t *rows, int nrows, int ncols, uint32_t *totals);
 

@@ -344,33 +344,30 @@ constexpr int kSegSortMax = 8192;
 constexpr int kSegWarps = 8;
 constexpr int kLongThreads = 1024;
 
-__global__ void target_counts(const uint64_t *__restrict__ v, int64_t n, int32_t *__restrict__ cnt) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    atomicAdd(cnt + (v[i] >> 32), 1);
-}
-
-// *mx = max over c of off[c + 1] - off[c].
-__global__ void segment_max(const int32_t *__restrict__ off, int64_t ncells,
-                            unsigned long long *__restrict__ mx) {
-  unsigned m = 0;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
-       c += (int64_t)gridDim.x * blockDim.x)
-    m = max(m, (unsigned)(off[c + 1] - off[c]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(mx, (unsigned long long)m);
+// v0[0, n0) into cnt0, v1[0, n1) into cnt1.
+__global__ void target_counts(const uint64_t *__restrict__ v0, int64_t n0,
+                              int32_t *__restrict__ cnt0, const uint64_t *__restrict__ v1,
+                              int64_t n1, int32_t *__restrict__ cnt1) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n0 + n1;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    if (i < n0)
+      atomicAdd(cnt0 + (v0[i] >> 32), 1);
+    else
+      atomicAdd(cnt1 + (v1[i - n0] >> 32), 1);
+  }
 }
 
 // Places each pair's source in its target's segment (order inside it
-// arbitrary).  cur starts as the segment offsets.
+// arbitrary).  cnt starts as the segments' sizes and counts down to 0.
 __global__ void scatter_by_target(const uint64_t *__restrict__ v, int64_t n,
-                                  int32_t *__restrict__ cur, uint32_t *__restrict__ src) {
+                                  const int32_t *__restrict__ off, int32_t *__restrict__ cnt,
+                                  uint32_t *__restrict__ src) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t x = v[i];
-    const int32_t pos = atomicAdd(cur + (x >> 32), 1);
-    src[pos] = (uint32_t)x;
+    const int64_t t = x >> 32;
+    const int32_t o = off[t];
+    src[o + atomicSub(cnt + t, 1) - 1] = (uint32_t)x;
   }
 }
 
@@ -497,7 +494,8 @@ int sort_segment_sources(tapas_b200_ctx *ctx, int w, unsigned long long longest)
   tb::DBuf<uint64_t> &L = w ? ctx->p2p : ctx->m2l;
   const int32_t *off = w ? ctx->p2p_off.p : ctx->m2l_off.p;
   TB_CUDA(ctx, cudaMemsetAsync(ctx->counters.p + 7, 0, sizeof(unsigned long long), s));
-  // the per-target cursors are spent: their buffer holds the long-segment list
+  // list 0's counts are spent (list 1's lie after them): their buffer holds the
+  // long-segment list
   sort_segments<<<grid_for(C, kSegWarps, ctx->num_sms * 8), kSegWarps * 32, 0, s>>>(
       ctx->list_src.p, off, C, b, L.p, ctx->list_cnt.p, ctx->counters.p + 7);
   TB_LAUNCH_CHECK(ctx);
@@ -661,24 +659,26 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
     ctx->list_shift = b;
     TB_CUDA(ctx, ctx->m2l_off.ensure(C + 1, s));
     TB_CUDA(ctx, ctx->p2p_off.ensure(C + 1, s));
-    TB_CUDA(ctx, ctx->list_cnt.ensure(C + 1, s));
+    TB_CUDA(ctx, ctx->list_cnt.ensure(2 * (C + 1), s));
     const int64_t nlist[2] = {ctx->n_m2l, ctx->n_p2p};
     tb::DBuf<uint64_t> *lists[2] = {&ctx->m2l, &ctx->p2p};
     tb::DBuf<int32_t> *offs[2] = {&ctx->m2l_off, &ctx->p2p_off};
-    // 1. per-target counts -> CSR offsets, and the longest segment
-    TB_CUDA(ctx, cudaMemsetAsync(ctx->counters.p + 5, 0, 2 * sizeof(unsigned long long), s));
-    for (int w = 0; w < 2; w++) {
-      TB_CUDA(ctx, cudaMemsetAsync(ctx->list_cnt.p, 0, sizeof(int32_t) * (C + 1), s));
-      if (nlist[w] > 0) {
-        target_counts<<<grid_for(nlist[w], kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
-            lists[w]->p, nlist[w], ctx->list_cnt.p);
-        TB_LAUNCH_CHECK(ctx);
-      }
-      TB_TRY(scan_exclusive(ctx, ctx->list_cnt.p, offs[w]->p, C, offs[w]->p + C));
-      segment_max<<<grid_for(C, kBlock, ctx->num_sms * 8), kBlock, 0, s>>>(offs[w]->p, C,
-                                                                          ctx->counters.p + 5 + w);
+    int32_t *const cnt[2] = {ctx->list_cnt.p, ctx->list_cnt.p + (C + 1)};
+    // 1. per-target counts -> CSR offsets, and the longest segment (counters 5
+    // and 6, zero unless the mutual expansion used them)
+    if (mutual)
+      TB_CUDA(ctx, cudaMemsetAsync(ctx->counters.p + 5, 0, 2 * sizeof(unsigned long long), s));
+    TB_CUDA(ctx, cudaMemsetAsync(cnt[0], 0, sizeof(int32_t) * 2 * (C + 1), s));
+    if (nlist[0] + nlist[1] > 0) {
+      target_counts<<<grid_for(nlist[0] + nlist[1], kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
+          ctx->m2l.p, nlist[0], cnt[0], ctx->p2p.p, nlist[1], cnt[1]);
       TB_LAUNCH_CHECK(ctx);
     }
+    const int32_t *const in[2] = {cnt[0], cnt[1]};
+    int32_t *const out[2] = {offs[0]->p, offs[1]->p};
+    int32_t *const tot[2] = {offs[0]->p + C, offs[1]->p + C};
+    unsigned long long *const longest[2] = {ctx->counters.p + 5, ctx->counters.p + 6};
+    TB_TRY(scan_exclusive2(ctx, in, out, C, tot, longest));
     TB_CUDA(ctx, cudaMemcpyAsync(hc + 5, ctx->counters.p + 5, 2 * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, s));
     TB_CUDA(ctx, cudaStreamSynchronize(s));
@@ -693,10 +693,8 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
       if (n == 0) continue;
       if (hc[5 + w] <= (unsigned long long)kSegSortMax) {
         TB_CUDA(ctx, ctx->list_src.ensure(n + 1, s));
-        TB_CUDA(ctx, cudaMemcpyAsync(ctx->list_cnt.p, offs[w]->p, sizeof(int32_t) * C,
-                                     cudaMemcpyDeviceToDevice, s));
         scatter_by_target<<<grid_for(n, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
-            L.p, n, ctx->list_cnt.p, ctx->list_src.p);
+            L.p, n, offs[w]->p, cnt[w], ctx->list_src.p);
         TB_LAUNCH_CHECK(ctx);
         if (w == 0 && !sort_m2l_sources) {
           // grouped by target only; sort_list_sources() completes the order
