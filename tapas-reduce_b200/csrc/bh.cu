@@ -688,7 +688,7 @@ int bh_interact(tapas_b200_ctx *ctx, double theta, double eps2, int precision) {
   }
   TB_LAUNCH_CHECK(ctx);
   unsigned long long *h = reinterpret_cast<unsigned long long *>(ctx->pinned.p);
-  TB_CUDA(ctx, ctx->pinned.ensure(256));
+  TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
   h = reinterpret_cast<unsigned long long *>(ctx->pinned.p);
   TB_CUDA(ctx, cudaMemcpyAsync(h, ctx->counters.p, 3 * sizeof(unsigned long long),
                                cudaMemcpyDeviceToHost, s));

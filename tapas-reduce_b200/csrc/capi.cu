@@ -187,6 +187,8 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
   ctx->direct_part.release();
   ctx->direct_out.release();
   ctx->pinned.release();
+  if (ctx->p2p_counted) cudaEventDestroy(ctx->p2p_counted);
+  if (ctx->m2l_done) cudaEventDestroy(ctx->m2l_done);
   if (ctx->upload_stream) cudaStreamDestroy(ctx->upload_stream);
   if (ctx->q_ready) cudaEventDestroy(ctx->q_ready);
   if (ctx->upload_fork) cudaEventDestroy(ctx->upload_fork);
@@ -387,7 +389,7 @@ int tapas_b200_set_owned_cells(tapas_b200_ctx *ctx, const uint8_t *mask, int mem
                                                            ctx->leaf_own.p, cnt);
     TB_LAUNCH_CHECK(ctx);
   }
-  TB_CUDA(ctx, ctx->pinned.ensure(256));
+  TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
   int *h = reinterpret_cast<int *>(ctx->pinned.p);
   TB_CUDA(ctx, cudaMemcpyAsync(h, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
   TB_CUDA(ctx, cudaStreamSynchronize(s));
@@ -643,6 +645,12 @@ int tapas_b200_get_lists(tapas_b200_ctx *ctx, int32_t *m2l_tgt, int32_t *m2l_src
   return TAPAS_B200_OK;
 }
 
+static int m2l_launch(tapas_b200_ctx *ctx, int precision) {
+  if (precision == TAPAS_B200_MIXED) return m2l_tensorcore(ctx);
+  TB_TRY(sort_list_sources(ctx, 0));  // the FP64 sums run in source order
+  return m2l_fp64(ctx);
+}
+
 int tapas_b200_m2l(tapas_b200_ctx *ctx, int precision) {
   TB_TRY(check_ctx(ctx));
   TB_TRY(check_precision(ctx, precision));
@@ -651,12 +659,8 @@ int tapas_b200_m2l(tapas_b200_ctx *ctx, int precision) {
     return TAPAS_B200_ERR_STATE;
   }
   PhaseTimer t(ctx, &ctx->timings.m2l);
-  if (precision == TAPAS_B200_MIXED) {
-    TB_TRY(m2l_tensorcore(ctx));
-  } else {
-    TB_TRY(sort_list_sources(ctx, 0));  // the FP64 sums run in source order
-    TB_TRY(m2l_fp64(ctx));
-  }
+  TB_TRY(m2l_launch(ctx, precision));
+  TB_TRY(m2l_status(ctx));
   ctx->have_L = true;
   return TAPAS_B200_OK;
 }
@@ -681,8 +685,25 @@ int tapas_b200_traverse(tapas_b200_ctx *ctx, double theta, int mutual, int preci
   // the mixed form needs the M2L list grouped by target, not each target's
   // sources sorted (it regroups the pairs by offset class)
   TB_TRY(build_lists(ctx, theta, mutual, precision != TAPAS_B200_MIXED));
-  TB_TRY(tapas_b200_m2l(ctx, precision));
-  return tapas_b200_p2p(ctx, precision);
+  if (!ctx->have_M) {
+    set_error(ctx, "m2l: needs upward and build_lists first");
+    return TAPAS_B200_ERR_STATE;
+  }
+  // The P2P item totals are read back while the M2L classes are, and the M2L's
+  // status once the P2P is launched: neither leaves the GPU without work.  1500
+  // bodies, mixed: 548 us, 567 us with each read where it is used.
+  TB_TRY(p2p_begin(ctx, precision));
+  int far;
+  {
+    PhaseTimer t(ctx, &ctx->timings.m2l);
+    far = m2l_launch(ctx, precision);
+  }
+  const int near = far ? far : tapas_b200_p2p(ctx, precision);
+  ctx->p2p_begun = false;  // whatever failed
+  TB_TRY(far);
+  TB_TRY(m2l_status(ctx));
+  ctx->have_L = true;
+  return near;
 }
 
 int tapas_b200_downward(tapas_b200_ctx *ctx, int precision) {

@@ -243,6 +243,7 @@ struct tapas_b200_ctx {
   tb::DBuf<double> p2p_part;            // partial sums of pieces of split leaves
   int64_t p2p_nitems = 0;
   bool p2p_split = false;
+  int64_t p2p_piece_pairs = 0;
   tb::TcState tc;                       // mixed: tensor-core M2L work state
   const uint32_t *m2l_pairs = nullptr;  // FP64 M2L of listed pairs: their list indices
   int64_t m2l_npairs = 0;
@@ -269,6 +270,14 @@ struct tapas_b200_ctx {
   tb::DBuf<double> direct_part, direct_out;
 
   tb::HBuf pinned;
+  // Read-backs a phase starts and a later one picks up: the P2P item totals and
+  // the tensor-core M2L's status, each with an event after its copy.  Their words
+  // of `pinned`, {items, piece rows, -, -, gave up, pairs}, are their own, and no
+  // request is so large that it would move the buffer under a copy.
+  static constexpr size_t kPinnedLater = 2048, kPinnedBytes = 4096;
+  cudaEvent_t p2p_counted = nullptr, m2l_done = nullptr;
+  bool p2p_begun = false, m2l_status_due = false;
+  int *pinned_later() const { return (int *)((char *)pinned.p + kPinnedLater); }
   // upload of the charges on a side stream while the keys are built and sorted
   cudaStream_t upload_stream = nullptr;
   cudaEvent_t q_ready = nullptr, upload_fork = nullptr;

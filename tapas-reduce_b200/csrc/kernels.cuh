@@ -25,7 +25,11 @@ int m2l_fp64_pairs(tapas_b200_ctx *ctx, const uint32_t *pairs, int64_t npairs);
 int downward_fp64(tapas_b200_ctx *ctx);
 // FP64 L2L, then L2P in FP32 added to the near field.
 int downward_fp32_l2p(tapas_b200_ctx *ctx);
-// Near field (p2p.cu).
+// After m2l_tensorcore: waits for it and reports a wait that gave up.
+int m2l_status(tapas_b200_ctx *ctx);
+// Near field (p2p.cu).  p2p_begin, which the others call if nobody has, counts the
+// work items of the current lists and starts the read-back of their totals.
+int p2p_begin(tapas_b200_ctx *ctx, int precision);
 int p2p_fp64(tapas_b200_ctx *ctx);
 int p2p_mixed(tapas_b200_ctx *ctx);
 }  // namespace tb

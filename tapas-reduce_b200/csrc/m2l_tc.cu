@@ -1127,7 +1127,7 @@ int m2l_classes(tapas_b200_ctx *ctx, size_t op_bytes, int64_t min_pairs, M2LClas
   // and the pairs that do not fit); only a first call or a miss runs the
   // separate range pass.
   TB_CUDA(ctx, T.err.ensure(8, s));
-  TB_CUDA(ctx, ctx->pinned.ensure(256));
+  TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
   int32_t *h = reinterpret_cast<int32_t *>(ctx->pinned.p);
   KeyPack kp;
   for (bool fresh = !T.kp_cached;; fresh = true) {
@@ -1301,7 +1301,6 @@ int m2l_tc_P(tapas_b200_ctx *ctx) {
     return TAPAS_B200_OK;
   }
   const int64_t ntc = ci.ntc, nitems = ci.nitems, n64 = ci.n64;
-  int32_t *h = reinterpret_cast<int32_t *>(ctx->pinned.p);
   if (ntc > 0) {
     TB_CUDA(ctx, T.ops.ensure((size_t)2 * S::OPS_FLOATS * ntc, s));
     build_operators<P><<<(unsigned)ntc, 256, 0, s>>>(T.tc_keys.p, T.ops.p);
@@ -1358,15 +1357,13 @@ int m2l_tc_P(tapas_b200_ctx *ctx) {
       C, ctx->cnb.p, ctx->cmin.p, ctx->cmax.p, T.Lt.p, ctx->L.p);
   TB_LAUNCH_CHECK(ctx);
   TB_TRY(m2l_fp64_pairs(ctx, T.pairs64.p, n64));
-  TB_CUDA(ctx, cudaMemcpyAsync(h, T.err.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-  TB_CUDA(ctx, cudaStreamSynchronize(s));
-  ctx->n_m2l_tc = h[1];
-  if (nitems > 0) {
-    if (h[0]) {
-      set_error(ctx, "m2l tensor-core kernel: a bounded wait on an MMA completion gave up");
-      return TAPAS_B200_ERR_TIMEOUT;
-    }
-  }
+  TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
+  if (!ctx->m2l_done)
+    TB_CUDA(ctx, cudaEventCreateWithFlags(&ctx->m2l_done, cudaEventDisableTiming));
+  TB_CUDA(ctx, cudaMemcpyAsync(ctx->pinned_later() + 4, T.err.p,
+                               2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  TB_CUDA(ctx, cudaEventRecord(ctx->m2l_done, s));
+  ctx->m2l_status_due = true;
   return TAPAS_B200_OK;
 }
 
@@ -1655,7 +1652,21 @@ int tc_tree_upward(tapas_b200_ctx *ctx) {
   return fp64_m2m_levels(ctx, 1 << 20);
 }
 
+int m2l_status(tapas_b200_ctx *ctx) {
+  if (!ctx->m2l_status_due) return TAPAS_B200_OK;
+  ctx->m2l_status_due = false;
+  TB_CUDA(ctx, cudaEventSynchronize(ctx->m2l_done));
+  const int *h = ctx->pinned_later() + 4;
+  ctx->n_m2l_tc = h[1];
+  if (h[0]) {
+    set_error(ctx, "m2l tensor-core kernel: a bounded wait on an MMA completion gave up");
+    return TAPAS_B200_ERR_TIMEOUT;
+  }
+  return TAPAS_B200_OK;
+}
+
 int m2l_tensorcore(tapas_b200_ctx *ctx) {
+  ctx->m2l_status_due = false;
   switch (ctx->P) {
     case 4: return m2l_tc_P<4>(ctx);
     case 5: return m2l_tc_P<5>(ctx);

@@ -673,12 +673,13 @@ __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
   }
 }
 
-// Builds the P2P work items of the current lists (ctx->p2p_items) and their
-// queue order (ctx->p2p_order: items by decreasing work).
-int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
+// Pieces of each leaf's list for a grid of warps_per_sm warps, and the read-back
+// of their totals.
+int count_items(tapas_b200_ctx *ctx, int warps_per_sm) {
   cudaStream_t s = ctx->stream;
   const int64_t piece_pairs = std::max<int64_t>(
       kMinPiecePairs, (int64_t)(ctx->n_p2p_int / ((uint64_t)ctx->num_sms * warps_per_sm * 8)));
+  ctx->p2p_piece_pairs = piece_pairs;
   int64_t nl = 0;
   const int32_t *leaves = work_leaves(ctx, nl);  // sharded: owned target leaves
   const uint64_t mask = (1ull << ctx->list_shift) - 1;
@@ -697,11 +698,25 @@ int p2p_items(tapas_b200_ctx *ctx, int warps_per_sm) {
   int32_t *const out[2] = {ctx->p2p_koff.p, ctx->p2p_poff.p};
   int32_t *const tot[2] = {ctx->p2p_counter.p + 1, ctx->p2p_counter.p + 2};
   TB_TRY(scan_exclusive2(ctx, in, out, nl, tot, nullptr));
-  TB_CUDA(ctx, ctx->pinned.ensure(256));
-  int32_t *h = reinterpret_cast<int32_t *>(ctx->pinned.p);
-  TB_CUDA(ctx, cudaMemcpyAsync(h, ctx->p2p_counter.p + 1, 2 * sizeof(int32_t),
+  TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
+  if (!ctx->p2p_counted)
+    TB_CUDA(ctx, cudaEventCreateWithFlags(&ctx->p2p_counted, cudaEventDisableTiming));
+  TB_CUDA(ctx, cudaMemcpyAsync(ctx->pinned_later(), ctx->p2p_counter.p + 1, 2 * sizeof(int32_t),
                                cudaMemcpyDeviceToHost, s));
-  TB_CUDA(ctx, cudaStreamSynchronize(s));
+  TB_CUDA(ctx, cudaEventRecord(ctx->p2p_counted, s));
+  return TAPAS_B200_OK;
+}
+
+// Builds the P2P work items that were counted (ctx->p2p_items) and their queue
+// order (ctx->p2p_order: items by decreasing work).
+int p2p_items(tapas_b200_ctx *ctx) {
+  cudaStream_t s = ctx->stream;
+  int64_t nl = 0;
+  const int32_t *leaves = work_leaves(ctx, nl);
+  const uint64_t mask = (1ull << ctx->list_shift) - 1;
+  const int64_t piece_pairs = ctx->p2p_piece_pairs;
+  TB_CUDA(ctx, cudaEventSynchronize(ctx->p2p_counted));
+  const int32_t *h = ctx->pinned_later();
   const int64_t ni = h[0], npart = h[1];
   if (ni < nl || npart < 0) {
     set_error(ctx, "p2p: work item count overflow");
@@ -764,13 +779,26 @@ static int zero_results_if_sharded(tapas_b200_ctx *ctx) {
   return TAPAS_B200_OK;
 }
 
+int p2p_begin(tapas_b200_ctx *ctx, int precision) {
+  int64_t nl = 0;
+  work_leaves(ctx, nl);
+  ctx->p2p_begun = true;
+  if (nl == 0) return TAPAS_B200_OK;
+  const int rc = count_items(ctx, precision == TAPAS_B200_MIXED ? kMixedBlocks * kMixedWarps
+                                                                : kFp64Blocks * kWarps);
+  ctx->p2p_begun = rc == TAPAS_B200_OK;
+  return rc;
+}
+
 int p2p_fp64(tapas_b200_ctx *ctx) {
   cudaStream_t s = ctx->stream;
   TB_TRY(zero_results_if_sharded(ctx));
   int64_t nl = 0;
   work_leaves(ctx, nl);
+  if (!ctx->p2p_begun) TB_TRY(p2p_begin(ctx, TAPAS_B200_FP64));
+  ctx->p2p_begun = false;
   if (nl == 0) return TAPAS_B200_OK;
-  TB_TRY(p2p_items(ctx, kFp64Blocks * kWarps));
+  TB_TRY(p2p_items(ctx));
   const uint64_t mask = (1ull << ctx->list_shift) - 1;
   p2p_fp64_kernel<<<p2p_grid(ctx, kWarps), kThreads, 0, s>>>(
       ctx->p2p_order.p, ctx->p2p_nitems, ctx->p2p_counter.p,
@@ -783,10 +811,12 @@ int p2p_fp64(tapas_b200_ctx *ctx) {
 int p2p_mixed(tapas_b200_ctx *ctx) {
   cudaStream_t s = ctx->stream;
   TB_TRY(zero_results_if_sharded(ctx));
-  int64_t nw = 0;
-  work_leaves(ctx, nw);
-  if (nw == 0) return TAPAS_B200_OK;
-  TB_TRY(p2p_items(ctx, kMixedBlocks * kMixedWarps));
+  int64_t nl = 0;
+  work_leaves(ctx, nl);
+  if (!ctx->p2p_begun) TB_TRY(p2p_begin(ctx, TAPAS_B200_MIXED));
+  ctx->p2p_begun = false;
+  if (nl == 0) return TAPAS_B200_OK;
+  TB_TRY(p2p_items(ctx));
   const uint64_t mask = (1ull << ctx->list_shift) - 1;
   p2p_mixed_kernel<kMixedBlocks><<<p2p_grid(ctx, kMixedWarps), kMixedThreads, 0, s>>>(
       ctx->p2p_order.p, ctx->p2p_nitems, ctx->p2p_counter.p,

@@ -553,7 +553,8 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
   TB_CUDA(ctx, ctx->trav_geo.ensure(C + 1, s));
   TB_CUDA(ctx, ctx->trav_meta.ensure(C + 1, s));
   TB_CUDA(ctx, ctx->counters.ensure(64, s));
-  TB_CUDA(ctx, ctx->pinned.ensure(512));
+  ctx->p2p_begun = false;  // counted for other lists
+  TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
   // First sizes: a list entry per cell and near or far neighbour of a
   // volume-filling tree for small trees, of a surface for large ones; a list that
   // outgrows its buffer is met below, and the buffers stay for the next call.

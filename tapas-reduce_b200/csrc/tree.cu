@@ -501,7 +501,7 @@ int build_tree(tapas_b200_ctx *ctx, int ncrit) {
     TB_TRY(sort_bodies(kSortLow));
   }
   PhaseTimer t(ctx, &ctx->timings.tree);
-  TB_CUDA(ctx, ctx->pinned.ensure(256));
+  TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
   uint32_t *h_total = reinterpret_cast<uint32_t *>(ctx->pinned.p);
   for (bool complete = false;;) {
     count_nonleaves<<<ntiles, kBlock, 0, s>>>(ctx->keys.p, n, ncrit, ntiles, cnt);
