@@ -407,8 +407,11 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
 }
 
 // A source leaf of the current batch: body i of the batch's stream of source
-// bodies is body b0 + i for the leaf that holds it; far: its box is far enough
-// for plain FP32 coordinates (see above).
+// bodies is body b0 + i for the leaf that holds it; far: 1 its box is far enough
+// for plain FP32 coordinates (see above), 0 its bodies are tested one by one, -1
+// it is the target leaf, whose bodies are near whatever their coordinates: the root
+// box can leave bodies outside (they go to the cells at its faces) and be a point,
+// and a far body is never compared with itself.
 struct __align__(8) LeafMeta {
   int b0, far;
 };
@@ -441,8 +444,8 @@ struct __align__(16) MixedWarp {
 // as splitting the sources over lane groups allows.
 template <int kR>
 __device__ __forceinline__ void mixed_tile(
-    int lane, int tb0, int nt, int L, int G, int e0, int e1, double tcx, double tcy, double tcz,
-    double tw, const uint64_t *__restrict__ list, uint64_t mask, const int32_t *__restrict__ cbeg,
+    int lane, int c, int tb0, int nt, int L, int G, int e0, int e1, double tcx, double tcy,
+    double tcz, double tw, const uint64_t *__restrict__ list, uint64_t mask, const int32_t *__restrict__ cbeg,
     const int32_t *__restrict__ cnb, const double *__restrict__ ccen,
     const double *__restrict__ cmin, const double *__restrict__ cmax,
     const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
@@ -502,7 +505,7 @@ __device__ __forceinline__ void mixed_tile(
       // boxes separated by gap along the farthest axis: every pair is >= gap apart
       const double sw = cmax[3 * s] - cmin[3 * s];
       const double gap = fmax(fabs(dcx), fmax(fabs(dcy), fabs(dcz))) - 0.5 * (tw + sw);
-      m.far = 3.0 * gap >= 0.5 * tw + sw ? 1 : 0;
+      m.far = s == c ? -1 : 3.0 * gap >= 0.5 * tw + sw ? 1 : 0;
     }
     int upto = ns;  // bodies of the batch's leaves 0 .. lane
 #pragma unroll
@@ -547,7 +550,8 @@ __device__ __forceinline__ void mixed_tile(
           hx = (float)dx;
           hy = (float)dy;
           hz = (float)dz;
-          farb = lm.far || fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz))) >= far_body;
+          farb = lm.far > 0 || (lm.far == 0 &&
+                                fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz))) >= far_body);
         }
         const unsigned fm = __ballot_sync(0xffffffffu, farb);
         const unsigned nm = __ballot_sync(0xffffffffu, valid && !farb);
@@ -663,7 +667,7 @@ __global__ void __launch_bounds__(kMixedThreads, kBlocks) p2p_mixed_kernel(
       int R, L, G;
       tile_shape<3, 2>(nt, R, L, G);
 #define TB_MIXED_TILE(RR)                                                                        \
-  mixed_tile<RR>(lane, tb0 + tbase, nt, L, G, e0, e1, tcx, tcy, tcz, tw, list, src_mask, cbeg,  \
+  mixed_tile<RR>(lane, c, tb0 + tbase, nt, L, G, e0, e1, tcx, tcy, tcz, tw, list, src_mask, cbeg,  \
                  cnb, ccen, cmin, cmax, sx, sy, sz, sq, sm[wi], out + tbase)
       if (R == 3) TB_MIXED_TILE(3);
       else if (R == 2) TB_MIXED_TILE(2);

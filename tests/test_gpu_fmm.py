@@ -655,3 +655,25 @@ def test_tree_bodies_close_in_one_cell(n, longest, tb, ctx, oracle_mod):
         if m > 1:
             x[idx[1]], y[idx[1]], z[idx[1]] = x[idx[0]], y[idx[0]], z[idx[0]]
     _check_tree(tb, ctx, oracle_mod, x, y, z, q, 4)
+
+
+@pytest.mark.parametrize("n", [1, 700, 30000])
+def test_near_field_counts_belong_to_their_call(n, tb, ctx):
+    """traverse() counts the near field's work ahead of the M2L; a p2p() call after
+    it, at the other precision or after new lists, counts its own: bit for bit the
+    result of a p2p() with nothing before it."""
+    b = tb.datasets.make("two_gaussians", n, 61)
+
+    def alone(theta, precision, before):
+        ctx.partition(*b, ncrit=16)
+        ctx.upward(4, tb.MIXED)
+        if before:
+            ctx.traverse(0.5, precision=tb.MIXED)
+        if theta is not None:
+            ctx.build_lists(theta)
+        ctx.p2p(precision)
+        return ctx.results()
+
+    for precision in (tb.FP64, tb.MIXED):
+        assert np.array_equal(alone(0.5, precision, False), alone(None, precision, True))
+        assert np.array_equal(alone(0.8, precision, False), alone(0.8, precision, True))
