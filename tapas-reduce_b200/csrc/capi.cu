@@ -811,7 +811,7 @@ int tapas_b200_direct(tapas_b200_ctx *ctx, const int64_t *targets, int64_t k, do
     dt = ctx->direct_tg.p;
     dout = ctx->direct_out.p;
   }
-  // about eight waves of blocks, at least 16 sources per thread
+  // about twelve waves of blocks, at least 16 sources per thread
   const int64_t nb = (k + kDirectTargets - 1) / kDirectTargets;
   const int64_t waves = ((int64_t)ctx->num_sms * 24 + nb - 1) / nb;
   const int nsplit = (int)std::max<int64_t>(

@@ -15,9 +15,12 @@ constexpr int kDirectTargets = 8;  // targets per block
 // order.  A target index outside [0, n) gives NaN.
 //
 // Bound: the FP64 pipe, 18 slots per pair with charge_over_distance: 4000 targets x
-// 1M bodies 5.4 ms, 71 % of that pipe.  A block per
-// target with 1.0 / sqrt(r2) took 13.6 ms.
-static __global__ void __launch_bounds__(kDirectThreads, 3) direct_tiles(
+// 1M bodies 5.06 ms, 76 % of that pipe.  All eight separations are in flight
+// at once, which takes 240 registers, so two blocks per SM: 5.44 ms with four and
+// three blocks (5.38 against 5.50 ms a call with the bodies out of L2), 5.00 with T = 7
+// or 10, 5.15 with sources loaded two steps ahead.  A
+// block per target with 1.0 / sqrt(r2) took 13.6 ms.
+static __global__ void __launch_bounds__(kDirectThreads, 2) direct_tiles(
     const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
     const double *__restrict__ q, int64_t n, const int64_t *__restrict__ targets, int64_t k,
     int nsplit, double *__restrict__ part) {
@@ -41,7 +44,7 @@ static __global__ void __launch_bounds__(kDirectThreads, 3) direct_tiles(
     const double4 b = next;
     if (j + step < n)
       next = make_double4(x[j + step], y[j + step], z[j + step], q[j + step]);
-    constexpr int G = 4;  // separations in flight
+    constexpr int G = T;  // separations in flight
 #pragma unroll
     for (int r0 = 0; r0 < T; r0 += G) {
       double dx[G], dy[G], dz[G], R2[G], qj[G], qr[G], inv[G];
