@@ -730,7 +730,7 @@ def config_bh_4m(tb, orc, ctx, torch, stream):
         res[name] = {"ms": ms, "interactions_per_s": (na + nd) / (ms * 1e-3),
                      "approx": na, "direct": nd,
                      "tree_build_ms": build_ms,
-                     "tree_build_gbs": 316.0 * n / (build_ms * 1e-3) / 1e9,
+                     "tree_build_gbs": 244.0 * n / (build_ms * 1e-3) / 1e9,
                      "rel_l2_force_vs_direct": _rel(r[tg, :3], d[:, :3]),
                      "rel_l2_pot_vs_direct": _rel(r[tg, 3], d[:, 3])}
     return res

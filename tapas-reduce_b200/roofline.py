@@ -7,7 +7,7 @@ Algorithmic work per unit (the figures `achieved` is computed from):
 * M2L   : 8 * sum_{j<P} (j+1)(P-j)^2 flop per translation (the reference's
           complex multiply-add count in LaplaceSphericalCPU_tapas.h:227-270);
           FP64 pipe (plain) or tensor pipe (mixed, split TF32).
-* sort  : 8 LSD passes x (read + write of u64 key + u32 index) = 192 B/body;
+* sort  : 5 LSD passes x (read + write of u64 key + u32 index) = 120 B/body;
           keys: 32 B read + 12 B written per body; HBM bound.
 Peaks: HBM from MEASURED_PEAKS.json; FP32/FP64 CUDA-core peaks are nominal
 (148 SMs x 128 FP32 / 64 FP64 FMA per clock x 2 x max SM clock), no measured
@@ -17,12 +17,13 @@ from __future__ import annotations
 
 
 # DRAM bytes of one p2p_mixed_kernel launch per body, from one ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum = 40.6 MB + 8.8 MB on a 1M-body
-# unit-sphere-surface set, P=15, theta=0.4, ncrit=128).  The kernel's DRAM
+# (dram__bytes_read.sum + dram__bytes_write.sum = 46.2 MB + 44.6 MB on a 1M-body
+# unit-sphere-surface set, P=12, theta=0.35, ncrit=128).  The kernel's DRAM
 # traffic is its body arrays read and results written (its source re-reads hit
 # L2), so a launch's traffic is this figure times the bodies.
-P2P_MIXED_DRAM_BYTES_PER_BODY = 49.4
-# Same capture, m2l_tc_kernel<15>: 540.5 MB + 45.8 MB for 1.04M translations
+P2P_MIXED_DRAM_BYTES_PER_BODY = 90.8
+# From one capture of the same set at P=15, theta=0.4, m2l_tc_kernel<15>: 540.5 MB +
+# 45.8 MB for 1.04M translations
 # (the operator and multipole rows grow with P).
 M2L_TC_DRAM_BYTES_PER_TRANSLATION = 565.0
 
@@ -89,7 +90,7 @@ def dominant(phases: dict, lists: dict, tree: dict, P: int, peaks: dict, peak_sr
                    peak_source=f"nominal fp64 at {smx:.0f} MHz", traffic=None,
                    work=f"{lists['n_m2l']} translations x {m2l_flops_per_translation(P)} flop")
     else:
-        per = {"sort": 192.0, "bbox_keys": 44.0 + 48.0, "tree": 16.0}.get(name)
+        per = {"sort": 120.0, "bbox_keys": 44.0 + 48.0, "tree": 16.0}.get(name)
         if per is None:
             out.update(bound="latency", note="no algorithmic byte/flop model for this phase")
             return out
