@@ -83,32 +83,42 @@ struct BhCells {
 // (bh.cc:148-149), from the hardware's approximation: refined to about an ulp
 // (the series of charge_over_distance), then one residual step each for the square
 // root and the reciprocal (Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", 1990): the residuals are exact in an
-// fma, so the results differ from the rounded exact ones only where those lie
-// within ~2^-104 of a rounding boundary.  12 FP64 operations where the two
-// library sequences take about 57 slots of the FP64 pipe.
+// the IBM RISC System/6000 processor", 1990).  The residuals are exact in an fma, so
+// before its rounding the root is off by less than 2^-103, relative, and the
+// reciprocal (its step taken to second order, e + e^2: y is up to an ulp off 1/s) by at
+// most 2^-106.  The arguments whose root lies that close to the middle of two
+// numbers, M^2 = r2 + j for odd 54-bit M and |j| <= 64, all come out rounded
+// right whatever the approximation's error (below 2^-20; enumerated); the one
+// reciprocal within 2^-106 of a middle that does not is that of an s with all
+// mantissa bits set (r2 just below a power of four: one step of a lattice of
+// spacing 1), which is tested for.  13 FP64 operations where the two library
+// sequences take about 57 slots of the FP64 pipe.
 // kN at once, with one branch for all: a branch each would keep their chains
 // from overlapping.
 template <int kN>
 __device__ __forceinline__ void rounded_inv_sqrt(const double (&r2)[kN], double (&inv)[kN]) {
+  // outside 2^-767 .. 2^768 the residuals could underflow
+  auto library = [](double r2, double s) {
+    return (unsigned)__double2hiint(r2) - 0x10000000u >= 0x60000000u || __double2loint(s) == -1;
+  };
+  double s[kN];
   bool odd = false;
 #pragma unroll
   for (int i = 0; i < kN; i++) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2[i]));
-    const double e = fma(-(r2[i] * y), y, 1.0);
+    double e = fma(-(r2[i] * y), y, 1.0);
     y = fma(y, e * fma(e, 0.375, 0.5), y);
     const double g = r2[i] * y;
-    const double s = fma(fma(-g, g, r2[i]), 0.5 * y, g);
-    inv[i] = fma(y, fma(-s, y, 1.0), y);
-    // outside 2^-767 .. 2^768 the residuals could underflow
-    odd |= (unsigned)__double2hiint(r2[i]) - 0x10000000u >= 0x60000000u;
+    s[i] = fma(fma(-g, g, r2[i]), 0.5 * y, g);
+    e = fma(-s[i], y, 1.0);
+    inv[i] = fma(y, fma(e, e, e), y);
+    odd |= library(r2[i], s[i]);
   }
   if (odd) {
 #pragma unroll
     for (int i = 0; i < kN; i++)
-      if ((unsigned)__double2hiint(r2[i]) - 0x10000000u >= 0x60000000u)
-        inv[i] = __ddiv_rn(1.0, __dsqrt_rn(r2[i]));
+      if (library(r2[i], s[i])) inv[i] = __ddiv_rn(1.0, __dsqrt_rn(r2[i]));
   }
 }
 

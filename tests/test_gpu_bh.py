@@ -105,3 +105,18 @@ def test_bh_massless_cells(tb, ctx, oracle_mod):
     np.testing.assert_array_equal(r, ref)
     r32 = ctx.bh_evaluate(x, y, z, m, ncrit=4, theta=0.3, eps2=1e-6, precision=tb.MIXED)
     assert np.array_equal(np.isnan(r32), np.isnan(r))
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -3, 1.0, 2.0 ** 5])
+@pytest.mark.parametrize("dx,eps2", [(1 - 2.0 ** -53, 2.0 ** -53), (1 - 2.0 ** -53, 1e-40),
+                                     (2 - 2.0 ** -52, 2.0 ** -51), (1.0, 3 * 2.0 ** -52)])
+def test_bh_fp64_distance_at_rounding_edge(dx, eps2, scale, tb, ctx, oracle_mod):
+    """Squared distances next to a power of four, where the rounded square root has
+    all mantissa bits set (or its exact value lies next to the middle of two numbers)
+    and the reciprocal next to a middle: bit for bit the sample's."""
+    x = np.array([0.0, dx * scale])
+    zero, m = np.zeros(2), np.array([1.0, 3.0])
+    args = dict(ncrit=1, theta=0.5, eps2=eps2 * scale * scale)
+    r = ctx.bh_evaluate(x, zero, zero, m, precision=tb.FP64, **args)
+    ref, _ = oracle_mod.barnes_hut(x, zero, zero, m, **args)
+    np.testing.assert_array_equal(r, ref)
