@@ -454,8 +454,8 @@ __device__ __forceinline__ float inv_sqrt32(float x) {
 // slots at a time are loaded by a lane each, whatever entry they belong to, into
 // shared memory with the lanes that add each half, then evaluated by all lanes.
 // Leaf bodies are stored as pairs {x0,x1,y0,y1},{z0,z1,m0,m1}, each leaf starting
-// a pair (an odd leaf's last one is padded with a massless copy of its first
-// body).  A slot's terms are evaluated by packed FP32 instructions, then added one
+// a pair (an odd leaf's last one is padded with a copy of its first body that no
+// lane adds).  A slot's terms are evaluated by packed FP32 instructions, then added one
 // after the other: an FP32 sum of 10^4 terms of one sign is rounded by 3e-5
 // somewhere, and only the walk's own order rounds it where this form always has.
 // Bound: issue slots and FP32 pipe; the union holds 1.37 times the bodies' own leaf
@@ -513,6 +513,7 @@ __global__ void __launch_bounds__(32, 32) bh_walk32(
       const int i = c0 + lane, k = lane_above(upto, i);
       const int p = __shfl_sync(0xffffffffu, r.x, k);
       const int p0 = __shfl_sync(0xffffffffu, upto - slots, k);
+      const int nb = __shfl_sync(0xffffffffu, r.y, k);
       const unsigned m0 = __shfl_sync(0xffffffffu, rm, k);
       const int pn = __shfl_sync(0xffffffffu, r.x, (k + 1) & 31);
       const unsigned mn = __shfl_sync(0xffffffffu, rm, (k + 1) & 31);
@@ -521,7 +522,8 @@ __global__ void __launch_bounds__(32, 32) bh_walk32(
           const float4 *src = pairs + 2 * ((int64_t)p + (i - p0));
           slot_a[lane] = __ldg(src);
           slot_b[lane] = __ldg(src + 1);
-          slot_lanes[lane] = make_uint2(m0, m0);
+          // no lane adds an odd leaf's padding: with eps2 = 0 its term is 0 * inf
+          slot_lanes[lane] = make_uint2(m0, 2 * (i - p0) + 1 < nb ? m0 : 0u);
         } else {
           const bool two = k < 31 && (cells >> (k + 1) & 1);
           const float4 u = __ldg(attr32 + ~p);
@@ -621,11 +623,10 @@ __global__ void __launch_bounds__(256) bh_pack(
     if (!pair_off || !is_leaf) continue;
     for (int k = sub; k < (nb + 1) >> 1; k += 8) {
       const int i = b0 + 2 * k;
-      const bool two = 2 * k + 1 < nb;
-      const int j = two ? i + 1 : b0;
+      const int j = 2 * k + 1 < nb ? i + 1 : b0;
       float4 *o = pairs + 2 * ((int64_t)pair_off[c] + k);
       o[0] = make_float4((float)sx[i], (float)sx[j], (float)sy[i], (float)sy[j]);
-      o[1] = make_float4((float)sz[i], (float)sz[j], (float)sm[i], two ? (float)sm[j] : 0.f);
+      o[1] = make_float4((float)sz[i], (float)sz[j], (float)sm[i], (float)sm[j]);
     }
   }
 }

@@ -120,3 +120,13 @@ def test_bh_fp64_distance_at_rounding_edge(dx, eps2, scale, tb, ctx, oracle_mod)
     r = ctx.bh_evaluate(x, zero, zero, m, precision=tb.FP64, **args)
     ref, _ = oracle_mod.barnes_hut(x, zero, zero, m, **args)
     np.testing.assert_array_equal(r, ref)
+
+
+@pytest.mark.parametrize("ncrit", [1, 4])
+def test_bh_fp32_unsoftened_potential_is_infinite(ncrit, tb, ctx):
+    """eps2 = 0: every body meets itself at distance zero, so its potential is
+    infinite (and no NaN) in either precision, whether its leaf is odd or even."""
+    x, y, z, m = tb.datasets.make("uniform_cube", 500, 84)
+    for precision in (tb.FP64, tb.MIXED):
+        r = ctx.bh_evaluate(x, y, z, m, ncrit=ncrit, theta=0.5, eps2=0.0, precision=precision)
+        assert np.all(r[:, 3] == np.inf), precision
