@@ -306,7 +306,9 @@ __global__ void __launch_bounds__(32 * kGemmWarps, 3) product_tiles64(
 }
 
 // The products of the pairs without an operator, one warp per pair, scaled
-// into the rows' units (w_t^(j+1)).
+// into the rows' units (w_t^(j+1)).  The translation is done in units of the power of
+// two below w_t, which changes no bit of it and leaves only powers of 1 <= f < 2 to
+// multiply by: w_t^16 itself overflows for cells wider than 2^64.
 template <int P>
 __global__ void __launch_bounds__(128) product_pairs64(
     const uint32_t *__restrict__ pairs, int64_t npairs, int64_t base, int64_t count,
@@ -330,26 +332,32 @@ __global__ void __launch_bounds__(128) product_pairs64(
     const uint64_t x = list[e + base];
     const int c = (int)(x >> shift), s = (int)(x & src_mask);
     if (cnb[s] == 0 || cnb[c] == 0) continue;  // not summed either
-    const Sph sp = sph_of(ccen[3 * c] - ccen[3 * s], ccen[3 * c + 1] - ccen[3 * s + 1],
-                          ccen[3 * c + 2] - ccen[3 * s + 2]);
+    const double w = cmax[3 * c] - cmin[3 * c];
+    const int ex = ilogb(w);
+    const double f = scalbn(w, -ex);
+    const Sph sp = sph_of(scalbn(ccen[3 * c] - ccen[3 * s], -ex),
+                          scalbn(ccen[3 * c + 1] - ccen[3 * s + 1], -ex),
+                          scalbn(ccen[3 * c + 2] - ccen[3 * s + 2], -ex));
     __syncwarp();
     if (lane < P) local_column<P>(lane, sp.r, sp.x, sp.y, sp.ei, Y);
-    for (int t = lane; t < S::NT; t += 32) {
+#pragma unroll
+    for (int r = 0; r < S::R; r++) {
+      const int t = lane + 32 * r;
+      if (t >= S::NT) continue;
       const double2 v = M[(int64_t)s * S::NT + t];
-      Mj[t] = cd{v.x, v.y};
+      Mj[t] = cd{scalbn(v.x, -ex * jj[r]), scalbn(v.y, -ex * jj[r])};
     }
     __syncwarp();
     cd acc[S::R];
 #pragma unroll
     for (int r = 0; r < S::R; r++) acc[r] = cd{0, 0};
     m2l_accumulate<P>(acc, jj, kk, lane, Mj, Y);
-    const double w = cmax[3 * c] - cmin[3 * c];
 #pragma unroll
     for (int r = 0; r < S::R; r++) {
       const int t = lane + 32 * r;
       if (t >= S::NT) continue;
-      double sc = w;
-      for (int k = 0; k < jj[r]; k++) sc *= w;
+      double sc = f;
+      for (int k = 0; k < jj[r]; k++) sc *= f;
       rows[e * S::NT + t] = make_double2(acc[r].x * sc, acc[r].y * sc);
     }
   }

@@ -677,3 +677,18 @@ def test_near_field_counts_belong_to_their_call(n, tb, ctx):
     for precision in (tb.FP64, tb.MIXED):
         assert np.array_equal(alone(0.5, precision, False), alone(None, precision, True))
         assert np.array_equal(alone(0.8, precision, False), alone(0.8, precision, True))
+
+
+@pytest.mark.parametrize("P,exponent", [(16, 66), (16, 40), (10, 101), (10, -95)])
+def test_fp64_evaluation_in_other_units(P, exponent, tb, ctx):
+    """Bodies in units so small or large that the powers of a cell's width leave the
+    FP64 range (cells of 2^64 and more at P = 16, as a galaxy's in metres): scaled by a
+    power of two the evaluation is the same up to the local coefficients that
+    become subnormal; those of degree 15 carry ~1e-6 of the field and keep 18 bits."""
+    x, y, z, q = tb.datasets.make("uniform_cube", 3000, 12)
+    args = dict(P=P, ncrit=16, theta=0.4, precision=tb.FP64)
+    a = ctx.evaluate(x, y, z, q, **args)
+    s = 2.0 ** exponent
+    b = ctx.evaluate(x * s, y * s, z * s, q, **args) * np.array([s, s * s, s * s, s * s])
+    assert np.isfinite(b).all()
+    assert _rel(b[:, 0], a[:, 0]) < 1e-8 and _rel(b[:, 1:], a[:, 1:]) < 1e-8
