@@ -1390,25 +1390,18 @@ constexpr int kFp64TreeLevels = 4;
 constexpr int kTcUpLevels = 3;
 constexpr int kTreeShift = 32;  // tree pair list entries: target << 32 | source
 
-// M2M operator classes o (octant o), in FP32 in the dense GEMM's layout.  child0: the first child of any non-leaf cell; the offsets
-// are its octants' centre offsets in child widths (exact: +-1/2).
+// M2M operator classes o (octant o), in FP32 in the dense GEMM's layout.  They belong to
+// no tree: the offsets are the octants' centre offsets in child widths.
 template <int P>
-__global__ void __launch_bounds__(256) build_tree_ops(const int32_t *__restrict__ cparent,
-                                                      const double *__restrict__ ccen,
-                                                      const double *__restrict__ cmin,
-                                                      const double *__restrict__ cmax,
-                                                      int64_t child0, float *__restrict__ ops) {
+__global__ void __launch_bounds__(256) build_tree_ops(float *__restrict__ ops) {
   using S = TcShape<P, true>;
   __shared__ cd Y[P * P];
   __shared__ unsigned char deg[S::NT], ord[S::NT];
   __shared__ int nr[S::NKC], co[S::NKC + 1];
   if (threadIdx.x == 0) chunk_tables<S>(nr, co);
   const int o = blockIdx.x;
-  const int64_t c = child0 + o;
-  const int p = cparent[c];
-  const double wc = cmax[3 * c] - cmin[3 * c];
   double d[3];
-  for (int k = 0; k < 3; k++) d[k] = (ccen[3 * p + k] - ccen[3 * c + k]) / wc;  // parent - child
+  for (int k = 0; k < 3; k++) d[k] = (o >> k & 1) ? -0.5 : 0.5;  // parent - child
   const Sph sp = sph_of(d[0], d[1], d[2]);
   if (threadIdx.x < P) multipole_column<P>(threadIdx.x, sp.r, sp.x, sp.y, sp.ei, Y);
   for (int t = threadIdx.x; t < S::NT; t += blockDim.x) {
@@ -1553,7 +1546,7 @@ int tree_parent_levels(const tapas_b200_ctx *ctx) {
 int first_tc_tree_level(int nlev) { return std::max(kFp64TreeLevels, nlev - kTcUpLevels); }
 
 // Pair lists, operators and the abort flag of the tree GEMMs; only for trees
-// with parent levels from kFp64TreeLevels on (level 1 exists).
+// with parent levels from kFp64TreeLevels on.
 template <int P>
 int tc_tree_prepare(tapas_b200_ctx *ctx) {
   using S = TcShape<P>;
@@ -1569,8 +1562,7 @@ int tc_tree_prepare(tapas_b200_ctx *ctx) {
   }
   if (T.tr_P != P) {
     TB_CUDA(ctx, T.ops_tr.ensure((size_t)2 * TcShape<P, true>::OPS_FLOATS * 8, s));
-    build_tree_ops<P><<<8, 256, 0, s>>>(ctx->cparent.p, ctx->ccen.p, ctx->cmin.p, ctx->cmax.p,
-                                        ctx->level_off[1], T.ops_tr.p);
+    build_tree_ops<P><<<8, 256, 0, s>>>(T.ops_tr.p);
     TB_LAUNCH_CHECK(ctx);
     T.tr_P = P;
   }

@@ -692,3 +692,20 @@ def test_fp64_evaluation_in_other_units(P, exponent, tb, ctx):
     b = ctx.evaluate(x * s, y * s, z * s, q, **args) * np.array([s, s * s, s * s, s * s])
     assert np.isfinite(b).all()
     assert _rel(b[:, 0], a[:, 0]) < 1e-8 and _rel(b[:, 1:], a[:, 1:]) < 1e-8
+
+
+def test_mixed_evaluation_after_a_zero_width_tree(tb):
+    """Bodies all at one point make a deep tree of zero-width cells; what a context
+    keeps from it (the M2M operators belong to an order, not to a tree) leaves the
+    next evaluation as in a context of its own."""
+    b = tb.datasets.make("plummer", 30000, 3)
+    point, ones = np.full(60, 0.25), np.ones(60)
+    args = dict(P=8, ncrit=8, theta=0.4, precision=tb.MIXED)
+    with tb.Context(0) as c:
+        ref = c.evaluate(*b, **args)
+    with tb.Context(0) as c:
+        c.evaluate(point, point, point, ones, **args)
+        got = c.evaluate(*b, **args)
+    assert np.isfinite(got).all()
+    # the mixed form's FP32 reductions are added in no fixed order
+    assert np.linalg.norm(got - ref, axis=0).max() <= 1e-6 * np.linalg.norm(ref, axis=0).max()
