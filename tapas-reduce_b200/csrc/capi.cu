@@ -590,6 +590,7 @@ int tapas_b200_set_multipoles(tapas_b200_ctx *ctx, const double *M, int mem) {
                                mem == TAPAS_B200_DEVICE ? cudaMemcpyDeviceToDevice
                                                         : cudaMemcpyHostToDevice,
                                ctx->stream));
+  ctx->tc.mt_ready = false;  // the mixed M2L's rows are those of the multipoles before
   TB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return TAPAS_B200_OK;
 }

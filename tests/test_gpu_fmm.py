@@ -709,3 +709,23 @@ def test_mixed_evaluation_after_a_zero_width_tree(tb):
     assert np.isfinite(got).all()
     # the mixed form's FP32 reductions are added in no fixed order
     assert np.linalg.norm(got - ref, axis=0).max() <= 1e-6 * np.linalg.norm(ref, axis=0).max()
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+def test_set_multipoles_after_upward(precision, tb, ctx):
+    """Multipoles given after a whole upward pass are the ones the M2L translates:
+    doubled, the local expansions double (exactly, but for the mixed form's FP32
+    reductions in no fixed order)."""
+    x, y, z, q = tb.datasets.make("uniform_cube", 20000, 3)
+    ctx.partition(x, y, z, q, ncrit=64)
+    ctx.upward(8, precision)
+    ctx.build_lists(0.4)
+    M = ctx.multipoles()
+    ctx.m2l(precision)
+    L1 = ctx.expansions()[1]
+    ctx.set_multipoles(np.stack([2 * M.real, 2 * M.imag], axis=-1))
+    ctx.m2l(precision)
+    L2 = ctx.expansions()[1]
+    ne = ctx.cells()["nb"] > 0
+    tol = 0.0 if precision == tb.FP64 else 1e-6
+    assert np.linalg.norm(L2[ne] - 2 * L1[ne]) <= tol * np.linalg.norm(L2[ne])
