@@ -842,6 +842,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
                              ? (nitems - 1 - (int64_t)blockIdx.x) / gridDim.x + 1
                              : 0;
   const int64_t nsteps = ntiles * S::NKC;
+  int64_t issued = 0;  // steps whose operator rows warp 25 has started to copy
   auto item_of = [&](int64_t jt) { return items[(int64_t)blockIdx.x + jt * gridDim.x]; };
 
   if (warp < kEpiWarp0) {
@@ -920,7 +921,6 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
     // ---------------- operator copies ----------------
     // per step the operator rows the chunk reaches, TF32 hi and lo; the warp
     // walks the steps together (uniform operands), one lane issues
-    int64_t issued = 0;
     int cls = 0, nxt_cls = ntiles > 0 ? item_of(0).cls : 0;
     for (int64_t step = 0; step < nsteps; step++) {
       const int st = (int)(step % NS);
@@ -943,15 +943,6 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
       }
       __syncwarp();
       issued = step + 1;
-    }
-    if (lane == 0 && *abort) {
-      // bulk copies of steps that may not have been consumed: let them land
-      for (int64_t s = issued > NS ? issued - NS : 0; s < issued; s++) {
-        const long long t0 = clock64();
-        while (!mbar_try_wait(&landed[s % NS], (uint32_t)((s / NS) & 1)) &&
-               clock64() - t0 < 200000000LL) {
-        }
-      }
     }
   } else if (warp == kMmaWarp) {
     // ---------------- MMA issue ----------------
@@ -1094,6 +1085,18 @@ __global__ void __launch_bounds__(kThreadsTc, 1) m2l_tc_kernel(
   }
   __syncthreads();
   if (tid == 0 && abort_sh) atomicExch(err, 1);
+  if (warp == kBulkWarp && lane == 0 && abort_sh) {
+    // no role will raise the abort flag from here on: bulk copies of steps that may not
+    // have been consumed land before the CTA gives up its shared memory (a stage whose
+    // rows' producers have left never completes its phase; its copies take far less
+    // than the wait)
+    for (int64_t s = issued > NS ? issued - NS : 0; s < issued; s++) {
+      const long long t0 = clock64();
+      while (!mbar_try_wait(&landed[s % NS], (uint32_t)((s / NS) & 1)) &&
+             clock64() - t0 < 200000000LL) {
+      }
+    }
+  }
   if (warp == kMmaWarp) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),

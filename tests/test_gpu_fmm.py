@@ -729,3 +729,32 @@ def test_set_multipoles_after_upward(precision, tb, ctx):
     ne = ctx.cells()["nb"] > 0
     tol = 0.0 if precision == tb.FP64 else 1e-6
     assert np.linalg.norm(L2[ne] - 2 * L1[ne]) <= tol * np.linalg.norm(L2[ne])
+
+
+@pytest.mark.parametrize("limit", [1, 1000, 3000])
+@pytest.mark.parametrize("P", [4, 16])
+def test_tensorcore_m2l_wait_timeout_with_copies_in_flight(P, limit, tb, ctx):
+    """Wait bounds around the time a copy takes, on lists of at most a tile or two per
+    CTA: the copying warp may have left its loop before another role gives up, and
+    its copies still have to land before the CTA ends.  Either the call reports the
+    timeout or it succeeds, and the next call with the default bound is right."""
+    x, y, z, q = tb.datasets.make("uniform_cube", 6000, 62)
+    ctx.partition(x, y, z, q, ncrit=32)
+    ctx.upward(P, tb.FP64)
+    ctx.build_lists(0.5)
+    ctx.m2l(tb.FP64)
+    _, L64 = ctx.expansions()
+    try:
+        ctx.set_wait_limit(limit)
+        for _ in range(3):
+            try:
+                ctx.m2l(tb.MIXED)
+            except tb.TapasError as e:
+                assert e.code == tb._lib.ERR_TIMEOUT
+    finally:
+        ctx.set_wait_limit(0)
+    ctx.m2l(tb.MIXED)
+    _, Lmx = ctx.expansions()
+    ne = (ctx.cells()["nb"] > 0) & (np.linalg.norm(L64, axis=1) > 0)
+    rel = np.linalg.norm(Lmx[ne] - L64[ne], axis=1) / np.linalg.norm(L64[ne], axis=1)
+    assert rel.max() < 2e-5
