@@ -318,12 +318,14 @@ inline cudaError_t check_launch() { return cudaGetLastError(); }
     }                                                                                \
   } while (0)
 
-// Phase timer: CUDA events on the context stream, only when profiling.
+// Phase timer: CUDA events on the context stream, only when profiling.  add: one part of
+// a phase of several.
 struct PhaseTimer {
   tapas_b200_ctx *ctx;
   double *slot;
+  bool add;
   cudaEvent_t a = nullptr, b = nullptr;
-  PhaseTimer(tapas_b200_ctx *c, double *s) : ctx(c), slot(s) {
+  PhaseTimer(tapas_b200_ctx *c, double *s, bool add = false) : ctx(c), slot(s), add(add) {
     if (ctx->profiling) {
       cudaEventCreate(&a);
       cudaEventCreate(&b);
@@ -336,7 +338,7 @@ struct PhaseTimer {
       cudaEventSynchronize(b);
       float ms = 0;
       cudaEventElapsedTime(&ms, a, b);
-      *slot = ms;
+      *slot = add ? *slot + ms : ms;
       cudaEventDestroy(a);
       cudaEventDestroy(b);
     }

@@ -503,12 +503,12 @@ __global__ void __launch_bounds__(kSortThreads) radix_block(
 
 // Completes the order of elements sorted on the bits from low_bits up: the run of
 // elements that agree there is put in order of all its bits by the thread of its
-// first element (stable insertion); *longest becomes at least the length of
-// any run too long for that, which is left as it is.
+// first element (stable insertion), or, longer than max_run, left as it is and listed.
 __global__ void __launch_bounds__(256) order_runs(uint64_t *__restrict__ keys,
                                                   uint32_t *__restrict__ vals, int64_t n,
                                                   int low_bits, int max_run,
-                                                  int *__restrict__ longest) {
+                                                  int2 *__restrict__ long_runs,
+                                                  unsigned long long *__restrict__ long_tally) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i + 1 < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     // only high bits are compared: a thread of another run may be reordering the
@@ -518,7 +518,19 @@ __global__ void __launch_bounds__(256) order_runs(uint64_t *__restrict__ keys,
     int64_t e = i + 2;
     while (e < n && e - i <= max_run && keys[e] >> low_bits == h) e++;
     if (e - i > max_run) {
-      atomicMax(longest, (int)(e - i));
+      int64_t hi = e;  // the run's end: e .. hi doubling, then halving
+      for (int64_t step = max_run; hi < n && keys[hi] >> low_bits == h; step *= 2) {
+        e = hi + 1;
+        hi += step;
+      }
+      hi = min(hi, n);
+      while (e < hi) {
+        const int64_t m = e + ((hi - e) >> 1);
+        if (keys[m] >> low_bits == h) e = m + 1; else hi = m;
+      }
+      const unsigned long long at =
+          atomicAdd(long_tally, (1ull << 32) + (unsigned long long)(e - i));
+      long_runs[at >> 32] = make_int2((int)i, (int)(at & 0xFFFFFFFFull));
       continue;
     }
     for (int64_t a = i + 1; a < e; a++) {
@@ -535,6 +547,51 @@ __global__ void __launch_bounds__(256) order_runs(uint64_t *__restrict__ keys,
   }
 }
 
+// The run that element i of the listed runs, one after another, belongs to.
+__device__ __forceinline__ int run_of(const int2 *__restrict__ runs, int nruns, int64_t i) {
+  int lo = 0, hi = nruns - 1;
+  while (lo < hi) {
+    const int m = (lo + hi + 1) >> 1;
+    if (runs[m].y <= i) lo = m; else hi = m - 1;
+  }
+  return lo;
+}
+
+// The listed runs' elements one run after another: keys {run, low bits} and values.
+__global__ void __launch_bounds__(256) collect_runs(const uint64_t *__restrict__ keys,
+                                                    const uint32_t *__restrict__ vals,
+                                                    const int2 *__restrict__ runs, int nruns,
+                                                    int64_t total, int low_bits,
+                                                    uint64_t *__restrict__ rkeys,
+                                                    uint32_t *__restrict__ rvals) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int r = run_of(runs, nruns, i);
+    const int64_t p = runs[r].x + (i - runs[r].y);
+    rkeys[i] = (uint64_t)r << low_bits | (keys[p] & ((1ull << low_bits) - 1));
+    rvals[i] = vals[p];
+  }
+}
+
+// Back to their places; at[i] = the place.
+__global__ void __launch_bounds__(256) return_runs(const uint64_t *__restrict__ rkeys,
+                                                   const uint32_t *__restrict__ rvals,
+                                                   const int2 *__restrict__ runs, int64_t total,
+                                                   int low_bits, uint64_t *__restrict__ keys,
+                                                   uint32_t *__restrict__ vals,
+                                                   uint32_t *__restrict__ at) {
+  const uint64_t low = (1ull << low_bits) - 1;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t k = rkeys[i];
+    const int2 run = runs[k >> low_bits];
+    const int64_t p = run.x + (i - run.y);
+    keys[p] = (keys[p] & ~low) | (k & low);  // a run's elements agree above
+    vals[p] = rvals[i];
+    at[i] = (uint32_t)p;
+  }
+}
+
 size_t scatter_smem_bytes() {
   return sizeof(uint32_t) * (kSortWarps * kRadix + 2 * kRadix) + sizeof(uint64_t) * kSortTile +
          sizeof(uint32_t) * kSortTile;
@@ -543,10 +600,28 @@ size_t scatter_smem_bytes() {
 }  // namespace
 
 int order_equal_runs(tapas_b200_ctx *ctx, uint64_t *keys, uint32_t *vals, int64_t n, int low_bits,
-                     int max_run, int *longest) {
-  order_runs<<<grid_for(n, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(keys, vals, n, low_bits,
-                                                                         max_run, longest);
+                     int max_run, int2 *long_runs, unsigned long long *long_tally) {
+  order_runs<<<grid_for(n, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+      keys, vals, n, low_bits, max_run, long_runs, long_tally);
   TB_LAUNCH_CHECK(ctx);
+  return TAPAS_B200_OK;
+}
+
+int order_long_runs(tapas_b200_ctx *ctx, uint64_t *keys, uint32_t *vals, const int2 *runs,
+                    int nruns, int64_t total, int begin_bit, int low_bits, uint64_t *const rk[2],
+                    uint32_t *const rv[2], const uint32_t *&at) {
+  cudaStream_t s = ctx->stream;
+  const int grid = grid_for(total, 256, ctx->num_sms * 16);
+  collect_runs<<<grid, 256, 0, s>>>(keys, vals, runs, nruns, total, low_bits, rk[0], rv[0]);
+  TB_LAUNCH_CHECK(ctx);
+  uint64_t *k = rk[0], *ka = rk[1];
+  uint32_t *v = rv[0], *va = rv[1];
+  int bits = low_bits;  // of the keys {run, low bits}
+  while (bits < 63 && (1ll << (bits - low_bits)) < nruns) bits++;
+  TB_TRY(radix_sort(ctx, k, ka, v, va, total, begin_bit, bits));
+  return_runs<<<grid, 256, 0, s>>>(k, v, runs, total, low_bits, keys, vals, va);
+  TB_LAUNCH_CHECK(ctx);
+  at = va;
   return TAPAS_B200_OK;
 }
 

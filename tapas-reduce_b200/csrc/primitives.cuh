@@ -24,9 +24,18 @@ int radix_sort(tapas_b200_ctx *ctx, uint64_t *&keys, uint64_t *&keys_alt, uint32
                uint32_t *&vals_alt, int64_t n, int begin_bit, int end_bit);
 
 // After a radix sort on the bits from low_bits up only: orders every run of keys
-// equal there by all bits (stable), except runs of more than max_run, of which
-// *longest (device, 0 before) is raised to a length above max_run.
+// equal there by all bits (stable), except runs of more than max_run, which are listed:
+// long_runs[r] = {first element, elements of the listed runs before it}, room for
+// n / (max_run + 1) of them; *long_tally (device, 0 before) = {their number, their
+// elements} in its high and low 32 bits.
 int order_equal_runs(tapas_b200_ctx *ctx, uint64_t *keys, uint32_t *vals, int64_t n, int low_bits,
-                     int max_run, int *longest);
+                     int max_run, int2 *long_runs, unsigned long long *long_tally);
+
+// The listed runs, `total` elements in all, put in order of the bits from begin_bit up
+// (stable): their elements are sorted by {run, low bits} in rk and rv (scratch for
+// `total` each) and put back.  at (in rv): the places they took.
+int order_long_runs(tapas_b200_ctx *ctx, uint64_t *keys, uint32_t *vals, const int2 *runs,
+                    int nruns, int64_t total, int begin_bit, int low_bits, uint64_t *const rk[2],
+                    uint32_t *const rv[2], const uint32_t *&at);
 
 }  // namespace tb

@@ -144,6 +144,22 @@ __global__ void __launch_bounds__(kBlock) gather_bodies(
   }
 }
 
+// The same for the bodies in m places only.
+__global__ void __launch_bounds__(kBlock) gather_places(
+    const double4 *__restrict__ packed, const uint32_t *__restrict__ idx,
+    const uint32_t *__restrict__ at, int64_t m, double *__restrict__ sx, double *__restrict__ sy,
+    double *__restrict__ sz, double *__restrict__ sq) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t p = at[i];
+    const double4 b = packed[idx[p]];
+    sx[p] = b.x;
+    sy[p] = b.y;
+    sz[p] = b.z;
+    sq[p] = b.w;
+  }
+}
+
 __global__ void init_root(int64_t n, int ncrit, const double *__restrict__ box,
                           uint64_t *ckey, int32_t *cbeg, int32_t *cnb, int32_t *cparent,
                           int32_t *cchild, int32_t *cleaf, int32_t *clevel, double *cmin,
@@ -178,9 +194,12 @@ __global__ void init_root(int64_t n, int ncrit, const double *__restrict__ box,
 // ---------------------------------------------------------------------------
 // The body sort takes the 40 highest of the 57 key bits (13 of 19 levels; five radix
 // passes instead of eight) and orders the few bodies that agree there by
-// insertion; more than kMaxRun of them in one place (1 in 10^4 of the root's
-// width) and the sort is run on all bits instead, which the read-back of the
-// level sizes tells.
+// insertion.  More than kMaxRun of them in one place (1 in 10^4 of the root's
+// width: the core of a Plummer sphere from some 5M bodies on, or clusters) are listed,
+// and only they are sorted on, by their low bits, once the read-back of the level sizes
+// has told of them: six launches more up to 4096 such bodies.  Tree build of 16M Plummer
+// 3.15 ms, of an 8M cube without and with 40 coincident bodies 1.31 and 1.38 ms; 5.17 and
+// 2.52 ms when all bodies were sorted again on all bits.
 constexpr int kSortLow = kDepthBits + 3 * kMaxDepth - 40;
 constexpr int kMaxRun = 32;
 
@@ -469,21 +488,28 @@ int build_tree(tapas_b200_ctx *ctx, int ncrit) {
     TB_LAUNCH_CHECK(ctx);
   }
   const int ntiles = (int)((n + kTreeTile - 1) / kTreeTile);
-  // counts per level and tile, level totals, longest unordered run
-  TB_CUDA(ctx, ctx->tree_cnt.ensure((size_t)kTreeLevels * (ntiles + 1) + 1, s));
-  uint32_t *cnt = ctx->tree_cnt.p, *d_total = cnt + (size_t)kTreeLevels * ntiles;
-  int *d_longest = reinterpret_cast<int *>(d_total + kTreeLevels);
-  // Sorts on the key bits from `low` up (bits 4..0, the depth, are 19 for every
-  // body), completes the order, and gathers the bodies.
-  auto sort_bodies = [&](int low) -> int {
+  // tally of the long unordered runs, level totals, counts per level and tile
+  constexpr int kTotals = 2 + kTreeLevels;
+  TB_CUDA(ctx, ctx->tree_cnt.ensure(kTotals + (size_t)kTreeLevels * ntiles, s));
+  unsigned long long *d_tally = reinterpret_cast<unsigned long long *>(ctx->tree_cnt.p);
+  uint32_t *d_total = ctx->tree_cnt.p + 2, *cnt = ctx->tree_cnt.p + kTotals;
+  // the long runs and the sort of their bodies live in the results' rows, which
+  // nothing holds yet: 24 n bytes of keys and values, then at most n / 33 runs
+  uint64_t *const rk[2] = {reinterpret_cast<uint64_t *>(ctx->trg.p),
+                           reinterpret_cast<uint64_t *>(ctx->trg.p) + n};
+  uint32_t *const rv[2] = {reinterpret_cast<uint32_t *>(rk[1] + n),
+                           reinterpret_cast<uint32_t *>(rk[1] + n) + n};
+  int2 *const runs = reinterpret_cast<int2 *>(rk[1] + 2 * n);
+  {
+    PhaseTimer t(ctx, &ctx->timings.sort);
+    // bits 4..0, the depth, are 19 for every body
     uint64_t *k = ctx->keys.p, *ka = ctx->keys_alt.p;
     uint32_t *v = ctx->idx.p, *va = ctx->idx_alt.p;
-    TB_TRY(radix_sort(ctx, k, ka, v, va, n, low, kDepthBits + 3 * kMaxDepth));
+    TB_TRY(radix_sort(ctx, k, ka, v, va, n, kSortLow, kDepthBits + 3 * kMaxDepth));
     if (k != ctx->keys.p) { std::swap(ctx->keys.p, ctx->keys_alt.p); std::swap(ctx->keys.cap, ctx->keys_alt.cap); }
     if (v != ctx->idx.p) { std::swap(ctx->idx.p, ctx->idx_alt.p); std::swap(ctx->idx.cap, ctx->idx_alt.cap); }
-    TB_CUDA(ctx, cudaMemsetAsync(d_longest, 0, sizeof(int), s));
-    if (low > kDepthBits)
-      TB_TRY(order_equal_runs(ctx, ctx->keys.p, ctx->idx.p, n, low, kMaxRun, d_longest));
+    TB_CUDA(ctx, cudaMemsetAsync(d_tally, 0, sizeof *d_tally, s));
+    TB_TRY(order_equal_runs(ctx, ctx->keys.p, ctx->idx.p, n, kSortLow, kMaxRun, runs, d_tally));
     if (ctx->q_pending) {  // the charges' copy ran alongside the keys and the sort
       TB_CUDA(ctx, cudaStreamWaitEvent(s, ctx->q_ready, 0));
       pack_charges<<<grid_for(n, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(ctx->q.p, n,
@@ -494,27 +520,35 @@ int build_tree(tapas_b200_ctx *ctx, int ncrit) {
     gather_bodies<<<grid_for(n, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
         ctx->body_pack.p, ctx->idx.p, n, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->sq.p);
     TB_LAUNCH_CHECK(ctx);
-    return TAPAS_B200_OK;
-  };
-  {
-    PhaseTimer t(ctx, &ctx->timings.sort);
-    TB_TRY(sort_bodies(kSortLow));
   }
-  PhaseTimer t(ctx, &ctx->timings.tree);
   TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
-  uint32_t *h_total = reinterpret_cast<uint32_t *>(ctx->pinned.p);
-  for (bool complete = false;;) {
+  const unsigned long long *h_tally = reinterpret_cast<unsigned long long *>(ctx->pinned.p);
+  const uint32_t *h_total = reinterpret_cast<uint32_t *>(ctx->pinned.p) + 2;
+  auto count_levels = [&]() -> int {
+    PhaseTimer t(ctx, &ctx->timings.tree, true);
     count_nonleaves<<<ntiles, kBlock, 0, s>>>(ctx->keys.p, n, ncrit, ntiles, cnt);
     TB_LAUNCH_CHECK(ctx);
     TB_TRY(scan_rows(ctx, cnt, kTreeLevels, ntiles, d_total));
-    TB_CUDA(ctx, cudaMemcpyAsync(h_total, d_total, (kTreeLevels + 1) * sizeof(uint32_t),
+    TB_CUDA(ctx, cudaMemcpyAsync(ctx->pinned.p, d_tally, kTotals * sizeof(uint32_t),
                                  cudaMemcpyDeviceToHost, s));
     TB_CUDA(ctx, cudaStreamSynchronize(s));
-    if (h_total[kTreeLevels] == 0 || complete) break;
-    // many bodies in one cell of level 13: sort on all bits
-    complete = true;
-    TB_TRY(sort_bodies(kDepthBits));
+    return TAPAS_B200_OK;
+  };
+  TB_TRY(count_levels());
+  if (*h_tally) {
+    {
+      PhaseTimer t(ctx, &ctx->timings.sort, true);
+      const int64_t total = (int64_t)(*h_tally & 0xFFFFFFFFull);
+      const uint32_t *at = nullptr;
+      TB_TRY(order_long_runs(ctx, ctx->keys.p, ctx->idx.p, runs, (int)(*h_tally >> 32), total,
+                             kDepthBits, kSortLow, rk, rv, at));
+      gather_places<<<grid_for(total, kBlock, ctx->num_sms * 16), kBlock, 0, s>>>(
+          ctx->body_pack.p, ctx->idx.p, at, total, ctx->sx.p, ctx->sy.p, ctx->sz.p, ctx->sq.p);
+      TB_LAUNCH_CHECK(ctx);
+    }
+    TB_TRY(count_levels());
   }
+  PhaseTimer t(ctx, &ctx->timings.tree, true);
   LevelRanks ranks;
   int64_t nnode = 0;
   int depth = 0;

@@ -758,3 +758,42 @@ def test_tensorcore_m2l_wait_timeout_with_copies_in_flight(P, limit, tb, ctx):
     ne = (ctx.cells()["nb"] > 0) & (np.linalg.norm(L64, axis=1) > 0)
     rel = np.linalg.norm(Lmx[ne] - L64[ne], axis=1) / np.linalg.norm(L64[ne], axis=1)
     assert rel.max() < 2e-5
+
+
+def _clustered(tb, n, clusters, seed=92):
+    """A cube with clusters far smaller than a cell of level 13, some bodies coincident."""
+    x, y, z, q = [a.copy() for a in tb.datasets.make("uniform_cube", n, seed)]
+    rng = np.random.default_rng(6)
+    free = rng.permutation(n)
+    for k, m in enumerate(clusters):
+        idx, free = free[:m], free[m:]
+        for a, c in ((x, 0.3), (y, -0.2), (z, 0.6)):
+            a[idx] = c - 0.007 * k + 3e-6 * rng.random(m)
+        for a in (x, y, z):
+            a[idx[m // 2:m // 2 + 5]] = a[idx[0]]
+    return x, y, z, q
+
+
+@pytest.mark.parametrize("n,clusters,ncrit", [
+    (2000, [33], 4), (4096, [33, 34, 1000], 4), (9000, [40] * 100, 16), (9000, [4096], 16),
+    (9000, [4097, 33], 64), (40000, [40, 17000, 33, 9000], 64), (5000, [5000], 8),
+    (70000, [35] * 300 + [30] * 300, 16)])
+def test_tree_long_runs_of_close_bodies(n, clusters, ncrit, tb, ctx, oracle_mod):
+    """Clusters whose bodies agree in all 40 key bits sorted first: longer than the
+    insertion takes, one or many, few bodies or all, on both sides of the one-block
+    sort's limit, against the oracle's tree, bit for bit."""
+    _check_tree(tb, ctx, oracle_mod, *_clustered(tb, n, clusters), ncrit)
+
+
+@pytest.mark.parametrize("n", [3000, 50000])
+def test_long_runs_do_not_sort_everything_again(n, tb, ctx):
+    """A few close bodies cost a sort of themselves (six launches more), not one of all
+    bodies on all bits (24 passes' launches)."""
+    launches = []
+    for clusters in ([30], [33]):
+        b = _clustered(tb, n, clusters)
+        ctx.partition(*b, ncrit=64)
+        ctx.kernel_launches(True)
+        ctx.partition(*b, ncrit=64)
+        launches.append(ctx.kernel_launches(True))
+    assert launches[1] - launches[0] == 6
