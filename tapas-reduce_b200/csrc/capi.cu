@@ -812,11 +812,8 @@ int tapas_b200_direct(tapas_b200_ctx *ctx, const int64_t *targets, int64_t k, do
     dt = ctx->direct_tg.p;
     dout = ctx->direct_out.p;
   }
-  // about twelve waves of blocks, at least 16 sources per thread
   const int64_t nb = (k + kDirectTargets - 1) / kDirectTargets;
-  const int64_t waves = ((int64_t)ctx->num_sms * 24 + nb - 1) / nb;
-  const int nsplit = (int)std::max<int64_t>(
-      1, std::min({waves, (int64_t)64, ctx->n / (16 * kDirectThreads)}));
+  const int nsplit = direct_splits(ctx->num_sms, ctx->n, k);
   TB_CUDA(ctx, ctx->direct_part.ensure((size_t)4 * k * nsplit, s));
   direct_tiles<<<dim3((unsigned)nb, nsplit), kDirectThreads, 0, s>>>(
       ctx->x.p, ctx->y.p, ctx->z.p, ctx->q.p, ctx->n, dt, k, nsplit, ctx->direct_part.p);

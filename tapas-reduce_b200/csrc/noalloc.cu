@@ -1,7 +1,8 @@
 // FP64 direct sum for sampled targets that allocates no memory.
 //
-// Why it exists: tapas_b200_direct stages its target list and per-target sums
-// in device buffers it allocates on every call.  Some callers cannot allow a
+// Why it exists: tapas_b200_direct keeps the partial sums (and a host call's
+// targets and results) in device buffers of its context, which a larger call
+// allocates anew.  Some callers cannot allow a
 // device allocation where they check accuracy: a time-stepping loop that
 // reserves all of its device memory up front (a cudaMalloc there can fail or
 // push the solver out of memory), or code that shares the GPU with other
@@ -12,7 +13,7 @@
 // Limits and sharing:
 //  - at most kMaxTargets targets per call; more are rejected with
 //    TAPAS_B200_ERR_CAPACITY and a message;
-//  - the scratch array (kMaxTargets x kSplit x 4 doubles = 2 MiB) exists once
+//  - the scratch array (kMaxRows x 4 doubles = 2 MiB) exists once
 //    per GPU that loads the library and is held until the process exits;
 //  - every call on a device uses the same array, and it keeps the last call's
 //    contents.  Each call writes every slot it later reads, so nothing needs
@@ -31,11 +32,11 @@ namespace tb {
 namespace {
 
 constexpr int kMaxTargets = 4096;
-constexpr int kSplit = 16;       // blocks per target, each over 1/kSplit of the sources
+constexpr int64_t kMaxRows = 65536;  // (target, split) pairs: 16 splits of the most targets
 constexpr int kMaxDevices = 64;
 
 // The scratch: per (target, split) the 4 partial sums.
-static __device__ __align__(256) double g_direct_scratch[(size_t)kMaxTargets * kSplit * 4];
+static __device__ __align__(256) double g_direct_scratch[(size_t)kMaxRows * 4];
 
 double *g_scratch_addr[kMaxDevices] = {nullptr};
 std::mutex g_scratch_mutex;
@@ -91,11 +92,23 @@ extern "C" int tapas_b200_direct_noalloc(const double *x, const double *y, const
               cudaGetErrorString(e));
     return TAPAS_B200_ERR_CUDA;
   }
-  direct_tiles<<<dim3((unsigned)((k + kDirectTargets - 1) / kDirectTargets), kSplit),
-                 kDirectThreads, 0, s>>>(x, y, z, q, n, targets, k, kSplit, scratch);
+  int num_sms = 0;
+  e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) {
+    set_error(nullptr, "direct_noalloc: %s", cudaGetErrorString(e));
+    return TAPAS_B200_ERR_CUDA;
+  }
+  // the scratch has room for 16 splits of any k: 4096 targets x 1M bodies 5.04 ms, 5.14 with
+  // the rule's 7, whose last wave of blocks is nearly empty
+  const int64_t most = std::max<int64_t>(1, n / (16 * kDirectThreads));
+  const int nsplit = (int)std::min<int64_t>(
+      kMaxRows / k, std::max<int64_t>(direct_splits(num_sms, n, k),
+                                      std::min<int64_t>(kMaxRows / kMaxTargets, most)));
+  direct_tiles<<<dim3((unsigned)((k + kDirectTargets - 1) / kDirectTargets), nsplit),
+                 kDirectThreads, 0, s>>>(x, y, z, q, n, targets, k, nsplit, scratch);
   e = cudaGetLastError();
   if (e == cudaSuccess) {
-    direct_finish<<<(unsigned)((k * 4 + 255) / 256), 256, 0, s>>>(scratch, k, kSplit, out4);
+    direct_finish<<<(unsigned)((k * 4 + 255) / 256), 256, 0, s>>>(scratch, k, nsplit, out4);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {

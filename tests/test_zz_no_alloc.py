@@ -93,3 +93,26 @@ def test_direct_noalloc_rejects_too_many_targets(tb):
     rc = _noalloc(L, dev, tg, k, out)
     assert rc == -5
     assert b"4096" in L.tapas_b200_last_error(None)
+
+
+@pytest.mark.parametrize("n", [40_000, 1_000_000])
+@pytest.mark.parametrize("k", [1, 7, 9, 600, 4096])
+def test_direct_noalloc_at_every_split(n, k, tb):
+    """A group's sources are shared out by a rule of the bodies and the targets, up to
+    64 ways for few targets, 16 ways and up for many: the fixed scratch holds the
+    shares of each, and their sums are the allocating entry point's, at its bar."""
+    torch = pytest.importorskip("torch")
+    L = tb.lib()
+    L.tapas_b200_last_error.restype = ctypes.c_char_p
+    b = tb.datasets.make("sphere_surface", n, 74)
+    dev = [torch.from_numpy(a).cuda() for a in b]
+    tg = np.random.default_rng(k).integers(0, n, k)
+    with tb.Context(0) as ctx:
+        ctx.partition(*b, ncrit=64)
+        ref = ctx.direct(tg)
+    tg_d = torch.from_numpy(tg).cuda()
+    out = torch.full((k, 4), 7.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert _noalloc(L, dev, tg_d, k, out) == 0, L.tapas_b200_last_error(None)
+    torch.cuda.synchronize()
+    assert np.all(np.abs(out.cpu().numpy() - ref) <= 1e-12 * np.max(np.abs(ref), axis=0))
