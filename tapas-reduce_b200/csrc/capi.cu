@@ -200,6 +200,7 @@ int tapas_b200_ctx_destroy(tapas_b200_ctx *ctx) {
 int tapas_b200_set_stream(tapas_b200_ctx *ctx, void *stream) {
   TB_TRY(check_ctx(ctx));
   ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
+  ctx->trav_blocks = 0;  // another stream may hold another share of the SMs
   return TAPAS_B200_OK;
 }
 

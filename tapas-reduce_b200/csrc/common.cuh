@@ -221,7 +221,7 @@ struct tapas_b200_ctx {
   int mutual = 0;                       // lists of the last build_lists came from a mutual traversal
   uint64_t n_p2p_int = 0;
   int trav_iters = 0;
-  int trav_blocks = 0;     // blocks of the traversal kernel the GPU holds at once
+  int trav_blocks = 0;     // blocks of the traversal kernel the stream holds at once (0: not known)
   int64_t trav_pairs = 0;  // (target, source) pairs the traversal classified
   int list_shift = 1;                   // packed list key = target << shift | source
   bool reference_lists = false;         // keep pairs with empty cells, as the reference visits them

@@ -30,6 +30,7 @@
 
 #include <algorithm>
 
+#include "coop.cuh"
 #include "primitives.cuh"
 #include "traverse.cuh"
 
@@ -581,7 +582,7 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
       ctx->trav_blocks = std::max(1, per_sm) * ctx->num_sms;
     }
     // few blocks for a small tree: the barrier costs more than their work
-    const int blocks =
+    int blocks =
         (int)std::min<int64_t>(ctx->trav_blocks, std::max<int64_t>(32, C * 8 / kBlock));
     TravState *h = reinterpret_cast<TravState *>(hc + 16);
     for (int attempt = 0;; attempt++) {
@@ -595,8 +596,12 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
       int prune = ctx->reference_lists ? 0 : 1, mut = mutual;
       TravState *state = st;
       void *args[] = {&cells, &bufs, &state, &prune, &mut};
-      TB_CUDA(ctx, cudaLaunchCooperativeKernel(reinterpret_cast<void *>(dtt_steps), dim3(blocks),
-                                               dim3(kBlock), args, 0, s));
+      const int asked = blocks;
+      TB_CUDA(ctx, launch_at_most(blocks, [&](int b) {
+                return cudaLaunchCooperativeKernel(reinterpret_cast<void *>(dtt_steps), dim3(b),
+                                                   dim3(kBlock), args, 0, s);
+              }));
+      if (blocks < asked) ctx->trav_blocks = blocks;  // what this stream holds
       count_launch(ctx);
       TB_CUDA(ctx, cudaMemcpyAsync(h, st, sizeof(TravState), cudaMemcpyDeviceToHost, s));
       TB_CUDA(ctx, cudaStreamSynchronize(s));

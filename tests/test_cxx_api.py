@@ -145,3 +145,18 @@ def test_user_functors_on_gpu(device_driver):
     d = json.loads(p.stdout.strip().splitlines()[-1])
     assert d["max_rel_user_p2p"] < 1e-12 and d["max_rel_mapreduce"] < 1e-13
     assert d["reduce_levels_ok"] and d["levels"] >= 4
+
+
+def test_cooperative_launch_fits_the_streams_share(tmp_path):
+    """A launch refused for its size is tried with fewer blocks, down to one, and any
+    other error is reported as it is (host code, against a fake launch)."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not pathlib.Path(nvcc).exists():
+        pytest.skip("no nvcc")
+    exe = tmp_path / "coop_launch_test"
+    subprocess.run([nvcc, "-std=c++17", "-x", "cu", "-I",
+                    str(ROOT / "tapas-reduce_b200" / "csrc"),
+                    str(ROOT / "tests" / "cxx" / "coop_launch_test.cxx"), "-o", str(exe)],
+                   check=True, capture_output=True, text=True)
+    p = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert p.returncode == 0, p.stdout
