@@ -557,13 +557,15 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
   ctx->p2p_begun = false;  // counted for other lists
   TB_CUDA(ctx, ctx->pinned.ensure(tapas_b200_ctx::kPinnedBytes));
   // First sizes: a list entry per cell and near or far neighbour of a
-  // volume-filling tree for small trees, of a surface for large ones; a list that
-  // outgrows its buffer is met below, and the buffers stay for the next call.
+  // volume-filling tree for small trees, of a surface for large ones, and the frontier
+  // of a step that has both (100k bodies of a cube, ncrit 64, theta 0.4: 667k pairs,
+  // 143 per cell); a list that outgrows its buffer is met below, and the buffers
+  // stay for the next call.
   auto room = [&](int64_t per_cell, int64_t large, int64_t extra) {
     return (size_t)(std::min(per_cell * C, large * C + extra) + 4096);
   };
-  TB_CUDA(ctx, ctx->front_a.ensure(room(64, 16, 2000000), s));
-  TB_CUDA(ctx, ctx->front_b.ensure(room(64, 16, 2000000), s));
+  TB_CUDA(ctx, ctx->front_a.ensure(room(160, 16, 2000000), s));
+  TB_CUDA(ctx, ctx->front_b.ensure(room(160, 16, 2000000), s));
   TB_CUDA(ctx, ctx->m2l.ensure(room(128, 40, 4000000), s));
   TB_CUDA(ctx, ctx->p2p.ensure(room(64, 24, 2000000), s));
   unsigned long long *hc = reinterpret_cast<unsigned long long *>(ctx->pinned.p);

@@ -797,3 +797,62 @@ def test_long_runs_do_not_sort_everything_again(n, tb, ctx):
         ctx.partition(*b, ncrit=64)
         launches.append(ctx.kernel_launches(True))
     assert launches[1] - launches[0] == 6
+
+
+def _pair_codes(keys, order, t, s):
+    """Sorted codes of (target, source) pairs, cells numbered by key (order: argsort)."""
+    rank = np.empty(len(keys), np.int64)
+    rank[order] = np.arange(len(keys))
+    return np.sort(rank[t] * len(keys) + rank[s])
+
+
+@pytest.mark.parametrize("mutual", [0, 1])
+@pytest.mark.parametrize("n,ncrit,theta,over", [
+    (3000, 16, 0.1, "frontier and P2P"), (40000, 16, 0.25, "frontier and M2L"),
+    (3000, 16, 0.4, "none")])
+def test_traversal_outgrows_its_first_buffers(n, ncrit, theta, over, mutual, tb, oracle_mod):
+    """Lists and frontiers longer than a fresh context's buffers end the traversal's
+    launch; it goes on from that step in larger ones.  The lists are the oracle's, from
+    a context whose first traversal this is and from one that has grown from a
+    smaller set's."""
+    x, y, z, q = tb.datasets.make("uniform_cube", n, 21)
+    o = oracle_mod.Oracle(x, y, z, q, P=2, ncrit=ncrit, theta=theta, mutual=mutual)
+    okeys = o.cells()["key"]
+    oo = np.argsort(okeys, kind="stable")
+    expected = []
+    for t, s in (o.m2l_list(), o.p2p_list()):
+        if mutual:  # the unordered pairs, both ways
+            other = t != s
+            t, s = np.concatenate([t, s[other]]), np.concatenate([s, t[other]])
+        expected.append(_pair_codes(okeys, oo, t, s))
+    for small_first in (False, True):
+        with tb.Context(0) as c:
+            c.set_reference_lists(True)
+            if small_first:
+                c.partition(*tb.datasets.make("uniform_cube", 200, 22), ncrit=16)
+                c.build_lists(0.5, mutual)
+            c.partition(x, y, z, q, ncrit=ncrit)
+            launches = []
+            for _ in range(2):
+                c.kernel_launches(True)
+                info = c.build_lists(theta, mutual)
+                launches.append(c.kernel_launches(True))
+                keys = c.cells()["key"]
+                go = np.argsort(keys, kind="stable")
+                for got, want in zip(c.lists(), expected):
+                    assert np.array_equal(_pair_codes(keys, go, *got), want)
+            assert (launches[0] > launches[1]) == (over != "none")
+            first = 1.125 * (128 * len(keys) + 4096) + 1024
+            assert (info["n_m2l"] / (1 + mutual) > first) == ("M2L" in over)
+
+
+def test_first_traversal_of_the_default_cube_runs_through(tb):
+    """100k bodies of a cube at the default setting fit a fresh context's buffers."""
+    with tb.Context(0) as c:
+        c.partition(*tb.datasets.make("uniform_cube", 100000, 3), ncrit=64)
+        launches = []
+        for _ in range(2):
+            c.kernel_launches(True)
+            c.build_lists(0.4)
+            launches.append(c.kernel_launches(True))
+        assert launches[0] == launches[1]
