@@ -35,6 +35,7 @@ void set_error(tapas_b200_ctx *ctx, const char *fmt, ...);
     if (e_ != cudaSuccess) {                                                       \
       ::tb::set_error((ctx), "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e_), \
                       __FILE__, __LINE__);                                         \
+      cudaGetLastError(); /* reported here, not by the next launch's check */      \
       return e_ == cudaErrorMemoryAllocation ? TAPAS_B200_ERR_NOMEM               \
                                              : TAPAS_B200_ERR_CUDA;               \
     }                                                                              \

@@ -856,3 +856,30 @@ def test_first_traversal_of_the_default_cube_runs_through(tb):
             c.build_lists(0.4)
             launches.append(c.kernel_launches(True))
         assert launches[0] == launches[1]
+
+
+def _all_but(mb):
+    """A tensor that takes the GPU's memory but for about `mb` MiB."""
+    import torch
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    return torch.empty(torch.cuda.mem_get_info()[0] - (mb << 20), dtype=torch.uint8, device="cuda")
+
+
+def test_out_of_memory_is_reported_once(tb):
+    """An allocation that fails is its own call's error, not also that of the next
+    call's first launch."""
+    b = tb.datasets.make("sphere_surface", 1000000, 9)
+    with tb.Context(0) as c:
+        c.partition(*b, ncrit=128)
+        hog = _all_but(24)
+        try:
+            with pytest.raises(tb.TapasError) as e:
+                c.build_lists(0.4)
+            assert e.value.code == tb._lib.ERR_NOMEM
+        finally:
+            del hog
+            import torch
+            torch.cuda.empty_cache()
+        c.partition(*b, ncrit=128)
+        assert c.build_lists(0.4)["n_p2p"] > 0
