@@ -532,7 +532,10 @@ int sort_list_sources(tapas_b200_ctx *ctx) {
   return sort_list_sources(ctx, 1);
 }
 
-int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sources) {
+// build_lists; roomy: with first sizes that hold most trees' lists, and half as much
+// again for one that grows, else with no more than each step needs.
+static int build_lists_in(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sources,
+                          bool roomy) {
   if (!ctx->have_tree) {
     set_error(ctx, "build_lists: no tree (call partition first)");
     return TAPAS_B200_ERR_STATE;
@@ -562,8 +565,9 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
   // 143 per cell); a list that outgrows its buffer is met below, and the buffers
   // stay for the next call.
   auto room = [&](int64_t per_cell, int64_t large, int64_t extra) {
-    return (size_t)(std::min(per_cell * C, large * C + extra) + 4096);
+    return (size_t)((roomy ? std::min(per_cell * C, large * C + extra) : 0) + 4096);
   };
+  auto grown = [&](unsigned long long need) { return (size_t)(need + (roomy ? need / 2 : 0)); };
   TB_CUDA(ctx, ctx->front_a.ensure(room(160, 16, 2000000), s));
   TB_CUDA(ctx, ctx->front_b.ensure(room(160, 16, 2000000), s));
   TB_CUDA(ctx, ctx->m2l.ensure(room(128, 40, 4000000), s));
@@ -614,11 +618,11 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
       }
       tb::DBuf<int2> &next = (h->steps & 1) ? ctx->front_a : ctx->front_b;
       if (h->need_front > next.cap)
-        TB_CUDA(ctx, next.ensure(h->need_front + h->need_front / 2, s));
+        TB_CUDA(ctx, next.ensure(grown(h->need_front), s));
       if (h->need_m2l > ctx->m2l.cap)
-        TB_CUDA(ctx, ctx->m2l.ensure(h->need_m2l + h->need_m2l / 2, s, true, h->m2l));
+        TB_CUDA(ctx, ctx->m2l.ensure(grown(h->need_m2l), s, true, h->m2l));
       if (h->need_p2p > ctx->p2p.cap)
-        TB_CUDA(ctx, ctx->p2p.ensure(h->need_p2p + h->need_p2p / 2, s, true, h->p2p));
+        TB_CUDA(ctx, ctx->p2p.ensure(grown(h->need_p2p), s, true, h->p2p));
       h->stop = 0;
       for (auto &set : h->cnt)
         for (auto &v : set) v = 0;
@@ -660,6 +664,10 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
     ctx->n_p2p_int = n_int;
     ctx->trav_iters = iters;
     ctx->trav_pairs = visited;
+    if (!roomy) {
+      ctx->front_a.release();
+      ctx->front_b.release();
+    }
   }
   {
     PhaseTimer tm(ctx, &ctx->timings.list_sort);
@@ -730,6 +738,18 @@ int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sou
   }
   ctx->have_lists = true;
   return TAPAS_B200_OK;
+}
+
+int build_lists(tapas_b200_ctx *ctx, double theta, int mutual, bool sort_m2l_sources) {
+  const int rc = build_lists_in(ctx, theta, mutual, sort_m2l_sources, true);
+  if (rc != TAPAS_B200_ERR_NOMEM) return rc;
+  // The GPU's memory does not hold the first sizes (1M sphere, ncrit 128: 122 MB in all,
+  // 44 with the least each step needs): give them back and start again.
+  ctx->front_a.release();
+  ctx->front_b.release();
+  for (auto *b : {&ctx->m2l, &ctx->p2p, &ctx->list_alt}) b->release();
+  ctx->list_src.release();
+  return build_lists_in(ctx, theta, mutual, sort_m2l_sources, false);
 }
 
 }  // namespace tb

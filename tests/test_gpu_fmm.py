@@ -7,6 +7,7 @@ Bars (stated per check):
 * mixed form: rel-L2 vs the FP64 form <= 2e-6, and vs direct sum the same
   accuracy class as FP64.
 """
+import contextlib
 import pathlib
 
 import numpy as np
@@ -858,12 +859,19 @@ def test_first_traversal_of_the_default_cube_runs_through(tb):
         assert launches[0] == launches[1]
 
 
-def _all_but(mb):
-    """A tensor that takes the GPU's memory but for about `mb` MiB."""
+@contextlib.contextmanager
+def _free_memory(mb):
+    """The GPU's memory taken but for about `mb` MiB."""
     import torch
     torch.cuda.empty_cache()
     torch.cuda.synchronize()
-    return torch.empty(torch.cuda.mem_get_info()[0] - (mb << 20), dtype=torch.uint8, device="cuda")
+    rest = torch.cuda.mem_get_info()[0] - (mb << 20)
+    hog = torch.empty(rest, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del hog
+        torch.cuda.empty_cache()
 
 
 def test_out_of_memory_is_reported_once(tb):
@@ -872,14 +880,27 @@ def test_out_of_memory_is_reported_once(tb):
     b = tb.datasets.make("sphere_surface", 1000000, 9)
     with tb.Context(0) as c:
         c.partition(*b, ncrit=128)
-        hog = _all_but(24)
-        try:
+        with _free_memory(24):
             with pytest.raises(tb.TapasError) as e:
                 c.build_lists(0.4)
             assert e.value.code == tb._lib.ERR_NOMEM
-        finally:
-            del hog
-            import torch
-            torch.cuda.empty_cache()
         c.partition(*b, ncrit=128)
         assert c.build_lists(0.4)["n_p2p"] > 0
+
+
+@pytest.mark.parametrize("mutual", [0, 1])
+def test_lists_where_memory_is_short(mutual, tb):
+    """Where the GPU's memory does not hold the traversal's first sizes (122 MB for
+    this tree), it runs with what each step needs: the same lists."""
+    b = tb.datasets.make("sphere_surface", 1000000, 9)
+    with tb.Context(0) as c:
+        c.partition(*b, ncrit=128)
+        c.build_lists(0.4, mutual)
+        want = c.lists()
+    with tb.Context(0) as c:
+        c.partition(*b, ncrit=128)
+        with _free_memory(80):
+            c.build_lists(0.4, mutual)
+            got = c.lists()
+        for g, w in zip(got, want):
+            assert np.array_equal(g[0], w[0]) and np.array_equal(g[1], w[1])
