@@ -700,7 +700,11 @@ int tapas_b200_traverse(tapas_b200_ctx *ctx, double theta, int mutual, int preci
     PhaseTimer t(ctx, &ctx->timings.m2l);
     far = m2l_launch(ctx, precision);
   }
-  const int near = far ? far : tapas_b200_p2p(ctx, precision);
+  int near = far ? far : tapas_b200_p2p(ctx, precision);
+  if (!far && near == TAPAS_B200_ERR_NOMEM && ctx->tc.rows64.cap > 0) {
+    ctx->tc.rows64.release();  // the FP64 M2L's rows took what was left: it is done with them
+    near = tapas_b200_p2p(ctx, precision);
+  }
   ctx->p2p_begun = false;  // whatever failed
   TB_TRY(far);
   TB_TRY(m2l_status(ctx));

@@ -32,6 +32,7 @@ namespace tb {
 namespace {
 
 constexpr size_t kRowBytes = (size_t)512 << 20;  // product rows kept at once
+constexpr size_t kLeastRowBytes = (size_t)8 << 20;  // the same where memory is short
 // Pairs a class needs for an operator of its own: building one and multiplying
 // a partly filled tile costs about as much as translating 16 pairs one by one.
 constexpr int64_t kMinClassPairs = 16;
@@ -426,31 +427,46 @@ int m2l_products_P(tapas_b200_ctx *ctx) {
   TB_CUDA(ctx, cudaMemsetAsync(ctx->L.p, 0, sizeof(double2) * (size_t)C * O::NT, s));
   ctx->tc_classes = 0;
   if (n == 0) return TAPAS_B200_OK;
-  const int64_t per_range =
-      std::min<int64_t>(n, std::max<int64_t>(1, (int64_t)(kRowBytes / (sizeof(double) * O::K))));
-  const int64_t nrange = (n + per_range - 1) / per_range;
+  int64_t per_range = std::min<int64_t>(n, (int64_t)(kRowBytes / (sizeof(double) * O::K)));
+  int64_t nrange = 1, parts = 0;
   M2LClassInfo ci;
   int64_t max_tiles = 0;
   {
     PhaseTimer t(ctx, &ctx->timings.m2l_setup);
     TB_TRY(m2l_classes(ctx, sizeof(double) * O::DOUBLES, kMinClassPairs, ci));
-    TB_CUDA(ctx, T.rows64.ensure((size_t)per_range * O::K, s));
     if (ci.ntc > 0) {
       TB_CUDA(ctx, T.ops64.ensure(O::DOUBLES * ci.ntc, s));
+      TB_CUDA(ctx, T.Mt64.ensure((size_t)C * O::KP, s));
+    }
+    // the tile tables and the rows, in shorter ranges where memory is too short for the rows
+    for (;; per_range = (per_range + 1) / 2) {
+      nrange = (n + per_range - 1) / per_range;
+      parts = ci.ntc * nrange;
+      max_tiles = n / kPairTile + parts;
+      auto room = [&]() -> cudaError_t {
+        cudaError_t e = T.cnt64.ensure(parts + 1, s);
+        if (e == cudaSuccess) e = T.off64.ensure(parts + 1, s);
+        if (e == cudaSuccess) e = T.part64.ensure(parts + 1, s);
+        if (e == cudaSuccess) e = T.items64.ensure(max_tiles + 1, s);
+        return e == cudaSuccess ? T.rows64.ensure((size_t)per_range * O::K, s) : e;
+      };
+      const cudaError_t e = room();
+      if (e == cudaErrorMemoryAllocation &&
+          (size_t)per_range * sizeof(double) * O::K > kLeastRowBytes) {
+        cudaGetLastError();
+        continue;
+      }
+      TB_CUDA(ctx, e);
+      break;
+    }
+    if (ci.ntc > 0) {
       build_operators64<P><<<(unsigned)ci.ntc, 256, 0, s>>>(T.tc_keys.p, T.ops64.p);
       TB_LAUNCH_CHECK(ctx);
-      TB_CUDA(ctx, T.Mt64.ensure((size_t)C * O::KP, s));
       normalize_M64<P><<<grid_for(C, 8, ctx->num_sms * 8), 256, 0, s>>>(
           C, ctx->cnb.p, ctx->cmin.p, ctx->cmax.p, ctx->M.p,
           reinterpret_cast<double2 *>(T.Mt64.p));
       TB_LAUNCH_CHECK(ctx);
       // tiles, ranges outermost
-      const int64_t parts = ci.ntc * nrange;
-      max_tiles = n / kPairTile + parts;
-      TB_CUDA(ctx, T.cnt64.ensure(parts + 1, s));
-      TB_CUDA(ctx, T.off64.ensure(parts + 1, s));
-      TB_CUDA(ctx, T.part64.ensure(parts + 1, s));
-      TB_CUDA(ctx, T.items64.ensure(max_tiles + 1, s));
       count_tiles64<<<grid_for(parts, 256), 256, 0, s>>>(T.cls_range.p, ci.ntc, nrange, per_range,
                                                          T.vals.p, T.cnt64.p, T.part64.p);
       TB_LAUNCH_CHECK(ctx);

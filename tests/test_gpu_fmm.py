@@ -904,3 +904,24 @@ def test_lists_where_memory_is_short(mutual, tb):
             got = c.lists()
         for g, w in zip(got, want):
             assert np.array_equal(g[0], w[0]) and np.array_equal(g[1], w[1])
+
+
+@pytest.mark.parametrize("mb", [850, 600])
+def test_fp64_m2l_where_memory_is_short(mb, tb):
+    """Where the GPU's memory does not hold the product rows' 512 MiB, the M2L takes
+    shorter ranges and leaves the near field its room: the same bits."""
+    b = tb.datasets.make("uniform_cube", 60000, 12)
+
+    def evaluate(c):
+        c.partition(*b, ncrit=16)
+        c.upward(14, tb.FP64)
+        with _free_memory(mb) if short else contextlib.nullcontext():
+            c.traverse(0.35, precision=tb.FP64)
+            c.downward(tb.FP64)
+            return c.results()
+
+    got = []
+    for short in (False, True):
+        with tb.Context(0) as c:
+            got.append(evaluate(c))
+    assert np.array_equal(*got)
