@@ -394,7 +394,8 @@ __host__ __device__ inline uint64_t finest_key(int ax, int ay, int az) {
 // both 0 for r2 = 0 (a body with itself).  The hardware's approximation y of
 // 1 / sqrt(r2) is refined once by the binomial series of (1 - e)^(-1/2),
 // e = 1 - r2 y^2, to third order (1 + e/2 + 3/8 e^2): e is below ~2^-20, so the
-// truncation is below 2^-60 and the result within about an ulp, for 5 FP64
+// truncation is below 2^-60 and the result within 1.01 ulp (half of it the last
+// rounding, the rest that of r2 y in e), for 5 FP64
 // operations (measured: rsqrt(r2) takes 10 slots of the FP64 pipe).  Zero,
 // subnormal, infinite and NaN r2, which the approximation flushes or the
 // refinement would turn into NaN, take rsqrt; one branch for all kN, since a

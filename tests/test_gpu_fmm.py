@@ -925,3 +925,33 @@ def test_fp64_m2l_where_memory_is_short(mb, tb):
         with tb.Context(0) as c:
             got.append(evaluate(c))
     assert np.array_equal(*got)
+
+
+@pytest.mark.parametrize("lo,hi", [(-30, 30), (-511.5, -510.5), (-537, -511.6), (-545, -538),
+                                   (509.0, 511.99), (512.01, 514)])
+def test_reciprocal_distance_within_its_bound(lo, hi, tb, ctx):
+    """charge_over_distance by itself: one unit charge at the origin, chargeless bodies at
+    distances 2^lo .. 2^hi, so a body's potential is 1/r alone.  In the ordinary
+    range, with r^2 on both sides of the smallest normal number and near the
+    largest, subnormal, zero (adds nothing) and infinite (nothing either).  Against
+    extended precision, from the rounded r^2: the refined 1/sqrt is off by its last
+    rounding (1/2 ulp), half the rounding of r^2 y (at most 1/2 ulp) and the
+    series' rest (0.003 ulp); rsqrt, which takes the rest, by 1 ulp.  The acceleration has
+    three such factors and three roundings."""
+    rng = np.random.default_rng(17)
+    n = 4000
+    d = 2.0 ** rng.uniform(lo, hi, n) * rng.choice([-1.0, 1.0], n)
+    x, q = np.concatenate([[0.0], d]), np.zeros(n + 1)
+    q[0] = 1.0
+    zero = np.zeros(n + 1)
+    ctx.partition(x, zero, zero, q, ncrit=64)
+    r = ctx.direct(np.arange(1, n + 1))
+    with np.errstate(all="ignore"):
+        r2 = d * d
+        exact = np.where(r2 == 0, 0, 1 / np.sqrt(r2.astype(np.longdouble)))
+    bound = np.spacing(np.maximum(exact.astype(np.float64), 1e-300)).astype(np.longdouble)
+    assert np.all(np.abs(r[:, 0].astype(np.longdouble) - exact) <= 1.01 * bound)
+    if lo >= -30 and hi <= 30:  # beyond, 1/r^3 leaves the FP64 range
+        acc = -d.astype(np.longdouble) * exact ** 3
+        assert np.all(np.abs(r[:, 1] - acc) <= 4.6 * 2.0 ** -52 * np.abs(acc))
+        assert np.all(r[:, 2:] == 0)
