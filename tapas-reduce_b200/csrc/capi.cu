@@ -674,7 +674,7 @@ int tapas_b200_p2p(tapas_b200_ctx *ctx, int precision) {
     set_error(ctx, "p2p: needs build_lists first");
     return TAPAS_B200_ERR_STATE;
   }
-  PhaseTimer t(ctx, &ctx->timings.p2p);
+  PhaseTimer t(ctx, &ctx->timings.p2p, ctx->p2p_begun);  // after its items were counted
   ctx->near_precision = precision;
   if (precision == TAPAS_B200_MIXED) return p2p_mixed(ctx);
   TB_TRY(sort_list_sources(ctx, 1));  // the FP64 sums run in source order
@@ -694,7 +694,10 @@ int tapas_b200_traverse(tapas_b200_ctx *ctx, double theta, int mutual, int preci
   // The P2P item totals are read back while the M2L classes are, and the M2L's
   // status once the P2P is launched: neither leaves the GPU without work.  1500
   // bodies, mixed: 548 us, 567 us with each read where it is used.
-  TB_TRY(p2p_begin(ctx, precision));
+  {
+    PhaseTimer t(ctx, &ctx->timings.p2p);
+    TB_TRY(p2p_begin(ctx, precision));
+  }
   int far;
   {
     PhaseTimer t(ctx, &ctx->timings.m2l);

@@ -55,27 +55,24 @@ static __global__ void __launch_bounds__(kDirectThreads, 2) direct_tiles(
     const double4 b = next;
     if (j + step < n)
       next = make_double4(x[j + step], y[j + step], z[j + step], q[j + step]);
-    constexpr int G = T;  // separations in flight
+    // all T separations in flight
+    double dx[T], dy[T], dz[T], R2[T], qj[T], qr[T], inv[T];
 #pragma unroll
-    for (int r0 = 0; r0 < T; r0 += G) {
-      double dx[G], dy[G], dz[G], R2[G], qj[G], qr[G], inv[G];
+    for (int i = 0; i < T; i++) {
+      dx[i] = xi[i] - b.x;
+      dy[i] = yi[i] - b.y;
+      dz[i] = zi[i] - b.z;
+      R2[i] = dx[i] * dx[i] + dy[i] * dy[i] + dz[i] * dz[i];
+      qj[i] = b.w;
+    }
+    charge_over_distance(R2, qj, qr, inv);
 #pragma unroll
-      for (int i = 0; i < G; i++) {
-        dx[i] = xi[r0 + i] - b.x;
-        dy[i] = yi[r0 + i] - b.y;
-        dz[i] = zi[r0 + i] - b.z;
-        R2[i] = dx[i] * dx[i] + dy[i] * dy[i] + dz[i] * dz[i];
-        qj[i] = b.w;
-      }
-      charge_over_distance(R2, qj, qr, inv);
-#pragma unroll
-      for (int i = 0; i < G; i++) {
-        const double s3 = qr[i] * inv[i] * inv[i];
-        p[r0 + i] += qr[i];
-        ax[r0 + i] = fma(-dx[i], s3, ax[r0 + i]);
-        ay[r0 + i] = fma(-dy[i], s3, ay[r0 + i]);
-        az[r0 + i] = fma(-dz[i], s3, az[r0 + i]);
-      }
+    for (int i = 0; i < T; i++) {
+      const double s3 = qr[i] * inv[i] * inv[i];
+      p[i] += qr[i];
+      ax[i] = fma(-dx[i], s3, ax[i]);
+      ay[i] = fma(-dy[i], s3, ay[i]);
+      az[i] = fma(-dz[i], s3, az[i]);
     }
   }
   __shared__ double red[kDirectThreads / 32][4 * T];

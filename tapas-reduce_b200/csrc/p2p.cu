@@ -579,7 +579,7 @@ __device__ __forceinline__ void mixed_tile(
       __syncwarp();
       if (active) {
         // loops short enough for the instruction cache nearest the scheduler: with
-        // three or four targets a lane has that many independent chains anyway
+        // two or three targets a lane has that many independent chains anyway
 #pragma unroll(kR == 1 ? 2 : 1)
         for (int k = 2 * g; k < nfar; k += 2 * G)
           far2(*reinterpret_cast<const float2 *>(sm.fx + k),

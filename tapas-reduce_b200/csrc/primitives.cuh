@@ -4,7 +4,7 @@
 
 namespace tb {
 
-// out[i] = sum(in[0..i)); *d_total (device, may be null) = sum(in).  n <= 4096^2.
+// out[i] = sum(in[0..i)); *d_total (device, may be null) = sum(in).  n < 2^31, sums too.
 int scan_exclusive(tapas_b200_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
                    int32_t *d_total);
 

@@ -437,7 +437,7 @@ int leaf_depth_histogram(tapas_b200_ctx *ctx, int nbins, int64_t *out) {
   return TAPAS_B200_OK;
 }
 
-int ensure_cells(tapas_b200_ctx *ctx, int64_t need) {
+static int ensure_cells(tapas_b200_ctx *ctx, int64_t need) {
   cudaStream_t s = ctx->stream;
   TB_CUDA(ctx, ctx->ckey.ensure(need, s));
   TB_CUDA(ctx, ctx->cbeg.ensure(need, s));

@@ -3,7 +3,6 @@
 #include "common.cuh"
 
 namespace tb {
-int ensure_cells(tapas_b200_ctx *ctx, int64_t need, int64_t used);
 // Builds the tree of the bodies already in ctx->x/y/z/q (ctx->n of them).
 int build_tree(tapas_b200_ctx *ctx, int ncrit);
 // Bodies per leaf depth (deeper leaves in the last bin), nbins <= 64, host out.
