@@ -156,6 +156,10 @@ __device__ __forceinline__ float warp_reduce_scatter16f(float (&buf)[16], int la
   return buf[0] + __shfl_xor_sync(0xffffffffu, buf[0], 1);
 }
 
+// The unit of a leaf's expansions in the mixed form: its width, or 1 where it has none
+// (the root of a single body is a point, and the body beside it).
+__device__ __forceinline__ double unit_of(double width) { return width > 0 ? width : 1.0; }
+
 // P2M of the mixed form: each body's terms in FP32, in units of the leaf width
 // w (rho' = rho / w <= ~0.87, so rho'^n stays in range at every n; M_n = w^n
 // times the sum), 8 complex terms at a time summed over the warp by one
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 6) p2m32_kernel(
   const int c = leaves[w];
   const int b0 = cbeg[c], nb = cnb[c];
   const double cx = ccen[3 * c], cy = ccen[3 * c + 1], cz = ccen[3 * c + 2];
-  const double width = cmax[3 * c] - cmin[3 * c], iw = 1.0 / width;
+  const double width = unit_of(cmax[3 * c] - cmin[3 * c]), iw = 1.0 / width;
   double acc[kGroups];  // lane l: component of slot (l >> 1) & 15 of group g
 #pragma unroll
   for (int g = 0; g < kGroups; g++) acc[g] = 0;
@@ -483,7 +487,7 @@ __global__ void __launch_bounds__(256) l2p32_prep(
   const int64_t w = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
   if (w >= nleaves) return;
   const int c = leaves[w];
-  const double width = cmax[3 * c] - cmin[3 * c];
+  const double width = unit_of(cmax[3 * c] - cmin[3 * c]);
   for (int t = lane; t < S::NT; t += 32) {
     int n, m;
     jk_of(t, n, m);

@@ -955,3 +955,13 @@ def test_reciprocal_distance_within_its_bound(lo, hi, tb, ctx):
         acc = -d.astype(np.longdouble) * exact ** 3
         assert np.all(np.abs(r[:, 1] - acc) <= 4.6 * 2.0 ** -52 * np.abs(acc))
         assert np.all(r[:, 2:] == 0)
+
+
+@pytest.mark.parametrize("P", [3, 6, 16])
+def test_one_body_feels_nothing(P, tb, ctx):
+    """A single body's root cell has no width, and the body lies beside it: no field in
+    either form."""
+    one = [np.array([v]) for v in (0.3, 0.2, 0.7, 1.5)]
+    for precision in (tb.FP64, tb.MIXED):
+        r = ctx.evaluate(*one, P=P, ncrit=64, theta=0.4, precision=precision)
+        assert np.array_equal(r, np.zeros((1, 4))), precision
