@@ -91,8 +91,8 @@ struct BhCells {
 // right whatever the approximation's error (below 2^-20; enumerated); the one
 // reciprocal within 2^-106 of a middle that does not is that of an s with all
 // mantissa bits set (r2 just below a power of four: one step of a lattice of
-// spacing 1), which is tested for.  13 FP64 operations where the two library
-// sequences take about 57 slots of the FP64 pipe.
+// spacing 1), which is tested for.  11 FP64 operations (y is halved in its
+// exponent) where the two library sequences take about 57 slots of the FP64 pipe.
 // kN at once, with one branch for all: a branch each would keep their chains
 // from overlapping.
 template <int kN>
@@ -110,7 +110,8 @@ __device__ __forceinline__ void rounded_inv_sqrt(const double (&r2)[kN], double 
     double e = fma(-(r2[i] * y), y, 1.0);
     y = fma(y, e * fma(e, 0.375, 0.5), y);
     const double g = r2[i] * y;
-    s[i] = fma(fma(-g, g, r2[i]), 0.5 * y, g);
+    const double half_y = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));
+    s[i] = fma(fma(-g, g, r2[i]), half_y, g);
     e = fma(-s[i], y, 1.0);
     inv[i] = fma(y, fma(e, e, e), y);
     odd |= library(r2[i], s[i]);
@@ -339,7 +340,8 @@ __device__ __forceinline__ int lane_above(int sums, int i) {
 // bodies: 625, one per scheduler), so the time is one warp's chain of dependent
 // loads and FP64 sequences; here a chain step serves up to 32 popped entries,
 // eight opened cells, 32 loads or four terms instead of one.  One warp per block,
-// so that few warps spread evenly over the SMs.  20k bodies, ncrit 1: 0.69 ms;
+// so that few warps spread evenly over the SMs.  20k bodies, ncrit 1: 0.67 ms (4M, ncrit 32:
+// 130 ms; 125 with the reciprocal's step to first order, which a few s round wrong by);
 // 0.81 ms with one entry popped at a time, 2.39 ms with one cell and one term at
 // a time, 1.68 ms without the box's tests.
 __global__ void __launch_bounds__(32) bh_walk64(
