@@ -527,6 +527,8 @@ __global__ void __launch_bounds__(kThreads) l2p32_bodies(
       if (rxy > 0.f) {
         cp = dx / rxy;
         sp = dy / rxy;
+      } else if (dz < 0.f) {
+        y = 1.2246468e-16f;  // sin(acos(-1)) in FP64, as the FP64 form gets it
       }
     }
     const float inv_y = 1.f / y, inv_r = 1.f / r;

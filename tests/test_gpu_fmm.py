@@ -965,3 +965,28 @@ def test_one_body_feels_nothing(P, tb, ctx):
     for precision in (tb.FP64, tb.MIXED):
         r = ctx.evaluate(*one, P=P, ncrit=64, theta=0.4, precision=precision)
         assert np.array_equal(r, np.zeros((1, 4))), precision
+
+
+@pytest.mark.parametrize("P", [4, 11])
+def test_mixed_bodies_on_a_leafs_axis(P, tb, ctx):
+    """Bodies of a lattice lie on the vertical axes through their leaves' centres.  The
+    field there is finite in the mixed form wherever it is in the FP64 form (below the
+    centre; at it and above it the reference's own angles give NaN)."""
+    rng = np.random.default_rng(11)
+    x, y, z = (rng.integers(-8, 9, (3, 4000)) / 8.0)
+    q = rng.uniform(-1, 1, 4000)
+    x[:2], y[:2], z[:2] = [-1, 1], [-1, 1], [-1, 1]
+    r64 = ctx.evaluate(x, y, z, q, P=P, ncrit=16, theta=0.5, precision=tb.FP64)
+    rmx = ctx.evaluate(x, y, z, q, P=P, ncrit=16, theta=0.5, precision=tb.MIXED)
+    cells, (order, _) = ctx.cells(), ctx.sorted_bodies()
+    on_axis = 0
+    for c in np.flatnonzero((cells["leaf"] != 0) & (cells["nb"] > 0)):
+        b = order[cells["bbeg"][c]:cells["bbeg"][c] + cells["nb"][c]]
+        cx, cy, cz = cells["center"][c]
+        on_axis += np.sum((x[b] == cx) & (y[b] == cy) & (z[b] < cz))
+    assert on_axis > 0
+    fine = np.isfinite(r64)
+    assert np.isfinite(rmx[fine]).all()
+    rows = fine.all(axis=1)
+    num = np.linalg.norm(rmx[rows] - r64[rows], axis=0)
+    assert np.all(num <= 2e-6 * np.linalg.norm(r64[rows], axis=0))
