@@ -97,11 +97,12 @@ struct BhCells {
 // from overlapping.
 template <int kN>
 __device__ __forceinline__ void rounded_inv_sqrt(const double (&r2)[kN], double (&inv)[kN]) {
-  // outside 2^-767 .. 2^768 the residuals could underflow
-  auto library = [](double r2, double s) {
-    return (unsigned)__double2hiint(r2) - 0x10000000u >= 0x60000000u || __double2loint(s) == -1;
+  // outside 2^-767 .. 2^768 the residuals could underflow; s has all mantissa bits set for
+  // the two numbers below a power of four only
+  auto library = [](double r2) {
+    return (unsigned)__double2hiint(r2) - 0x10000000u >= 0x60000000u ||
+           (unsigned)__double2loint(r2) >= 0xfffffffeu;
   };
-  double s[kN];
   bool odd = false;
 #pragma unroll
   for (int i = 0; i < kN; i++) {
@@ -111,15 +112,15 @@ __device__ __forceinline__ void rounded_inv_sqrt(const double (&r2)[kN], double 
     y = fma(y, e * fma(e, 0.375, 0.5), y);
     const double g = r2[i] * y;
     const double half_y = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));
-    s[i] = fma(fma(-g, g, r2[i]), half_y, g);
-    e = fma(-s[i], y, 1.0);
+    const double s = fma(fma(-g, g, r2[i]), half_y, g);
+    e = fma(-s, y, 1.0);
     inv[i] = fma(y, fma(e, e, e), y);
-    odd |= library(r2[i], s[i]);
+    odd |= library(r2[i]);
   }
   if (odd) {
 #pragma unroll
     for (int i = 0; i < kN; i++)
-      if (library(r2[i], s[i])) inv[i] = __ddiv_rn(1.0, __dsqrt_rn(r2[i]));
+      if (library(r2[i])) inv[i] = __ddiv_rn(1.0, __dsqrt_rn(r2[i]));
   }
 }
 
@@ -341,7 +342,7 @@ __device__ __forceinline__ int lane_above(int sums, int i) {
 // loads and FP64 sequences; here a chain step serves up to 32 popped entries,
 // eight opened cells, 32 loads or four terms instead of one.  One warp per block,
 // so that few warps spread evenly over the SMs.  20k bodies, ncrit 1: 0.67 ms (4M, ncrit 32:
-// 130 ms; 125 with the reciprocal's step to first order, which a few s round wrong by);
+// 128 ms; 125 with the reciprocal's step to first order, which a few s round wrong by);
 // 0.81 ms with one entry popped at a time, 2.39 ms with one cell and one term at
 // a time, 1.68 ms without the box's tests.
 __global__ void __launch_bounds__(32) bh_walk64(
