@@ -86,12 +86,12 @@ struct BhCells {
 // the IBM RISC System/6000 processor", 1990).  The residuals are exact in an fma, so
 // before its rounding the root is off by less than 2^-103, relative, and the
 // reciprocal (its step taken to second order, e + e^2: y is up to an ulp off 1/s) by at
-// most 2^-106.  The arguments whose root lies that close to the middle of two
-// numbers, M^2 = r2 + j for odd 54-bit M and |j| <= 64, all come out rounded
-// right whatever the approximation's error (below 2^-20; enumerated); the one
-// reciprocal within 2^-106 of a middle that does not is that of an s with all
-// mantissa bits set (r2 just below a power of four: one step of a lattice of
-// spacing 1), which is tested for.  11 FP64 operations (y is halved in its
+// most 2^-106.  The roots that lie so close to the middle of two numbers, squares of odd
+// 54-bit integers within 128 of a multiple of 2^54 or 2^55, were enumerated: all round
+// right whatever the approximation's error (below 2^-20).  The one reciprocal within
+// 2^-106 of a middle that does not is that of an s with all mantissa bits set (r2 just
+// below a power of four, as for a unit step of a lattice summed up from tenths),
+// which is tested for.  11 FP64 operations (y is halved in its
 // exponent) where the two library sequences take about 57 slots of the FP64 pipe.
 // kN at once, with one branch for all: a branch each would keep their chains
 // from overlapping.
